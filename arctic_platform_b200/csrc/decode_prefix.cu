@@ -17,8 +17,8 @@
 // block j+1 before it waits for the probabilities of block j, and P V accumulates over all blocks in ONE output
 // buffer in tensor memory that the softmax warps read only once, at the end.  The running maximum is therefore a
 // REFERENCE maximum: a row rescales its output (read, multiply, write back -- after the previous P V has landed)
-// only when its true maximum has moved more than 2^8 above the reference; otherwise the probabilities are taken
-// against the stale reference (at most 256, harmless in bf16 / fp32) and nothing is rescaled.  Per block a softmax
+// only when its true maximum, or that of another row of its warp, has moved more than 2^8 above the reference; otherwise
+// the probabilities are taken against the stale reference (at most 256, harmless in bf16 / fp32) and nothing is rescaled.  Per block a softmax
 // thread thus reads its 128 scores once, takes 128 exponentials and writes 64 packed words -- the per-block read-out
 // and fold of the output (and the second pass over the scores) of the earlier versions set the pace of the kernel.
 #include "common.cuh"
@@ -228,7 +228,8 @@ decode_prefix_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
         for (int i = 0; i < 32; ++i)
           if (c * 32 + i < limit) mx = fmaxf(mx, __uint_as_float(sc[c][i]));
       const float m_new = fmaxf(m_ref, mx * p.scale_log2);
-      if (m_new > m_ref + kDpRescaleSlack || m_ref == -INFINITY) {
+      // one row that is behind moves the references of its whole warp: tensor-memory loads and stores are warp collectives
+      if (__any_sync(0xffffffffu, m_new > m_ref + kDpRescaleSlack || m_ref == -INFINITY)) {
         // move the reference.  Everything accumulated so far is in the old units: the row sum here, the output
         // row in tensor memory (once the previous block's P V has landed; block 0 has nothing to rescale)
         const float alpha = (m_ref == -INFINITY) ? 0.f : exp2f(m_ref - m_new);

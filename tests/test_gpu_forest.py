@@ -15,6 +15,34 @@ def _scratch(B, Hq, D, splits):
             [torch.empty((B, Hq, splits, 2), **f32) for _ in range(4)])
 
 
+def test_shared_pass_when_single_rows_meet_much_larger_scores_late():
+    """The running reference of a row moves when its scores outgrow it by 2^8; here some rows of a warp do, others never, in
+    several blocks.  bf16 weights (2^-9 each) and outputs (2^-9) against fp32."""
+    from arctic_platform_b200.ops import _lib
+    from arctic_platform_b200.ops import forest_attention as fa
+    B, Hq, Hkv, D, tokens = 12, 32, 8, 128, 1216
+    g = torch.Generator(device="cuda").manual_seed(5)
+    n = tokens // PAGE
+    kc, vc = (torch.randn((n + B, Hkv, PAGE, D), generator=g, device="cuda").to(torch.bfloat16) for _ in range(2))
+    q = torch.randn((B, Hq, D), generator=g, device="cuda")
+    q[::3] *= 6                                    # scores of every third sequence spread six times as far ...
+    kc[3 * n // 8:3 * n // 8 + 2] *= 3             # ... and grow in two of the ten blocks
+    kc[7 * n // 8:7 * n // 8 + 1] *= 5
+    q = q.to(torch.bfloat16)
+    pages = np.arange(n, dtype=np.int32)
+    own = [np.array([n + b], dtype=np.int32) for b in range(B)]
+    forest = fa.build_forest_tables([fa.ForestNode(0, list(range(B)), pages, tokens)], B, n + 1, 32, "cuda")
+    i32 = dict(device="cuda", dtype=torch.int32)
+    table = torch.zeros((B, n + 1), **i32)
+    table[:, 0] = torch.arange(n, n + B, **i32)
+    part_o, part_ml = _scratch(B, Hq, D, 2)
+    out = fa.forest_decode_attention(q, kc, vc, forest, torch.arange(B, **i32), torch.ones(B, **i32), table,
+                                     torch.full((B,), 5, **i32), part_o, part_ml, 2, 2)
+    _lib.check_status("forest")
+    ref = fa.forest_decode_reference(q, kc, vc, [[(pages, tokens), (own[b], 5)] for b in range(B)])
+    assert (out.float() - ref).norm() <= 2 ** -7 * ref.norm()
+
+
 @pytest.mark.parametrize("Hq,Hkv", [(32, 8), (16, 8), (8, 8)])
 def test_three_level_forest_matches_dense_attention(Hq, Hkv):
     """Headers shared by several prompts, prompts shared by their rollouts, private tails; one sequence without a
