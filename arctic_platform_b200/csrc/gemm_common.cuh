@@ -204,4 +204,52 @@ __device__ __forceinline__ void gemm_store_chunk(const GemmParams& p, int row, i
   }
 }
 
+// ---------------------------------------------------------------- lm-head epilogues
+// One record (max, sum exp, sum exp * z, label's z) of a row's 128 columns from `n0` on.
+__device__ __forceinline__ void lmhead_partial_128(const GemmParams& p, int row, bool row_ok, const uint32_t (&acc)[4][32], int n0) {
+  const float rs = p.alpha * ((p.row_scale && row_ok) ? p.row_scale[row] : 1.f);
+  const int label = (row_ok ? p.labels[row] : -1) - n0, cols = p.N - n0;
+  float m = -INFINITY, lab = -INFINITY, s = 0.f, e = 0.f;
+#pragma unroll
+  for (int j = 0; j < 128; ++j) {
+    const float z = __uint_as_float(acc[j / 32][j % 32]) * rs;
+    if (j < cols) m = fmaxf(m, z);
+    if (j == label) lab = z;
+  }
+#pragma unroll
+  for (int j = 0; j < 128; ++j) {
+    const float z = __uint_as_float(acc[j / 32][j % 32]) * rs;
+    const float x = j < cols ? __expf(z - m) : 0.f;
+    s += x;
+    e += x * z;
+  }
+  if (row_ok)
+    *(reinterpret_cast<float4*>(p.partial) + static_cast<long long>(row) * ((p.N + 127) / 128) + n0 / 128) = make_float4(m, s, e, lab);
+}
+
+// What d loss / d logits of a row needs besides the logit.
+struct LmheadRow {
+  float rs = 0.f, lse = 0.f, ent = 0.f, glp = 0.f, gent = 0.f;
+  int label = -1;
+};
+__device__ __forceinline__ LmheadRow lmhead_row(const GemmParams& p, int row, bool row_ok) {
+  LmheadRow r;
+  r.rs = p.alpha * ((p.row_scale && row_ok) ? p.row_scale[row] : 1.f);
+  if (row_ok) {
+    r.label = p.labels[row];
+    r.lse = p.row_lse[row];
+    r.ent = p.row_ent[row];
+    r.glp = p.row_glp[row];
+    if (p.row_gent) r.gent = p.row_gent[row];
+  }
+  return r;
+}
+__device__ __forceinline__ float lmhead_dlogit(const LmheadRow& r, float acc, int col) {
+  const float z = acc * r.rs;
+  const float pj = __expf(z - r.lse);
+  float g = -r.glp * pj - r.gent * pj * (z - r.lse + r.ent);
+  if (col == r.label) g += r.glp;
+  return g * r.rs;
+}
+
 }  // namespace apb

@@ -297,57 +297,19 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tma_a, const CUtens
       const int row = m0 + quarter * 32 + lane;
       const bool row_ok = row < m_end;
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * Cfg::kAccStride;
-      if (p.epi == kEpiLogprobPartial) {
-        // BN == 128 here: one partial record per row and tile
-        const float rs = p.alpha * ((p.row_scale && row_ok) ? p.row_scale[row] : 1.f);
-        const int label = row_ok ? p.labels[row] : -1;
-        float m_run = -INFINITY, s_run = 0.f, e_run = 0.f, lab = -INFINITY;
-#pragma unroll 1
-        for (int c = 0; c < BN / 32; ++c) {
-          const int col0 = n0 + c * 32;
-          if (col0 >= p.N) break;
-          uint32_t r[32];
-          tmem_ld_32x32(taddr + c * 32, r);
-          tmem_ld_wait();
-          float z[32];
-          float cm = -INFINITY;
+      if (BN == 128 && p.epi == kEpiLogprobPartial) {      // one record per row and tile
+        uint32_t acc[4][32];
 #pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            z[j] = (col0 + j < p.N) ? __uint_as_float(r[j]) * rs : -INFINITY;
-            cm = fmaxf(cm, z[j]);
-            if (col0 + j == label) lab = z[j];
-          }
-          const float m_new = fmaxf(m_run, cm);
-          const float corr = __expf(m_run - m_new);
-          float cs = 0.f, ce = 0.f;
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const float ex = (col0 + j < p.N) ? __expf(z[j] - m_new) : 0.f;
-            cs += ex;
-            ce += (col0 + j < p.N) ? ex * z[j] : 0.f;
-          }
-          s_run = s_run * corr + cs;
-          e_run = e_run * corr + ce;
-          m_run = m_new;
-        }
-        if (row_ok) {
-          const int tiles_n_ = (p.N + BN - 1) / BN;
-          float4* dst = reinterpret_cast<float4*>(p.partial) + static_cast<long long>(row) * tiles_n_ + n0 / BN;
-          *dst = make_float4(m_run, s_run, e_run, lab);
-        }
+        for (int c = 0; c < 4; ++c) tmem_ld_32x32(taddr + c * 32, acc[c]);
+        tmem_ld_wait();
+        lmhead_partial_128(p, row, row_ok, acc, n0);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&tempty_bar[buf]);
         continue;
       }
       if (p.epi == kEpiDlogits) {
-        const float it = (p.row_scale && row_ok) ? p.row_scale[row] : 1.f;
-        const float rs = p.alpha * it;
-        const int label = row_ok ? p.labels[row] : -1;
-        const float lse = row_ok ? p.row_lse[row] : 0.f;
-        const float ent = row_ok ? p.row_ent[row] : 0.f;
-        const float glp = row_ok ? p.row_glp[row] : 0.f;
-        const float gent = (row_ok && p.row_gent) ? p.row_gent[row] : 0.f;
+        const LmheadRow lm = lmhead_row(p, row, row_ok);
 #pragma unroll 1
         for (int c = 0; c < BN / 32; ++c) {
           const int col0 = n0 + c * 32;
@@ -356,25 +318,15 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tma_a, const CUtens
           tmem_ld_32x32(taddr + c * 32, r);
           tmem_ld_wait();
           if (!row_ok) continue;
-          float v[32];
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const float z = __uint_as_float(r[j]) * rs;
-            const float pj = __expf(z - lse);
-            float g = -glp * pj - gent * pj * (z - lse + ent);
-            if (col0 + j == label) g += glp;
-            v[j] = g * rs;
-          }
           __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(p.C) + static_cast<long long>(row) * p.ldc + col0;
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
             if (col0 + q * 8 < p.N) {
-              uint4 o;
-              o.x = pack_bf16x2(v[q * 8 + 0], v[q * 8 + 1]);
-              o.y = pack_bf16x2(v[q * 8 + 2], v[q * 8 + 3]);
-              o.z = pack_bf16x2(v[q * 8 + 4], v[q * 8 + 5]);
-              o.w = pack_bf16x2(v[q * 8 + 6], v[q * 8 + 7]);
-              *reinterpret_cast<uint4*>(dst + q * 8) = o;
+              float v[8];
+#pragma unroll
+              for (int j = 0; j < 8; ++j) v[j] = lmhead_dlogit(lm, __uint_as_float(r[q * 8 + j]), col0 + q * 8 + j);
+              *reinterpret_cast<uint4*>(dst + q * 8) = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]),
+                                                                  pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
             }
           }
         }
@@ -503,6 +455,8 @@ extern "C" int apb_gemm_bf16_pair_glu(const void* A, const void* B, void* C, int
                                   const void* bias, void* C2, long long ldc2, float glu_limit, cudaStream_t stream);
 
 namespace apb {
+int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, cudaStream_t stream);
+
 static bool pair_kernel_enabled() {
   static int on = -1;
   if (on < 0) {
@@ -770,9 +724,14 @@ __global__ void lmhead_combine_kernel(const float4* __restrict__ partial, int ti
   }
 }
 
+// More than one 128-row tile of rows goes to CTA pairs (256 x 256 tiles): a one-CTA tile of 128 x 128 reads 32 KB of operands
+// from shared memory for every 1 MMAC and reaches 660 TFLOP/s at 16384 x 151936 x 2560 (19.3 ms), the pair 1420 (8.9 ms).
+// Up to 128 rows half of a pair's tile would be padding and the product waits for the weights anyway.
 static int lmhead_launch(const void* hidden, const void* weight, int M, int V, int H, long long ldh, long long ldw,
                          GemmParams& p, int bn, cudaStream_t stream) {
   if ((ldh % 8) || (ldw % 8) || (V % 8)) return kBadArgument;
+  const bool pair = M > kBM && pair_kernel_enabled();
+  if (pair) bn = 128;                          // rows of B that one CTA of the pair stages
   CUtensorMap ta, tb;
   int rc = make_tmap_2d(&ta, hidden, 2, M, H, ldh, 64, kBM);
   if (rc) return 1000 + rc;
@@ -790,6 +749,7 @@ static int lmhead_launch(const void* hidden, const void* weight, int M, int V, i
   p.tile_map = nullptr;
   p.num_map_tiles = 0;
   p.status = status_device_ptr();
+  if (pair) return launch_gemm_pair(ta, tb, p, stream);
   return bn == 256 ? launch_gemm<256>(ta, tb, p, 0, stream) : launch_gemm<128>(ta, tb, p, 0, stream);
 }
 

@@ -1,22 +1,27 @@
-// bf16 GEMM on CTA pairs: two SMs work on one 256 x 256 output tile with tcgen05.mma.cta_group::2.
+// bf16 GEMM on CTA pairs: two SMs work on one output tile of 256 x 256 or 256 x 512 with tcgen05.mma.cta_group::2.
 //
-// Why a pair.  With one CTA per 128 x 256 tile every MMA of 128 x 256 x 16 reads 4 KB of A and 8 KB of B
-// from shared memory while TMA writes the same amount, which saturates the SM's shared-memory port at about
-// three quarters of the tensor-core rate.  In a pair each CTA stages its own 128 rows of A and only HALF of
-// the B tile (128 of the 256 columns); the instruction issued by the leader CTA multiplies the 256 x 16 A
-// slab spread over both SMs with the 256 x 16 B slab spread over both SMs, so each SM reads 8 KB per
-// 128 cycles instead of 12 KB and the tensor cores stay fed.
+// What bounds it: the operand stream from L2 to the SMs.  A 256 x 256 tile moves 64 B per SM and tensor cycle, which L2 delivers
+// at little more than half of the tensor rate (all-zero operands, where power does not matter: 1290 TFLOP/s at 1965 MHz); with
+// real operands the card also sits at its power limit, and every byte moved costs clock.  A 256 x 512 tile moves a quarter less.
+// It fills all 512 columns of tensor memory, so the two accumulators cannot belong to two tiles; they are the two halves of one
+// (see "Halves").
 //
 // Layout of the protocol (cluster of 2 CTAs, rank 0 = leader):
-//   warp 0   TMA producer of ITS CTA: A rows [m0 + 128*rank, +128), B rows [n0 + 128*rank, +128) per k-block.
-//            Loads are plain per-CTA copies (no multicast qualifier); the peer's copies signal the LEADER's
+//   warp 0   TMA producer of ITS CTA: A rows [m0 + 128*rank, +128) and, of every 256 columns of the tile, 128 rows of B per
+//            k-block.  Loads are plain per-CTA copies (no multicast qualifier); the peer's copies signal the LEADER's
 //            "full" barrier (cp.async.bulk.tensor ... cta_group::2), which expects the bytes of both CTAs.
 //   warp 1   leader only: issues the MMAs, then commits to the "empty" barrier of the stage in BOTH CTAs and,
-//            at the end of a tile, to the "accumulator full" barrier in both CTAs.  Owns the TMEM allocation
+//            at the end of an accumulator, to its "full" barrier in both CTAs.  Owns the TMEM allocation
 //            (both CTAs execute the paired alloc / dealloc).
-//   warps 2-5 epilogue of ITS CTA: its 128 accumulator rows (TMEM lanes) x 256 columns -> registers -> global;
-//            releases the accumulator buffer by arriving on the leader's barrier (8 arrivals: 4 warps x 2 CTAs).
-// Two accumulator buffers (2 x 256 TMEM columns) overlap the epilogue of tile i with the main loop of tile i+1.
+//   warps 2-9 epilogue of ITS CTA, two warps per 32 accumulator rows: each takes 128 of the accumulator's 256 columns into
+//            registers at once and gives the accumulator back (16 arrivals on the leader's barrier: 8 warps x 2 CTAs) before
+//            it computes and stores.  Results leave through 4 KB of shared memory per warp and TMA stores (or TMA additions,
+//            carried out by L2, for "+="): a row per thread would cost one L1 wavefront per 16 bytes, four times the main loop of a
+//            weight gradient over 549 tokens.
+// Halves.  NT = 256: a tile uses one of two accumulators in turn, its epilogue overlaps the next tile's main loop.  NT = 512: the
+// columns [0, 256) and [256, 512) of a tile are accumulator 0 and 1.  The last k-blocks of a tile are multiplied for half 0
+// first, then for half 1, and so are the first ones of the next tile: half 0 is read out while half 1 is finished, half 1 while the
+// next tile's half 0 is begun, and the tensor cores do not wait for either.
 // Every mbarrier wait is bounded; a CTA whose wait runs out records a status code and unwinds, its partner's
 // waits then run out as well, and both meet at the cluster barrier before TMEM is released.
 //
@@ -29,13 +34,21 @@
 namespace apb {
 
 constexpr int kPairBK = 64;
-constexpr int kPairStages = 6;
-constexpr int kPairABytes = 128 * kPairBK * 2;   // this CTA's 128 rows of A
-constexpr int kPairBBytes = 128 * kPairBK * 2;   // this CTA's 128 of the tile's 256 columns of B
-constexpr int kPairStageBytes = kPairABytes + kPairBBytes;
-constexpr int kPairSmem = kPairStages * kPairStageBytes + 1024 /*align*/ + 256 /*barriers*/;
-constexpr int kPairThreads = 192;
-constexpr int kPairTmemCols = 512;               // two fp32 accumulators of 256 columns
+constexpr int kPairBoxBytes = 128 * kPairBK * 2;   // 128 rows of A, or of one half of B
+constexpr int kPairEpiWarps = 8;
+constexpr int kPairThreads = 64 + 32 * kPairEpiWarps;
+constexpr int kPairOutBytes = 4096;                // a warp's 32 rows x 128 bytes on their way out
+constexpr int kPairTmemCols = 512;                 // two fp32 accumulators of 256 columns
+constexpr int kPairGroupM = 16;                    // row tiles that are walked before the next column tile
+
+template <int NT>
+struct PairCfg {
+  static constexpr int kHalves = NT / 256;
+  static constexpr int kStageBytes = (1 + kHalves) * kPairBoxBytes;
+  static constexpr int kStages = NT == 256 ? 6 : 4;
+  static constexpr int kSmem = kStages * kStageBytes + kPairEpiWarps * kPairOutBytes + 1024 /*align*/ + 256 /*barriers*/;
+};
+static_assert(PairCfg<256>::kSmem <= 227 * 1024 && PairCfg<512>::kSmem <= 227 * 1024, "shared memory of one CTA");
 
 __device__ __forceinline__ uint32_t cluster_cta_rank() {
   uint32_t r;
@@ -93,14 +106,131 @@ __device__ __forceinline__ void tc_commit_pair(uint32_t bar_cluster_addr) {
                : "memory");
 }
 
+// TMA store / addition of one staged box (32 rows x 128 bytes), and the wait until the previous one has left shared memory.
+__device__ __forceinline__ void tma_out_2d(const CUtensorMap* map, const void* smem_src, int x, int y, bool add) {
+  if (add)
+    asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3}], [%1];" ::"l"(
+                     reinterpret_cast<uint64_t>(map)),
+                 "r"(smem_u32(smem_src)), "r"(x), "r"(y)
+                 : "memory");
+  else
+    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%2, %3}], [%1];" ::"l"(
+                     reinterpret_cast<uint64_t>(map)),
+                 "r"(smem_u32(smem_src)), "r"(x), "r"(y)
+                 : "memory");
+  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+__device__ __forceinline__ void tma_out_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void tma_out_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+
+// One staged box of a warp: eight 16-byte units per row, swizzled as the tensor map expects them.
+struct PairOut {
+  uint8_t* buf;
+  int lane;
+  __device__ __forceinline__ void begin() const {
+    if (lane == 0) tma_out_wait_read();
+    __syncwarp();
+  }
+  __device__ __forceinline__ void put(int unit, const uint4& v) const {
+    *reinterpret_cast<uint4*>(buf + lane * 128 + ((unit ^ (lane & 7)) << 4)) = v;
+  }
+  __device__ __forceinline__ void send(const CUtensorMap* map, int x, int y, bool add) const {
+    fence_proxy_async_smem();
+    __syncwarp();
+    if (lane == 0) tma_out_2d(map, buf, x, y, add);
+  }
+};
+
+// What a variant of the kernel does with its accumulators.  A kernel holds one of them: with all in one kernel the unrolled code of
+// the untaken ones pushed the taken one out of the instruction cache (gate/up of 18432 tokens: 2.6 ms against 0.9).
+enum PairEpi : int { kPairBf16, kPairF32, kPairSwiGLU, kPairGeGLU, kPairClampGLU, kPairPartial, kPairDlogits };
+
+// 128 accumulator columns from `nb` on of the rows [row0, row0 + 32), this lane's row in `acc`.  Columns and rows outside the
+// output are clipped by the tensor maps; a box that would begin outside is not sent.
+template <int EPI>
+__device__ __forceinline__ void pair_epilogue(const GemmParams& p, const CUtensorMap& tma_c, const CUtensorMap& tma_c2,
+                                              const PairOut& out, int row0, int nb, const uint32_t (&acc)[4][32]) {
+  const int row = row0 + out.lane;
+  const bool row_ok = row < p.M;
+  if constexpr (EPI == kPairPartial) {
+    lmhead_partial_128(p, row, row_ok, acc, nb);
+  } else if constexpr (EPI == kPairF32) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      if (nb + c * 32 >= p.N) break;
+      out.begin();
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        float4 f;
+        f.x = __uint_as_float(acc[c][u * 4]) * p.alpha;
+        f.y = __uint_as_float(acc[c][u * 4 + 1]) * p.alpha;
+        f.z = __uint_as_float(acc[c][u * 4 + 2]) * p.alpha;
+        f.w = __uint_as_float(acc[c][u * 4 + 3]) * p.alpha;
+        out.put(u, *reinterpret_cast<const uint4*>(&f));
+      }
+      out.send(&tma_c, nb + c * 32, row0, p.epi != kEpiF32);
+    }
+  } else {
+    constexpr bool glu = EPI == kPairSwiGLU || EPI == kPairGeGLU || EPI == kPairClampGLU;
+    if (!glu || p.C != nullptr) {
+      LmheadRow lm;
+      if constexpr (EPI == kPairDlogits) lm = lmhead_row(p, row, row_ok);
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const int col0 = nb + c * 64;
+        if (col0 >= p.N) break;
+        out.begin();
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          float v[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const float a = __uint_as_float(acc[c * 2 + u / 4][(u % 4) * 8 + j]);
+            v[j] = EPI == kPairDlogits ? lmhead_dlogit(lm, a, col0 + u * 8 + j) : a * p.alpha;
+          }
+          if (EPI != kPairDlogits && p.bias && col0 + u * 8 < p.N) {     // N is a multiple of 8
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] += __bfloat162float(p.bias[col0 + u * 8 + j]);
+          }
+          out.put(u, make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7])));
+        }
+        out.send(&tma_c, col0, row0, false);
+      }
+    }
+    if constexpr (glu) {
+      out.begin();
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        float a[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const int i = u * 16 + 2 * j;
+          float g = __uint_as_float(acc[i / 32][i % 32]) * p.alpha, x = __uint_as_float(acc[i / 32][i % 32 + 1]) * p.alpha;
+          if (p.C && p.bias && nb + i < p.N) {
+            g += __bfloat162float(p.bias[nb + i]);
+            x += __bfloat162float(p.bias[nb + i + 1]);
+          }
+          a[j] = EPI == kPairSwiGLU ? silu_f(g) * x : EPI == kPairGeGLU ? gelu_tanh_f(g) * x : clamped_glu_f(g, x, p.glu_limit);
+        }
+        out.put(u, make_uint4(pack_bf16x2(a[0], a[1]), pack_bf16x2(a[2], a[3]), pack_bf16x2(a[4], a[5]), pack_bf16x2(a[6], a[7])));
+      }
+      out.send(&tma_c2, nb / 2, row0, false);
+    }
+  }
+}
+
+template <int NT, int EPI>
 __global__ void __launch_bounds__(kPairThreads, 1)
 gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
-                      const GemmParams p) {
+                      const __grid_constant__ CUtensorMap tma_c, const __grid_constant__ CUtensorMap tma_c2, const GemmParams p) {
+  using Cfg = PairCfg<NT>;
+  constexpr int kStages = Cfg::kStages;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + kPairStages * kPairStageBytes);
-  uint64_t* empty_bar = full_bar + kPairStages;
-  uint64_t* tfull_bar = empty_bar + kPairStages;
+  uint8_t* smem_out = smem + kStages * Cfg::kStageBytes;
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem_out + kPairEpiWarps * kPairOutBytes);
+  uint64_t* empty_bar = full_bar + kStages;
+  uint64_t* tfull_bar = empty_bar + kStages;
   uint64_t* tempty_bar = tfull_bar + 2;
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(tempty_bar + 2);
 
@@ -112,19 +242,19 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
   const int num_pairs = gridDim.x >> 1;
 
   const int tiles_m = (p.M + 255) / 256;
-  const int tiles_n = (p.N + 255) / 256;
+  const int tiles_n = (p.N + NT - 1) / NT;
   const int mn_tiles = tiles_m * tiles_n;
   const int total_tiles = mn_tiles * p.splits;   // work units: output tiles x K splits (split-K adds into C)
   const int k_blocks = (p.K + kPairBK - 1) / kPairBK;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kPairStages; ++s) {
+    for (int s = 0; s < kStages; ++s) {
       mbar_init(&full_bar[s], 1);    // the leader's arrive.expect_tx; bytes come from both CTAs
       mbar_init(&empty_bar[s], 1);   // one commit by the leader's MMA thread
     }
     for (int b = 0; b < 2; ++b) {
-      mbar_init(&tfull_bar[b], 1);   // one commit by the leader's MMA thread
-      mbar_init(&tempty_bar[b], 8);  // 4 epilogue warps of each CTA (used in the leader only)
+      mbar_init(&tfull_bar[b], 1);                    // one commit by the leader's MMA thread
+      mbar_init(&tempty_bar[b], 2 * kPairEpiWarps);   // the epilogue warps of both CTAs (used in the leader only)
     }
     mbar_fence_init();
   }
@@ -142,21 +272,22 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
 
-  // Tile order: 8 m-tiles of one n-band at a time, so pairs running together share B in L2.
+  // Tile order: kPairGroupM m-tiles of one n-band at a time, so pairs running together share B in L2.
   auto decode = [&](int unit, int& m0, int& n0, int& kb0, int& kb1) {
     const int split = unit / mn_tiles;
     const int t = unit - split * mn_tiles;
     kb0 = static_cast<int>((static_cast<long long>(k_blocks) * split) / p.splits);
     kb1 = static_cast<int>((static_cast<long long>(k_blocks) * (split + 1)) / p.splits);
-    constexpr int G = 8;
-    const int per_group = G * tiles_n;
+    const int per_group = kPairGroupM * tiles_n;
     const int g = t / per_group;
-    const int first_m = g * G;
-    const int gsize = min(tiles_m - first_m, G);
+    const int first_m = g * kPairGroupM;
+    const int gsize = min(tiles_m - first_m, kPairGroupM);
     const int r = t - g * per_group;
     m0 = (first_m + r % gsize) * 256;
-    n0 = (r / gsize) * 256;
+    n0 = (r / gsize) * NT;
   };
+  // accumulators of a tile: its second half may lie outside the output
+  auto halves_of = [&](int n0) { return NT == 512 && n0 + 256 < p.N ? 2 : 1; };
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer (both CTAs)
@@ -167,6 +298,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
       for (int t = pair; t < total_tiles && ok; t += num_pairs) {
         int m0, n0, kb0, kb1;
         decode(t, m0, n0, kb0, kb1);
+        const int halves = halves_of(n0);
         const int my_m = m0 + static_cast<int>(cta) * 128;
         const int my_n = n0 + static_cast<int>(cta) * 128;
         // All tiles walk K in the same order: pairs that share a row or a column of tiles in one wave then hit the
@@ -177,10 +309,9 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
             ok = false;
             break;
           }
-          uint8_t* sa = smem + stage * kPairStageBytes;
-          uint8_t* sb = sa + kPairABytes;
+          uint8_t* sa = smem + stage * Cfg::kStageBytes;
           const uint32_t bar = map_to_cta(smem_u32(&full_bar[stage]), 0);
-          if (leader) mbar_expect_tx(&full_bar[stage], 2 * kPairStageBytes);
+          if (leader) mbar_expect_tx(&full_bar[stage], 2 * (1 + halves) * kPairBoxBytes);
           if (!p.a_mn) {
             tma_load_2d_pair(sa, &tma_a, bar, kb * kPairBK, my_m);
           } else {
@@ -188,14 +319,17 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
             for (int c = 0; c < 2; ++c)
               tma_load_2d_pair(sa + c * (64 * kPairBK * 2), &tma_a, bar, my_m + c * 64, kb * kPairBK);
           }
-          if (!p.b_mn) {
-            tma_load_2d_pair(sb, &tma_b, bar, kb * kPairBK, my_n);
-          } else {
+          for (int h = 0; h < halves; ++h) {
+            uint8_t* sb = sa + (1 + h) * kPairBoxBytes;
+            if (!p.b_mn) {
+              tma_load_2d_pair(sb, &tma_b, bar, kb * kPairBK, my_n + h * 256);
+            } else {
 #pragma unroll
-            for (int c = 0; c < 2; ++c)
-              tma_load_2d_pair(sb + c * (64 * kPairBK * 2), &tma_b, bar, my_n + c * 64, kb * kPairBK);
+              for (int c = 0; c < 2; ++c)
+                tma_load_2d_pair(sb + c * (64 * kPairBK * 2), &tma_b, bar, my_n + h * 256 + c * 64, kb * kPairBK);
+            }
           }
-          if (++stage == kPairStages) {
+          if (++stage == kStages) {
             stage = 0;
             phase ^= 1;
           }
@@ -210,87 +344,129 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (leader CTA only)
-    if (leader && lane == 0) {
+    // The whole warp walks the loop and one elected lane issues: stage numbers and descriptors are then uniform, and an MMA
+    // costs two additions in front of it.  Built by a lone lane in a divergent branch, every operand went through a copy into
+    // uniform registers, and the issue took longer than the 128 cycles of the MMA.
+    if (leader) {
       const uint32_t idesc = umma_idesc_bf16(256, 256, p.a_mn, p.b_mn);
-      int stage = 0;
-      uint32_t phase = 0;
+      const uint32_t base = smem_u32(smem) >> 4;
+      const uint64_t desc_a = umma_smem_desc(0, p.a_mn ? 64 * kPairBK * 2 : 0, 1024) + base;
+      const uint64_t desc_b = umma_smem_desc(0, p.b_mn ? 64 * kPairBK * 2 : 0, 1024) + base + (kPairBoxBytes >> 4);
+      const uint32_t step_a = (p.a_mn ? 2048 : 32) >> 4, step_b = (p.b_mn ? 2048 : 32) >> 4;
+      const uint32_t peer_bars = map_to_cta(smem_u32(full_bar), 1) - smem_u32(full_bar);
+      uint32_t stage = 0, phase = 0;
+      uint32_t used[2] = {0, 0};      // times that each accumulator has been filled
       int it = 0;
       bool ok = true;
+      auto wait_full = [&](uint32_t s, uint32_t ph) {
+        const bool r = __all_sync(0xffffffffu, mbar_wait(&full_bar[s], ph, p.status, kTimeoutFull));
+        tc_fence_after();
+        return r;
+      };
+      auto wait_acc = [&](int slot) {
+        const bool r = __all_sync(0xffffffffu, mbar_wait(&tempty_bar[slot], (used[slot] & 1) ^ 1, p.status, kTimeoutTmemEmpty));
+        ++used[slot];
+        tc_fence_after();
+        return r;
+      };
+      // the MMAs of one stage; `release`: the stage is free in both CTAs once they have read it; `publish`: so is the accumulator
+      auto mma = [&](uint32_t s, int half, int slot, bool first, bool release, bool publish) {
+        const uint64_t da = desc_a + s * (Cfg::kStageBytes >> 4);
+        const uint64_t db = desc_b + s * (Cfg::kStageBytes >> 4) + half * (kPairBoxBytes >> 4);
+        if (elect_one()) {
+#pragma unroll
+          for (int k = 0; k < kPairBK / 16; ++k)
+            umma_bf16_ss_pair(tmem_base + slot * 256, da + k * step_a, db + k * step_b, idesc, (!first || k > 0) ? 1u : 0u);
+          if (release) {
+            const uint32_t eb = smem_u32(&empty_bar[s]);
+            tc_commit_pair(eb);
+            tc_commit_pair(eb + peer_bars);
+          }
+          if (publish) {
+            const uint32_t tb = smem_u32(&tfull_bar[slot]);
+            tc_commit_pair(tb);
+            tc_commit_pair(tb + peer_bars);
+          }
+        }
+        __syncwarp();
+      };
       for (int t = pair; t < total_tiles && ok; t += num_pairs, ++it) {
         int m0, n0, kb0, kb1;
         decode(t, m0, n0, kb0, kb1);
-        const int buf = it & 1;
-        const uint32_t acc_phase = (it >> 1) & 1;
-        if (!mbar_wait(&tempty_bar[buf], acc_phase ^ 1, p.status, kTimeoutTmemEmpty)) {
+        const int n = kb1 - kb0, halves = halves_of(n0);
+        const int slot0 = NT == 512 ? 0 : (it & 1);
+        if (!wait_acc(slot0)) {
           ok = false;
           break;
         }
-        tc_fence_after();
-        const uint32_t tmem_d = tmem_base + buf * 256;
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(&full_bar[stage], phase, p.status, kTimeoutFull)) {
-            ok = false;
-            break;
+        // runs of k-blocks: the first and the last kStages of them are walked once per half, the others once
+        for (int b = 0; b < n && ok;) {
+          const int last = max(kStages, n - kStages);
+          const int run = halves == 1 ? 1 : b == 0 ? min(n, kStages) : b >= last ? n - b : 1;
+          const bool end = b + run == n;
+          uint32_t s = stage, ph = phase;
+          for (int i = 0; i < run && ok; ++i) {
+            ok = wait_full(s, ph);
+            if (!ok) break;
+            mma(s, 0, slot0, b + i == 0, halves == 1, end && i == run - 1);
+            if (++s == kStages) {
+              s = 0;
+              ph ^= 1;
+            }
           }
-          tc_fence_after();
-          const uint32_t sa = smem_u32(smem + stage * kPairStageBytes);
-          const uint32_t sb = sa + kPairABytes;
-#pragma unroll
-          for (int k = 0; k < kPairBK / 16; ++k) {
-            const uint64_t da = p.a_mn ? umma_smem_desc(sa + k * 2048, 64 * kPairBK * 2, 1024)
-                                       : umma_smem_desc(sa + k * 32, 0, 1024);
-            const uint64_t db = p.b_mn ? umma_smem_desc(sb + k * 2048, 64 * kPairBK * 2, 1024)
-                                       : umma_smem_desc(sb + k * 32, 0, 1024);
-            umma_bf16_ss_pair(tmem_d, da, db, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+          if (!ok) break;
+          if (halves == 2) {
+            if (b == 0 && !wait_acc(1)) {
+              ok = false;
+              break;
+            }
+            uint32_t s1 = stage;
+            for (int i = 0; i < run; ++i) {
+              mma(s1, 1, 1, b + i == 0, true, end && i == run - 1);
+              if (++s1 == kStages) s1 = 0;
+            }
           }
-          // the stage is free in both CTAs once these MMAs have read it
-          const uint32_t eb = smem_u32(&empty_bar[stage]);
-          tc_commit_pair(eb);
-          tc_commit_pair(map_to_cta(eb, 1));
-          if (++stage == kPairStages) {
-            stage = 0;
-            phase ^= 1;
-          }
-        }
-        if (ok) {
-          const uint32_t tb = smem_u32(&tfull_bar[buf]);
-          tc_commit_pair(tb);
-          tc_commit_pair(map_to_cta(tb, 1));
+          stage = s;
+          phase = ph;
+          b += run;
         }
       }
     }
   } else {
     // ------------------------------------------------------------ epilogue (both CTAs)
-    const int quarter = warp & 3;  // TMEM lanes this warp may read
+    const int quarter = warp & 3;              // TMEM lanes this warp may read
+    const int part = (warp - 2) >> 2;          // columns [128 part, +128) of every accumulator
+    const PairOut out{smem_out + (warp - 2) * kPairOutBytes, lane};
+    uint32_t used[2] = {0, 0};
     int it = 0;
     bool ok = true;
     for (int t = pair; t < total_tiles && ok; t += num_pairs, ++it) {
       int m0, n0, kb0, kb1;
       decode(t, m0, n0, kb0, kb1);
-      const int buf = it & 1;
-      const uint32_t acc_phase = (it >> 1) & 1;
-      if (!mbar_wait(&tfull_bar[buf], acc_phase, p.status, kTimeoutTmemFull)) {
-        ok = false;
-        break;
-      }
-      tc_fence_after();
-      const int row = m0 + static_cast<int>(cta) * 128 + quarter * 32 + lane;
-      const bool row_ok = row < p.M;
-      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * 256;
-#pragma unroll 1
-      for (int c = 0; c < 256 / 32; ++c) {
-        const int col0 = n0 + c * 32;
-        if (col0 >= p.N) break;  // uniform across the warp
-        uint32_t r[32];
-        tmem_ld_32x32(taddr + c * 32, r);
+      const int row0 = m0 + static_cast<int>(cta) * 128 + quarter * 32;
+      const int halves = halves_of(n0);
+      for (int h = 0; h < halves; ++h) {
+        const int slot = NT == 512 ? h : (it & 1);
+        ok = mbar_wait(&tfull_bar[slot], used[slot] & 1, p.status, kTimeoutTmemFull);
+        if (!__all_sync(0xffffffffu, ok)) {
+          ok = false;
+          break;
+        }
+        ++used[slot];
+        tc_fence_after();
+        const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + slot * 256 + part * 128;
+        uint32_t acc[4][32];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) tmem_ld_32x32(taddr + c * 32, acc[c]);
         tmem_ld_wait();
-        if (!row_ok) continue;
-        gemm_store_chunk(p, row, col0, r);
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&tempty_bar[slot]), 0));
+        const int nb = n0 + h * 256 + part * 128;
+        if (row0 < p.M && nb < p.N) pair_epilogue<EPI>(p, tma_c, tma_c2, out, row0, nb, acc);
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&tempty_bar[buf]), 0));
     }
+    if (lane == 0) tma_out_wait_all();
   }
 
   // ---------------------------------------------------------------- teardown
@@ -301,6 +477,89 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
     tc_fence_after();
     tmem_dealloc_pair(tmem_base, kPairTmemCols);
   }
+}
+
+// Pairs that can be resident at once (SMs of a pair must sit in one cluster-capable group, so this can be fewer than half the
+// SM count).  The grid never exceeds it: a pair that had to wait for a second wave would still take a full share of the tiles.
+template <int NT, int EPI>
+static int pair_capacity(cudaLaunchConfig_t cfg) {
+  static int resident[64] = {0};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!resident[dev & 63]) {
+    if (cudaFuncSetAttribute(gemm_bf16_pair_kernel<NT, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairCfg<NT>::kSmem) != cudaSuccess)
+      return -static_cast<int>(cudaGetLastError());
+    cfg.gridDim = dim3(2 * (sm_count() / 2));
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, gemm_bf16_pair_kernel<NT, EPI>, &cfg) != cudaSuccess || n <= 0) {
+      cudaGetLastError();
+      n = sm_count() / 2 - 4;        // conservative when the query is unavailable
+    }
+    resident[dev & 63] = n < sm_count() / 2 ? n : sm_count() / 2;
+  }
+  return resident[dev & 63];
+}
+
+template <int NT, int EPI>
+static int launch_pair_as(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const CUtensorMap& tc2,
+                       const GemmParams& p, cudaStream_t stream) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.blockDim = dim3(kPairThreads);
+  cfg.dynamicSmemBytes = PairCfg<NT>::kSmem;
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const int room = pair_capacity<NT, EPI>(cfg);
+  if (room <= 0) return room < 0 ? -room : kBadArgument;
+  const long long total = static_cast<long long>((p.M + 255) / 256) * ((p.N + NT - 1) / NT) * p.splits;
+  cfg.gridDim = dim3(2 * static_cast<int>(total < room ? total : room));
+  cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_bf16_pair_kernel<NT, EPI>, ta, tb, tc, tc2, p);
+  if (e != cudaSuccess) return static_cast<int>(e);
+  return static_cast<int>(cudaGetLastError());
+}
+
+template <int NT>
+static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const CUtensorMap& tc2,
+                       const GemmParams& p, cudaStream_t s) {
+  switch (p.epi) {
+    case kEpiBf16: return launch_pair_as<NT, kPairBf16>(ta, tb, tc, tc2, p, s);
+    case kEpiF32:
+    case kEpiF32Accum:
+    case kEpiF32Atomic: return launch_pair_as<NT, kPairF32>(ta, tb, tc, tc2, p, s);
+    case kEpiSwiGLU: return launch_pair_as<NT, kPairSwiGLU>(ta, tb, tc, tc2, p, s);
+    case kEpiGeGLU: return launch_pair_as<NT, kPairGeGLU>(ta, tb, tc, tc2, p, s);
+    case kEpiClampGLU: return launch_pair_as<NT, kPairClampGLU>(ta, tb, tc, tc2, p, s);
+    case kEpiLogprobPartial: return launch_pair_as<NT, kPairPartial>(ta, tb, tc, tc2, p, s);
+    case kEpiDlogits: return launch_pair_as<NT, kPairDlogits>(ta, tb, tc, tc2, p, s);
+    default: return kBadArgument;
+  }
+}
+
+// Launches the kernel on filled-in operands: A and B as boxes of 64 x 128 (64 x 64 transposed).
+int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, cudaStream_t stream) {
+  CUtensorMap tc = ta, tc2 = ta;               // outputs that the epilogue does not write keep a valid map
+  const bool f32 = p.epi == kEpiF32 || p.epi == kEpiF32Accum || p.epi == kEpiF32Atomic;
+  if (p.C) {
+    const int rc = make_tmap_2d(&tc, p.C, f32 ? 4 : 2, p.M, p.N, p.ldc, f32 ? 32 : 64, 32);
+    if (rc) return 3000 + rc;
+  }
+  if (p.C2) {
+    const int rc = make_tmap_2d(&tc2, p.C2, 2, p.M, p.N / 2, p.ldc2, 64, 32);
+    if (rc) return 4000 + rc;
+  }
+  // The width whose waves take less time.  Twice as wide is 0.9 of twice as long where the main loop is long or the weights'
+  // gradient is formed (under the power limit, 18432 x 2560 x 19456: 1.40 ms against 1.54; 151936 x 2560 x 16384: 10.8 against
+  // 12.4), and a few percent more than twice where its start and end show (18432 x 6144 x 2560: 0.448 ms against 0.427).
+  const long long pairs = sm_count() / 2, tm = (p.M + 255) / 256;
+  auto waves = [&](int nt) { return (tm * ((p.N + nt - 1) / nt) * p.splits + pairs - 1) / pairs; };
+  const bool steady = (p.K + kPairBK - 1) / kPairBK / p.splits >= 96 || (f32 && p.a_mn && p.M >= 4 * p.K);
+  if (waves(512) * (steady ? 1.8 : 2.1) < waves(256)) return launch_pair<512>(ta, tb, tc, tc2, p, stream);
+  return launch_pair<256>(ta, tb, tc, tc2, p, stream);
 }
 
 }  // namespace apb
@@ -386,42 +645,7 @@ int apb_gemm_bf16_pair_glu(const void* A, const void* B, void* C, int M, int N, 
   p.glu_limit = glu_limit;
   p.status = status_device_ptr();
 
-  // How many pairs can be resident at once (SMs of a pair must sit in one cluster-capable group, so this can be
-  // fewer than half the SM count).  The grid never exceeds it: a pair that had to wait for a second wave would
-  // still take a full share of the tiles.
-  static int resident_pairs[64] = {0};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.blockDim = dim3(kPairThreads);
-  cfg.dynamicSmemBytes = kPairSmem;
-  cfg.stream = stream;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  if (!resident_pairs[dev & 63]) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_bf16_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    cfg.gridDim = dim3(2 * (sm_count() / 2));
-    int n = 0;
-    e = cudaOccupancyMaxActiveClusters(&n, gemm_bf16_pair_kernel, &cfg);
-    if (e != cudaSuccess || n <= 0) {
-      cudaGetLastError();
-      n = sm_count() / 2 - 4;        // conservative when the query is unavailable
-    }
-    resident_pairs[dev & 63] = n < sm_count() / 2 ? n : sm_count() / 2;
-  }
-  const long long total = static_cast<long long>((M + 255) / 256) * ((N + 255) / 256) * p.splits;
-  const int max_pairs = resident_pairs[dev & 63];
-  const int pairs = static_cast<int>(total < max_pairs ? total : max_pairs);
-  cfg.gridDim = dim3(2 * pairs);
-  cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_bf16_pair_kernel, ta, tb, p);
-  if (e != cudaSuccess) return static_cast<int>(e);
-  return static_cast<int>(cudaGetLastError());
+  return launch_gemm_pair(ta, tb, p, stream);
 }
 
 int apb_gemm_bf16_pair(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,

@@ -80,6 +80,15 @@ def _fwd_cuda(hidden, weight, labels, inv_temp_t, inv_temp_s):
     return lp, ent, lse
 
 
+def _bwd_rows(N: int, V: int, budget: int = 5 << 30) -> int:
+    """Rows of d(logits) that are formed at a time: as many as ``budget`` bytes of bf16 hold, in chunks of equal size.  Every
+    chunk reads and writes the fp32 weight gradient once, and the tiles of a chunk's ``[rows, H]`` gradient should fill the
+    GPU several times over: at V = 151936, H = 2560 chunks of 4096 rows make 160 tiles on 74 CTA pairs (2.2 waves), chunks of
+    16384 rows 640 (8.6 waves)."""
+    parts = -(-N * V * 2 // budget)
+    return min(N, (-(-N // parts) + 255) // 256 * 256)
+
+
 class _LmHeadLogprobFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, hidden, weight, labels, inv_temp_t, inv_temp_s, with_entropy, bwd_chunk):
@@ -104,7 +113,7 @@ class _LmHeadLogprobFn(torch.autograd.Function):
         d_hidden = torch.empty_like(hidden)
         acc = getattr(weight, "grad_f32", None)
         dw32 = acc if acc is not None else torch.zeros((V, H), device=hidden.device, dtype=torch.float32)
-        chunk = ctx.bwd_chunk
+        chunk = ctx.bwd_chunk or _bwd_rows(N, V)
         buf = torch.empty((min(chunk, N), V), device=hidden.device, dtype=torch.bfloat16)
         for s in range(0, N, chunk):
             n = min(chunk, N - s)
@@ -123,10 +132,11 @@ class _LmHeadLogprobFn(torch.autograd.Function):
 
 
 def lm_head_logprobs(hidden: torch.Tensor, weight: torch.Tensor, labels: torch.Tensor,
-                     inv_temperature=1.0, with_entropy: bool = True, bwd_chunk: int = 4096
+                     inv_temperature=1.0, with_entropy: bool = True, bwd_chunk: Optional[int] = None
                      ) -> Tuple[torch.Tensor, Optional[torch.Tensor]]:
     """``hidden [N,H]``, ``weight [V,H]``, ``labels [N]`` -> ``(logprob [N] fp32, entropy [N] fp32 or None)``.
-    ``inv_temperature`` is a float or a per-row tensor ``[N]`` multiplying the logits."""
+    ``inv_temperature`` is a float or a per-row tensor ``[N]`` multiplying the logits.  ``bwd_chunk``: rows of d(logits) that the
+    backward forms at a time (None: :func:`_bwd_rows`)."""
     if not hidden.is_cuda:
         return logprobs_entropy_ref(hidden, weight, labels, inv_temperature, with_entropy)
     if hidden.shape[0] == 0:

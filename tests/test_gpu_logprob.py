@@ -28,3 +28,29 @@ def test_logprob_forward_backward(N, H, V, per_row_temp):
         err = (got.float() - ref).abs().max().item()
         sc = ref.abs().max().item()
         assert err <= 3e-2 * sc + 1e-3, f"{nm}: {err} vs scale {sc}"
+
+
+@pytest.mark.parametrize("N,H,V", [(129, 64, 1032), (256, 72, 1280), (385, 2560, 4232), (700, 1024, 136)])
+def test_row_and_column_remainders_of_pair_tiles(N, H, V):
+    """More than one 128-row tile runs on CTA pairs of 256 x 256: odd rows, a last tile of 8, 128 or 136 columns.  The logits of
+    both sides have the same bf16 operands, so log-probabilities differ by fp32 rounding of sums and exponentials (V terms of
+    2^-22 relative, 1e-4 with room); gradients pass through bf16 once per d(logits) and once per result (2^-8 each)."""
+    from arctic_platform_b200.ops import _lib
+    from arctic_platform_b200.ops.logprob import lm_head_logprobs, logprobs_entropy_ref
+    g = torch.Generator(device="cuda").manual_seed(N)
+    hidden = torch.randn(N, H, device="cuda", generator=g).bfloat16().requires_grad_()
+    weight = (torch.randn(V, H, device="cuda", generator=g) * 2 * H ** -0.5).bfloat16().requires_grad_()
+    labels = torch.randint(0, V, (N,), device="cuda", generator=g)
+    labels[:2] = torch.tensor([0, V - 1], device="cuda")
+    g1, g2 = (torch.randn(N, device="cuda", generator=g) for _ in range(2))
+    lp, ent = lm_head_logprobs(hidden, weight, labels)
+    ((lp * g1).sum() + 0.1 * (ent * g2).sum()).backward()
+    _lib.check_status("lmhead")
+    hr, wr = (t.detach().double().requires_grad_() for t in (hidden, weight))
+    z = torch.log_softmax(hr @ wr.T, -1)
+    lpr, entr = z.gather(1, labels[:, None])[:, 0], -(z.exp() * z).sum(-1)
+    ((lpr * g1).sum() + 0.1 * (entr * g2).sum()).backward()
+    for got, ref in ((lp, lpr), (ent, entr)):
+        assert (got - ref).abs().max() <= 1e-4 * max(1.0, ref.abs().max().item())
+    for got, ref in ((hidden.grad, hr.grad), (weight.grad, wr.grad)):
+        assert (got.double() - ref).norm() <= 2 ** -7 * ref.norm()
