@@ -1,24 +1,28 @@
 // Segment attention backward on tcgen05 tensor cores (see attention_fwd.cu for
 // the segment model).  One CTA owns one key block (128 rows of one KV head) and
-// walks every 64-row query tile that can see it -- all query heads of the KV
+// walks every 128-row query tile that can see it -- all query heads of the KV
 // head, and under ZoRRo all rollouts that share the prompt the block belongs to
 // -- so dK and dV of a shared prompt are accumulated in tensor memory and written
 // once.  The reference gets these sums from autograd through torch.cat copies of
 // the prompt K/V (arctic_platform/rl/zorro_train/zorro_train.py:857-912).
 //
-// Per query tile, with everything transposed so that TMEM lanes are key rows:
+// Per query tile, with S and dP transposed so that TMEM lanes are key rows:
 //   S^T  = K  Q^T          dP^T = V dO^T                     (tensor core)
-//   P^T  = exp2(S^T*c - lse[q])     dS^T = P^T*(dP^T - delta[q])*scale   (128 threads)
-//   dV  += P^T dO          dK  += dS^T Q        dQ^T = K^T dS^T          (tensor core)
+//   P^T  = exp2(S^T*c - lse[q])     dS^T = P^T*(dP^T - delta[q])     (two groups of 128 threads, 64 columns each)
+//   dV  += P^T dO          dK  += dS^T Q        dQ = dS K          (tensor core)
 // P^T overwrites S^T in TMEM and is the TMEM A operand of the dV product; dS^T goes
-// to shared memory once and is read by two products (K-major for dK, MN-major for
-// dQ^T).  dQ^T is added to an fp32 accumulator in global memory with coalesced
-// red.add (lanes = head-dim index).
+// to shared memory once and is read by two products (K-major for dK, M-major for
+// dQ).  The softmax scale that dS lacks is applied to dK and dQ where they leave.
 //
-// Two gradient warpgroups take alternate query tiles, so the tensor core works on tile i+1 while the other group is
-// still in the exponentials / dS of tile i.  Tensor memory (512 columns): per group one 64-column slot that holds
-// S^T, then P^T, then dQ^T of its tile, and one 64-column slot for dP^T; dK and dV take 128 columns each.
-#include "common.cuh"
+// What bounds it: five products of 128 x 128 x 128, 2560 tensor cycles per tile.  Tensor memory (512 columns) holds S^T / P^T,
+// dP^T, dK and dV; dQ takes dP^T's place once dS^T has been formed.  The products are issued in the order
+//   S(i+1)  dQ(i)  dK(i)  dP(i+1)  dV(i+1)
+// so that each waits for something that was ready earlier: the exponentials of tile i+1 have the time of three products, dS(i) that
+// of dV(i) and S(i+1), the read-out of dQ(i) that of dK(i).  dQ is read by a group of its own and leaves as TMA additions of
+// 32 x 32 boxes.  One sequence of 16384 tokens, 32 query and 8 key heads: 5.7 ms (960 TFLOP/s; the products alone 4.3).  Before:
+// 64-row tiles (their 64-wide products alone 6.8 ms, since the operands saturate shared memory) 10.3 with dQ added by TMA, 13 with
+// red.add of one float per lane.
+#include "attention_common.cuh"
 #include "host_utils.cuh"
 
 namespace apb {
@@ -30,55 +34,60 @@ struct AttnBwdParams {
   float scale, scale_log2;
   const float* lse;    // [Hq, T]
   const float* delta;  // [Hq, T]
-  float* dq_acc;       // [T, Hq*D] fp32, zero-initialised by the caller
-  long long ld_dq;
   __nv_bfloat16* dk;   // [T, Hkv*D]
   __nv_bfloat16* dv;
   long long ld_dk, ld_dv;
   int* status;
 };
 
-constexpr int kBwdThreads = 320;  // producer, MMA issuer, two gradient groups of four warps
-constexpr int kBwdQTile = 64;
-constexpr int kBwdStages = 3;
+// Four warpgroups: producer and MMA issuer; two for P and dS; one for dQ.  Registers are moved from the first to the others:
+// 56 + 3 * 152 = 4 * 128, what the block was launched with.
+constexpr int kBwdThreads = 512;
+constexpr int kBwdRegsIssue = 56, kBwdRegsWork = 152;
+constexpr int kBwdTile = 128;            // query rows and key rows
 constexpr int kBigDiag = 1 << 27;
 
 template <int D>
 struct AttnBwdCfg {
-  static constexpr int kKvTileBytes = 128 * D * 2;
-  static constexpr int kQTileBytes = kBwdQTile * D * 2;
-  static constexpr int kStageBytes = 2 * kQTileBytes + 512;  // Q, dO, lse[64], delta[64]
-  static constexpr int kDsBytes = 128 * kBwdQTile * 2;
-  static constexpr int kSmemBytes = 2 * kKvTileBytes + kBwdStages * (2 * kQTileBytes) + 2 * kDsBytes +
-                                    kBwdStages * 512 + 1024 + 256;
+  static_assert(D == 128, "tensor memory and the dQ boxes are laid out for heads of 128");
+  static constexpr int kTileBytes = kBwdTile * D * 2;
+  static constexpr int kHeadBytes = 2 * 128 * 4 + 2 * 128 * 4 + 128;   // -lse and -delta of two tiles, barriers
+  // statistics and barriers lie in front, the tiles from the next multiple of 1024 on
+  static constexpr int kSmemBytes = 3072 + 6 * kTileBytes /*K, V, 2 Q, dO, dS*/ + 8 * kStagedBoxBytes;
+  static_assert(kHeadBytes <= 3072 - 896 && kSmemBytes <= 227 * 1024, "shared memory of one CTA");
 };
 
 template <int D>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant__ CUtensorMap tma_do,
                 const __grid_constant__ CUtensorMap tma_k, const __grid_constant__ CUtensorMap tma_v,
-                const AttnBwdParams p) {
+                const __grid_constant__ CUtensorMap tma_dq, const AttnBwdParams p) {
   using Cfg = AttnBwdCfg<D>;
-  constexpr int QCH = Cfg::kQTileBytes / (D / 64);  // bytes of one 64-wide chunk of a Q/dO tile (8192)
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  constexpr int kTileBytes = Cfg::kTileBytes;
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  float* smem_lse = reinterpret_cast<float*>(smem_raw);        // [2][128]
+  float* smem_delta = smem_lse + 256;                          // [2][128]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem_delta + 256);
+  uint64_t* q_full = bars;            // [2]  copy and statistics
+  uint64_t* q_empty = bars + 2;       // [2]
+  uint64_t* do_full = bars + 4;       // copy and statistics
+  uint64_t* do_empty = bars + 5;
+  uint64_t* kv_full = bars + 6;
+  uint64_t* s_full = bars + 7;        // S^T of a tile is there
+  uint64_t* p_full = bars + 8;        // (256 arrivals) P^T written
+  uint64_t* dp_full = bars + 9;       // dP^T is there
+  uint64_t* ds_full = bars + 10;      // (256 arrivals) dS^T in shared memory, dP^T read
+  uint64_t* dq_full = bars + 11;      // dQ is there
+  uint64_t* dq_read = bars + 12;      // (128 arrivals) dQ has been read
+  uint64_t* dkv_full = bars + 13;
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 14);
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + Cfg::kHeadBytes + 1023) & ~uintptr_t(1023));
   uint8_t* smem_k = smem;
-  uint8_t* smem_v = smem_k + Cfg::kKvTileBytes;
-  uint8_t* smem_qdo = smem_v + Cfg::kKvTileBytes;                       // [stage][Q | dO]
-  uint8_t* smem_ds = smem_qdo + kBwdStages * 2 * Cfg::kQTileBytes;      // [2][128 x 64 bf16]
-  float* smem_stat = reinterpret_cast<float*>(smem_ds + 2 * Cfg::kDsBytes);  // [stage][lse 64 | delta 64]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(smem_stat) + kBwdStages * 512);
-  uint64_t* full = bars;                    // [stages]
-  uint64_t* empty = full + kBwdStages;      // [stages]
-  uint64_t* kv_full = empty + kBwdStages;   // 1
-  uint64_t* s_full = kv_full + 1;           // [2]  S^T of a tile is in its group's slot
-  uint64_t* dp_full = s_full + 2;           // [2]  dP^T likewise
-  uint64_t* p_full = dp_full + 2;           // [2]  (128 arrivals) P^T written
-  uint64_t* ds_full = p_full + 2;           // [2]  (128 arrivals) dS^T in shared memory, dP^T slot free
-  uint64_t* dq_full = ds_full + 2;          // [2]  dQ^T of the tile is in the slot
-  uint64_t* dq_read = dq_full + 2;          // [2]  (128 arrivals) slot free again
-  uint64_t* dkv_full = dq_read + 2;         // 1
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(dkv_full + 1);
+  uint8_t* smem_v = smem + kTileBytes;
+  uint8_t* smem_q = smem + 2 * kTileBytes;       // [2]
+  uint8_t* smem_do = smem + 4 * kTileBytes;
+  uint8_t* smem_ds = smem + 5 * kTileBytes;      // [column half][128 key rows][64 bf16]
+  uint8_t* smem_out = smem + 6 * kTileBytes;     // [warp][2] boxes of dQ on their way out
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -88,19 +97,19 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
   const int n_iter = list_cnt * ratio;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kBwdStages; ++s) {
-      mbar_init(&full[s], 1);
-      mbar_init(&empty[s], 1);
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&q_full[s], 2);
+      mbar_init(&q_empty[s], 1);
     }
+    mbar_init(do_full, 2);
+    mbar_init(do_empty, 1);
     mbar_init(kv_full, 1);
-    for (int g = 0; g < 2; ++g) {
-      mbar_init(&s_full[g], 1);
-      mbar_init(&dp_full[g], 1);
-      mbar_init(&p_full[g], 128);
-      mbar_init(&ds_full[g], 128);
-      mbar_init(&dq_full[g], 1);
-      mbar_init(&dq_read[g], 128);
-    }
+    mbar_init(s_full, 1);
+    mbar_init(p_full, 256);
+    mbar_init(dp_full, 1);
+    mbar_init(ds_full, 256);
+    mbar_init(dq_full, 1);
+    mbar_init(dq_read, 128);
     mbar_init(dkv_full, 1);
     mbar_fence_init();
   }
@@ -112,264 +121,319 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
-  constexpr uint32_t kColSlot = 0, kColDP = 128, kColDK = 256, kColDV = 384;  // slot / dP: + 64 * group
+  constexpr uint32_t kColS = 0, kColDP = 128, kColDK = 256, kColDV = 384;
 
-  if (warp == 0) {
-    // ---------------------------------------------------------------- producer (whole warp)
-    if (n_iter > 0) {
+  // a wait of a whole warp
+  auto wait = [&](uint64_t* bar, uint32_t parity, int code) {
+    const bool r = __all_sync(0xffffffffu, mbar_wait(bar, parity, p.status, code));
+    tc_fence_after();
+    return r;
+  };
+
+  if (warp < 4) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kBwdRegsIssue));
+    if (warp == 0 && n_iter > 0) {
+      // ---------------------------------------------------------------- producer (whole warp)
       if (lane == 0) {
-        mbar_expect_tx(kv_full, 2 * Cfg::kKvTileBytes);
+        mbar_expect_tx(kv_full, 2 * kTileBytes);
         for (int ch = 0; ch < D / 64; ++ch) {
           tma_load_2d(smem_k + ch * 16384, &tma_k, kv_full, kvh * D + ch * 64, kv_row0);
           tma_load_2d(smem_v + ch * 16384, &tma_v, kv_full, kvh * D + ch * 64, kv_row0);
         }
       }
       bool ok = true;
-      for (int it = 0; it < n_iter; ++it) {
-        const int s = it % kBwdStages;
-        const uint32_t ph = (it / kBwdStages) & 1;
-        int okw = 1;
-        if (lane == 0) okw = mbar_wait(&empty[s], ph ^ 1, p.status, kTimeoutEmpty) ? 1 : 0;
-        okw = __shfl_sync(0xffffffffu, okw, 0);
-        if (!okw) {
-          ok = false;
-          break;
-        }
-        const int* e = p.list + static_cast<long long>(list_off + it / ratio) * 4;
+      int hd = 0;
+      const int* e = p.list + static_cast<long long>(list_off) * 4;
+      for (int i = 0; i < n_iter && ok; ++i) {
+        const int s = i & 1;
         const int q_row0 = e[0];
-        const int head = kvh * ratio + it % ratio;
-        float* st = smem_stat + s * 128;
+        const int head = kvh * ratio + hd;
+        if (++hd == ratio) {
+          hd = 0;
+          e += 4;
+        }
+        // the statistics are on their way while the buffers are waited for
+        const float* lse = p.lse + static_cast<long long>(head) * p.T + q_row0;
+        const float* delta = p.delta + static_cast<long long>(head) * p.T + q_row0;
+        float a[4], d[4];
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          const int idx = lane + 32 * i;
-          const long long t = static_cast<long long>(q_row0) + idx;
-          const bool in = t < p.T;
-          st[idx] = in ? p.lse[static_cast<long long>(head) * p.T + t] * 1.4426950408889634f : 0.f;
-          st[64 + idx] = in ? p.delta[static_cast<long long>(head) * p.T + t] : 0.f;
+        for (int j = 0; j < 4; ++j) {
+          const bool in = q_row0 + lane + 32 * j < p.T;
+          a[j] = in ? -lse[lane + 32 * j] * 1.4426950408889634f : 0.f;
+          d[j] = in ? -delta[lane + 32 * j] : 0.f;
         }
-        __syncwarp();
+        ok = wait(&q_empty[s], ((i >> 1) & 1) ^ 1, kTimeoutEmpty);
+        if (!ok) break;
         if (lane == 0) {
-          uint8_t* sq = smem_qdo + s * 2 * Cfg::kQTileBytes;
-          uint8_t* sdo = sq + Cfg::kQTileBytes;
-          mbar_expect_tx(&full[s], 2 * Cfg::kQTileBytes);
-          for (int ch = 0; ch < D / 64; ++ch) {
-            tma_load_2d(sq + ch * QCH, &tma_q, &full[s], head * D + ch * 64, q_row0);
-            tma_load_2d(sdo + ch * QCH, &tma_do, &full[s], head * D + ch * 64, q_row0);
-          }
+          mbar_expect_tx(&q_full[s], kTileBytes);
+          for (int ch = 0; ch < D / 64; ++ch)
+            tma_load_2d(smem_q + s * kTileBytes + ch * 16384, &tma_q, &q_full[s], head * D + ch * 64, q_row0);
         }
+        // (tile i - 2's -lse and -delta were read before its P^T and dS^T were published, and dK(i - 2) came after both)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) smem_lse[s * 128 + lane + 32 * j] = a[j];
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&q_full[s]);
+        ok = wait(do_empty, (i & 1) ^ 1, kTimeoutEmpty);
+        if (!ok) break;
+        if (lane == 0) {
+          mbar_expect_tx(do_full, kTileBytes);
+          for (int ch = 0; ch < D / 64; ++ch) tma_load_2d(smem_do + ch * 16384, &tma_do, do_full, head * D + ch * 64, q_row0);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) smem_delta[s * 128 + lane + 32 * j] = d[j];
+        __syncwarp();
+        if (lane == 0) mbar_arrive(do_full);
       }
       if (!ok && lane == 0) {
         const uint64_t t0 = global_timer_ns();
         while (global_timer_ns() - t0 < 100000ull) {
         }
       }
-    }
-  } else if (warp == 1) {
-    // ---------------------------------------------------------------- MMA issuer
-    if (lane == 0 && n_iter > 0) {
-      const uint32_t idesc_st = umma_idesc_bf16(128, kBwdQTile, 0, 0);  // S^T, dP^T : A K-major, B K-major
-      const uint32_t idesc_dv = umma_idesc_bf16(128, D, 0, 1);          // dV, dK    : A K-major, B MN-major
-      const uint32_t idesc_dq = umma_idesc_bf16(128, kBwdQTile, 1, 1);  // dQ^T      : A MN-major, B MN-major
-      const uint32_t ka = smem_u32(smem_k), va = smem_u32(smem_v);
-      auto stage_q = [&](int s) { return smem_u32(smem_qdo + s * 2 * Cfg::kQTileBytes); };
-      auto issue_st = [&](uint32_t a_base, uint32_t b_base, uint32_t tcol) {
+    } else if (warp == 1 && n_iter > 0) {
+      // -------------------------------------------------------------- MMA issuer (whole warp, one elected lane issues: see
+      // gemm_tcgen05_2cta.cu)
+      const uint32_t idesc_kk = umma_idesc_bf16(128, 128, 0, 0);        // S^T, dP^T : A K-major, B K-major
+      const uint32_t idesc_kn = umma_idesc_bf16(128, 128, 0, 1);        // dV, dK    : A K-major, B N-major
+      const uint32_t idesc_mn = umma_idesc_bf16(128, 128, 1, 1);        // dQ        : A M-major, B N-major
+      auto kmajor = [&](const uint8_t* t) { return umma_smem_desc(smem_u32(t), 0, 1024); };
+      auto nmajor = [&](const uint8_t* t) { return umma_smem_desc(smem_u32(t), 16384, 1024); };
+      const uint64_t k_k = kmajor(smem_k), v_k = kmajor(smem_v), k_n = nmajor(smem_k), q_k = kmajor(smem_q), q_n = nmajor(smem_q),
+                     do_k = kmajor(smem_do), do_n = nmajor(smem_do), ds_k = kmajor(smem_ds), ds_m = nmajor(smem_ds);
+      constexpr uint32_t kTile = kTileBytes >> 4;
+      // by the elected lane: one product, eight steps of 16; a K-major operand advances within 64-column chunks, an M- or
+      // N-major one by 16 rows
+      auto product = [&](uint32_t col, uint64_t a, bool a_rows, uint64_t b, bool b_rows, uint32_t idesc, bool first) {
 #pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-          const uint32_t aoff = (k / 4) * 16384 + (k % 4) * 32;
-          const uint32_t boff = (k / 4) * QCH + (k % 4) * 32;
-          umma_bf16_ss(tmem_base + tcol, umma_smem_desc(a_base + aoff, 0, 1024),
-                       umma_smem_desc(b_base + boff, 0, 1024), idesc_st, k > 0 ? 1u : 0u);
-        }
+        for (int k = 0; k < 8; ++k)
+          umma_bf16_ss(tmem_base + col, a + (a_rows ? k * 128 : (k / 4) * 1024 + (k % 4) * 2),
+                       b + (b_rows ? k * 128 : (k / 4) * 1024 + (k % 4) * 2), idesc, (!first || k > 0) ? 1u : 0u);
       };
-      bool ok = mbar_wait(kv_full, 0, p.status, kTimeoutFull);
-      // S^T and dP^T of the first tile of each group
-      for (int j = 0; j < 2 && j < n_iter && ok; ++j) {
-        ok = mbar_wait(&full[j % kBwdStages], 0, p.status, kTimeoutFull);
-        if (!ok) break;
-        tc_fence_after();
-        issue_st(ka, stage_q(j % kBwdStages), kColSlot + j * 64);
-        tc_commit(&s_full[j]);
-        issue_st(va, stage_q(j % kBwdStages) + Cfg::kQTileBytes, kColDP + j * 64);
-        tc_commit(&dp_full[j]);
-      }
-      for (int it = 0; it < n_iter && ok; ++it) {
-        const int s = it % kBwdStages;
-        const int g = it & 1;
-        const uint32_t par = (it >> 1) & 1;
-        const uint32_t sq = stage_q(s), sdo = sq + Cfg::kQTileBytes;
-        const uint32_t slot = tmem_base + kColSlot + g * 64;
-        // dV += P^T dO
-        if (!mbar_wait(&p_full[g], par, p.status, kTimeoutTmemEmpty)) { ok = false; break; }
-        tc_fence_after();
-#pragma unroll
-        for (int k = 0; k < kBwdQTile / 16; ++k)
-          umma_bf16_ts(tmem_base + kColDV, slot + k * 8, umma_smem_desc(sdo + k * 2048, QCH, 1024), idesc_dv,
-                       (it > 0 || k > 0) ? 1u : 0u);
-        // S^T and dP^T of the other group's next tile (its slot is free once dQ^T of tile it-1 has been read)
-        if (it >= 1 && it + 1 < n_iter) {
-          const int it1 = it + 1, g1 = g ^ 1, s1 = it1 % kBwdStages;
-          if (!mbar_wait(&dq_read[g1], ((it - 1) >> 1) & 1, p.status, kTimeoutTmemEmpty) ||
-              !mbar_wait(&full[s1], (it1 / kBwdStages) & 1, p.status, kTimeoutFull)) { ok = false; break; }
-          tc_fence_after();
-          issue_st(ka, stage_q(s1), kColSlot + g1 * 64);
-          tc_commit(&s_full[g1]);
-          issue_st(va, stage_q(s1) + Cfg::kQTileBytes, kColDP + g1 * 64);
-          tc_commit(&dp_full[g1]);
+      auto scores_of = [&](uint32_t s) {
+        if (elect_one()) {
+          product(kColS, k_k, false, q_k + s * kTile, false, idesc_kk, true);
+          tc_commit(s_full);
         }
-        // dK += dS^T Q ; dQ^T = K^T dS^T (into the slot, whose P^T the dV product above has consumed: the
-        // tensor core executes one CTA's MMAs in issue order)
-        if (!mbar_wait(&ds_full[g], par, p.status, kTimeoutTmemEmpty)) { ok = false; break; }
-        tc_fence_after();
-        const uint32_t dsa = smem_u32(smem_ds + g * Cfg::kDsBytes);
+        __syncwarp();
+      };
+      auto dp_of = [&]() {
+        if (elect_one()) {
+          product(kColDP, v_k, false, do_k, false, idesc_kk, true);
+          tc_commit(dp_full);
+        }
+        __syncwarp();
+      };
+      auto dv_of = [&](bool first) {       // P^T: columns [0, 64) in TMEM columns [0, 32), columns [64, 128) in [64, 96)
+        if (elect_one()) {
 #pragma unroll
-        for (int k = 0; k < kBwdQTile / 16; ++k)
-          umma_bf16_ss(tmem_base + kColDK, umma_smem_desc(dsa + k * 32, 0, 1024),
-                       umma_smem_desc(sq + k * 2048, QCH, 1024), idesc_dv, (it > 0 || k > 0) ? 1u : 0u);
-#pragma unroll
-        for (int k = 0; k < 128 / 16; ++k)
-          umma_bf16_ss(slot, umma_smem_desc(ka + k * 2048, 16384, 1024), umma_smem_desc(dsa + k * 2048, 0, 1024),
-                       idesc_dq, k > 0 ? 1u : 0u);
-        tc_commit(&dq_full[g]);
-        tc_commit(&empty[s]);
+          for (int k = 0; k < 8; ++k)
+            umma_bf16_ts(tmem_base + kColDV, tmem_base + kColS + (k / 4) * 64 + (k % 4) * 8, do_n + k * 128, idesc_kn,
+                         (!first || k > 0) ? 1u : 0u);
+          tc_commit(do_empty);
+        }
+        __syncwarp();
+      };
+      bool ok = wait(kv_full, 0, kTimeoutFull) && wait(&q_full[0], 0, kTimeoutFull);
+      if (ok) {
+        scores_of(0);
+        ok = wait(do_full, 0, kTimeoutFull);
       }
-      if (ok) tc_commit(dkv_full);
+      if (ok) {
+        dp_of();
+        ok = wait(p_full, 0, kTimeoutTmemEmpty);
+      }
+      if (ok) dv_of(true);
+      for (int i = 0; i < n_iter && ok; ++i) {
+        const uint32_t par = i & 1, s = i & 1;
+        const bool next = i + 1 < n_iter;
+        // S(i+1) over P(i), which dV(i) has read: the tensor core executes one CTA's MMAs in issue order
+        if (next) {
+          ok = wait(&q_full[s ^ 1], ((i + 1) >> 1) & 1, kTimeoutFull);
+          if (!ok) break;
+          scores_of(s ^ 1);
+        }
+        ok = wait(ds_full, par, kTimeoutTmemEmpty);
+        if (!ok) break;
+        if (elect_one()) {
+          product(kColDP, ds_m, true, k_n, true, idesc_mn, true);
+          tc_commit(dq_full);
+          product(kColDK, ds_k, false, q_n + s * kTile, true, idesc_kn, i == 0);
+          tc_commit(&q_empty[s]);
+          if (!next) tc_commit(dkv_full);
+        }
+        __syncwarp();
+        if (next) {
+          ok = wait(do_full, par ^ 1, kTimeoutFull) && wait(dq_read, par, kTimeoutTmemEmpty);
+          if (!ok) break;
+          dp_of();
+          ok = wait(p_full, par ^ 1, kTimeoutTmemEmpty);
+          if (!ok) break;
+          dv_of(false);
+        }
+      }
     }
-  } else {
-    // ---------------------------------------------------------------- softmax / gradient group
+  } else if (warp < 12) {
+    // ------------------------------------------------------------------ P and dS: 64 columns of every tile per group
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kBwdRegsWork));
     const int quarter = warp & 3;
-    const int grp = (warp - 2) >> 2;    // gradient group: tiles grp, grp + 2, ...
-    const int r = quarter * 32 + lane;  // key row of the block (and head-dim index for dQ^T)
+    const int grp = (warp >> 2) - 1;
+    const int r = quarter * 32 + lane;  // key row of the block
     const uint32_t lane_off = static_cast<uint32_t>(quarter * 32) << 16;
     const bool row_ok = r < kv_valid;
+    const uint32_t t_s = tmem_base + lane_off + kColS + grp * 64, t_dp = tmem_base + lane_off + kColDP + grp * 64;
+    uint8_t* ds_row = smem_ds + grp * 16384 + r * 128;
+    const uint64_t c2 = xtc_pair(p.scale_log2, p.scale_log2);
     bool ok = true;
-    for (int it = grp; it < n_iter; it += 2) {
-      const uint32_t par = (it >> 1) & 1;
-      const int s = it % kBwdStages;
-      const int* e = p.list + static_cast<long long>(list_off + it / ratio) * 4;
-      const int q_row0 = e[0], q_valid = e[1], diag = e[2];
-      const int head = kvh * ratio + it % ratio;
-      const int c_min = (diag >= kBigDiag) ? 0 : max(0, r - diag);
-      const float* st = smem_stat + s * 128;
-      if (!mbar_wait(&full[s], (it / kBwdStages) & 1, p.status, kTimeoutFull) ||
-          !mbar_wait(&s_full[grp], par, p.status, kTimeoutTmemFull)) {
-        ok = false;
-        break;
+    int hd = 0;
+    const int4* e = reinterpret_cast<const int4*>(p.list) + list_off;
+    for (int i = 0; i < n_iter; ++i) {
+      const int s = i & 1;
+      const uint32_t par = i & 1;
+      const int q_valid = e->y - grp * 64, diag = e->z + grp * 64;      // of this group's columns
+      if (++hd == ratio) {
+        hd = 0;
+        ++e;
       }
-      tc_fence_after();
-      const uint32_t t_s = tmem_base + lane_off + kColSlot + grp * 64;
-      float pr[kBwdQTile];
+      // Columns that some rows do not see (the diagonal, the block's and the tile's end) take the masked form
+      const bool all = kv_valid == kBwdTile && q_valid >= 64 && diag >= 127;
+      const int c_min = !row_ok ? 64 : diag >= kBigDiag ? 0 : r - diag;
+      ok = wait(&q_full[s], (i >> 1) & 1, kTimeoutFull) && wait(s_full, par, kTimeoutTmemFull);
+      if (!ok) break;
+      uint64_t pr[32];                  // P^T in pairs of columns
+      {
+        const ulonglong2* nlse = reinterpret_cast<const ulonglong2*>(smem_lse + s * 128 + grp * 64);
+        uint32_t v[2][32], pk[32];
+        tmem_ld_32x32(t_s, v[0]);
+        tmem_ld_32x32(t_s + 32, v[1]);
+        tmem_ld_wait(v[0]);
+        tmem_ld_wait(v[1]);
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        uint32_t v[32];
-        tmem_ld_32x32(t_s + h * 32, v);
-        tmem_ld_wait();
-        uint32_t pk[16];
+        for (int u = 0; u < 16; ++u) {
+          const ulonglong2 n = nlse[u];
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          const int col = h * 32 + i;
-          const bool vis = row_ok && col >= c_min && col < q_valid;
-          pr[col] = vis ? exp2f(__uint_as_float(v[i]) * p.scale_log2 - st[col]) : 0.f;
+          for (int h = 0; h < 2; ++h) {
+            const int col = 4 * u + 2 * h;
+            float2 f = xtc_unpair(xtc_fma2(xtc_pair(__uint_as_float(v[col / 32][col % 32]), __uint_as_float(v[col / 32][col % 32 + 1])),
+                                           c2, h ? n.y : n.x));
+            f.x = xtc_ex2(f.x);
+            f.y = xtc_ex2(f.y);
+            if (!all) {
+              if (col < c_min || col >= q_valid) f.x = 0.f;
+              if (col + 1 < c_min || col + 1 >= q_valid) f.y = 0.f;
+            }
+            pr[col / 2] = xtc_pair(f.x, f.y);
+            pk[col / 2] = pack_bf16x2(f.x, f.y);
+          }
         }
-#pragma unroll
-        for (int i = 0; i < 16; ++i) pk[i] = pack_bf16x2(pr[h * 32 + 2 * i], pr[h * 32 + 2 * i + 1]);
-        tmem_st_32x16(t_s + h * 16, pk);
+        tmem_st_32x32(t_s, pk);
+        tmem_st_wait();
       }
-      tmem_st_wait();
       tc_fence_before();
-      mbar_arrive(&p_full[grp]);
-      // dS^T
-      if (!mbar_wait(&dp_full[grp], par, p.status, kTimeoutTmemFull)) {
-        ok = false;
-        break;
-      }
-      tc_fence_after();
-      uint8_t* ds_row = smem_ds + grp * Cfg::kDsBytes + r * 128;
+      mbar_arrive(p_full);
+      ok = wait(do_full, par, kTimeoutFull) && wait(dp_full, par, kTimeoutTmemFull);
+      if (!ok) break;
+      const ulonglong2* ndelta = reinterpret_cast<const ulonglong2*>(smem_delta + s * 128 + grp * 64);
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
+      for (int half = 0; half < 2; ++half) {
         uint32_t v[32];
-        tmem_ld_32x32(tmem_base + lane_off + kColDP + grp * 64 + h * 32, v);
-        tmem_ld_wait();
+        tmem_ld_32x32(t_dp + half * 32, v);
+        tmem_ld_wait(v);
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
           uint32_t o[4];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const int col = h * 32 + u * 8 + 2 * i;
-            const float a = pr[col] > 0.f ? pr[col] * (__uint_as_float(v[u * 8 + 2 * i]) - st[64 + col]) * p.scale : 0.f;
-            const float b = pr[col + 1] > 0.f
-                                ? pr[col + 1] * (__uint_as_float(v[u * 8 + 2 * i + 1]) - st[64 + col + 1]) * p.scale
-                                : 0.f;
-            o[i] = pack_bf16x2(a, b);
+          for (int h = 0; h < 2; ++h) {
+            const ulonglong2 n = ndelta[half * 8 + u * 2 + h];
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+              const int col = u * 8 + h * 4 + j * 2;
+              const uint64_t w = pr[half * 16 + col / 2];
+              float2 f = xtc_unpair(
+                  xtc_mul2(w, xtc_add2(xtc_pair(__uint_as_float(v[col]), __uint_as_float(v[col + 1])), j ? n.y : n.x)));
+              if (!all) {                            // whatever dP^T holds where a row does not see the column
+                const float2 q = xtc_unpair(w);
+                if (q.x == 0.f) f.x = 0.f;
+                if (q.y == 0.f) f.y = 0.f;
+              }
+              o[h * 2 + j] = pack_bf16x2(f.x, f.y);
+            }
           }
-          const int unit = (h * 4 + u) ^ (r & 7);
-          *reinterpret_cast<uint4*>(ds_row + unit * 16) = make_uint4(o[0], o[1], o[2], o[3]);
+          *reinterpret_cast<uint4*>(ds_row + (((half * 4 + u) ^ (r & 7)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
         }
       }
       fence_proxy_async_smem();
       tc_fence_before();
-      mbar_arrive(&ds_full[grp]);
-      // dQ^T -> global accumulator (this thread holds head-dim index r for 64 query rows)
-      if (!mbar_wait(&dq_full[grp], par, p.status, kTimeoutTmemFull)) {
-        ok = false;
-        break;
-      }
-      tc_fence_after();
-      float* dq = p.dq_acc + static_cast<long long>(q_row0) * p.ld_dq + static_cast<long long>(head) * D + r;
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        uint32_t v[32];
-        tmem_ld_32x32(t_s + h * 32, v);
-        tmem_ld_wait();
-        if (r < D) {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const int col = h * 32 + i;
-            if (col < q_valid) atomicAdd(dq + static_cast<long long>(col) * p.ld_dq, __uint_as_float(v[i]));
-          }
-        }
-      }
-      tc_fence_before();
-      mbar_arrive(&dq_read[grp]);
+      mbar_arrive(ds_full);
     }
-    // dK / dV of this block.  The TMEM loads are warp collectives: every lane runs them, only the
+    // dK (first group) and dV (second) of this block.  The TMEM loads are warp collectives: every lane runs them, only the
     // global stores are predicated on the row being inside the block.
-    ok = __all_sync(0xffffffffu, ok ? 1 : 0) != 0;
+    if (ok && n_iter > 0) ok = wait(dkv_full, 0, kTimeoutTmemFull);
     if (ok) {
-      if (n_iter > 0) ok = mbar_wait(dkv_full, 0, p.status, kTimeoutTmemFull);
-      ok = __all_sync(0xffffffffu, ok ? 1 : 0) != 0;
-      tc_fence_after();
-      if (ok) {
-        __nv_bfloat16* dkp = p.dk + (static_cast<long long>(kv_row0) + r) * p.ld_dk + static_cast<long long>(kvh) * D;
-        __nv_bfloat16* dvp = p.dv + (static_cast<long long>(kv_row0) + r) * p.ld_dv + static_cast<long long>(kvh) * D;
-        {
-          const int which = grp;  // group 0 stores dK, group 1 stores dV
-          __nv_bfloat16* dst = which ? dvp : dkp;
-          const uint32_t col0 = which ? kColDV : kColDK;
+      __nv_bfloat16* dst = grp ? p.dv + (static_cast<long long>(kv_row0) + r) * p.ld_dv : p.dk + (static_cast<long long>(kv_row0) + r) * p.ld_dk;
+      dst += static_cast<long long>(kvh) * D;
+      const float scale = grp ? 1.f : p.scale;
 #pragma unroll 1
-          for (int h = 0; h < D / 32; ++h) {
-            uint32_t v[32];
-            if (n_iter > 0) {  // uniform across the CTA
-              tmem_ld_32x32(tmem_base + lane_off + col0 + h * 32, v);
-              tmem_ld_wait();
-            } else {
+      for (int h = 0; h < D / 32; ++h) {
+        uint32_t v[32];
+        if (n_iter > 0) {  // uniform across the CTA
+          tmem_ld_32x32(tmem_base + lane_off + (grp ? kColDV : kColDK) + h * 32, v);
+          tmem_ld_wait(v);
+        } else {
 #pragma unroll
-              for (int i = 0; i < 32; ++i) v[i] = 0u;
-            }
-            if (row_ok) {
+          for (int j = 0; j < 32; ++j) v[j] = 0u;
+        }
+        if (row_ok) {
 #pragma unroll
-              for (int q = 0; q < 4; ++q) {
-                uint4 o;
-                o.x = pack_bf16x2(__uint_as_float(v[q * 8 + 0]), __uint_as_float(v[q * 8 + 1]));
-                o.y = pack_bf16x2(__uint_as_float(v[q * 8 + 2]), __uint_as_float(v[q * 8 + 3]));
-                o.z = pack_bf16x2(__uint_as_float(v[q * 8 + 4]), __uint_as_float(v[q * 8 + 5]));
-                o.w = pack_bf16x2(__uint_as_float(v[q * 8 + 6]), __uint_as_float(v[q * 8 + 7]));
-                *reinterpret_cast<uint4*>(dst + h * 32 + q * 8) = o;
-              }
-            }
+          for (int q = 0; q < 4; ++q) {
+            uint4 o;
+            o.x = pack_bf16x2(__uint_as_float(v[q * 8 + 0]) * scale, __uint_as_float(v[q * 8 + 1]) * scale);
+            o.y = pack_bf16x2(__uint_as_float(v[q * 8 + 2]) * scale, __uint_as_float(v[q * 8 + 3]) * scale);
+            o.z = pack_bf16x2(__uint_as_float(v[q * 8 + 4]) * scale, __uint_as_float(v[q * 8 + 5]) * scale);
+            o.w = pack_bf16x2(__uint_as_float(v[q * 8 + 6]) * scale, __uint_as_float(v[q * 8 + 7]) * scale);
+            *reinterpret_cast<uint4*>(dst + h * 32 + q * 8) = o;
           }
         }
       }
     }
+  } else {
+    // ------------------------------------------------------------------ dQ: one query row per thread
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kBwdRegsWork));
+    const int quarter = warp & 3;
+    const uint32_t t_dq = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + kColDP;
+    uint8_t* boxes = smem_out + quarter * 2 * kStagedBoxBytes;
+    int hd = 0;
+    const int4* e = reinterpret_cast<const int4*>(p.list) + list_off;
+    for (int i = 0; i < n_iter; ++i) {
+      const int q_row0 = e->x, rows = e->y - quarter * 32;      // rows of this warp that belong to the tile
+      const int head = kvh * ratio + hd;
+      if (++hd == ratio) {
+        hd = 0;
+        ++e;
+      }
+      if (!wait(dq_full, i & 1, kTimeoutTmemFull)) break;
+      uint32_t v[4][32];
+#pragma unroll
+      for (int b = 0; b < 4; ++b) tmem_ld_32x32(t_dq + b * 32, v[b]);
+#pragma unroll
+      for (int b = 0; b < 4; ++b) tmem_ld_wait(v[b]);
+      tc_fence_before();
+      mbar_arrive(dq_read);
+      if (rows <= 0) continue;
+#pragma unroll
+      for (int b = 0; b < 4; ++b) {
+        const StagedBox out{boxes + (b & 1) * kStagedBoxBytes, lane};
+        out.begin<1>();
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          float4 f = make_float4(__uint_as_float(v[b][u * 4]) * p.scale, __uint_as_float(v[b][u * 4 + 1]) * p.scale,
+                                 __uint_as_float(v[b][u * 4 + 2]) * p.scale, __uint_as_float(v[b][u * 4 + 3]) * p.scale);
+          if (lane >= rows) f = make_float4(0.f, 0.f, 0.f, 0.f);       // rows of another segment: whatever dS holds there
+          out.put(u, *reinterpret_cast<const uint4*>(&f));
+        }
+        out.send(&tma_dq, head * D + b * 32, q_row0 + quarter * 32, true);
+      }
+    }
+    if (lane == 0) tma_out_wait_all();
   }
 
   tc_fence_before();
@@ -414,7 +478,7 @@ int apb_attn_bwd(const void* q, const void* k, const void* v, const void* o, con
                  long long ld_dq, long long ld_dk, long long ld_dv, float scale, cudaStream_t stream) {
   using namespace apb;
   if (n_cta <= 0 || T <= 0) return 0;
-  if (D != 128 || (ldq % 8) || (ldk % 8) || (ldv % 8) || (lddo % 8) || (ld_dk % 8) || (ld_dv % 8) || Hq % Hkv)
+  if (D != 128 || (ld_dq % 4) || (ldq % 8) || (ldk % 8) || (ldv % 8) || (lddo % 8) || (ld_dk % 8) || (ld_dv % 8) || Hq % Hkv)
     return kBadArgument;
   {
     const long long warps = static_cast<long long>(T) * Hq;
@@ -422,15 +486,17 @@ int apb_attn_bwd(const void* q, const void* k, const void* v, const void* o, con
     attn_delta_kernel<<<grid, 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(o), ldo,
                                                 static_cast<const __nv_bfloat16*>(d_o), lddo, delta, T, Hq, D);
   }
-  CUtensorMap tq, tdo, tk, tv;
-  int rc = make_tmap_2d(&tq, q, 2, T, static_cast<uint64_t>(Hq) * D, ldq, 64, kBwdQTile);
+  CUtensorMap tq, tdo, tk, tv, tdq;
+  int rc = make_tmap_2d(&tq, q, 2, T, static_cast<uint64_t>(Hq) * D, ldq, 64, kBwdTile);
   if (rc) return 1000 + rc;
-  rc = make_tmap_2d(&tdo, d_o, 2, T, static_cast<uint64_t>(Hq) * D, lddo, 64, kBwdQTile);
+  rc = make_tmap_2d(&tdo, d_o, 2, T, static_cast<uint64_t>(Hq) * D, lddo, 64, kBwdTile);
   if (rc) return 2000 + rc;
   rc = make_tmap_2d(&tk, k, 2, T, static_cast<uint64_t>(Hkv) * D, ldk, 64, 128);
   if (rc) return 3000 + rc;
   rc = make_tmap_2d(&tv, v, 2, T, static_cast<uint64_t>(Hkv) * D, ldv, 64, 128);
   if (rc) return 4000 + rc;
+  rc = make_tmap_2d(&tdq, dq_acc, 4, T, static_cast<uint64_t>(Hq) * D, ld_dq, 32, 32);
+  if (rc) return 5000 + rc;
   AttnBwdParams p;
   p.cta = cta;
   p.list = list;
@@ -441,8 +507,6 @@ int apb_attn_bwd(const void* q, const void* k, const void* v, const void* o, con
   p.scale_log2 = scale * 1.4426950408889634f;
   p.lse = lse;
   p.delta = delta;
-  p.dq_acc = dq_acc;
-  p.ld_dq = ld_dq;
   p.dk = static_cast<__nv_bfloat16*>(dk);
   p.dv = static_cast<__nv_bfloat16*>(dv);
   p.ld_dk = ld_dk;
@@ -457,7 +521,7 @@ int apb_attn_bwd(const void* q, const void* k, const void* v, const void* o, con
     if (e != cudaSuccess) return static_cast<int>(e);
     configured[dev & 63] = true;
   }
-  attn_bwd_kernel<128><<<n_cta, kBwdThreads, AttnBwdCfg<128>::kSmemBytes, stream>>>(tq, tdo, tk, tv, p);
+  attn_bwd_kernel<128><<<n_cta, kBwdThreads, AttnBwdCfg<128>::kSmemBytes, stream>>>(tq, tdo, tk, tv, tdq, p);
   return static_cast<int>(cudaGetLastError());
 }
 }

@@ -131,67 +131,66 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
       }
     }
   } else if (warp == 1) {
-    // ---------------------------------------------------------------- MMA issuer
-    if (lane == 0 && n_blocks > 0) {
+    // ---------------------------------------------------------------- MMA issuer (whole warp, one elected lane issues: see
+    // gemm_tcgen05_2cta.cu)
+    if (n_blocks > 0) {
       const uint32_t idesc_s = umma_idesc_bf16(128, kKvBlock, 0, 0);
       const uint32_t idesc_o = umma_idesc_bf16(128, D, 0, 1);
-      bool ok = mbar_wait(q_full, 0, p.status, kTimeoutFull);
-      auto issue_s = [&](int g, int slot) {
-        const uint32_t qa = smem_u32(smem_q + g * Cfg::kTileBytes);
-        const uint32_t ka = smem_u32(smem_kv + slot * Cfg::kTileBytes);
+      const uint64_t desc_q = umma_smem_desc(smem_u32(smem_q), 0, 1024), desc_k = umma_smem_desc(smem_u32(smem_kv), 0, 1024);
+      const uint64_t desc_v = umma_smem_desc(smem_u32(smem_kv), 16384, 1024);
+      constexpr uint32_t kTile = Cfg::kTileBytes >> 4;
+      auto wait = [&](uint64_t* bar, uint32_t parity, int code) {
+        const bool r = __all_sync(0xffffffffu, mbar_wait(bar, parity, p.status, code));
+        tc_fence_after();
+        return r;
+      };
+      bool ok = wait(q_full, 0, kTimeoutFull);
+      auto issue_s = [&](uint32_t g, uint32_t slot) {      // by the elected lane
 #pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-          const uint32_t off = (k / 4) * 16384 + (k % 4) * 32;
-          umma_bf16_ss(tmem_base + g * 128, umma_smem_desc(qa + off, 0, 1024), umma_smem_desc(ka + off, 0, 1024),
-                       idesc_s, k > 0 ? 1u : 0u);
-        }
+        for (int k = 0; k < D / 16; ++k)
+          umma_bf16_ss(tmem_base + g * 128, desc_q + g * kTile + (k / 4) * 1024 + (k % 4) * 2,
+                       desc_k + slot * kTile + (k / 4) * 1024 + (k % 4) * 2, idesc_s, k > 0 ? 1u : 0u);
         tc_commit(&s_full[g]);
       };
-      auto issue_o = [&](int g, int slot) {
-        const uint32_t va = smem_u32(smem_kv + slot * Cfg::kTileBytes);
+      auto issue_o = [&](uint32_t g, uint32_t slot) {
 #pragma unroll
-        for (int k = 0; k < kKvBlock / 16; ++k) {
-          umma_bf16_ts(tmem_base + 256 + g * 128, tmem_base + g * 128 + k * 8,
-                       umma_smem_desc(va + k * 2048, 16384, 1024), idesc_o, k > 0 ? 1u : 0u);
-        }
+        for (int k = 0; k < kKvBlock / 16; ++k)
+          umma_bf16_ts(tmem_base + 256 + g * 128, tmem_base + g * 128 + k * 8, desc_v + slot * kTile + k * 128, idesc_o,
+                       k > 0 ? 1u : 0u);
         tc_commit(&o_full[g]);
       };
       // K_j sits in ring position 2j, V_j in 2j+1.
-      auto wait_slot = [&](int n) {
-        return mbar_wait(&kv_full[n % Cfg::kSlots], (n / Cfg::kSlots) & 1, p.status, kTimeoutFull);
-      };
+      auto wait_slot = [&](int n) { return wait(&kv_full[n % Cfg::kSlots], (n / Cfg::kSlots) & 1, kTimeoutFull); };
       if (ok) ok = wait_slot(0);
-      if (ok) {
-        tc_fence_after();
+      if (ok && elect_one()) {
         for (int g = 0; g < n_groups; ++g) issue_s(g, 0);
         // K_0 is released once both S_0 are done; later K_j are released after the second group's S_j.
         tc_commit(&kv_empty[0]);
       }
+      __syncwarp();
       for (int j = 0; j < n_blocks && ok; ++j) {
         const int nv = 2 * j + 1;
         const int nk = 2 * j + 2;
-        if (!wait_slot(nv)) {
-          ok = false;
-          break;
-        }
         const bool more = j + 1 < n_blocks;
-        if (more && !wait_slot(nk)) {
+        if (!wait_slot(nv) || (more && !wait_slot(nk))) {
           ok = false;
           break;
         }
-        tc_fence_after();
         for (int g = 0; g < n_groups; ++g) {
-          if (!mbar_wait(&p_full[g], j & 1, p.status, kTimeoutTmemEmpty)) {
+          if (!wait(&p_full[g], j & 1, kTimeoutTmemEmpty)) {
             ok = false;
             break;
           }
-          tc_fence_after();
-          issue_o(g, nv % Cfg::kSlots);
-          if (more) issue_s(g, nk % Cfg::kSlots);
+          if (elect_one()) {
+            issue_o(g, nv % Cfg::kSlots);
+            if (more) issue_s(g, nk % Cfg::kSlots);
+            if (g == n_groups - 1) {
+              tc_commit(&kv_empty[nv % Cfg::kSlots]);
+              if (more) tc_commit(&kv_empty[nk % Cfg::kSlots]);
+            }
+          }
+          __syncwarp();
         }
-        if (!ok) break;
-        tc_commit(&kv_empty[nv % Cfg::kSlots]);
-        if (more) tc_commit(&kv_empty[nk % Cfg::kSlots]);
       }
     }
   } else if (n_blocks > 0) {

@@ -37,7 +37,6 @@ constexpr int kPairBK = 64;
 constexpr int kPairBoxBytes = 128 * kPairBK * 2;   // 128 rows of A, or of one half of B
 constexpr int kPairEpiWarps = 8;
 constexpr int kPairThreads = 64 + 32 * kPairEpiWarps;
-constexpr int kPairOutBytes = 4096;                // a warp's 32 rows x 128 bytes on their way out
 constexpr int kPairTmemCols = 512;                 // two fp32 accumulators of 256 columns
 constexpr int kPairGroupM = 16;                    // row tiles that are walked before the next column tile
 
@@ -46,7 +45,7 @@ struct PairCfg {
   static constexpr int kHalves = NT / 256;
   static constexpr int kStageBytes = (1 + kHalves) * kPairBoxBytes;
   static constexpr int kStages = NT == 256 ? 6 : 4;
-  static constexpr int kSmem = kStages * kStageBytes + kPairEpiWarps * kPairOutBytes + 1024 /*align*/ + 256 /*barriers*/;
+  static constexpr int kSmem = kStages * kStageBytes + kPairEpiWarps * kStagedBoxBytes + 1024 /*align*/ + 256 /*barriers*/;
 };
 static_assert(PairCfg<256>::kSmem <= 227 * 1024 && PairCfg<512>::kSmem <= 227 * 1024, "shared memory of one CTA");
 
@@ -106,41 +105,6 @@ __device__ __forceinline__ void tc_commit_pair(uint32_t bar_cluster_addr) {
                : "memory");
 }
 
-// TMA store / addition of one staged box (32 rows x 128 bytes), and the wait until the previous one has left shared memory.
-__device__ __forceinline__ void tma_out_2d(const CUtensorMap* map, const void* smem_src, int x, int y, bool add) {
-  if (add)
-    asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3}], [%1];" ::"l"(
-                     reinterpret_cast<uint64_t>(map)),
-                 "r"(smem_u32(smem_src)), "r"(x), "r"(y)
-                 : "memory");
-  else
-    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%2, %3}], [%1];" ::"l"(
-                     reinterpret_cast<uint64_t>(map)),
-                 "r"(smem_u32(smem_src)), "r"(x), "r"(y)
-                 : "memory");
-  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-}
-__device__ __forceinline__ void tma_out_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-__device__ __forceinline__ void tma_out_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-
-// One staged box of a warp: eight 16-byte units per row, swizzled as the tensor map expects them.
-struct PairOut {
-  uint8_t* buf;
-  int lane;
-  __device__ __forceinline__ void begin() const {
-    if (lane == 0) tma_out_wait_read();
-    __syncwarp();
-  }
-  __device__ __forceinline__ void put(int unit, const uint4& v) const {
-    *reinterpret_cast<uint4*>(buf + lane * 128 + ((unit ^ (lane & 7)) << 4)) = v;
-  }
-  __device__ __forceinline__ void send(const CUtensorMap* map, int x, int y, bool add) const {
-    fence_proxy_async_smem();
-    __syncwarp();
-    if (lane == 0) tma_out_2d(map, buf, x, y, add);
-  }
-};
-
 // What a variant of the kernel does with its accumulators.  A kernel holds one of them: with all in one kernel the unrolled code of
 // the untaken ones pushed the taken one out of the instruction cache (gate/up of 18432 tokens: 2.6 ms against 0.9).
 enum PairEpi : int { kPairBf16, kPairF32, kPairSwiGLU, kPairGeGLU, kPairClampGLU, kPairPartial, kPairDlogits };
@@ -149,7 +113,7 @@ enum PairEpi : int { kPairBf16, kPairF32, kPairSwiGLU, kPairGeGLU, kPairClampGLU
 // output are clipped by the tensor maps; a box that would begin outside is not sent.
 template <int EPI>
 __device__ __forceinline__ void pair_epilogue(const GemmParams& p, const CUtensorMap& tma_c, const CUtensorMap& tma_c2,
-                                              const PairOut& out, int row0, int nb, const uint32_t (&acc)[4][32]) {
+                                              const StagedBox& out, int row0, int nb, const uint32_t (&acc)[4][32]) {
   const int row = row0 + out.lane;
   const bool row_ok = row < p.M;
   if constexpr (EPI == kPairPartial) {
@@ -228,7 +192,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* smem_out = smem + kStages * Cfg::kStageBytes;
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem_out + kPairEpiWarps * kPairOutBytes);
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem_out + kPairEpiWarps * kStagedBoxBytes);
   uint64_t* empty_bar = full_bar + kStages;
   uint64_t* tfull_bar = empty_bar + kStages;
   uint64_t* tempty_bar = tfull_bar + 2;
@@ -436,7 +400,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
     // ------------------------------------------------------------ epilogue (both CTAs)
     const int quarter = warp & 3;              // TMEM lanes this warp may read
     const int part = (warp - 2) >> 2;          // columns [128 part, +128) of every accumulator
-    const PairOut out{smem_out + (warp - 2) * kPairOutBytes, lane};
+    const StagedBox out{smem_out + (warp - 2) * kStagedBoxBytes, lane};
     uint32_t used[2] = {0, 0};
     int it = 0;
     bool ok = true;
@@ -458,7 +422,8 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
         uint32_t acc[4][32];
 #pragma unroll
         for (int c = 0; c < 4; ++c) tmem_ld_32x32(taddr + c * 32, acc[c]);
-        tmem_ld_wait();
+#pragma unroll
+        for (int c = 0; c < 4; ++c) tmem_ld_wait(acc[c]);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&tempty_bar[slot]), 0));

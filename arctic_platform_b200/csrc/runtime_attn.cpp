@@ -8,7 +8,7 @@
 //
 // Forward table: one entry per (query tile of 128 rows, KV head, pair of query
 // heads), longest first.  Backward table: one entry per (key block of 128 rows,
-// KV head) with the list of 64-row query tiles that can see the block, so that
+// KV head) with the list of 128-row query tiles that can see the block, so that
 // dK/dV of a shared prompt block are accumulated by ONE CTA over all rollouts of
 // the group and written once, without atomics and without replicated K/V.
 #include <algorithm>
@@ -20,7 +20,7 @@
 namespace {
 constexpr int kQTileFwd = 128;
 constexpr int kKvBlock = 128;
-constexpr int kQTileBwd = 64;
+constexpr int kQTileBwd = 128;
 constexpr int kBig = 1 << 28;
 
 struct Seg {

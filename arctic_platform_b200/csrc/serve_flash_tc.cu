@@ -51,7 +51,7 @@ __device__ __forceinline__ uint64_t flash_weights(uint32_t t_s, uint64_t scale2,
 #pragma unroll
   for (int c = 0; c < 4; ++c) {                        // the next 32 scores are on their way while these are worked on
     uint32_t(&r)[32] = stage[c & 1];
-    xtc_wait_load(r);
+    tmem_ld_wait(r);
     if (c < 3) tmem_ld_32x32(t_s + (c + 1) * 32, stage[(c + 1) & 1]);
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
@@ -122,7 +122,7 @@ __device__ __forceinline__ uint64_t flash_capped_weights(uint32_t t_s, const Cap
     uint32_t r[32];
     uint64_t v[16];
     tmem_ld_32x32(t_s + c * 32, r);
-    xtc_wait_load(r);
+    tmem_ld_wait(r);
     capped_exponents(r, k, off, v);
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
@@ -151,7 +151,7 @@ __device__ __forceinline__ uint64_t flash_fixed_weights(uint32_t t_s, const CapS
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
     uint32_t(&r)[32] = stage[c & 1];
-    xtc_wait_load(r);
+    tmem_ld_wait(r);
     if (c < 3) tmem_ld_32x32(t_s + (c + 1) * 32, stage[(c + 1) & 1]);
     uint64_t v[16];
     capped_exponents(r, k, off, v);
@@ -408,7 +408,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
           for (int c = 0; c < p.E; c += 32) {
             uint32_t o[32];
             tmem_ld_32x32(t_o + c, o);
-            xtc_wait_load(o);
+            tmem_ld_wait(o);
 #pragma unroll
             for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * f);
             tmem_st_32x32(t_o + c, o);
@@ -441,7 +441,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
       for (int c = 0; c < p.E; c += 32) {
         uint32_t o[32];
         tmem_ld_32x32(t_o + c, o);
-        xtc_wait_load(o);
+        tmem_ld_wait(o);
         if (!live) continue;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {

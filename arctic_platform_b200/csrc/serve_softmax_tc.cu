@@ -206,7 +206,7 @@ softmax_attn_tc_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_c
       for (int c = 0; c < kXtcKeys / 32; ++c) {        // the next 32 scores are on their way while these are worked on
         uint32_t(&r)[32] = ring[c & 1];
         uint32_t pk[16];
-        xtc_wait_load(r);
+        tmem_ld_wait(r);
         if (c + 1 < kXtcKeys / 32) tmem_ld_32x32(t_s + (c + 1) * 32, ring[(c + 1) & 1]);
         uint64_t v[16];                                // log2 weights of neighbouring keys
         float top = 0.f;

@@ -85,3 +85,44 @@ def test_zorro_matches_replicated_layout():
         assert torch.allclose(o2[P:].float(), o[t:t + r].float(), atol=1e-2, rtol=1e-2)
         t += r
     _lib.check_status("attn zorro")
+
+
+@pytest.mark.parametrize("Hq,Hkv", [(3, 3), (4, 1), (10, 2), (16, 2)])
+@pytest.mark.parametrize("sharp", [1.0, 4.0])
+def test_tile_edges_and_sharp_scores_against_64_bits(Hq, Hkv, sharp):
+    """Lengths around the 128-row tiles, prompts shared by several responses, every number of query heads per key head, and scores
+    wide enough that running maxima and references move.  o, P and dS are bf16 operands (2^-9 each) of sums that cancel in dS: a
+    few times 2^-8 of a gradient's norm."""
+    from arctic_platform_b200.ops import _lib
+    from arctic_platform_b200.ops.attention import AttnLayout, attention_ref, segment_attention
+    segs, t = [], 0
+    for plen, rlens in ((127, ()), (128, ()), (129, (1, 127)), (257, (128, 129, 33)), (64, (65,)), (1, (1,)), (384, (300,))):
+        p0 = t
+        segs.append([p0, plen, 0, 0, p0, plen])
+        t += plen
+        for r in rlens:
+            segs.append([t, r, p0, plen, t, r])
+            t += r
+    layout = AttnLayout(np.array(segs, dtype=np.int32), t)
+    torch.manual_seed(Hq)
+    q, k, v = _rand((t, Hq, 128), sharp).requires_grad_(), _rand((t, Hkv, 128)).requires_grad_(), _rand((t, Hkv, 128)).requires_grad_()
+    d_o = _rand((t, Hq, 128))
+    o = segment_attention(q, k, v, layout)
+    o.backward(d_o)
+    _lib.check_status("attention")
+    qr, kr, vr = (x.detach().double().requires_grad_() for x in (q, k, v))
+    ref = _attention64(qr, kr, vr, layout)
+    ref.backward(d_o.double())
+    assert (o.double() - ref).norm() <= 2 ** -7 * ref.norm()
+    for got, want in ((q.grad, qr.grad), (k.grad, kr.grad), (v.grad, vr.grad)):
+        assert (got.double() - want).norm() <= 2 ** -6 * want.norm()
+
+
+def _attention64(q, k, v, layout):
+    rep, out = q.shape[1] // k.shape[1], []
+    for qs, ql, ps, pl, os_, ol in layout.segs.tolist():
+        kk, vv = (torch.cat([x[ps:ps + pl], x[os_:os_ + ol]]).repeat_interleave(rep, 1) for x in (k, v))
+        s = torch.einsum("qhd,khd->hqk", q[qs:qs + ql], kk) * q.shape[-1] ** -0.5
+        seen = torch.arange(pl + ol, device=q.device)[None] <= pl + ol - ql + torch.arange(ql, device=q.device)[:, None]
+        out.append(torch.einsum("hqk,khd->qhd", torch.softmax(s.masked_fill(~seen, float("-inf")), -1), vv))
+    return torch.cat(out)
