@@ -11,14 +11,20 @@
 //  arctic_platform/rl/zorro_train/zorro_train.py:857-912); here the key tile index
 // is resolved in the kernel and nothing is replicated.
 //
-// CTA = 320 threads: warp 0 TMA producer, warp 1 MMA issuer, warps 2-5 and 6-9 two
-// softmax groups.  The two groups hold two query heads of the same KV head (same
+// CTA = 384 threads, one per SM, walking its share of the work table (longest tiles first): warp 0 TMA producer, warp 1 MMA
+// issuer, warps 4-7 and 8-11 two softmax groups.  The two groups hold two query heads of the same KV head (same
 // 128 query rows), so they walk the same K/V tiles and ping-pong on the tensor
 // core: while one group does softmax on S_j the other group's P*V and next S run.
 // S (fp32) lives in TMEM, P (bf16) overwrites it in place and feeds the P*V MMA as
-// the TMEM A operand, the P*V product is read back and accumulated in registers
-// with the usual online-softmax rescale.
-#include "common.cuh"
+// the TMEM A operand; P*V accumulates in TMEM.
+//
+// What bounds it: 2048 tensor cycles per pair of 128 x 128 blocks, and as many of the exponential unit (16 per cycle and SM) if it
+// took them all; the groups' exponentials hide behind each other's products, other instructions (one read of S,
+// maxima, packed fp32 arithmetic) behind both.  Weights are taken relative to a reference that follows a row's maximum only when
+// it, or that of another row of its warp, has moved by more than 2^8; O is rescaled on those occasions, in tensor memory, and read
+// once per tile.  Reading O after every block, scores twice, and one CTA per tile took 7200 cycles per pair of blocks
+// (8 x 4096 tokens, 32 / 8 heads: 1.74 ms, 630 TFLOP/s), this 4300 (1.04 ms, 1060; one sequence of 32768: 1180).
+#include "attention_common.cuh"
 #include "host_utils.cuh"
 
 namespace apb {
@@ -35,8 +41,12 @@ struct AttnFwdParams {
   int* status;
 };
 
-constexpr int kAttnThreads = 320;
+// Three warpgroups: issue and two of softmax.  Registers move from the first to the others: 56 + 2 * 224 = 3 * 168, what the block
+// was launched with.
+constexpr int kAttnThreads = 384;
+constexpr int kAttnRegsIssue = 56, kAttnRegsSoftmax = 224;
 constexpr int kKvBlock = 128;
+constexpr float kAttnSlack = 8.f;       // log2 units by which a row's maximum may exceed its reference
 
 template <int D>
 struct AttnCfg {
@@ -46,43 +56,49 @@ struct AttnCfg {
   static constexpr int kSmemBytes = 2 * kTileBytes + kSlots * kTileBytes + 1024 + 256;
 };
 
+struct AttnItem {
+  int q_row0, q_valid, pre_start, pre_len, own_start, own_len, diag, head0, n_groups, n_pre, n_blocks;
+  __device__ __forceinline__ explicit AttnItem(const int* w) {
+    const int4 a = *reinterpret_cast<const int4*>(w), b = *reinterpret_cast<const int4*>(w + 4);
+    q_row0 = a.x, q_valid = a.y, pre_start = a.z, pre_len = a.w;
+    own_start = b.x, own_len = b.y, diag = b.z;
+    head0 = b.w & 0xFFFF;
+    n_groups = (b.w >> 16) ? 2 : 1;
+    n_pre = (pre_len + kKvBlock - 1) / kKvBlock;
+    n_blocks = n_pre + (own_len + kKvBlock - 1) / kKvBlock;
+  }
+};
+
 template <int D>
 __global__ void __launch_bounds__(kAttnThreads, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant__ CUtensorMap tma_k,
                 const __grid_constant__ CUtensorMap tma_v, const AttnFwdParams p) {
   using Cfg = AttnCfg<D>;
+  constexpr int kSlots = Cfg::kSlots;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* smem_q = smem;                              // 2 tiles
   uint8_t* smem_kv = smem + 2 * Cfg::kTileBytes;       // ring
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem_kv + Cfg::kSlots * Cfg::kTileBytes);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem_kv + kSlots * Cfg::kTileBytes);
   uint64_t* kv_full = bars;                 // [kSlots]
-  uint64_t* kv_empty = bars + Cfg::kSlots;  // [kSlots]
-  uint64_t* q_full = bars + 2 * Cfg::kSlots;
-  uint64_t* s_full = q_full + 1;  // [2]
-  uint64_t* p_full = s_full + 2;  // [2]
-  uint64_t* o_full = p_full + 2;  // [2]
+  uint64_t* kv_empty = bars + kSlots;       // [kSlots]
+  uint64_t* q_full = bars + 2 * kSlots;
+  uint64_t* q_empty = q_full + 1;
+  uint64_t* s_full = q_empty + 1;  // [2]
+  uint64_t* p_full = s_full + 2;   // [2]
+  uint64_t* o_full = p_full + 2;   // [2]  once per work item
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(o_full + 2);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
 
-  const int* w = p.work + static_cast<long long>(blockIdx.x) * 8;
-  const int q_row0 = w[0], q_valid = w[1], pre_start = w[2], pre_len = w[3], own_start = w[4], own_len = w[5],
-            diag = w[6];
-  const int head0 = w[7] & 0xFFFF;
-  const int n_groups = (w[7] >> 16) ? 2 : 1;
-  const int kvh = head0 / (p.Hq / p.Hkv);
-  const int n_pre = (pre_len + kKvBlock - 1) / kKvBlock;
-  const int n_own = (own_len + kKvBlock - 1) / kKvBlock;
-  const int n_blocks = n_pre + n_own;
-
   if (threadIdx.x == 0) {
-    for (int s = 0; s < Cfg::kSlots; ++s) {
+    for (int s = 0; s < kSlots; ++s) {
       mbar_init(&kv_full[s], 1);
       mbar_init(&kv_empty[s], 1);
     }
     mbar_init(q_full, 1);
+    mbar_init(q_empty, 1);
     for (int g = 0; g < 2; ++g) {
       mbar_init(&s_full[g], 1);
       mbar_init(&p_full[g], 128);
@@ -98,53 +114,71 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
-  // TMEM map: S/P of group g at columns [g*128, g*128+128), P*V of group g at [256 + g*128, ...+D)
+  // TMEM map: S/P of group g at columns [g*128, g*128+128), O of group g at [256 + g*128, ...+D)
 
-  auto block_row = [&](int b) { return b < n_pre ? pre_start + b * kKvBlock : own_start + (b - n_pre) * kKvBlock; };
+  // This CTA's items: one of every gridDim.x, from the front and from the back in turn, so that the CTA with the longest item
+  // of one round gets the shortest of the next.
+  const int rounds = (p.num_work + gridDim.x - 1) / gridDim.x;
+  auto item_at = [&](int round) {
+    const int i = round * gridDim.x + ((round & 1) ? gridDim.x - 1 - blockIdx.x : blockIdx.x);
+    return i < p.num_work ? i : -1;
+  };
+  auto wait = [&](uint64_t* bar, uint32_t parity, int code) {      // of a whole warp
+    const bool r = __all_sync(0xffffffffu, mbar_wait(bar, parity, p.status, code));
+    tc_fence_after();
+    return r;
+  };
 
-  if (warp == 0) {
-    // ---------------------------------------------------------------- producer
-    if (lane == 0 && n_blocks > 0) {
-      mbar_expect_tx(q_full, n_groups * Cfg::kTileBytes);
-      for (int g = 0; g < n_groups; ++g)
-        for (int c = 0; c < Cfg::kChunks; ++c)
-          tma_load_2d(smem_q + g * Cfg::kTileBytes + c * 16384, &tma_q, q_full, (head0 + g) * D + c * 64, q_row0);
-      bool ok = true;
-      for (int n = 0; n < 2 * n_blocks && ok; ++n) {
-        const int slot = n % Cfg::kSlots;
-        const uint32_t phase = (n / Cfg::kSlots) & 1;
-        if (!mbar_wait(&kv_empty[slot], phase ^ 1, p.status, kTimeoutEmpty)) {
-          ok = false;
-          break;
+  if (warp < 4) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kAttnRegsIssue));
+    if (warp == 0) {
+      // ---------------------------------------------------------------- producer
+      if (lane == 0) {
+        bool ok = true;
+        int slot = 0;
+        uint32_t phase = 0, items = 0;
+        for (int round = 0; round < rounds && ok; ++round) {
+          const int at = item_at(round);
+          if (at < 0) continue;
+          const AttnItem w(p.work + static_cast<long long>(at) * 8);
+          if (w.n_blocks == 0) continue;
+          const int kvh = w.head0 / (p.Hq / p.Hkv);
+          ok = mbar_wait(q_empty, (items & 1) ^ 1, p.status, kTimeoutEmpty);
+          if (!ok) break;
+          ++items;
+          mbar_expect_tx(q_full, w.n_groups * Cfg::kTileBytes);
+          for (int g = 0; g < w.n_groups; ++g)
+            for (int c = 0; c < Cfg::kChunks; ++c)
+              tma_load_2d(smem_q + g * Cfg::kTileBytes + c * 16384, &tma_q, q_full, (w.head0 + g) * D + c * 64, w.q_row0);
+          for (int n = 0; n < 2 * w.n_blocks; ++n) {
+            ok = mbar_wait(&kv_empty[slot], phase ^ 1, p.status, kTimeoutEmpty);
+            if (!ok) break;
+            const int b = n >> 1;
+            const int row = b < w.n_pre ? w.pre_start + b * kKvBlock : w.own_start + (b - w.n_pre) * kKvBlock;
+            uint8_t* dst = smem_kv + slot * Cfg::kTileBytes;
+            mbar_expect_tx(&kv_full[slot], Cfg::kTileBytes);
+            const CUtensorMap* map = (n & 1) ? &tma_v : &tma_k;
+            for (int c = 0; c < Cfg::kChunks; ++c) tma_load_2d(dst + c * 16384, map, &kv_full[slot], kvh * D + c * 64, row);
+            if (++slot == kSlots) {
+              slot = 0;
+              phase ^= 1;
+            }
+          }
         }
-        const int row = block_row(n >> 1);
-        uint8_t* dst = smem_kv + slot * Cfg::kTileBytes;
-        mbar_expect_tx(&kv_full[slot], Cfg::kTileBytes);
-        const CUtensorMap* map = (n & 1) ? &tma_v : &tma_k;
-        for (int c = 0; c < Cfg::kChunks; ++c)
-          tma_load_2d(dst + c * 16384, map, &kv_full[slot], kvh * D + c * 64, row);
-      }
-      if (!ok) {
-        const uint64_t t0 = global_timer_ns();
-        while (global_timer_ns() - t0 < 100000ull) {
+        if (!ok) {
+          const uint64_t t0 = global_timer_ns();
+          while (global_timer_ns() - t0 < 100000ull) {
+          }
         }
       }
-    }
-  } else if (warp == 1) {
-    // ---------------------------------------------------------------- MMA issuer (whole warp, one elected lane issues: see
-    // gemm_tcgen05_2cta.cu)
-    if (n_blocks > 0) {
+    } else if (warp == 1) {
+      // -------------------------------------------------------------- MMA issuer (whole warp, one elected lane issues: see
+      // gemm_tcgen05_2cta.cu)
       const uint32_t idesc_s = umma_idesc_bf16(128, kKvBlock, 0, 0);
       const uint32_t idesc_o = umma_idesc_bf16(128, D, 0, 1);
       const uint64_t desc_q = umma_smem_desc(smem_u32(smem_q), 0, 1024), desc_k = umma_smem_desc(smem_u32(smem_kv), 0, 1024);
       const uint64_t desc_v = umma_smem_desc(smem_u32(smem_kv), 16384, 1024);
       constexpr uint32_t kTile = Cfg::kTileBytes >> 4;
-      auto wait = [&](uint64_t* bar, uint32_t parity, int code) {
-        const bool r = __all_sync(0xffffffffu, mbar_wait(bar, parity, p.status, code));
-        tc_fence_after();
-        return r;
-      };
-      bool ok = wait(q_full, 0, kTimeoutFull);
       auto issue_s = [&](uint32_t g, uint32_t slot) {      // by the elected lane
 #pragma unroll
         for (int k = 0; k < D / 16; ++k)
@@ -152,146 +186,182 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
                        desc_k + slot * kTile + (k / 4) * 1024 + (k % 4) * 2, idesc_s, k > 0 ? 1u : 0u);
         tc_commit(&s_full[g]);
       };
-      auto issue_o = [&](uint32_t g, uint32_t slot) {
+      auto issue_o = [&](uint32_t g, uint32_t slot, bool first) {
 #pragma unroll
         for (int k = 0; k < kKvBlock / 16; ++k)
           umma_bf16_ts(tmem_base + 256 + g * 128, tmem_base + g * 128 + k * 8, desc_v + slot * kTile + k * 128, idesc_o,
-                       k > 0 ? 1u : 0u);
-        tc_commit(&o_full[g]);
+                       (!first || k > 0) ? 1u : 0u);
       };
-      // K_j sits in ring position 2j, V_j in 2j+1.
-      auto wait_slot = [&](int n) { return wait(&kv_full[n % Cfg::kSlots], (n / Cfg::kSlots) & 1, kTimeoutFull); };
-      if (ok) ok = wait_slot(0);
-      if (ok && elect_one()) {
-        for (int g = 0; g < n_groups; ++g) issue_s(g, 0);
-        // K_0 is released once both S_0 are done; later K_j are released after the second group's S_j.
-        tc_commit(&kv_empty[0]);
-      }
-      __syncwarp();
-      for (int j = 0; j < n_blocks && ok; ++j) {
-        const int nv = 2 * j + 1;
-        const int nk = 2 * j + 2;
-        const bool more = j + 1 < n_blocks;
-        if (!wait_slot(nv) || (more && !wait_slot(nk))) {
-          ok = false;
-          break;
+      uint32_t slot = 0, phase = 0, items = 0, done[2] = {0, 0};       // done: blocks of each group whose P has been awaited
+      auto wait_slot = [&]() {         // the ring's next tile; its slot
+        const uint32_t s = slot;
+        const bool r = wait(&kv_full[s], phase, kTimeoutFull);
+        if (++slot == kSlots) {
+          slot = 0;
+          phase ^= 1;
         }
-        for (int g = 0; g < n_groups; ++g) {
-          if (!wait(&p_full[g], j & 1, kTimeoutTmemEmpty)) {
-            ok = false;
-            break;
-          }
-          if (elect_one()) {
-            issue_o(g, nv % Cfg::kSlots);
-            if (more) issue_s(g, nk % Cfg::kSlots);
-            if (g == n_groups - 1) {
-              tc_commit(&kv_empty[nv % Cfg::kSlots]);
-              if (more) tc_commit(&kv_empty[nk % Cfg::kSlots]);
+        return r;
+      };
+      bool ok = true;
+      for (int round = 0; round < rounds && ok; ++round) {
+        const int at = item_at(round);
+        if (at < 0) continue;
+        const AttnItem w(p.work + static_cast<long long>(at) * 8);
+        if (w.n_blocks == 0) continue;
+        uint32_t sk = slot;
+        ok = wait(q_full, items & 1, kTimeoutFull) && wait_slot();
+        if (!ok) break;
+        ++items;
+        if (elect_one()) {
+          for (int g = 0; g < w.n_groups; ++g) issue_s(g, sk);
+          tc_commit(&kv_empty[sk]);
+          if (w.n_blocks == 1) tc_commit(q_empty);
+        }
+        __syncwarp();
+        for (int j = 0; j < w.n_blocks && ok; ++j) {
+          const bool more = j + 1 < w.n_blocks;
+          const uint32_t sv = slot;
+          ok = wait_slot();
+          sk = slot;
+          if (ok && more) ok = wait_slot();
+          if (!ok) break;
+          for (int g = 0; g < w.n_groups && ok; ++g) {
+            ok = wait(&p_full[g], done[g] & 1, kTimeoutTmemEmpty);
+            if (!ok) break;
+            ++done[g];
+            if (elect_one()) {
+              issue_o(g, sv, j == 0);
+              if (more)
+                issue_s(g, sk);      // over P, which the product above reads first: the tensor core keeps the order of issue
+              else
+                tc_commit(&o_full[g]);
+              if (g == w.n_groups - 1) {
+                tc_commit(&kv_empty[sv]);
+                if (more) tc_commit(&kv_empty[sk]);
+                if (j + 2 == w.n_blocks) tc_commit(q_empty);
+              }
             }
+            __syncwarp();
           }
-          __syncwarp();
         }
       }
     }
-  } else if (n_blocks > 0) {
-    // ---------------------------------------------------------------- softmax groups
-    const int g = (warp - 2) >> 2;
-    if (g < n_groups) {
-      const int quarter = warp & 3;
-      const int row = quarter * 32 + lane;  // row inside the query tile
-      const uint32_t lane_off = static_cast<uint32_t>(quarter * 32) << 16;
-      const uint32_t t_s = tmem_base + lane_off + g * 128;
-      const uint32_t t_o = tmem_base + lane_off + 256 + g * 128;
-      float o_acc[D];
-#pragma unroll
-      for (int i = 0; i < D; ++i) o_acc[i] = 0.f;
-      float m_run = -INFINITY, l_run = 0.f;
-      bool ok = true;
-      for (int j = 0; j < n_blocks; ++j) {
-        if (!mbar_wait(&s_full[g], j & 1, p.status, kTimeoutTmemFull)) {
-          ok = false;
-          break;
-        }
-        tc_fence_after();
-        int limit;  // number of visible key columns of this block for this row
-        if (j < n_pre) {
-          limit = pre_len - j * kKvBlock;
+  } else {
+    // ------------------------------------------------------------------ softmax groups
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kAttnRegsSoftmax));
+    const int g = (warp >> 2) - 1;
+    const int quarter = warp & 3;
+    const int row = quarter * 32 + lane;  // row inside the query tile
+    const uint32_t lane_off = static_cast<uint32_t>(quarter * 32) << 16;
+    const uint32_t t_s = tmem_base + lane_off + g * 128;
+    const uint32_t t_o = tmem_base + lane_off + 256 + g * 128;
+    const uint64_t c2 = xtc_pair(p.scale_log2, p.scale_log2);
+    uint32_t blocks = 0, items = 0;       // of this group so far
+    bool ok = true;
+    for (int round = 0; round < rounds && ok; ++round) {
+      const int at = item_at(round);
+      if (at < 0) continue;
+      const AttnItem w(p.work + static_cast<long long>(at) * 8);
+      if (w.n_blocks == 0 || g >= w.n_groups) continue;
+      float m_ref = -INFINITY;
+      uint64_t l2 = 0;                    // row sum in two halves
+      for (int j = 0; j < w.n_blocks; ++j) {
+        ok = wait(&s_full[g], blocks & 1, kTimeoutTmemFull);
+        if (!ok) break;
+        ++blocks;
+        // visible key columns of this block: of this row, and of the tile's first row
+        int limit, least;
+        if (j < w.n_pre) {
+          limit = least = w.pre_len - j * kKvBlock;
         } else {
-          const int b0 = (j - n_pre) * kKvBlock;
-          limit = min(own_len - b0, row + diag - b0 + 1);
+          const int b0 = (j - w.n_pre) * kKvBlock;
+          least = min(w.own_len - b0, w.diag - b0 + 1);
+          limit = min(w.own_len - b0, row + w.diag - b0 + 1);
         }
-        limit = max(0, min(limit, kKvBlock));
-        // pass 1: row maximum
-        float mx = -INFINITY;
-#pragma unroll 1
-        for (int c = 0; c < kKvBlock / 32; ++c) {
-          uint32_t r[32];
-          tmem_ld_32x32(t_s + c * 32, r);
-          tmem_ld_wait();
+        uint32_t v[4][32];
 #pragma unroll
-          for (int i = 0; i < 32; ++i)
-            if (c * 32 + i < limit) mx = fmaxf(mx, __uint_as_float(r[i]));
+        for (int c = 0; c < 4; ++c) tmem_ld_32x32(t_s + c * 32, v[c]);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) tmem_ld_wait(v[c]);
+        if (least < kKvBlock) {
+#pragma unroll
+          for (int c = 0; c < kKvBlock; ++c)
+            if (c >= limit) v[c / 32][c % 32] = 0xff800000u;
         }
-        const float m_new = fmaxf(m_run, mx * p.scale_log2);
-        const float m_use = (m_new == -INFINITY) ? 0.f : m_new;
-        const float alpha = exp2f(m_run - m_use);  // m_run = -inf -> 0
-        // pass 2: probabilities, written over S as packed bf16 (two per 32-bit column)
-        float rowsum = 0.f;
+        float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+        for (int c = 0; c < kKvBlock; c += 2)
+          mx[(c >> 1) & 3] = fmaxf(fmaxf(mx[(c >> 1) & 3], __uint_as_float(v[c / 32][c % 32])), __uint_as_float(v[c / 32][c % 32 + 1]));
+        // the scale is positive: the maximum of the scaled scores is the scaled maximum
+        const float m_new = fmaxf(m_ref, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * p.scale_log2);
+        if (__any_sync(0xffffffffu, m_new > m_ref + kAttnSlack || m_ref == -INFINITY)) {
+          if (j > 0) {           // O holds the blocks before this one: their product was issued ahead of this S
+            const float alpha = m_ref == -INFINITY ? 0.f : xtc_ex2(m_ref - m_new);
+            l2 = xtc_mul2(l2, xtc_pair(alpha, alpha));
 #pragma unroll 1
-        for (int c = 0; c < kKvBlock / 32; ++c) {
-          uint32_t r[32];
-          tmem_ld_32x32(t_s + c * 32, r);
-          tmem_ld_wait();
+            for (int c = 0; c < D / 32; ++c) {
+              uint32_t o[32];
+              tmem_ld_32x32(t_o + c * 32, o);
+              tmem_ld_wait(o);
+#pragma unroll
+              for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+              tmem_st_32x32(t_o + c * 32, o);
+            }
+          }
+          m_ref = m_new;
+        }
+        const float m_use = m_ref == -INFINITY ? 0.f : m_ref;
+        const uint64_t nm2 = xtc_pair(-m_use, -m_use);
+        uint64_t sum[2] = {0, 0};
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
           uint32_t pk[16];
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
-            float p0 = exp2f(__uint_as_float(r[2 * i]) * p.scale_log2 - m_use);
-            float p1 = exp2f(__uint_as_float(r[2 * i + 1]) * p.scale_log2 - m_use);
-            if (c * 32 + 2 * i >= limit) p0 = 0.f;
-            if (c * 32 + 2 * i + 1 >= limit) p1 = 0.f;
-            rowsum += p0 + p1;
-            pk[i] = pack_bf16x2(p0, p1);
+            float2 f = xtc_unpair(
+                xtc_fma2(xtc_pair(__uint_as_float(v[c][2 * i]), __uint_as_float(v[c][2 * i + 1])), c2, nm2));
+            f.x = xtc_ex2(f.x);
+            f.y = xtc_ex2(f.y);
+            sum[i & 1] = xtc_add2(sum[i & 1], xtc_pair(f.x, f.y));
+            pk[i] = pack_bf16x2(f.x, f.y);
           }
           tmem_st_32x16(t_s + c * 16, pk);
         }
         tmem_st_wait();
         tc_fence_before();
         mbar_arrive(&p_full[g]);
-        l_run = l_run * alpha + rowsum;
-        m_run = m_new;
-        // accumulate P*V of this block
-        if (!mbar_wait(&o_full[g], j & 1, p.status, kTimeoutTmemFull)) {
-          ok = false;
-          break;
-        }
-        tc_fence_after();
-#pragma unroll
-        for (int c = 0; c < D / 32; ++c) {
-          uint32_t r[32];
-          tmem_ld_32x32(t_o + c * 32, r);
-          tmem_ld_wait();
-#pragma unroll
-          for (int i = 0; i < 32; ++i) o_acc[c * 32 + i] = o_acc[c * 32 + i] * alpha + __uint_as_float(r[i]);
-        }
-        tc_fence_before();
+        l2 = xtc_add2(l2, xtc_add2(sum[0], sum[1]));
       }
-      if (ok && row < q_valid) {
-        const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
-        const long long t = static_cast<long long>(q_row0) + row;
-        __nv_bfloat16* dst = p.O + t * p.ldo + static_cast<long long>(head0 + g) * D;
+      if (!ok) break;
+      ok = wait(&o_full[g], items & 1, kTimeoutTmemFull);
+      if (!ok) break;
+      ++items;
+      const float2 l = xtc_unpair(l2);
+      const float l_run = l.x + l.y;
+      const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
+      const long long t = static_cast<long long>(w.q_row0) + row;
+      __nv_bfloat16* dst = p.O + t * p.ldo + static_cast<long long>(w.head0 + g) * D;
+#pragma unroll 1
+      for (int c = 0; c < D / 32; ++c) {
+        uint32_t o[32];
+        tmem_ld_32x32(t_o + c * 32, o);
+        tmem_ld_wait(o);
+        if (row < w.q_valid) {
 #pragma unroll
-        for (int q = 0; q < D / 8; ++q) {
-          uint4 o;
-          o.x = pack_bf16x2(o_acc[q * 8 + 0] * inv, o_acc[q * 8 + 1] * inv);
-          o.y = pack_bf16x2(o_acc[q * 8 + 2] * inv, o_acc[q * 8 + 3] * inv);
-          o.z = pack_bf16x2(o_acc[q * 8 + 4] * inv, o_acc[q * 8 + 5] * inv);
-          o.w = pack_bf16x2(o_acc[q * 8 + 6] * inv, o_acc[q * 8 + 7] * inv);
-          *reinterpret_cast<uint4*>(dst + q * 8) = o;
+          for (int q = 0; q < 4; ++q) {
+            uint4 x;
+            x.x = pack_bf16x2(__uint_as_float(o[q * 8 + 0]) * inv, __uint_as_float(o[q * 8 + 1]) * inv);
+            x.y = pack_bf16x2(__uint_as_float(o[q * 8 + 2]) * inv, __uint_as_float(o[q * 8 + 3]) * inv);
+            x.z = pack_bf16x2(__uint_as_float(o[q * 8 + 4]) * inv, __uint_as_float(o[q * 8 + 5]) * inv);
+            x.w = pack_bf16x2(__uint_as_float(o[q * 8 + 6]) * inv, __uint_as_float(o[q * 8 + 7]) * inv);
+            *reinterpret_cast<uint4*>(dst + c * 32 + q * 8) = x;
+          }
         }
-        if (p.lse)
-          p.lse[static_cast<long long>(head0 + g) * p.T + t] =
-              l_run > 0.f ? (m_run + log2f(l_run)) * 0.6931471805599453f : -INFINITY;
       }
+      tc_fence_before();
+      if (p.lse && row < w.q_valid)
+        p.lse[static_cast<long long>(w.head0 + g) * p.T + t] =
+            l_run > 0.f ? (m_ref + log2f(l_run)) * 0.6931471805599453f : -INFINITY;
     }
   }
 
@@ -333,6 +403,7 @@ int apb_attn_fwd(const void* q, const void* k, const void* v, void* o, float* ls
   p.lse = lse;
   p.T = T;
   p.status = status_device_ptr();
+  const int grid = num_work < sm_count() ? num_work : sm_count();
   static bool configured[2][64] = {{false}};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -343,7 +414,7 @@ int apb_attn_fwd(const void* q, const void* k, const void* v, void* o, float* ls
       if (e != cudaSuccess) return static_cast<int>(e);
       configured[0][dev & 63] = true;
     }
-    attn_fwd_kernel<128><<<num_work, kAttnThreads, AttnCfg<128>::kSmemBytes, stream>>>(tq, tk, tv, p);
+    attn_fwd_kernel<128><<<grid, kAttnThreads, AttnCfg<128>::kSmemBytes, stream>>>(tq, tk, tv, p);
   } else {
     if (!configured[1][dev & 63]) {
       cudaError_t e = cudaFuncSetAttribute(attn_fwd_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -351,7 +422,7 @@ int apb_attn_fwd(const void* q, const void* k, const void* v, void* o, float* ls
       if (e != cudaSuccess) return static_cast<int>(e);
       configured[1][dev & 63] = true;
     }
-    attn_fwd_kernel<64><<<num_work, kAttnThreads, AttnCfg<64>::kSmemBytes, stream>>>(tq, tk, tv, p);
+    attn_fwd_kernel<64><<<grid, kAttnThreads, AttnCfg<64>::kSmemBytes, stream>>>(tq, tk, tv, p);
   }
   return static_cast<int>(cudaGetLastError());
 }
