@@ -49,21 +49,6 @@ struct PairCfg {
 };
 static_assert(PairCfg<256>::kSmem <= 227 * 1024 && PairCfg<512>::kSmem <= 227 * 1024, "shared memory of one CTA");
 
-__device__ __forceinline__ uint32_t cluster_cta_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// Address of `local_shared_addr` in the shared memory of CTA `rank` of this cluster.
-__device__ __forceinline__ uint32_t map_to_cta(uint32_t local_shared_addr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local_shared_addr), "r"(rank));
-  return r;
-}
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
@@ -589,7 +574,7 @@ int apb_gemm_bf16_pair_glu(const void* A, const void* B, void* C, int M, int N, 
     };
     int best = 1;
     double best_eff = wave_eff(1);
-    for (int s = 2; s <= 4; ++s) {
+    for (int s = 2; s <= 16; ++s) {
       if (k_blocks / s < 32) break;
       const double e = wave_eff(s);
       if (e > best_eff + 0.04) {

@@ -230,64 +230,61 @@ struct MoePlanOut {
   int max_tiles[4];
 };
 
-__global__ void __launch_bounds__(256)
+// One CTA per expert: it sums the experts before it and writes its own records (one CTA for all walked 512 columns of tiles per
+// expert and table in each thread, 94 us at 128 experts of 2048 x 768).
+__global__ void __launch_bounds__(128)
 moe_plan_kernel(const int* __restrict__ counts, int E, int H, int I, MoePlanOut out, int* __restrict__ seg_start,
                 int* __restrict__ n_tiles) {
-  __shared__ int row_off[513];
-  __shared__ int blk_off[513];
-  if (threadIdx.x == 0) {
-    int r = 0, b = 0;
-    for (int e = 0; e < E; ++e) {
-      row_off[e] = r;
-      blk_off[e] = b;
-      const int padded = (max(counts[e], 0) + 63) / 64 * 64;
-      r += padded;
-      b += (padded + 127) / 128;
-    }
-    row_off[E] = r;
-    blk_off[E] = b;
+  __shared__ int before[2];
+  const int e = blockIdx.x, tid = threadIdx.x, n = blockDim.x;
+  if (tid < 2) before[tid] = 0;
+  __syncthreads();
+  int rows = 0, blocks = 0;
+  for (int i = tid; i < e; i += n) {
+    const int padded = (max(counts[i], 0) + 63) / 64 * 64;
+    rows += padded;
+    blocks += (padded + 127) / 128;
+  }
+  if (rows) {
+    atomicAdd(&before[0], rows);
+    atomicAdd(&before[1], blocks);
   }
   __syncthreads();
+  const int r0 = before[0], r1 = r0 + (max(counts[e], 0) + 63) / 64 * 64;
+  const int b0 = before[1], b1 = b0 + (r1 - r0 + 127) / 128;
   const int I2 = 2 * I;
   const int nt[4] = {(I2 + 127) / 128, (H + 127) / 128, (I + 127) / 128, (H + 127) / 128};
   const int b_off_mul[4] = {I2, H, 0, 0};      // b_row_offset = e * this
   const int bk_mul[4] = {0, 0, H, I2};         // bk_off = e * this
-  for (int e = threadIdx.x; e <= E; e += blockDim.x) seg_start[e] = row_off[e];
-  for (int e = threadIdx.x; e < E; e += blockDim.x) {
-    const int r0 = row_off[e], r1 = row_off[e + 1];
-    int b = blk_off[e];
-    for (int m0 = r0; m0 < r1; m0 += 128, ++b) {
 #pragma unroll
-      for (int g = 0; g < 4; ++g) {
-        for (int t = 0; t < nt[g]; ++t) {
-          const int i = b * nt[g] + t;
-          if (i < out.max_tiles[g]) {
-            out.map[g][i] = make_int4(m0, r1, e * b_off_mul[g], t);
-            out.ext[g][i] = make_int4(0, 0, -1, e * bk_mul[g]);
-          }
-        }
+  for (int g = 0; g < 4; ++g) {
+    for (int k = tid; k < (b1 - b0) * nt[g]; k += n) {
+      const int i = b0 * nt[g] + k;
+      if (i < out.max_tiles[g]) {
+        out.map[g][i] = make_int4(r0 + k / nt[g] * 128, r1, e * b_off_mul[g], k % nt[g]);
+        out.ext[g][i] = make_int4(0, 0, -1, e * bk_mul[g]);
       }
     }
-    // weight gradients: tile (e, mt, nt) at a fixed position
-    const int kb0 = r0 / 64, kb1 = r1 / 64;
-    const int mt_dn = (H + 127) / 128, nt_dn = (I + 127) / 128;
-    for (int mt = 0; mt < mt_dn; ++mt)
-      for (int t = 0; t < nt_dn; ++t) {
-        const int i = (e * mt_dn + mt) * nt_dn + t;
-        out.map[4][i] = make_int4(mt * 128, H, 0, t);
-        out.ext[4][i] = make_int4(e * H, kb0, kb1, 0);
-      }
-    const int mt_gu = (I2 + 127) / 128, nt_gu = (H + 127) / 128;
-    for (int mt = 0; mt < mt_gu; ++mt)
-      for (int t = 0; t < nt_gu; ++t) {
-        const int i = (e * mt_gu + mt) * nt_gu + t;
-        out.map[5][i] = make_int4(mt * 128, I2, 0, t);
-        out.ext[5][i] = make_int4(e * I2, kb0, kb1, 0);
-      }
   }
-  if (threadIdx.x == 0) {
+  // weight gradients: tile (e, mt, nt) at a fixed position
+  const int kb0 = r0 / 64, kb1 = r1 / 64;
+  const int mt_dn = (H + 127) / 128, nt_dn = (I + 127) / 128;
+  for (int k = tid; k < mt_dn * nt_dn; k += n) {
+    out.map[4][e * mt_dn * nt_dn + k] = make_int4(k / nt_dn * 128, H, 0, k % nt_dn);
+    out.ext[4][e * mt_dn * nt_dn + k] = make_int4(e * H, kb0, kb1, 0);
+  }
+  const int mt_gu = (I2 + 127) / 128, nt_gu = (H + 127) / 128;
+  for (int k = tid; k < mt_gu * nt_gu; k += n) {
+    out.map[5][e * mt_gu * nt_gu + k] = make_int4(k / nt_gu * 128, I2, 0, k % nt_gu);
+    out.ext[5][e * mt_gu * nt_gu + k] = make_int4(e * I2, kb0, kb1, 0);
+  }
+  if (tid == 0) {
+    seg_start[e] = r0;
+    if (e == E - 1) {
+      seg_start[E] = r1;
 #pragma unroll
-    for (int g = 0; g < 4; ++g) n_tiles[g] = min(blk_off[E] * nt[g], out.max_tiles[g]);
+      for (int g = 0; g < 4; ++g) n_tiles[g] = min(b1 * nt[g], out.max_tiles[g]);
+    }
   }
 }
 
@@ -310,7 +307,7 @@ int apb_moe_plan(const int* counts, int E, int H, int I, void* const* maps, void
     o.ext[g] = static_cast<int4*>(exts[g]);
   }
   for (int g = 0; g < 4; ++g) o.max_tiles[g] = max_tiles[g];
-  moe_plan_kernel<<<1, 256, 0, s>>>(counts, E, H, I, o, seg_start, n_tiles);
+  moe_plan_kernel<<<E, 128, 0, s>>>(counts, E, H, I, o, seg_start, n_tiles);
   return static_cast<int>(cudaGetLastError());
 }
 

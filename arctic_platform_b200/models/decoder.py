@@ -21,7 +21,7 @@ from typing import Dict, Iterator, List, Optional, Tuple
 import torch
 from torch import nn
 
-from ..ops import gemm, norm
+from ..ops import gemm, norm, rows
 from ..ops.attention import AttnLayout, segment_attention
 from .config import DecoderConfig
 
@@ -312,7 +312,7 @@ class DecoderLM(nn.Module):
             finally:
                 for m in moes:
                     m.routed_experts = None
-        x = torch.nn.functional.embedding(input_ids, self.embed)
+        x = rows.embedding(input_ids, self.embed)
         rope = self.rope(x.device)
         positions = positions.to(torch.int32) if x.is_cuda else positions
         stream = None
@@ -361,7 +361,7 @@ def token_logprobs(model: DecoderLM, packed, inv_temperature=1.0, with_entropy: 
     if routed_experts is not None:          # [B, S, L_moe, k] aligned with the input grid -> packed token order
         routed_experts = packed.gather_inputs(routed_experts)
     hidden = model.forward_hidden(packed.input_ids, packed.positions, packed.layout, routed_experts)
-    pred = hidden.index_select(0, packed.pred_index)
+    pred = rows.gather_rows(hidden, packed.pred_index)
     if action_masks is not None:
         from ..utils.action_masks import masked_logprobs
         return masked_logprobs(pred, model.output_weight, packed.labels, action_masks, inv_temperature, with_entropy)

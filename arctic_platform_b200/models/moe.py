@@ -19,7 +19,7 @@ from typing import Optional, Tuple
 import torch
 from torch import nn
 
-from ..ops import gemm
+from ..ops import gemm, rows
 from .config import DecoderConfig
 
 
@@ -174,14 +174,6 @@ class MoEPlan:
             cap = torch.tensor(self.max_tiles, dtype=torch.int64, device=self.n_tiles.device)
             if bool((self.n_tiles.to(torch.int64) > cap).any()):
                 raise checked.TableError(f"moe_plan: tile counts {self.n_tiles.tolist()} exceed the tables {self.max_tiles}")
-
-    def padded_rows(self, sorted_expert: torch.Tensor) -> torch.Tensor:
-        """Padded row of every pair of an expert-sorted list (``sorted_expert [P]`` int64, ascending)."""
-        c64 = self.counts.to(torch.int64)
-        first = c64.cumsum(0) - c64
-        P = sorted_expert.numel()
-        within = torch.arange(P, device=sorted_expert.device) - first[sorted_expert]
-        return self.seg_start.to(torch.int64)[sorted_expert] + within
 
 
 _PLAN_FNS = {}
@@ -421,21 +413,24 @@ class MoEFeedForward(nn.Module):
         if self.ep is not None:
             return self.ep.forward(self, x, w, idx)
         k = cfg.num_experts_per_tok
+        planned = torch.is_grad_enabled() and padded_plan_supported(x, self.wgu)
+        if rows.moe_rows_supported(x, cfg.num_experts):
+            # rows go straight to their expert's place and come back weighted; with gradients the places are those of the padded
+            # plan, whose grouped GEMMs run forward and backward
+            counts, place = rows.moe_place(idx, cfg.num_experts, 64 if planned else 1)
+            self.last_tokens_per_expert = counts.detach()
+            if planned:
+                plan = MoEPlan(counts, place.numel(), H, self.wgu.shape[1] // 2)
+                ys = _GroupedFFNPaddedFn.apply(rows.moe_spread(x, place, plan.rows_cap, True), self.wgu, self.wdown, plan)
+            else:
+                ys = grouped_ffn(rows.moe_spread(x, place, place.numel()), self.wgu, self.wdown, counts)
+            return rows.moe_collect(ys, place, w, planned)
         flat_e = idx.reshape(-1)
         order = torch.argsort(flat_e, stable=True)
         counts = _expert_histogram(flat_e, cfg.num_experts)
         self.last_tokens_per_expert = counts.detach()
         src_tok = torch.div(order, k, rounding_mode="floor")
-        if torch.is_grad_enabled() and padded_plan_supported(x, self.wgu):
-            # training: padded expert-major rows, forward and backward as grouped GEMMs planned on the device
-            plan = MoEPlan(counts.to(torch.int32), flat_e.numel(), H, self.wgu.shape[1] // 2)
-            pos = plan.padded_rows(flat_e.index_select(0, order))
-            x_pad = torch.zeros((plan.rows_cap, H), device=x.device, dtype=x.dtype).index_copy(
-                0, pos, x.index_select(0, src_tok))
-            ys = _GroupedFFNPaddedFn.apply(x_pad, self.wgu, self.wdown, plan).index_select(0, pos)
-        else:
-            xs = x.index_select(0, src_tok)
-            ys = grouped_ffn(xs, self.wgu, self.wdown, counts)
+        ys = grouped_ffn(x.index_select(0, src_tok), self.wgu, self.wdown, counts)
         wflat = w.reshape(-1).index_select(0, order).to(ys.dtype)
         out = torch.zeros((T, H), device=x.device, dtype=torch.float32 if x.is_cuda else x.dtype)
         out.index_add_(0, src_tok, (ys * wflat[:, None]).to(out.dtype))
