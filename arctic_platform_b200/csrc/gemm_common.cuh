@@ -70,6 +70,7 @@ struct GemmParams {
   int heads, a_step, c_step;
   const __nv_bfloat16* gate;   // kEpiSigmoidGate
   long long ldg;
+  int staged;              // one-CTA kernel: fp32 results leave by TMA (set by the launcher)
   int chained;             // 1: launched in chained mode -- B (weights nobody in the chain writes) is prefetched
                            // before the wait for the previous kernel, everything else after it
 };
@@ -90,12 +91,17 @@ __device__ __forceinline__ float clamped_glu_f(float g, float u, float limit) {
 // epilogue except the two lm-head ones, which keep running state across the chunks of a tile.
 // `ncols` (32, or 16 for the last chunk of a tile width that is not a multiple of 32) clips the chunk at the tile
 // edge; columns at or beyond p.N are never written either.  `c_shift`: first column of the head in C (products per head).
+// MASK: the epilogue kinds (bits) that the calling kernel can have; code of the others is left out.  The unrolled code of all kinds is
+// longer than the instruction cache, and a kernel of one tile per CTA fetches what it jumps around as well.
+template <uint32_t MASK = ~0u>
 __device__ __forceinline__ void gemm_store_chunk(const GemmParams& p, int row, int col0, const uint32_t (&r)[32],
                                                  int ncols = 32, int c_shift = 0) {
+  auto is = [&](int epi) { return ((MASK >> epi) & 1u) && p.epi == epi; };
+  const bool glu = is(kEpiSwiGLU) || is(kEpiGeGLU) || is(kEpiClampGLU);
   float v[32];
 #pragma unroll
   for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]) * p.alpha;
-  if (p.epi == kEpiSigmoidGate) {
+  if (is(kEpiSigmoidGate)) {
     const __nv_bfloat16* g = p.gate + static_cast<long long>(row) * p.ldg + c_shift + col0;
 #pragma unroll
     for (int j = 0; j < 32; j += 8)
@@ -110,7 +116,7 @@ __device__ __forceinline__ void gemm_store_chunk(const GemmParams& p, int row, i
         }
       }
   }
-  if (p.epi == kEpiBf16 || p.epi == kEpiSigmoidGate || (is_glu_epilogue(p.epi) && p.C != nullptr)) {
+  if (is(kEpiBf16) || is(kEpiSigmoidGate) || (glu && p.C != nullptr)) {
     if (p.bias) {
 #pragma unroll
       for (int j = 0; j < 32; ++j)
@@ -129,7 +135,7 @@ __device__ __forceinline__ void gemm_store_chunk(const GemmParams& p, int row, i
       }
     }
   }
-  if (is_glu_epilogue(p.epi)) {
+  if (glu) {
     __nv_bfloat16* dst =
         static_cast<__nv_bfloat16*>(p.C2) + static_cast<long long>(row) * p.ldc2 + (col0 >> 1);
 #pragma unroll
@@ -139,7 +145,7 @@ __device__ __forceinline__ void gemm_store_chunk(const GemmParams& p, int row, i
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const float g = v[q * 16 + 2 * j], u = v[q * 16 + 2 * j + 1];
-          a[j] = p.epi == kEpiSwiGLU ? silu_f(g) * u : p.epi == kEpiGeGLU ? gelu_tanh_f(g) * u : clamped_glu_f(g, u, p.glu_limit);
+          a[j] = is(kEpiGeGLU) ? gelu_tanh_f(g) * u : is(kEpiClampGLU) ? clamped_glu_f(g, u, p.glu_limit) : silu_f(g) * u;
         }
         uint4 o;
         o.x = pack_bf16x2(a[0], a[1]);
@@ -149,13 +155,13 @@ __device__ __forceinline__ void gemm_store_chunk(const GemmParams& p, int row, i
         *reinterpret_cast<uint4*>(dst + q * 8) = o;
       }
     }
-  } else if (p.epi == kEpiF32 || p.epi == kEpiF32Accum) {
+  } else if (is(kEpiF32) || is(kEpiF32Accum)) {
     float* dst = static_cast<float*>(p.C) + static_cast<long long>(row) * p.ldc + col0;
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
       if (q * 4 < ncols && col0 + q * 4 < p.N) {
         float4 o = make_float4(v[q * 4], v[q * 4 + 1], v[q * 4 + 2], v[q * 4 + 3]);
-        if (p.epi == kEpiF32Accum) {
+        if (is(kEpiF32Accum)) {
           const float4 old = *reinterpret_cast<const float4*>(dst + q * 4);
           o.x += old.x;
           o.y += old.y;
@@ -165,7 +171,7 @@ __device__ __forceinline__ void gemm_store_chunk(const GemmParams& p, int row, i
         *reinterpret_cast<float4*>(dst + q * 4) = o;
       }
     }
-  } else if (p.epi == kEpiF32AtomicPeer) {
+  } else if (is(kEpiF32AtomicPeer)) {
     const int owner = min(row / p.rows_per_rank, p.world - 1);
     float* dst = static_cast<float*>(p.c_peers[owner]) +
                  static_cast<long long>(row - owner * p.rows_per_rank) * p.ldc + col0;
@@ -175,7 +181,7 @@ __device__ __forceinline__ void gemm_store_chunk(const GemmParams& p, int row, i
         atomicAdd(reinterpret_cast<float4*>(dst + q * 4),
                   make_float4(v[q * 4], v[q * 4 + 1], v[q * 4 + 2], v[q * 4 + 3]));
     }
-  } else if (p.epi == kEpiBf16ScatterPeer) {
+  } else if (is(kEpiBf16ScatterPeer)) {
     const int2 to = p.row_map[row];
     if (to.x >= p.world || to.y < 0) {
       atomicCAS(p.status, 0, kBadRouting);
@@ -193,7 +199,7 @@ __device__ __forceinline__ void gemm_store_chunk(const GemmParams& p, int row, i
         }
       }
     }
-  } else if (p.epi == kEpiF32Atomic) {
+  } else if (is(kEpiF32Atomic)) {
     float* dst = static_cast<float*>(p.C) + static_cast<long long>(row) * p.ldc + col0;
 #pragma unroll
     for (int q = 0; q < 8; ++q) {

@@ -24,30 +24,46 @@ namespace apb {
 constexpr int kBM = 128;
 constexpr int kBK = 64;
 constexpr int kGemmThreads = 192;
+constexpr int kFewRows = 32;      // rows of A up to which only that many are staged
 
 // ST = 0 picks the deepest ring that fits one CTA per SM; ST = 3 is the "two CTAs per SM" variant for skinny
 // (decode) problems whose tile count falls between one and two waves of SMs.
-template <int BN, int ST = 0>
+//
+// AR: rows of A that are staged.  A product of at most 32 rows (decoding few sequences) waits for the first touch of the weights, and
+// a full tile's 96 rows of zeros would take half of the ring: with 32 rows ten stages fit instead of six, and more of the weights are
+// on their way before the kernel that produces A has ended.  The MMA still multiplies 128 rows; the other 96 are whatever lies behind
+// the staged ones in the ring, and nobody reads their results.
+template <int BN, int ST = 0, int AR = kBM>
 struct GemmCfg {
-  static constexpr int kABytes = kBM * kBK * 2;
+  static constexpr int kABytes = AR * kBK * 2;
   static constexpr int kBBytes = BN * kBK * 2;
   static constexpr int kStageBytes = kABytes + kBBytes;
+  static_assert(kStageBytes >= kBM * kBK * 2, "the 128 rows that an MMA reads stay inside the stage");
+  // fp32 results leave through shared memory and TMA where the ring leaves room (4 KB per epilogue warp)
+  static constexpr bool kStaged = ST == 0 && BN != 208;
+  static constexpr int kRest = (kStaged ? 4 * kStagedBoxBytes : 0) + 1024 /*align*/ + 384 /*barriers*/;
   // deepest ring that fits: widths 144 and 208 (one wave of SMs for column counts such as 19456 or 151936 that
   // 128- or 256-wide tiles cut into "one wave and a bit") are 16-column multiples between the power-of-two widths
-  static constexpr int kStages = ST ? ST : (BN == 256) ? 4 : (BN > 144) ? 5 : (BN > 64) ? 6 : 8;
-  static constexpr int kSmemBytes = kStages * kStageBytes + 1024 /*align*/ + 256 /*barriers*/;
+  static constexpr int kStages = ST ? ST : (227 * 1024 - kRest) / kStageBytes;
+  static constexpr int kSmemBytes = kStages * kStageBytes + kRest;
+  static_assert(kSmemBytes <= 227 * 1024 && (2 * kStages + 4) * 8 + 8 <= 384, "shared memory of one CTA");
   static constexpr int kTmemCols = BN <= 64 ? 128 : (BN <= 128 ? 256 : 512);   // a power of two, two accumulators
   static constexpr int kAccStride = kTmemCols / 2;
   static constexpr int kChunks = (BN + 31) / 32;                                // 32-column epilogue chunks
 };
 
-template <int BN, int ST = 0>
+// Epilogue kinds of a kernel variant (see gemm_store_chunk).
+constexpr uint32_t kAnyEpi = ~0u, kBf16Epi = 1u << kEpiBf16, kSwiGluEpi = 1u << kEpiSwiGLU,
+                   kF32Epi = 1u << kEpiF32 | 1u << kEpiF32Atomic | 1u << kEpiF32Accum;
+
+template <int BN, int ST = 0, int AR = kBM, uint32_t MASK = kAnyEpi>
 __device__ __forceinline__ void gemm_body(const CUtensorMap& tma_a, const CUtensorMap& tma_b,
-                                          const CUtensorMap* a_peer_maps, const GemmParams& p) {
-  using Cfg = GemmCfg<BN, ST>;
+                                          const CUtensorMap* a_peer_maps, const CUtensorMap* tma_c, const GemmParams& p) {
+  using Cfg = GemmCfg<BN, ST, AR>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + Cfg::kStages * Cfg::kStageBytes);
+  uint8_t* smem_out = smem + Cfg::kStages * Cfg::kStageBytes;
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem_out + (Cfg::kStaged ? 4 * kStagedBoxBytes : 0));
   uint64_t* empty_bar = full_bar + Cfg::kStages;
   uint64_t* tfull_bar = empty_bar + Cfg::kStages;
   uint64_t* tempty_bar = tfull_bar + 2;
@@ -230,50 +246,45 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tma_a, const CUtens
       }
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      pdl_wait();
-      const uint32_t idesc = umma_idesc_bf16(kBM, BN, p.a_mn, p.b_mn);
-      int stage = 0;
-      uint32_t phase = 0;
-      int it = 0;
-      bool ok = true;
-      for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
-        int m0, m_end, b_row, n0, kb0, kb1;
-        decode(t, m0, m_end, b_row, n0, kb0, kb1);
-        if (kb1 <= kb0) continue;              // a group without rows: no loads, no accumulator, nothing stored
-        const int buf = it & 1;
-        const uint32_t acc_phase = (it >> 1) & 1;
-        ++it;
-        if (!mbar_wait(&tempty_bar[buf], acc_phase ^ 1, p.status, kTimeoutTmemEmpty)) {
-          ok = false;
-          break;
-        }
+    // ------------------------------------------------------------ MMA issuer: the whole warp walks the loop and one elected
+    // lane issues, so that stage numbers and descriptors are uniform (see gemm_tcgen05_2cta.cu)
+    pdl_wait();
+    const uint32_t idesc = umma_idesc_bf16(kBM, BN, p.a_mn, p.b_mn);
+    const uint32_t base = smem_u32(smem) >> 4;
+    const uint64_t desc_a = umma_smem_desc(0, p.a_mn ? 64 * kBK * 2 : 0, 1024) + base;
+    const uint64_t desc_b = umma_smem_desc(0, p.b_mn ? 64 * kBK * 2 : 0, 1024) + base + (Cfg::kABytes >> 4);
+    const uint32_t step_a = (p.a_mn ? 2048 : 32) >> 4, step_b = (p.b_mn ? 2048 : 32) >> 4;
+    uint32_t stage = 0, phase = 0;
+    int it = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
+      int m0, m_end, b_row, n0, kb0, kb1;
+      decode(t, m0, m_end, b_row, n0, kb0, kb1);
+      if (kb1 <= kb0) continue;              // a group without rows: no loads, no accumulator, nothing stored
+      const int buf = it & 1;
+      const uint32_t acc_phase = (it >> 1) & 1;
+      ++it;
+      ok = __all_sync(0xffffffffu, mbar_wait(&tempty_bar[buf], acc_phase ^ 1, p.status, kTimeoutTmemEmpty));
+      if (!ok) break;
+      tc_fence_after();
+      const uint32_t tmem_d = tmem_base + buf * Cfg::kAccStride;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        ok = __all_sync(0xffffffffu, mbar_wait(&full_bar[stage], phase, p.status, kTimeoutFull));
+        if (!ok) break;
         tc_fence_after();
-        const uint32_t tmem_d = tmem_base + buf * Cfg::kAccStride;
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(&full_bar[stage], phase, p.status, kTimeoutFull)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t sa = smem_u32(smem + stage * Cfg::kStageBytes);
-          const uint32_t sb = sa + Cfg::kABytes;
+        const uint64_t da = desc_a + stage * (Cfg::kStageBytes >> 4), db = desc_b + stage * (Cfg::kStageBytes >> 4);
+        if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < kBK / 16; ++k) {
-            const uint64_t da = p.a_mn ? umma_smem_desc(sa + k * 2048, 64 * kBK * 2, 1024)
-                                       : umma_smem_desc(sa + k * 32, 0, 1024);
-            const uint64_t db = p.b_mn ? umma_smem_desc(sb + k * 2048, 64 * kBK * 2, 1024)
-                                       : umma_smem_desc(sb + k * 32, 0, 1024);
-            umma_bf16_ss(tmem_d, da, db, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
-          }
+          for (int k = 0; k < kBK / 16; ++k)
+            umma_bf16_ss(tmem_d, da + k * step_a, db + k * step_b, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
           tc_commit(&empty_bar[stage]);
-          if (++stage == Cfg::kStages) {
-            stage = 0;
-            phase ^= 1;
-          }
+          if (kb + 1 == kb1) tc_commit(&tfull_bar[buf]);
         }
-        if (ok) tc_commit(&tfull_bar[buf]);
+        __syncwarp();
+        if (++stage == Cfg::kStages) {
+          stage = 0;
+          phase ^= 1;
+        }
       }
     }
   } else {
@@ -297,7 +308,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tma_a, const CUtens
       const int row = m0 + quarter * 32 + lane;
       const bool row_ok = row < m_end;
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * Cfg::kAccStride;
-      if (BN == 128 && p.epi == kEpiLogprobPartial) {      // one record per row and tile
+      if (MASK == kAnyEpi && BN == 128 && p.epi == kEpiLogprobPartial) {      // one record per row and tile
         uint32_t acc[4][32];
 #pragma unroll
         for (int c = 0; c < 4; ++c) tmem_ld_32x32(taddr + c * 32, acc[c]);
@@ -308,7 +319,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tma_a, const CUtens
         if (lane == 0) mbar_arrive(&tempty_bar[buf]);
         continue;
       }
-      if (p.epi == kEpiDlogits) {
+      if (MASK == kAnyEpi && p.epi == kEpiDlogits) {
         const LmheadRow lm = lmhead_row(p, row, row_ok);
 #pragma unroll 1
         for (int c = 0; c < BN / 32; ++c) {
@@ -353,13 +364,30 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tma_a, const CUtens
           tmem_ld_32x32(taddr + c * 32, r);
           tmem_ld_wait();
         }
+        if (MASK == kF32Epi && Cfg::kStaged && p.staged) {
+          // a box of 32 x 32 per warp; what it holds beyond the tile's rows or columns is added as zeros
+          const int row0 = m0 + quarter * 32;
+          if (row0 >= m_end) continue;
+          const StagedBox out{smem_out + quarter * kStagedBoxBytes, lane};
+          out.begin();
+#pragma unroll
+          for (int u = 0; u < 8; ++u) {
+            float4 f = make_float4(__uint_as_float(r[u * 4]) * p.alpha, __uint_as_float(r[u * 4 + 1]) * p.alpha,
+                                   __uint_as_float(r[u * 4 + 2]) * p.alpha, __uint_as_float(r[u * 4 + 3]) * p.alpha);
+            if (!row_ok || u * 4 >= ncols) f = make_float4(0.f, 0.f, 0.f, 0.f);
+            out.put(u, *reinterpret_cast<const uint4*>(&f));
+          }
+          out.send(tma_c, col0, row0 + c_off, p.epi != kEpiF32);
+          continue;
+        }
         if (!row_ok) continue;
-        gemm_store_chunk(p, row + c_off, col0, r, ncols, c_col);
+        gemm_store_chunk<MASK>(p, row + c_off, col0, r, ncols, c_col);
       }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tempty_bar[buf]);
     }
+    if (MASK == kF32Epi && Cfg::kStaged && p.staged && lane == 0) tma_out_wait_all();
   }
 
   // ---------------------------------------------------------------- teardown
@@ -371,11 +399,11 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tma_a, const CUtens
   }
 }
 
-template <int BN>
+template <int BN, int AR, uint32_t MASK>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
-                 const GemmParams p) {
-  gemm_body<BN>(tma_a, tma_b, nullptr, p);
+                 const __grid_constant__ CUtensorMap tma_c, const GemmParams p) {
+  gemm_body<BN, 0, AR, MASK>(tma_a, tma_b, nullptr, &tma_c, p);
 }
 
 // Two CTAs per SM with a 3-stage ring each (see GemmCfg).
@@ -383,7 +411,7 @@ template <int BN>
 __global__ void __launch_bounds__(kGemmThreads, 2)
 gemm_bf16_x2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                     const GemmParams p) {
-  gemm_body<BN, 3>(tma_a, tma_b, nullptr, p);
+  gemm_body<BN, 3>(tma_a, tma_b, nullptr, nullptr, p);
 }
 
 // Variant whose A operand is gathered from the other ranks' memory tile by tile (all-gather -> GEMM).
@@ -391,7 +419,7 @@ template <int BN>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_bf16_ag_kernel(const __grid_constant__ PeerTensorMaps a_maps, const __grid_constant__ CUtensorMap tma_b,
                     const GemmParams p) {
-  gemm_body<BN>(a_maps.m[0], tma_b, a_maps.m, p);
+  gemm_body<BN>(a_maps.m[0], tma_b, a_maps.m, nullptr, p);
 }
 
 }  // namespace apb
@@ -401,15 +429,14 @@ gemm_bf16_ag_kernel(const __grid_constant__ PeerTensorMaps a_maps, const __grid_
 // ---------------------------------------------------------------------------
 namespace apb {
 
-template <int BN>
-static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int max_ctas,
-                       cudaStream_t stream) {
-  using Cfg = GemmCfg<BN>;
+template <int BN, int AR, uint32_t MASK>
+static int launch_gemm_as(const CUtensorMap& ta, const CUtensorMap& tb, GemmParams p, int max_ctas, cudaStream_t stream) {
+  using Cfg = GemmCfg<BN, 0, AR>;
   static bool configured[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
   if (!configured[dev & 63]) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel<BN, AR, MASK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          Cfg::kSmemBytes);
     if (e != cudaSuccess) return static_cast<int>(e);
     configured[dev & 63] = true;
@@ -421,8 +448,36 @@ static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const GemmP
   int grid = static_cast<int>(total < sm_count() ? total : sm_count());
   if (max_ctas > 0 && grid > max_ctas) grid = max_ctas;
   if (grid <= 0) return 0;
-  return static_cast<int>(launch_kernel(gemm_bf16_kernel<BN>, dim3(grid), dim3(kGemmThreads), Cfg::kSmemBytes, stream,
-                                        ta, tb, p));
+  // fp32 results go out by TMA (a weight gradient of few rows is bound by them: as rows per thread every 16 bytes were an L1
+  // wavefront of their own).  Boxes have 32 rows and columns: slabs of a stacked C start at multiples of that, and a store (which
+  // cannot pad with zeros) ends with the tile.
+  CUtensorMap tc = ta;
+  const bool add = p.epi == kEpiF32Atomic || p.epi == kEpiF32Accum;
+  if (MASK == kF32Epi && Cfg::kStaged && p.C && p.heads == 0 && (p.ldc % 4) == 0 &&
+      (reinterpret_cast<uintptr_t>(p.C) & 15) == 0 && (!p.tile_ext || p.M % 32 == 0) &&
+      (add || (BN % 32 == 0 && !p.tile_map))) {
+    // with slabs, no box reaches beyond the rows of its own one, and their number is the caller's
+    const uint64_t c_rows = p.tile_ext && !p.num_tiles_dev ? uint64_t{1} << 24 : static_cast<uint64_t>(p.M);
+    if (make_tmap_2d(&tc, p.C, 4, c_rows, p.N, p.ldc, 32, 32) == 0) p.staged = 1;
+  }
+  return static_cast<int>(launch_kernel(gemm_bf16_kernel<BN, AR, MASK>, dim3(grid), dim3(kGemmThreads), Cfg::kSmemBytes, stream,
+                                        ta, tb, tc, p));
+}
+
+// The variant that holds the epilogue's code and little else (gate/up of 128 rows, 19456 x 2560: 38 us with the code of all kinds,
+// 32 with its own; 8 rows 40 and 27).  `few`: see GemmCfg; only for those kinds.
+static bool own_variant(const GemmParams& p) {
+  return ((kF32Epi >> p.epi) & 1u) || ((p.epi == kEpiSwiGLU || p.epi == kEpiBf16) && !p.bias);
+}
+template <int BN, int AR = kBM>
+static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int max_ctas, cudaStream_t stream) {
+  if (own_variant(p)) {
+    if (p.epi == kEpiSwiGLU) return launch_gemm_as<BN, AR, kSwiGluEpi>(ta, tb, p, max_ctas, stream);
+    if (p.epi == kEpiBf16) return launch_gemm_as<BN, AR, kBf16Epi>(ta, tb, p, max_ctas, stream);
+    return launch_gemm_as<BN, AR, kF32Epi>(ta, tb, p, max_ctas, stream);
+  }
+  if constexpr (AR == kBM) return launch_gemm_as<BN, AR, kAnyEpi>(ta, tb, p, max_ctas, stream);
+  return kBadArgument;
 }
 
 template <int BN>
@@ -503,10 +558,12 @@ static int gemm_bf16_impl(const void* A, const void* B, void* C, int M, int N, i
   if (splits > 1 && epi != kEpiF32Atomic) return kBadArgument;
   // Large plain problems go to the CTA-pair kernel (256 x 256 tiles, half of B per SM): at least one full wave
   // of pairs, automatic tile choice, no grid cap.  APB_GEMM_PAIR=0 keeps everything on the one-CTA kernel.
+  // Sums that add into C may also be cut along K (the pair kernel does so itself), which makes up for missing tiles.
+  const long long pair_cuts = epi == kEpiF32Accum ? (k_blocks / 32 < 1 ? 1 : k_blocks / 32 > 16 ? 16 : k_blocks / 32) : 1;
   if (bn == 0 && splits == 1 && !tile_map && max_ctas <= 0 && pair_kernel_enabled() &&
       (epi == kEpiBf16 || epi == kEpiF32 || epi == kEpiF32Accum || glu) &&
       !(epi == kEpiBf16 && !C) && M >= 512 &&
-      static_cast<long long>((M + 255) / 256) * ((N + 255) / 256) >= sm_count() / 2)
+      static_cast<long long>((M + 255) / 256) * ((N + 255) / 256) * pair_cuts >= sm_count() / 2)
     return apb_gemm_bf16_pair_glu(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, epi, alpha, bias, C2, ldc2, glu_limit, stream);
   if (bn == 0) {
     const long long tm = (M + kBM - 1) / kBM;
@@ -516,6 +573,14 @@ static int gemm_bf16_impl(const void* A, const void* B, void* C, int M, int N, i
     // skinny problems (decode): narrower tiles put more SMs on the weight stream
     if (bn == 128 && t128 * 10 < sm_count() * 7 && N >= 128) bn = 64;
     if (tile_map) bn = 128;
+    // "+=" of few tiles: parts of K add into C, at least four k-blocks each (weight gradient 768 x 256 of 4292 rows: 12 tiles of
+    // 128 x 128 took 31 us, 132 parts 10)
+    if (epi == kEpiF32Accum && splits == 1 && !tile_map && max_ctas <= 0 && N >= 128 && 2 * t128 <= sm_count() && k_blocks >= 8) {
+      bn = 128;
+      const int cuts = static_cast<int>(sm_count() / t128);
+      splits = cuts < k_blocks / 4 ? cuts : k_blocks / 4;
+      epi = kEpiF32Atomic;
+    }
     // one row tile (decode): the width that covers N in the fewest waves of SMs, then the fewest idle SMs
     if (!tile_map && tm == 1 && splits == 1 && !b_mn && N >= 1024 && epi != kEpiLogprobPartial && epi != kEpiDlogits) {
       const int cand[5] = {256, 208, 144, 128, 64};
@@ -541,10 +606,12 @@ static int gemm_bf16_impl(const void* A, const void* B, void* C, int M, int N, i
   if ((bn == 144 || bn == 208) && (b_mn || tile_map || epi == kEpiLogprobPartial || epi == kEpiDlogits))
     return kBadArgument;
 
+  const bool few = M <= kFewRows && !a_mn && !tile_map && !x2 && bn >= 128 &&     // see GemmCfg
+                   (((kF32Epi >> epi) & 1u) || ((epi == kEpiSwiGLU || epi == kEpiBf16) && !bias));
   CUtensorMap ta, tb;
   int rc;
   if (!a_mn)
-    rc = make_tmap_2d(&ta, A, 2, static_cast<uint64_t>(M), static_cast<uint64_t>(K), lda, 64, kBM);
+    rc = make_tmap_2d(&ta, A, 2, static_cast<uint64_t>(M), static_cast<uint64_t>(K), lda, 64, few ? kFewRows : kBM);
   else
     rc = make_tmap_2d(&ta, A, 2, static_cast<uint64_t>(K), static_cast<uint64_t>(M), lda, 64, 64);
   if (rc) return 1000 + rc;
@@ -581,6 +648,12 @@ static int gemm_bf16_impl(const void* A, const void* B, void* C, int M, int N, i
   p.row_lse = p.row_ent = p.row_glp = p.row_gent = nullptr;
   p.chained = chained_launch_on() && !tile_map ? 1 : 0;
   if (x2) return bn == 64 ? launch_gemm_x2<64>(ta, tb, p, stream) : launch_gemm_x2<128>(ta, tb, p, stream);
+  if (few) {
+    if (bn == 128) return launch_gemm<128, kFewRows>(ta, tb, p, max_ctas, stream);
+    if (bn == 144) return launch_gemm<144, kFewRows>(ta, tb, p, max_ctas, stream);
+    if (bn == 208) return launch_gemm<208, kFewRows>(ta, tb, p, max_ctas, stream);
+    return launch_gemm<256, kFewRows>(ta, tb, p, max_ctas, stream);
+  }
   if (bn == 64) return launch_gemm<64>(ta, tb, p, max_ctas, stream);
   if (bn == 144) return launch_gemm<144>(ta, tb, p, max_ctas, stream);
   if (bn == 208) return launch_gemm<208>(ta, tb, p, max_ctas, stream);

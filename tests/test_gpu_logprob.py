@@ -34,7 +34,7 @@ def test_logprob_forward_backward(N, H, V, per_row_temp):
 def test_row_and_column_remainders_of_pair_tiles(N, H, V):
     """More than one 128-row tile runs on CTA pairs of 256 x 256: odd rows, a last tile of 8, 128 or 136 columns.  The logits of
     both sides have the same bf16 operands, so log-probabilities differ by fp32 rounding of sums and exponentials (V terms of
-    2^-22 relative, 1e-4 with room); gradients pass through bf16 once per d(logits) and once per result (2^-8 each)."""
+    2^-22 relative, 1e-4 with room); gradients pass through bf16 once per d(logits) and once per result (2^-8 at most each, half of that in the mean)."""
     from arctic_platform_b200.ops import _lib
     from arctic_platform_b200.ops.logprob import lm_head_logprobs, logprobs_entropy_ref
     g = torch.Generator(device="cuda").manual_seed(N)
