@@ -444,24 +444,27 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
   }
 }
 
-// delta[h, t] = sum_d dO[t,h,d] * O[t,h,d]; one warp per (t, h).
-__global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ o, long long ldo,
-                                  const __nv_bfloat16* __restrict__ d_o, long long lddo, float* __restrict__ delta,
-                                  int T, int Hq, int D) {
-  const long long gw = (blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (gw >= static_cast<long long>(T) * Hq) return;
-  const int t = static_cast<int>(gw / Hq), h = static_cast<int>(gw % Hq);
-  const __nv_bfloat16* a = o + t * ldo + static_cast<long long>(h) * D;
-  const __nv_bfloat16* b = d_o + t * lddo + static_cast<long long>(h) * D;
+// delta[h, t] = sum_d dO[t,h,d] * O[t,h,d] for heads of 128; 16 lanes per (t, h), 16 bytes of each per lane.
+__global__ void __launch_bounds__(256)
+attn_delta_kernel(const __nv_bfloat16* __restrict__ o, long long ldo, const __nv_bfloat16* __restrict__ d_o, long long lddo,
+                  float* __restrict__ delta, int T, int Hq) {
+  const long long gw = (blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) >> 4;
+  const int lane = threadIdx.x & 15;
+  const bool ok = gw < static_cast<long long>(T) * Hq;
+  const int t = ok ? static_cast<int>(gw / Hq) : 0, h = ok ? static_cast<int>(gw % Hq) : 0;
+  const uint4 x = *reinterpret_cast<const uint4*>(o + t * ldo + static_cast<long long>(h) * 128 + lane * 8);
+  const uint4 y = *reinterpret_cast<const uint4*>(d_o + t * lddo + static_cast<long long>(h) * 128 + lane * 8);
+  const uint32_t xs[4] = {x.x, x.y, x.z, x.w}, ys[4] = {y.x, y.y, y.z, y.w};
   float acc = 0.f;
-  for (int i = lane * 2; i < D; i += 64) {
-    const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(a + i));
-    const float2 y = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(b + i));
-    acc += x.x * y.x + x.y * y.y;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&xs[i]));
+    const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&ys[i]));
+    acc += a.x * b.x + a.y * b.y;
   }
-  acc = warp_sum(acc);
-  if (lane == 0) delta[static_cast<long long>(h) * T + t] = acc;
+#pragma unroll
+  for (int s = 8; s > 0; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
+  if (ok && lane == 0) delta[static_cast<long long>(h) * T + t] = acc;
 }
 
 }  // namespace apb
@@ -478,13 +481,13 @@ int apb_attn_bwd(const void* q, const void* k, const void* v, const void* o, con
                  long long ld_dq, long long ld_dk, long long ld_dv, float scale, cudaStream_t stream) {
   using namespace apb;
   if (n_cta <= 0 || T <= 0) return 0;
-  if (D != 128 || (ld_dq % 4) || (ldq % 8) || (ldk % 8) || (ldv % 8) || (lddo % 8) || (ld_dk % 8) || (ld_dv % 8) || Hq % Hkv)
+  if (D != 128 || (ld_dq % 4) || (ldq % 8) || (ldk % 8) || (ldv % 8) || (ldo % 8) || (lddo % 8) || (ld_dk % 8) || (ld_dv % 8) || Hq % Hkv ||
+      ((reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(d_o)) & 15))
     return kBadArgument;
   {
-    const long long warps = static_cast<long long>(T) * Hq;
-    const int grid = static_cast<int>((warps * 32 + 255) / 256);
+    const int grid = static_cast<int>((static_cast<long long>(T) * Hq * 16 + 255) / 256);
     attn_delta_kernel<<<grid, 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(o), ldo,
-                                                static_cast<const __nv_bfloat16*>(d_o), lddo, delta, T, Hq, D);
+                                                static_cast<const __nv_bfloat16*>(d_o), lddo, delta, T, Hq);
   }
   CUtensorMap tq, tdo, tk, tv, tdq;
   int rc = make_tmap_2d(&tq, q, 2, T, static_cast<uint64_t>(Hq) * D, ldq, 64, kBwdTile);

@@ -91,8 +91,8 @@ def test_zorro_matches_replicated_layout():
 @pytest.mark.parametrize("sharp", [1.0, 4.0])
 def test_tile_edges_and_sharp_scores_against_64_bits(Hq, Hkv, sharp):
     """Lengths around the 128-row tiles, prompts shared by several responses, every number of query heads per key head, and scores
-    wide enough that running maxima and references move.  o, P and dS are bf16 operands (2^-9 each) of sums that cancel in dS: a
-    few times 2^-8 of a gradient's norm."""
+    wide enough that running maxima and references move.  o, P and dS are bf16 operands (2^-8 at most each) of sums that cancel in
+    dS: a few times that of a gradient's norm."""
     from arctic_platform_b200.ops import _lib
     from arctic_platform_b200.ops.attention import AttnLayout, attention_ref, segment_attention
     segs, t = [], 0

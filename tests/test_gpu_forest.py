@@ -17,7 +17,8 @@ def _scratch(B, Hq, D, splits):
 
 def test_shared_pass_when_single_rows_meet_much_larger_scores_late():
     """The running reference of a row moves when its scores outgrow it by 2^8; here some rows of a warp do, others never, in
-    several blocks.  bf16 weights (2^-9 each) and outputs (2^-9) against fp32."""
+    several blocks.  bf16 weights and outputs (2^-8 at most each, half of that in the
+    mean) against fp32."""
     from arctic_platform_b200.ops import _lib
     from arctic_platform_b200.ops import forest_attention as fa
     B, Hq, Hkv, D, tokens = 12, 32, 8, 128, 1216
