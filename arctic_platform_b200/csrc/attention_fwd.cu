@@ -11,19 +11,24 @@
 //  arctic_platform/rl/zorro_train/zorro_train.py:857-912); here the key tile index
 // is resolved in the kernel and nothing is replicated.
 //
-// CTA = 384 threads, one per SM, walking its share of the work table (longest tiles first): warp 0 TMA producer, warp 1 MMA
-// issuer, warps 4-7 and 8-11 two softmax groups.  The two groups hold two query heads of the same KV head (same
-// 128 query rows), so they walk the same K/V tiles and ping-pong on the tensor
+// CTA = 384 threads, one per SM, walking its share of the work table (longest tiles first): warp 0 TMA producer,
+// warp 1 MMA issuer, warps 4-7 and 8-11 two softmax groups.  The two groups hold two query heads of the same KV head
+// (same 128 query rows), so they walk the same K/V tiles and ping-pong on the tensor
 // core: while one group does softmax on S_j the other group's P*V and next S run.
 // S (fp32) lives in TMEM, P (bf16) overwrites it in place and feeds the P*V MMA as
-// the TMEM A operand; P*V accumulates in TMEM.
+// the TMEM A operand, the P*V product is read back and accumulated in registers
+// with the usual online-softmax rescale.
 //
-// What bounds it: 2048 tensor cycles per pair of 128 x 128 blocks, and as many of the exponential unit (16 per cycle and SM) if it
-// took them all; the groups' exponentials hide behind each other's products, other instructions (one read of S,
-// maxima, packed fp32 arithmetic) behind both.  Weights are taken relative to a reference that follows a row's maximum only when
-// it, or that of another row of its warp, has moved by more than 2^8; O is rescaled on those occasions, in tensor memory, and read
-// once per tile.  Reading O after every block, scores twice, and one CTA per tile took 7200 cycles per pair of blocks
-// (8 x 4096 tokens, 32 / 8 heads: 1.74 ms, 630 TFLOP/s), this 4300 (1.04 ms, 1060; one sequence of 32768: 1180).
+// What bounds it: 2048 tensor cycles per pair of 128 x 128 blocks, and as many of the exponential unit (16 per
+// cycle and SM).  A group's other instructions (maxima, packed fp32 arithmetic, the read of the previous P*V) hide
+// behind the other group's products; loads from tensor memory are 32 columns at a time, the next one on its way
+// while one is worked on, because 128 registers hold O.  P*V of block j - 1 is read when S_j is there (it was issued
+// before S_j), so nobody waits for it.  Masks are applied only where a block has any.  Reading O behind every block,
+// masks everywhere, unpacked arithmetic and one CTA per tile took 7200 cycles per pair of blocks (8 x 4096 tokens,
+// 32 / 8 heads: 1.74 ms, 630 TFLOP/s), this 5500 (1.34 ms, 820; 32768 tokens 850 TFLOP/s).  Adding the previous P*V
+// between the exponentials instead, 16 columns at a time, spilled and took 1.46 ms.  Keeping O in tensor memory
+// behind a reference that lags the maximum took 4300 cycles, but rounds P and O differently from block to block;
+// routers downstream turn such last bits into other experts, so results stay those of the exact running maximum.
 #include "attention_common.cuh"
 #include "host_utils.cuh"
 
@@ -46,7 +51,6 @@ struct AttnFwdParams {
 constexpr int kAttnThreads = 384;
 constexpr int kAttnRegsIssue = 56, kAttnRegsSoftmax = 224;
 constexpr int kKvBlock = 128;
-constexpr float kAttnSlack = 8.f;       // log2 units by which a row's maximum may exceed its reference
 
 template <int D>
 struct AttnCfg {
@@ -186,11 +190,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
                        desc_k + slot * kTile + (k / 4) * 1024 + (k % 4) * 2, idesc_s, k > 0 ? 1u : 0u);
         tc_commit(&s_full[g]);
       };
-      auto issue_o = [&](uint32_t g, uint32_t slot, bool first) {
+      auto issue_o = [&](uint32_t g, uint32_t slot) {
 #pragma unroll
         for (int k = 0; k < kKvBlock / 16; ++k)
           umma_bf16_ts(tmem_base + 256 + g * 128, tmem_base + g * 128 + k * 8, desc_v + slot * kTile + k * 128, idesc_o,
-                       (!first || k > 0) ? 1u : 0u);
+                       k > 0 ? 1u : 0u);
       };
       uint32_t slot = 0, phase = 0, items = 0, done[2] = {0, 0};       // done: blocks of each group whose P has been awaited
       auto wait_slot = [&]() {         // the ring's next tile; its slot
@@ -230,7 +234,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
             if (!ok) break;
             ++done[g];
             if (elect_one()) {
-              issue_o(g, sv, j == 0);
+              issue_o(g, sv);
               if (more)
                 issue_s(g, sk);      // over P, which the product above reads first: the tensor core keeps the order of issue
               else
@@ -258,13 +262,23 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
     const uint64_t c2 = xtc_pair(p.scale_log2, p.scale_log2);
     uint32_t blocks = 0, items = 0;       // of this group so far
     bool ok = true;
+    uint64_t o[D / 2];                    // pairs of columns
+    uint32_t buf[2][32];
     for (int round = 0; round < rounds && ok; ++round) {
       const int at = item_at(round);
       if (at < 0) continue;
       const AttnItem w(p.work + static_cast<long long>(at) * 8);
       if (w.n_blocks == 0 || g >= w.n_groups) continue;
-      float m_ref = -INFINITY;
-      uint64_t l2 = 0;                    // row sum in two halves
+      float m_run = -INFINITY, l_run = 0.f, alpha = 0.f;
+#pragma unroll
+      for (int i = 0; i < D / 2; ++i) o[i] = 0;
+      // o = o * alpha + P*V, 32 columns that are in `v`
+      auto add = [&](int c, const uint32_t (&v)[32]) {
+        const uint64_t a2 = xtc_pair(alpha, alpha);
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+          o[c * 16 + i] = xtc_fma2(o[c * 16 + i], a2, xtc_pair(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])));
+      };
       for (int j = 0; j < w.n_blocks; ++j) {
         ok = wait(&s_full[g], blocks & 1, kTimeoutTmemFull);
         if (!ok) break;
@@ -278,90 +292,100 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
           least = min(w.own_len - b0, w.diag - b0 + 1);
           limit = min(w.own_len - b0, row + w.diag - b0 + 1);
         }
-        uint32_t v[4][32];
+        const bool masked = least < kKvBlock;
+        auto mask = [&](int c, uint32_t (&v)[32]) {
+          if (masked) {
 #pragma unroll
-        for (int c = 0; c < 4; ++c) tmem_ld_32x32(t_s + c * 32, v[c]);
+            for (int i = 0; i < 32; ++i)
+              if (c * 32 + i >= limit) v[i] = 0xff800000u;
+          }
+        };
+        // the product of the block before, which was issued ahead of this S
+        if (j > 0) {
+          tmem_ld_32x32(t_o, buf[0]);
+          tmem_ld_wait(buf[0]);
 #pragma unroll
-        for (int c = 0; c < 4; ++c) tmem_ld_wait(v[c]);
-        if (least < kKvBlock) {
-#pragma unroll
-          for (int c = 0; c < kKvBlock; ++c)
-            if (c >= limit) v[c / 32][c % 32] = 0xff800000u;
+          for (int c = 0; c < D / 32; ++c) {
+            if (c + 1 < D / 32) tmem_ld_32x32(t_o + (c + 1) * 32, buf[(c + 1) & 1]);
+            else tmem_ld_32x32(t_s, buf[(c + 1) & 1]);
+            add(c, buf[c & 1]);
+            tmem_ld_wait(buf[(c + 1) & 1]);
+          }
+        } else {
+          tmem_ld_32x32(t_s, buf[0]);
+          tmem_ld_wait(buf[0]);
         }
+        // pass 1: row maximum (buf[c & 1] holds columns [32 c, +32) at the start of step c: D / 32 is even)
         float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-        for (int c = 0; c < kKvBlock; c += 2)
-          mx[(c >> 1) & 3] = fmaxf(fmaxf(mx[(c >> 1) & 3], __uint_as_float(v[c / 32][c % 32])), __uint_as_float(v[c / 32][c % 32 + 1]));
-        // the scale is positive: the maximum of the scaled scores is the scaled maximum
-        const float m_new = fmaxf(m_ref, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * p.scale_log2);
-        if (__any_sync(0xffffffffu, m_new > m_ref + kAttnSlack || m_ref == -INFINITY)) {
-          if (j > 0) {           // O holds the blocks before this one: their product was issued ahead of this S
-            const float alpha = m_ref == -INFINITY ? 0.f : xtc_ex2(m_ref - m_new);
-            l2 = xtc_mul2(l2, xtc_pair(alpha, alpha));
-#pragma unroll 1
-            for (int c = 0; c < D / 32; ++c) {
-              uint32_t o[32];
-              tmem_ld_32x32(t_o + c * 32, o);
-              tmem_ld_wait(o);
+        for (int c = 0; c < 4; ++c) {
+          tmem_ld_32x32(t_s + ((c + 1) & 3) * 32, buf[(c + 1) & 1]);
+          mask(c, buf[c & 1]);
 #pragma unroll
-              for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-              tmem_st_32x32(t_o + c * 32, o);
-            }
-          }
-          m_ref = m_new;
+          for (int i = 0; i < 32; i += 2)
+            mx[(i >> 1) & 3] = fmaxf(fmaxf(mx[(i >> 1) & 3], __uint_as_float(buf[c & 1][i])), __uint_as_float(buf[c & 1][i + 1]));
+          tmem_ld_wait(buf[(c + 1) & 1]);
         }
-        const float m_use = m_ref == -INFINITY ? 0.f : m_ref;
+        const float m_new = fmaxf(m_run, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * p.scale_log2);
+        const float m_use = (m_new == -INFINITY) ? 0.f : m_new;
+        alpha = xtc_ex2(m_run - m_use);  // m_run = -inf -> 0
+        // pass 2: probabilities, written over S as packed bf16 (two per 32-bit column)
         const uint64_t nm2 = xtc_pair(-m_use, -m_use);
-        uint64_t sum[2] = {0, 0};
+        float rowsum = 0.f;
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
+          if (c < 3) tmem_ld_32x32(t_s + (c + 1) * 32, buf[(c + 1) & 1]);
+          mask(c, buf[c & 1]);
           uint32_t pk[16];
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
             float2 f = xtc_unpair(
-                xtc_fma2(xtc_pair(__uint_as_float(v[c][2 * i]), __uint_as_float(v[c][2 * i + 1])), c2, nm2));
+                xtc_fma2(xtc_pair(__uint_as_float(buf[c & 1][2 * i]), __uint_as_float(buf[c & 1][2 * i + 1])), c2, nm2));
             f.x = xtc_ex2(f.x);
             f.y = xtc_ex2(f.y);
-            sum[i & 1] = xtc_add2(sum[i & 1], xtc_pair(f.x, f.y));
+            rowsum += f.x + f.y;
             pk[i] = pack_bf16x2(f.x, f.y);
           }
+          if (c < 3) tmem_ld_wait(buf[(c + 1) & 1]);
           tmem_st_32x16(t_s + c * 16, pk);
         }
         tmem_st_wait();
         tc_fence_before();
         mbar_arrive(&p_full[g]);
-        l2 = xtc_add2(l2, xtc_add2(sum[0], sum[1]));
+        l_run = fmaf(l_run, alpha, rowsum);
+        m_run = m_new;
       }
       if (!ok) break;
       ok = wait(&o_full[g], items & 1, kTimeoutTmemFull);
       if (!ok) break;
       ++items;
-      const float2 l = xtc_unpair(l2);
-      const float l_run = l.x + l.y;
+#pragma unroll
+      for (int c = 0; c < D / 32; ++c) {
+        tmem_ld_32x32(t_o + c * 32, buf[0]);
+        tmem_ld_wait(buf[0]);
+        add(c, buf[0]);
+      }
+      tc_fence_before();
       const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
       const long long t = static_cast<long long>(w.q_row0) + row;
       __nv_bfloat16* dst = p.O + t * p.ldo + static_cast<long long>(w.head0 + g) * D;
-#pragma unroll 1
-      for (int c = 0; c < D / 32; ++c) {
-        uint32_t o[32];
-        tmem_ld_32x32(t_o + c * 32, o);
-        tmem_ld_wait(o);
-        if (row < w.q_valid) {
+      if (row < w.q_valid) {
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            uint4 x;
-            x.x = pack_bf16x2(__uint_as_float(o[q * 8 + 0]) * inv, __uint_as_float(o[q * 8 + 1]) * inv);
-            x.y = pack_bf16x2(__uint_as_float(o[q * 8 + 2]) * inv, __uint_as_float(o[q * 8 + 3]) * inv);
-            x.z = pack_bf16x2(__uint_as_float(o[q * 8 + 4]) * inv, __uint_as_float(o[q * 8 + 5]) * inv);
-            x.w = pack_bf16x2(__uint_as_float(o[q * 8 + 6]) * inv, __uint_as_float(o[q * 8 + 7]) * inv);
-            *reinterpret_cast<uint4*>(dst + c * 32 + q * 8) = x;
-          }
+        for (int q = 0; q < D / 8; ++q) {
+          float2 f[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) f[i] = xtc_unpair(o[q * 4 + i]);
+          uint4 x;
+          x.x = pack_bf16x2(f[0].x * inv, f[0].y * inv);
+          x.y = pack_bf16x2(f[1].x * inv, f[1].y * inv);
+          x.z = pack_bf16x2(f[2].x * inv, f[2].y * inv);
+          x.w = pack_bf16x2(f[3].x * inv, f[3].y * inv);
+          *reinterpret_cast<uint4*>(dst + q * 8) = x;
         }
       }
-      tc_fence_before();
       if (p.lse && row < w.q_valid)
         p.lse[static_cast<long long>(w.head0 + g) * p.T + t] =
-            l_run > 0.f ? (m_ref + log2f(l_run)) * 0.6931471805599453f : -INFINITY;
+            l_run > 0.f ? (m_run + log2f(l_run)) * 0.6931471805599453f : -INFINITY;
     }
   }
 
