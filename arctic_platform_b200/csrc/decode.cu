@@ -220,12 +220,14 @@ paged_decode_kernel(const __nv_bfloat16* __restrict__ q, const int* __restrict__
 // 3-deep shared-memory ring (XOR-swizzled 16-byte chunks), reads fragments with ldmatrix and runs S = Q K^T and
 // O += P V as m16n8k16 MMAs whose 16 rows hold up to 16 / R queries x R heads.  Per page that is 32 MMAs and 16
 // ldmatrix instead of ~850 scalar instructions, which leaves the load pipeline as the only limiter.
-// Output format is the same un-normalised (numerator, max, sum) partial as the scalar kernel.
+// Output format is the same un-normalised (numerator, max, sum) partial as the scalar kernel; with `out`, the parts of a row are a
+// cluster that joins them through shared memory and writes the normalised result (no partials in memory, no merge launch).
 // ---------------------------------------------------------------------------
 constexpr int kMmaStages = 3;
 constexpr int kMmaPageBytes = kPage * 128 * 2;                    // one K or V page of one head
 constexpr int kMmaWarpBytes = kMmaStages * 2 * kMmaPageBytes;     // K+V ring of one warp
 constexpr int kMmaSmem = 4 * kMmaWarpBytes;                       // 96 KB
+constexpr int kMaxSeqSplits = 4;                                  // parts that one cluster joins
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
@@ -272,13 +274,13 @@ paged_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, const int* __restri
                         const int* __restrict__ q_count, const int* __restrict__ pages, int max_pages,
                         const int* __restrict__ kv_len, const __nv_bfloat16* __restrict__ kcache,
                         const __nv_bfloat16* __restrict__ vcache, float* __restrict__ out_o, float* __restrict__ out_ml,
-                        int Hq, int Hkv, int splits, float scale_log2) {
+                        __nv_bfloat16* __restrict__ out, int Hq, int Hkv, int splits, float scale_log2) {
   pdl_entry();
   constexpr int D = 128;
   extern __shared__ __align__(128) uint8_t dec_smem[];
-  const int g = blockIdx.x / Hkv;
-  const int kvh = blockIdx.x % Hkv;
-  const int split = blockIdx.y;
+  const int split = blockIdx.x % splits;       // the CTAs of one (group, head) are neighbours, with `out` one cluster
+  const int g = blockIdx.x / splits / Hkv;
+  const int kvh = blockIdx.x / splits % Hkv;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int R = Hq / Hkv;
   const int nq = q_count[g];
@@ -291,6 +293,10 @@ paged_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, const int* __restri
   const uint32_t ring = smem_u32(dec_smem) + warp * kMmaWarpBytes;
   const int n_my = (p1 - p0 - warp + 3) / 4;  // pages p0 + warp, p0 + warp + 4, ... (<= 0: none)
   const int q_per_pass = 16 / R;              // queries whose R heads fit the 16 MMA rows
+  if (out && nq <= 0 && split == 0) {         // a slot without a sequence: finite rows for the layers behind
+    for (int i = threadIdx.x; i < R * D; i += kDecThreads)
+      out[(static_cast<long long>(qs) * Hq + kvh * R) * D + i] = __float2bfloat16(0.f);
+  }
   const int quad_row = lane >> 2, quad_col = (lane & 3) * 2;
 
   for (int q0 = 0; q0 < nq; q0 += q_per_pass) {
@@ -418,6 +424,8 @@ paged_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, const int* __restri
     float* red_o = reinterpret_cast<float*>(dec_smem);                 // [4][16][D]
     float* red_m = red_o + 4 * 16 * D;                                 // [4][16]
     float* red_l = red_m + 4 * 16;                                     // [4][16]
+    float* part_o = red_l + 4 * 16;                                    // [16][D]  this CTA's part for its cluster
+    float* part_ml = part_o + 16 * D;                                  // [16][2]
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       const int rr = quad_row + 8 * h;
@@ -446,12 +454,49 @@ paged_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, const int* __restri
         ll += red_l[w * 16 + rr] * scw;
       }
       const long long qrow = qs + q0 + rr / R;
-      const long long base = ((qrow * Hq + kvh * R + rr % R) * splits + split);
-      out_o[base * D + d] = ov;
-      if (d == 0) {
-        out_ml[base * 2] = mm;
-        out_ml[base * 2 + 1] = ll;
+      const long long head = qrow * Hq + kvh * R + rr % R;
+      if (out && splits == 1) {
+        out[head * D + d] = __float2bfloat16(ll > 0.f ? ov / ll : 0.f);
+      } else if (out) {
+        part_o[i] = ov;
+        if (d == 0) {
+          part_ml[rr * 2] = mm;
+          part_ml[rr * 2 + 1] = ll;
+        }
+      } else {
+        const long long base = head * splits + split;
+        out_o[base * D + d] = ov;
+        if (d == 0) {
+          out_ml[base * 2] = mm;
+          out_ml[base * 2 + 1] = ll;
+        }
       }
+    }
+    if (out && splits > 1) {
+      // the cluster's parts, joined by all its CTAs: each takes every splits-th run of 128 values
+      cluster_sync_all();
+      for (int rr = split; rr < rows_valid; rr += splits) {
+        const int d = threadIdx.x;
+        float pm[kMaxSeqSplits], pl[kMaxSeqSplits], mm = -INFINITY, ov = 0.f, ll = 0.f;
+        #pragma unroll
+        for (int k = 0; k < kMaxSeqSplits; ++k) {
+          if (k >= splits) break;
+          const uint32_t ml = map_to_cta(smem_u32(part_ml + rr * 2), k);
+          pm[k] = ld_cluster_f32(ml);
+          pl[k] = ld_cluster_f32(ml + 4);
+          mm = fmaxf(mm, pm[k]);
+        }
+        #pragma unroll
+        for (int k = 0; k < kMaxSeqSplits; ++k) {
+          if (k >= splits) break;
+          const float f = pm[k] == -INFINITY ? 0.f : exp2f(pm[k] - mm);
+          ov += ld_cluster_f32(map_to_cta(smem_u32(part_o + rr * D + d), k)) * f;
+          ll += pl[k] * f;
+        }
+        const long long qrow = qs + q0 + rr / R;
+        out[(qrow * Hq + kvh * R + rr % R) * D + d] = __float2bfloat16(ll > 0.f ? ov / ll : 0.f);
+      }
+      cluster_sync_all();
     }
     __syncthreads();  // the ring is written again by the next pass
   }
@@ -798,35 +843,60 @@ sample_threshold_kernel(const float* __restrict__ logits, long long ldl, const f
   if (threadIdx.x == 0) thr[b] = best_thr;
 }
 
-// One block per row.  logits [B, V] fp32 (row stride ldl).  temperature[b] <= 0 -> greedy.
+// What a part of a row knows: the largest key with its token and logit, and the softmax statistics.
+struct SampleRec {
+  float best, best_z, m, s;
+  int best_i;
+};
+__device__ __forceinline__ void sample_join(SampleRec& a, float best, int best_i, float best_z, float m, float s) {
+  if (best > a.best || (best == a.best && best_i < a.best_i)) {
+    a.best = best;
+    a.best_i = best_i;
+    a.best_z = best_z;
+  }
+  const float mn = fmaxf(a.m, m);
+  a.s = (a.m == -INFINITY ? 0.f : a.s * __expf(a.m - mn)) + (m == -INFINITY ? 0.f : s * __expf(m - mn));
+  a.m = mn;
+}
+__device__ __forceinline__ void sample_join_warp(SampleRec& a) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const float best = __shfl_xor_sync(0xffffffffu, a.best, o), best_z = __shfl_xor_sync(0xffffffffu, a.best_z, o);
+    const int best_i = __shfl_xor_sync(0xffffffffu, a.best_i, o);
+    const float m = __shfl_xor_sync(0xffffffffu, a.m, o), s = __shfl_xor_sync(0xffffffffu, a.s, o);
+    sample_join(a, best, best_i, best_z, m, s);
+  }
+}
+
+// One cluster of CTAs per row, each on a part of it.  logits [B, V] fp32 (row stride ldl).  temperature[b] <= 0 -> greedy.
 // Gumbel-max sampling: argmax(z + g), z = logit / T, over the tokens with z >= thr[b] when a cut-off is given.
 // Also returns log softmax(z)[token] under the UNFILTERED distribution (what the trainer's old_log_probs expect).
+// Bound by the exponentials and loads that one CTA has in flight: a CTA per row of 151936 took 52 us at 8 rows and 36 at 128
+// (78 MB), parts of the row 11 and 31.
 __global__ void __launch_bounds__(1024)
 sample_kernel(const float* __restrict__ logits, long long ldl, const float* __restrict__ temperature, int V,
               uint32_t seed, const int* __restrict__ step_dev, const float* __restrict__ thr,
-              int* __restrict__ tokens, float* __restrict__ logprobs) {
+              int* __restrict__ tokens, float* __restrict__ logprobs, int parts) {
   pdl_entry();
-  const int b = blockIdx.x;
+  const int b = blockIdx.x / parts, part = blockIdx.x % parts;
   const uint32_t step = step_dev ? static_cast<uint32_t>(*step_dev) : 0u;
   const float T = temperature[b];
   const bool greedy = !(T > 0.f);
   const float invT = greedy ? 1.f : 1.f / T;
   const float* row = logits + b * ldl;
   const float cut = (thr && !greedy) ? thr[b] : -INFINITY;
-  float best = -INFINITY, best_z = 0.f;
-  int best_i = 0;
-  float m = -INFINITY, s = 0.f;
+  SampleRec r{-INFINITY, 0.f, -INFINITY, 0.f, 0};
   // one hash per element: the per-(seed, step, row) part is mixed once, the column enters by a Weyl step
   const uint32_t base = hash_u32(seed ^ (step * 0x9E3779B9u)) ^ hash_u32(static_cast<uint32_t>(b) * 0x85ebca6bU + 1u);
   auto consider = [&](float raw, int i) {
     const float z = raw * invT;
     // running softmax statistics with ONE exponential per element (the rescaling branch is taken only when a new
     // maximum appears, which becomes rare after the first few elements of a thread)
-    if (z > m) {
-      s = s * __expf(m - z) + 1.f;
-      m = z;
+    if (z > r.m) {
+      r.s = r.s * __expf(r.m - z) + 1.f;
+      r.m = z;
     } else if (z > -INFINITY) {
-      s += __expf(z - m);
+      r.s += __expf(z - r.m);
     }
     float key = z;
     if (!greedy) {
@@ -838,81 +908,75 @@ sample_kernel(const float* __restrict__ logits, long long ldl, const float* __re
         key = -INFINITY;  // outside the top-k / top-p set
       }
     }
-    if (key > best) {
-      best = key;
-      best_i = i;
-      best_z = z;
+    if (key > r.best) {
+      r.best = key;
+      r.best_i = i;
+      r.best_z = z;
     }
   };
-  if ((ldl & 3) == 0 && (reinterpret_cast<uintptr_t>(logits) & 15) == 0) {
-    const float4* row4 = reinterpret_cast<const float4*>(row);
-    const int n4 = V >> 2;
-    for (int i4 = threadIdx.x; i4 < n4; i4 += blockDim.x) {
-      const float4 v = row4[i4];
-      consider(v.x, 4 * i4);
-      consider(v.y, 4 * i4 + 1);
-      consider(v.z, 4 * i4 + 2);
-      consider(v.w, 4 * i4 + 3);
-    }
+  // parts are whole vectors; the last one also takes what is left of the row
+  const bool vec = (ldl & 3) == 0 && (reinterpret_cast<uintptr_t>(logits) & 15) == 0;
+  const int n4 = vec ? V >> 2 : 0;
+  const int per = (n4 + parts - 1) / parts, i1 = min(n4, (part + 1) * per);
+  const float4* row4 = reinterpret_cast<const float4*>(row);
+  int i4 = part * per + threadIdx.x;
+  for (; i4 + static_cast<int>(blockDim.x) < i1; i4 += 2 * blockDim.x) {
+    const int k4 = i4 + blockDim.x;
+    const float4 v = row4[i4], w = row4[k4];
+    consider(v.x, 4 * i4);
+    consider(v.y, 4 * i4 + 1);
+    consider(v.z, 4 * i4 + 2);
+    consider(v.w, 4 * i4 + 3);
+    consider(w.x, 4 * k4);
+    consider(w.y, 4 * k4 + 1);
+    consider(w.z, 4 * k4 + 2);
+    consider(w.w, 4 * k4 + 3);
+  }
+  if (i4 < i1) {
+    const float4 v = row4[i4];
+    consider(v.x, 4 * i4);
+    consider(v.y, 4 * i4 + 1);
+    consider(v.z, 4 * i4 + 2);
+    consider(v.w, 4 * i4 + 3);
+  }
+  if (part == parts - 1)
     for (int i = 4 * n4 + threadIdx.x; i < V; i += blockDim.x) consider(row[i], i);
-  } else {
-    for (int i = threadIdx.x; i < V; i += blockDim.x) consider(row[i], i);
-  }
-  __shared__ float sb[32], sz[32], sm[32], ss[32];
-  __shared__ int si[32];
+
+  __shared__ SampleRec warp_rec[32], cta_rec;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-    const int oi = __shfl_xor_sync(0xffffffffu, best_i, o);
-    const float oz = __shfl_xor_sync(0xffffffffu, best_z, o);
-    if (ob > best || (ob == best && oi < best_i)) {
-      best = ob;
-      best_i = oi;
-      best_z = oz;
-    }
-    const float om = __shfl_xor_sync(0xffffffffu, m, o);
-    const float os = __shfl_xor_sync(0xffffffffu, s, o);
-    const float mn = fmaxf(m, om);
-    s = (m == -INFINITY ? 0.f : s * __expf(m - mn)) + (om == -INFINITY ? 0.f : os * __expf(om - mn));
-    m = mn;
-  }
-  if (lane == 0) {
-    sb[warp] = best;
-    si[warp] = best_i;
-    sz[warp] = best_z;
-    sm[warp] = m;
-    ss[warp] = s;
-  }
+  const SampleRec none{-INFINITY, 0.f, -INFINITY, 0.f, 0x7fffffff};
+  sample_join_warp(r);
+  if (lane == 0) warp_rec[warp] = r;
   __syncthreads();
   if (warp == 0) {
-    const int nw = blockDim.x >> 5;
-    best = lane < nw ? sb[lane] : -INFINITY;
-    best_i = lane < nw ? si[lane] : 0x7fffffff;
-    best_z = lane < nw ? sz[lane] : 0.f;
-    m = lane < nw ? sm[lane] : -INFINITY;
-    s = lane < nw ? ss[lane] : 0.f;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-      const int oi = __shfl_xor_sync(0xffffffffu, best_i, o);
-      const float oz = __shfl_xor_sync(0xffffffffu, best_z, o);
-      if (ob > best || (ob == best && oi < best_i)) {
-        best = ob;
-        best_i = oi;
-        best_z = oz;
-      }
-      const float om = __shfl_xor_sync(0xffffffffu, m, o);
-      const float os = __shfl_xor_sync(0xffffffffu, s, o);
-      const float mn = fmaxf(m, om);
-      s = (m == -INFINITY ? 0.f : s * __expf(m - mn)) + (om == -INFINITY ? 0.f : os * __expf(om - mn));
-      m = mn;
+    r = lane < static_cast<int>(blockDim.x >> 5) ? warp_rec[lane] : none;
+    sample_join_warp(r);
+    if (lane == 0) cta_rec = r;
+  }
+  cluster_sync_all();
+  if (part == 0 && warp == 0) {
+    r = none;
+    if (lane < parts) {
+      const uint32_t from = map_to_cta(smem_u32(&cta_rec), lane);
+      r.best = ld_cluster_f32(from);
+      r.best_z = ld_cluster_f32(from + 4);
+      r.m = ld_cluster_f32(from + 8);
+      r.s = ld_cluster_f32(from + 12);
+      r.best_i = __float_as_int(ld_cluster_f32(from + 16));
     }
+    sample_join_warp(r);
     if (lane == 0) {
-      tokens[b] = best_i;
-      logprobs[b] = best_z - (m + __logf(s));
+      tokens[b] = r.best_i;
+      logprobs[b] = r.best_z - (r.m + __logf(r.s));
     }
   }
+  cluster_sync_all();       // nobody leaves while its record may be read
+}
+
+// CTAs per row: as many as one wave of two CTAs per SM has room for, at most a portable cluster.
+static int sample_parts(int B) {
+  const int room = 2 * sm_count() / (B > 0 ? B : 1);
+  return room >= 8 ? 8 : room >= 4 ? 4 : room >= 2 ? 2 : 1;
 }
 
 }  // namespace apb
@@ -955,6 +1019,36 @@ int apb_decode_qkv_post(float* acc, long long ld_acc, const void* wq, const void
 static int g_decode_scalar = 0;
 void apb_decode_use_scalar(int on) { g_decode_scalar = on; }
 
+static int launch_decode_mma(const void* q, const int* q_start, const int* q_count, const int* pages, int max_pages, const int* kv_len,
+                             const void* kcache, const void* vcache, float* out_o, float* out_ml, void* out, int G, int Hq, int Hkv,
+                             int splits, float scale_log2, cudaStream_t s) {
+  static bool configured[64] = {false};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!configured[dev & 63]) {
+    cudaError_t e = cudaFuncSetAttribute(paged_decode_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMmaSmem);
+    if (e != cudaSuccess) return static_cast<int>(e);
+    configured[dev & 63] = true;
+  }
+  return static_cast<int>(launch_kernel_clusters(paged_decode_mma_kernel, dim3(G * Hkv * splits), dim3(kDecThreads), kMmaSmem,
+                                                 out ? splits : 1, s, static_cast<const __nv_bfloat16*>(q), q_start, q_count, pages,
+                                                 max_pages, kv_len, static_cast<const __nv_bfloat16*>(kcache),
+                                                 static_cast<const __nv_bfloat16*>(vcache), out_o, out_ml,
+                                                 static_cast<__nv_bfloat16*>(out), Hq, Hkv, splits, scale_log2));
+}
+
+// Decode attention of one token per sequence over its whole page table, normalised: out [Bq, Hq, D] bf16 (zeros in the row q_start[g] of
+// a group without queries).  D = 128, the query heads of a key head divide 16, 1, 2 or 4 splits.  Arguments as
+// apb_paged_decode_partial's.
+int apb_paged_decode(const void* q, const int* q_start, const int* q_count, const int* pages, int max_pages, const int* kv_len,
+                     const void* kcache, const void* vcache, void* out, int G, int Hq, int Hkv, int D, int splits, float scale,
+                     cudaStream_t s) {
+  if (G <= 0) return 0;
+  if (D != 128 || Hkv <= 0 || Hq % Hkv || 16 % (Hq / Hkv) || !out || (splits != 1 && splits != 2 && splits != 4)) return kBadArgument;
+  return launch_decode_mma(q, q_start, q_count, pages, max_pages, kv_len, kcache, vcache, nullptr, nullptr, out, G, Hq, Hkv, splits,
+                           scale * 1.4426950408889634f, s);
+}
+
 // Partial attention of G query groups (see paged_decode_kernel).  out_o / out_ml are fp32 scratch
 // [Bq, Hq, splits, D] and [Bq, Hq, splits, 2].
 int apb_paged_decode_partial(const void* q, const int* q_start, const int* q_count, const int* pages, int max_pages,
@@ -965,21 +1059,9 @@ int apb_paged_decode_partial(const void* q, const int* q_start, const int* q_cou
   const int R = Hq / Hkv;
   const dim3 grid(G * Hkv, splits);
   const float sl2 = scale * 1.4426950408889634f;
-  if (16 % R == 0 && !g_decode_scalar) {
-    static bool configured[64] = {false};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (!configured[dev & 63]) {
-      cudaError_t e = cudaFuncSetAttribute(paged_decode_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMmaSmem);
-      if (e != cudaSuccess) return static_cast<int>(e);
-      configured[dev & 63] = true;
-    }
-    return static_cast<int>(launch_kernel(paged_decode_mma_kernel, grid, dim3(kDecThreads), kMmaSmem, s,
-                                          static_cast<const __nv_bfloat16*>(q), q_start, q_count, pages, max_pages,
-                                          kv_len, static_cast<const __nv_bfloat16*>(kcache),
-                                          static_cast<const __nv_bfloat16*>(vcache), out_o, out_ml, Hq, Hkv, splits,
-                                          sl2));
-  }
+  if (16 % R == 0 && !g_decode_scalar)
+    return launch_decode_mma(q, q_start, q_count, pages, max_pages, kv_len, kcache, vcache, out_o, out_ml, nullptr, G, Hq, Hkv, splits,
+                             sl2, s);
 #define APB_DEC(RR)                                                                                           \
   paged_decode_kernel<RR, 128><<<grid, kDecThreads, 0, s>>>(                                                  \
       static_cast<const __nv_bfloat16*>(q), q_start, q_count, pages, max_pages, kv_len,                      \
@@ -1042,9 +1124,10 @@ int apb_decode_advance(const int* new_tok, const float* new_lp, int* active, int
 int apb_sample(const float* logits, long long ldl, const float* temperature, int B, int V, unsigned seed,
                const int* step_dev, int* tokens, float* logprobs, cudaStream_t s) {
   if (B <= 0) return 0;
-  return static_cast<int>(launch_kernel(sample_kernel, dim3(B), dim3(1024), 0, s, logits, ldl, temperature, V,
-                                        static_cast<uint32_t>(seed), step_dev, static_cast<const float*>(nullptr),
-                                        tokens, logprobs));
+  const int parts = sample_parts(B);
+  return static_cast<int>(launch_kernel_clusters(sample_kernel, dim3(B * parts), dim3(1024), 0, parts, s, logits, ldl, temperature, V,
+                                                 static_cast<uint32_t>(seed), step_dev, static_cast<const float*>(nullptr), tokens,
+                                                 logprobs, parts));
 }
 
 // Sampling restricted to the top-k tokens and to the smallest set of tokens with probability mass >= top_p.
@@ -1057,8 +1140,9 @@ int apb_sample_filtered(const float* logits, long long ldl, const float* tempera
   cudaError_t e = launch_kernel(sample_threshold_kernel, dim3(B), dim3(1024), 0, s, logits, ldl, temperature, V, top_k,
                                 top_p, thr);
   if (e != cudaSuccess) return static_cast<int>(e);
-  return static_cast<int>(launch_kernel(sample_kernel, dim3(B), dim3(1024), 0, s, logits, ldl, temperature, V,
-                                        static_cast<uint32_t>(seed), step_dev, static_cast<const float*>(thr), tokens,
-                                        logprobs));
+  const int parts = sample_parts(B);
+  return static_cast<int>(launch_kernel_clusters(sample_kernel, dim3(B * parts), dim3(1024), 0, parts, s, logits, ldl, temperature, V,
+                                                 static_cast<uint32_t>(seed), step_dev, static_cast<const float*>(thr), tokens,
+                                                 logprobs, parts));
 }
 }

@@ -144,6 +144,7 @@ def _fn(name: str):
         vp, i, ll, f, u = c.c_void_p, c.c_int, c.c_longlong, c.c_float, c.c_uint
         _FN["kvw"] = _lib.declare("apb_kv_cache_write", [vp, ll, vp, ll, vp, vp, vp, i, i, i, vp])
         _FN["dec"] = _lib.declare("apb_paged_decode_partial", [vp, vp, vp, vp, i, vp, vp, vp, vp, vp, i, i, i, i, i, f, vp])
+        _FN["dec_out"] = _lib.declare("apb_paged_decode", [vp, vp, vp, vp, i, vp, vp, vp, vp, i, i, i, i, i, f, vp])
         _FN["merge"] = _lib.declare("apb_decode_merge", [vp, vp, vp, i, vp, vp, vp, i, i, i, vp])
         _FN["sample"] = _lib.declare("apb_sample", [vp, ll, vp, i, i, u, vp, vp, vp, vp])
         _FN["sample_f"] = _lib.declare("apb_sample_filtered", [vp, ll, vp, i, i, u, vp, vp, vp, vp, vp, vp, vp])
@@ -447,7 +448,7 @@ class SamplerEngine:
         if os.environ.get("APB_DECODE_SEQ_SPLITS"):               # tuning knob for A/B timing
             seq_splits = max(1, min(self.splits, int(os.environ["APB_DECODE_SEQ_SPLITS"])))
         out = torch.empty((B, c.num_heads, c.head_dim), device=self.device, dtype=torch.bfloat16)
-        if self._cascade_on():
+        if self._cascade_on() and self.n_groups > 0:
             # shared pass: as many KV splits as keep all its CTAs (nodes x KV heads x splits) within one wave of SMs
             nodes = self._group_bucket()
             node_splits = max(1, min(self.splits, self._sm_count // max(1, nodes * c.num_kv_heads)))
@@ -455,6 +456,13 @@ class SamplerEngine:
                                            self.d_priv_table, self.d_priv_len, self.part_o, self.part_ml, node_splits,
                                            seq_splits, scale, out=out, n_nodes=nodes)
         s = _lib.stream_ptr()
+        if c.head_dim == 128 and 16 % (c.num_heads // c.num_kv_heads) == 0:
+            # one source: the splits of a row are a cluster that joins them (a power of two), nothing is left to merge
+            _lib.check(_fn("dec_out")(_lib.ptr(q), _lib.ptr(self.d_q_start), _lib.ptr(self.d_active), _lib.ptr(self.d_page_table),
+                                      self.max_pages, _lib.ptr(self.d_len), _lib.ptr(kc), _lib.ptr(vc), _lib.ptr(out), B,
+                                      c.num_heads, c.num_kv_heads, c.head_dim, 1 << (seq_splits.bit_length() - 1), scale, s),
+                       "paged_decode")
+            return out
         _lib.check(_fn("dec")(_lib.ptr(q), _lib.ptr(self.d_q_start), _lib.ptr(self.d_active), _lib.ptr(self.d_page_table),
                               self.max_pages, _lib.ptr(self.d_len), _lib.ptr(kc), _lib.ptr(vc), _lib.ptr(self.part_o[0]),
                               _lib.ptr(self.part_ml[0]), B, c.num_heads, c.num_kv_heads, c.head_dim, seq_splits, scale, s),
@@ -485,9 +493,9 @@ class SamplerEngine:
 
     def _group_bucket(self) -> int:
         """Rows of the node tables in use, rounded up to a power of two: the grid of the shared-node pass (and the
-        key of the captured graph) changes only when the count crosses a bucket."""
-        n = max(1, int(self.n_groups))
-        return min(self.n_node_rows, 1 << (n - 1).bit_length())
+        key of the captured graph) changes only when the count crosses a bucket; 0 when nothing is shared."""
+        n = int(self.n_groups)
+        return min(self.n_node_rows, 1 << (n - 1).bit_length()) if n > 0 else 0
 
     def _decode_logits(self, B: int) -> torch.Tensor:
         """Feeds the pending token of slots [0, B) through the model; logits ``[B, V]`` fp32 in ``d_logits``."""
@@ -787,6 +795,11 @@ class SamplerEngine:
                 slots_free.sort()
                 first_of_run = True
                 for r, P, n_full, priv_pages in per_prompt:
+                    if sp.n == 1:
+                        # one sample: nobody shares the prompt, so its pages belong to the per-sequence pass.  On a tile of
+                        # the shared pass 128 rows would stand for one sequence (41 prompts of 500 to 1500 tokens, 8 key
+                        # heads: 66 us a layer for the shared pass alone, 38 for a per-sequence pass that reads everything)
+                        n_full, priv_pages = 0, n_full + priv_pages
                     shared = self.pages.alloc(n_full)
                     gid = next_group
                     next_group += 1
@@ -911,8 +924,7 @@ class SamplerEngine:
             for _gid, mem in run["prompts"]:
                 s0 = live[mem[0]]
                 rem = prompts_np[s0.req][hlen:]
-                tail = s0.prompt_len % PAGE
-                pages = s0.shared_pages if tail == 0 else np.concatenate([s0.shared_pages, s0.private_pages[:1]])
+                pages = np.concatenate([s0.shared_pages, s0.private_pages])
                 q0 = t
                 put(rem, hlen, pages.astype(np.int64))
                 segs.append((q0, len(rem), hstart if hlen else 0, hlen, q0, len(rem)))
