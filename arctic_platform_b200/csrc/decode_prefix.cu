@@ -152,26 +152,31 @@ decode_prefix_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
     }
   } else if (warp == 1) {
     pdl_wait();
-    if (lane == 0 && n_blocks > 0) {
+    // the whole warp walks the loop and one elected lane issues, so that descriptors are uniform (see gemm_tcgen05_2cta.cu)
+    if (n_blocks > 0) {
       const uint32_t idesc_s = umma_idesc_bf16(128, 128, 0, 0);
       const uint32_t idesc_o = umma_idesc_bf16(128, D, 0, 1);
-      bool ok = mbar_wait(q_full, 0, p.status, kTimeoutFull);
-      const uint32_t qa = smem_u32(smem_q);
+      const uint64_t desc_q = umma_smem_desc(smem_u32(smem_q), 0, 1024), desc_k = umma_smem_desc(smem_u32(smem_kv), 0, 1024);
+      const uint64_t desc_v = umma_smem_desc(smem_u32(smem_kv), 16384, 1024);
+      auto wait = [&](uint64_t* bar, uint32_t parity, int code) {
+        const bool r = __all_sync(0xffffffffu, mbar_wait(bar, parity, p.status, code));
+        tc_fence_after();
+        return r;
+      };
+      bool ok = wait(q_full, 0, kTimeoutFull);
       // S(j) = Q K(j)^T into score buffer j & 1
       auto issue_qk = [&](int j) -> bool {
-        const int nk = 2 * j;
-        if (!mbar_wait(&kv_full[nk % kDpSlots], (nk / kDpSlots) & 1, p.status, kTimeoutFull)) return false;
-        tc_fence_after();
-        const uint32_t ka = smem_u32(smem_kv + (nk % kDpSlots) * kDpTile);
-        const uint32_t t_s = tmem_base + (j & 1) * 128;
+        const uint32_t slot = (2 * j) % kDpSlots;
+        if (!wait(&kv_full[slot], ((2 * j) / kDpSlots) & 1, kTimeoutFull)) return false;
+        if (elect_one()) {
 #pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-          const uint32_t off = (k / 4) * 16384 + (k % 4) * 32;
-          umma_bf16_ss(t_s, umma_smem_desc(qa + off, 0, 1024), umma_smem_desc(ka + off, 0, 1024), idesc_s,
-                       k > 0 ? 1u : 0u);
+          for (int k = 0; k < D / 16; ++k)
+            umma_bf16_ss(tmem_base + (j & 1) * 128, desc_q + (k / 4) * 1024 + (k % 4) * 2,
+                         desc_k + slot * (kDpTile >> 4) + (k / 4) * 1024 + (k % 4) * 2, idesc_s, k > 0 ? 1u : 0u);
+          tc_commit(&s_full[j & 1]);
+          tc_commit(&kv_empty[slot]);
         }
-        tc_commit(&s_full[j & 1]);
-        tc_commit(&kv_empty[nk % kDpSlots]);
+        __syncwarp();
         return true;
       };
       if (ok) ok = issue_qk(0);
@@ -182,21 +187,20 @@ decode_prefix_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
           ok = false;
           break;
         }
-        const int nv = 2 * j + 1, b = j & 1;
-        if (!mbar_wait(&kv_full[nv % kDpSlots], (nv / kDpSlots) & 1, p.status, kTimeoutFull) ||
-            !mbar_wait(&p_full[b], (j >> 1) & 1, p.status, kTimeoutTmemEmpty)) {
+        const uint32_t slot = (2 * j + 1) % kDpSlots, b = j & 1;
+        if (!wait(&kv_full[slot], ((2 * j + 1) / kDpSlots) & 1, kTimeoutFull) || !wait(&p_full[b], (j >> 1) & 1, kTimeoutTmemEmpty)) {
           ok = false;
           break;
         }
-        tc_fence_after();
-        const uint32_t va = smem_u32(smem_kv + (nv % kDpSlots) * kDpTile);
-        const uint32_t t_p = tmem_base + b * 128, t_o = tmem_base + 256;
+        if (elect_one()) {
 #pragma unroll
-        for (int k = 0; k < 128 / 16; ++k)
-          umma_bf16_ts(t_o, t_p + k * 8, umma_smem_desc(va + k * 2048, 16384, 1024), idesc_o,
-                       (j > 0 || k > 0) ? 1u : 0u);
-        tc_commit(&o_full[0]);
-        tc_commit(&kv_empty[nv % kDpSlots]);
+          for (int k = 0; k < 128 / 16; ++k)
+            umma_bf16_ts(tmem_base + 256, tmem_base + b * 128 + k * 8, desc_v + slot * (kDpTile >> 4) + k * 128, idesc_o,
+                         (j > 0 || k > 0) ? 1u : 0u);
+          tc_commit(&o_full[0]);
+          tc_commit(&kv_empty[slot]);
+        }
+        __syncwarp();
       }
     }
   } else {
