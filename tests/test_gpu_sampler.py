@@ -193,3 +193,92 @@ def test_engine_generates_with_top_k_and_top_p():
     assert all(o["token_ids"] == greedy for o in tiny_p)
     free = eng.generate([prompt], {"n": 8, "temperature": 1.0, "max_tokens": 8, "top_k": 50, "top_p": 0.95, "seed": 5})
     assert len({tuple(o["token_ids"]) for o in free}) > 1
+
+
+@pytest.mark.parametrize("Hq,Hkv,splits", [(32, 8, 1), (32, 8, 2), (32, 8, 4), (16, 1, 2), (8, 8, 4), (16, 8, 2)])
+def test_paged_decode_joined_by_its_cluster(Hq, Hkv, splits):
+    """One launch that writes normalised rows, against softmax in 64 bits: ranges that leave parts empty, that end inside a
+    page, idle slots (zeros).  P and the result are rounded to bf16 (2^-8 each at most), V's mean is of order one or less."""
+    import math
+    from arctic_platform_b200.engine.sampler import _fn
+    from arctic_platform_b200.ops import _lib
+    dev, D, PAGE = "cuda", 128, 16
+    g = torch.Generator(device=dev).manual_seed(Hq + Hkv + splits)
+    lens, active = [0, 1, 15, 16, 17, 64, 65, 1023, 300, 500], [1, 1, 1, 1, 1, 1, 1, 1, 0, 1]
+    G, max_pages = len(lens), 64
+    kc, vc = (torch.randn(G * max_pages, Hkv, PAGE, D, device=dev, generator=g).bfloat16() for _ in range(2))
+    pages = torch.randperm(G * max_pages, device=dev, generator=g).to(torch.int32).view(G, max_pages)
+    q = torch.randn(G, Hq, D, device=dev, generator=g).bfloat16()
+    i32 = dict(device=dev, dtype=torch.int32)
+    start, count, kv_len = torch.arange(G, **i32), torch.tensor(active, **i32), torch.tensor(lens, **i32)
+    out = torch.full((G, Hq, D), float("nan"), device=dev, dtype=torch.bfloat16)
+
+    def run(n):
+        return _fn("dec_out")(_lib.ptr(q), _lib.ptr(start), _lib.ptr(count), _lib.ptr(pages), max_pages, _lib.ptr(kv_len),
+                              _lib.ptr(kc), _lib.ptr(vc), _lib.ptr(out), G, Hq, Hkv, D, n, 1 / math.sqrt(D), _lib.stream_ptr())
+
+    _lib.check(run(splits), "paged_decode")
+    _lib.check_status("paged_decode")
+    assert run(3) != 0 and run(8) != 0
+    for i, L in enumerate(lens):
+        if not active[i] or L == 0:
+            assert (out[i] == 0).all()
+            continue
+        pg = pages[i, :(L + PAGE - 1) // PAGE].long()
+        K, V = (c[pg].transpose(0, 1).reshape(Hkv, -1, D)[:, :L].double() for c in (kc, vc))
+        s = torch.einsum("hrd,hld->hrl", q[i].double().view(Hkv, -1, D), K) / math.sqrt(D)
+        p = torch.softmax(s, -1)
+        ref, mag = (torch.einsum("hrl,hld->hrd", p, x).reshape(Hq, D) for x in (V, V.abs()))
+        assert ((out[i].double() - ref).abs() <= 2 ** -8 * (ref.abs() + mag) + 1e-5).all(), (i, L)
+
+
+@pytest.mark.parametrize("B", [1, 37, 38, 74, 75, 148, 149])
+@pytest.mark.parametrize("V,pad", [(151936, 0), (1003, 1), (1001, 3), (31, 1), (3, 1)])
+def test_sampling_when_several_ctas_take_a_row(B, V, pad):
+    """Greedy tokens (the first of equal logits) and log-probs for every number of parts, rows that start off a 16-byte
+    boundary, parts without a vector and the remainder of a row.  Sums of V fp32 exponentials in 64 bits; 2^-21 each."""
+    from arctic_platform_b200.engine.sampler import _fn
+    from arctic_platform_b200.ops import _lib
+    dev = "cuda"
+    g = torch.Generator(device=dev).manual_seed(B + V)
+    logits = torch.randn(B, V + pad, device=dev, generator=g).mul_(4)[:, :V]
+    top = torch.randint(0, V, (B, 2), device=dev, generator=g)
+    logits.scatter_(1, top, 25.0)                                     # two equal maxima, anywhere in the row
+    temp = torch.zeros(B, device=dev)
+    tok, lp = torch.full((B,), -1, device=dev, dtype=torch.int32), torch.zeros(B, device=dev)
+    step = torch.zeros(1, device=dev, dtype=torch.int32)
+
+    def run():
+        _lib.check(_fn("sample")(_lib.ptr(logits), logits.stride(0), _lib.ptr(temp), B, V, 11, _lib.ptr(step), _lib.ptr(tok),
+                                 _lib.ptr(lp), _lib.stream_ptr()), "sample")
+
+    run()
+    assert torch.equal(tok.long(), top.min(1).values)
+    # |z| <= 25 enters exp and log with 2^-24 relative, the exponential's own error and the sums' are below 2^-19
+    tol = 25 * 2 ** -23 + 2 ** -18
+    assert (lp.double() - torch.log_softmax(logits.double(), -1).gather(1, tok.long()[:, None])[:, 0]).abs().max() < tol
+    temp.fill_(1.5)
+    run()
+    assert ((tok >= 0) & (tok < V)).all()
+    ref = torch.log_softmax(logits.double() / 1.5, -1).gather(1, tok.long()[:, None])[:, 0]
+    assert (lp.double() - ref).abs().max() < tol
+
+
+def test_single_samples_with_and_without_a_shared_header():
+    """One sample a prompt keeps its pages to itself: the same greedy tokens' log-probs with the shared pass on and off."""
+    from arctic_platform_b200.ops import _lib
+    rng = np.random.default_rng(3)
+    header = rng.integers(1, 200, size=48).tolist()
+    prompts = [header + rng.integers(1, 200, size=k).tolist() for k in (5, 16, 33)]
+    prompts += [rng.integers(1, 200, size=k).tolist() for k in (3, 16, 32, 75)]
+    outs = []
+    for cascade in (True, False):
+        _, _, eng = _engine(cascade, True)
+        outs.append(eng.generate(prompts, {"n": 1, "temperature": 0.0, "max_tokens": 20}))
+        _lib.check_status("generate")
+        assert eng.pages.free_count() == eng.num_pages
+    for a, b in zip(*outs):
+        same = next((i for i, (x, y) in enumerate(zip(a["token_ids"], b["token_ids"])) if x != y), 20)
+        assert same > 0
+        # bf16 logits of the two orders of summation: the bound of the scoring test above
+        assert np.abs(np.array(a["logprobs"][:same]) - np.array(b["logprobs"][:same])).max() < 0.08
