@@ -77,13 +77,15 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 }
 // Bounded wait.  Returns false (and records `code`) after kWaitLimitNs.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* status, int code) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const uint64_t t0 = global_timer_ns();
+  // the clock is read only by waits that have lasted: a read takes longer than most waits do
+  uint64_t t0 = 0;
   for (;;) {
 #pragma unroll 1
     for (int i = 0; i < 128; ++i)
       if (mbar_try_wait(bar, parity)) return true;
-    if (global_timer_ns() - t0 > kWaitLimitNs) {
+    const uint64_t now = global_timer_ns();
+    if (t0 == 0) t0 = now;
+    if (now - t0 > kWaitLimitNs) {
       if (status) atomicCAS(status, 0, code);
       return false;
     }
