@@ -176,9 +176,10 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tma_a, const CUtens
         int m0, m_end, b_row, n0, kb0, kb1;
         decode(blockIdx.x, m0, m_end, b_row, n0, kb0, kb1);
         prefetched = min(Cfg::kStages, kb1 - kb0);
-        const int rot = k_rotation(blockIdx.x, kb1 - kb0);
+        int next = kb0 + k_rotation(blockIdx.x, kb1 - kb0);
         for (int i = 0; i < prefetched; ++i) {
-          const int kb = kb0 + (i + rot) % (kb1 - kb0);
+          const int kb = next;
+          if (++next == kb1) next = kb0;
           uint8_t* sb = smem + i * Cfg::kStageBytes + Cfg::kABytes;
           mbar_expect_tx(&full_bar[i], Cfg::kStageBytes);
           if (!p.b_mn) {
@@ -194,9 +195,10 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tma_a, const CUtens
       for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
         int m0, m_end, b_row, n0, kb0, kb1;
         decode(t, m0, m_end, b_row, n0, kb0, kb1);
-        const int rot = k_rotation(t, kb1 - kb0);
+        int next = kb0 + k_rotation(t, kb1 - kb0);
         for (int it = 0; it < kb1 - kb0; ++it) {
-          const int kb = kb0 + (it + rot) % (kb1 - kb0);
+          const int kb = next;
+          if (++next == kb1) next = kb0;
           const bool b_done = prefetched > 0;      // this stage's barrier is armed and its B tile requested already
           if (b_done) --prefetched;
           if (!b_done && !mbar_wait(&empty_bar[stage], phase ^ 1, p.status, kTimeoutEmpty)) {
