@@ -1,8 +1,9 @@
 // bf16 GEMM on CTA pairs: two SMs work on one output tile of 256 x 256 or 256 x 512 with tcgen05.mma.cta_group::2.
 //
-// What bounds it: the operand stream from L2 to the SMs.  A 256 x 256 tile moves 64 B per SM and tensor cycle, which L2 delivers
-// at little more than half of the tensor rate (all-zero operands, where power does not matter: 1290 TFLOP/s at 1965 MHz); with
-// real operands the card also sits at its power limit, and every byte moved costs clock.  A 256 x 512 tile moves a quarter less.
+// What bounds it: the card's power limit.  With real operands the clock falls until it fits, and every byte moved costs clock: a
+// 256 x 512 tile moves a quarter less from L2 than a 256 x 256 tile, whose 64 B per SM and tensor cycle are also close to what L2
+// delivers.  With all-zero operands, where power does not matter, it runs at 2090 TFLOP/s; products issued by a lone lane (see the
+// issuer) stopped at 1290, real operands at 1100 to 1360, now 1270 to 1560 (Qwen3-4B shapes, 8192 to 18432 rows).
 // It fills all 512 columns of tensor memory, so the two accumulators cannot belong to two tiles; they are the two halves of one
 // (see "Halves").
 //
