@@ -229,3 +229,48 @@ def test_in_between_tile_widths(M, N, K, bn):
     auto = gemm.matmul_nt(a, b)                      # the automatic choice for one row tile may be one of these widths
     _lib.check_status("gemm auto")
     _close(auto, ref, K)
+
+
+@pytest.mark.parametrize("M", [1, 31, 32, 33])
+@pytest.mark.parametrize("bn", [128, 144, 208, 256])
+def test_few_rows_at_every_width(M, bn):
+    """At most 32 rows stage 32 of A, the 33rd takes the full tile: fp32, bf16 and SwiGLU results, columns that end inside a tile, K
+    that ends inside a k-block.  fp32 sums of K products: 2^-22 of the sum of magnitudes; bf16 rounding 2^-9 of the result."""
+    from arctic_platform_b200.ops import _lib, gemm
+    N, K = 304, 584
+    g = torch.Generator(device="cuda").manual_seed(M + bn)
+    x, w = (torch.randn(r, K, generator=g, device="cuda").bfloat16() for r in (M, N))
+    ref, mag = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    f32, b16 = torch.full((M, N), 7.0, device="cuda"), torch.empty(M, N, device="cuda", dtype=torch.bfloat16)
+    act = torch.empty(M, N // 2, device="cuda", dtype=torch.bfloat16)
+    gemm.gemm_raw(x, w, f32, M=M, N=N, K=K, epi=gemm.EPI_F32, bn=bn)
+    assert ((f32.double() - ref).abs() <= 2 ** -22 * mag).all()
+    gemm.gemm_raw(x, w, b16, M=M, N=N, K=K, epi=gemm.EPI_BF16, bn=bn)
+    assert ((b16.double() - ref).abs() <= 2 ** -22 * mag + 2 ** -8 * ref.abs()).all()
+    f32.fill_(0.5)
+    gemm.gemm_raw(x, w, f32, M=M, N=N, K=K, epi=gemm.EPI_F32_ATOMIC, splits=3, bn=bn)
+    assert ((f32.double() - ref - 0.5).abs() <= 2 ** -22 * (mag + 1)).all()
+    gemm.gemm_raw(x, w, None, M=M, N=N, K=K, epi=gemm.EPI_SWIGLU, out2=act, bn=bn)
+    a32, b32 = ref[:, 0::2], ref[:, 1::2]
+    want = a32 * torch.sigmoid(a32) * b32
+    # gate and up are rounded to bf16 before the product (2^-9 each; silu changes by at most 1.1 times that), then the result
+    slack = 2 ** -8 * (a32.abs() * b32.abs() * 1.1 + want.abs()) + 2 ** -20 * mag.max() * (a32.abs() + b32.abs())
+    assert ((act.double() - want).abs() <= 2 * slack).all()
+    _lib.check_status("gemm")
+
+
+@pytest.mark.parametrize("M,N,K", [(256, 768, 4292), (8, 128, 512), (130, 136, 513), (768, 264, 2000)])
+def test_sums_of_few_tiles_are_cut_along_k(M, N, K):
+    """"+=" whose tiles leave most SMs without work adds parts of K: whole and ragged tiles, K that ends inside a k-block."""
+    from arctic_platform_b200.ops import _lib, gemm
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    Kp = (K + 7) // 8 * 8
+    a, b = (torch.zeros(r, Kp, device="cuda", dtype=torch.bfloat16) for r in (M, N))
+    for t in (a, b):
+        t[:, :K] = torch.randn(t.shape[0], K, generator=g, device="cuda").bfloat16()
+    c0 = torch.randn(M, N, generator=g, device="cuda")
+    out = c0.clone()
+    gemm.gemm_raw(a, b, out, M=M, N=N, K=K, epi=gemm.EPI_F32_ACCUM)
+    mag = a.double().abs() @ b.double().abs().T + c0.double().abs()
+    assert ((out.double() - c0.double() - a.double() @ b.double().T).abs() <= 2 ** -21 * mag).all()
+    _lib.check_status("gemm")
