@@ -456,7 +456,7 @@ paged_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, const int* __restri
       const long long qrow = qs + q0 + rr / R;
       const long long head = qrow * Hq + kvh * R + rr % R;
       if (out && splits == 1) {
-        out[head * D + d] = __float2bfloat16(ll > 0.f ? ov / ll : 0.f);
+        out[head * D + d] = __float2bfloat16(ov * (ll > 0.f ? 1.f / ll : 0.f));
       } else if (out) {
         part_o[i] = ov;
         if (d == 0) {
@@ -473,7 +473,8 @@ paged_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, const int* __restri
       }
     }
     if (out && splits > 1) {
-      // the cluster's parts, joined by all its CTAs: each takes every splits-th run of 128 values
+      // the cluster's parts, joined by all its CTAs in the order and with the roundings of decode_merge_kernel: each takes every
+      // splits-th run of 128 values
       cluster_sync_all();
       for (int rr = split; rr < rows_valid; rr += splits) {
         const int d = threadIdx.x;
@@ -494,7 +495,7 @@ paged_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, const int* __restri
           ll += pl[k] * f;
         }
         const long long qrow = qs + q0 + rr / R;
-        out[(qrow * Hq + kvh * R + rr % R) * D + d] = __float2bfloat16(ll > 0.f ? ov / ll : 0.f);
+        out[(qrow * Hq + kvh * R + rr % R) * D + d] = __float2bfloat16(ov * (ll > 0.f ? 1.f / ll : 0.f));
       }
       cluster_sync_all();
     }
@@ -1018,6 +1019,7 @@ int apb_decode_qkv_post(float* acc, long long ld_acc, const void* wq, const void
 // Selects the scalar (CUDA-core) paged decode kernel instead of the MMA one: numerics cross-check and A/B timing.
 static int g_decode_scalar = 0;
 void apb_decode_use_scalar(int on) { g_decode_scalar = on; }
+int apb_decode_scalar() { return g_decode_scalar; }
 
 static int launch_decode_mma(const void* q, const int* q_start, const int* q_count, const int* pages, int max_pages, const int* kv_len,
                              const void* kcache, const void* vcache, float* out_o, float* out_ml, void* out, int G, int Hq, int Hkv,
@@ -1038,8 +1040,8 @@ static int launch_decode_mma(const void* q, const int* q_start, const int* q_cou
 }
 
 // Decode attention of one token per sequence over its whole page table, normalised: out [Bq, Hq, D] bf16 (zeros in the row q_start[g] of
-// a group without queries).  D = 128, the query heads of a key head divide 16, 1, 2 or 4 splits.  Arguments as
-// apb_paged_decode_partial's.
+// a group without queries), to the bit what apb_paged_decode_partial and apb_decode_merge make of the same splits.  D = 128, the
+// query heads of a key head divide 16, 1, 2 or 4 splits.  Arguments as apb_paged_decode_partial's.
 int apb_paged_decode(const void* q, const int* q_start, const int* q_count, const int* pages, int max_pages, const int* kv_len,
                      const void* kcache, const void* vcache, void* out, int G, int Hq, int Hkv, int D, int splits, float scale,
                      cudaStream_t s) {

@@ -456,12 +456,13 @@ class SamplerEngine:
                                            self.d_priv_table, self.d_priv_len, self.part_o, self.part_ml, node_splits,
                                            seq_splits, scale, out=out, n_nodes=nodes)
         s = _lib.stream_ptr()
-        if c.head_dim == 128 and 16 % (c.num_heads // c.num_kv_heads) == 0:
-            # one source: the splits of a row are a cluster that joins them (a power of two), nothing is left to merge
+        if (c.head_dim == 128 and 16 % (c.num_heads // c.num_kv_heads) == 0 and seq_splits != 3
+                and not _lib.cuda_lib().apb_decode_scalar()):
+            # one source: the splits of a row (a power of two) are a cluster that joins them, nothing is left to merge; the same
+            # bits as the two launches below
             _lib.check(_fn("dec_out")(_lib.ptr(q), _lib.ptr(self.d_q_start), _lib.ptr(self.d_active), _lib.ptr(self.d_page_table),
                                       self.max_pages, _lib.ptr(self.d_len), _lib.ptr(kc), _lib.ptr(vc), _lib.ptr(out), B,
-                                      c.num_heads, c.num_kv_heads, c.head_dim, 1 << (seq_splits.bit_length() - 1), scale, s),
-                       "paged_decode")
+                                      c.num_heads, c.num_kv_heads, c.head_dim, seq_splits, scale, s), "paged_decode")
             return out
         _lib.check(_fn("dec")(_lib.ptr(q), _lib.ptr(self.d_q_start), _lib.ptr(self.d_active), _lib.ptr(self.d_page_table),
                               self.max_pages, _lib.ptr(self.d_len), _lib.ptr(kc), _lib.ptr(vc), _lib.ptr(self.part_o[0]),
@@ -795,10 +796,12 @@ class SamplerEngine:
                 slots_free.sort()
                 first_of_run = True
                 for r, P, n_full, priv_pages in per_prompt:
-                    if sp.n == 1:
+                    if sp.n == 1 and not self.cfg.is_moe:
                         # one sample: nobody shares the prompt, so its pages belong to the per-sequence pass.  On a tile of
                         # the shared pass 128 rows would stand for one sequence (41 prompts of 500 to 1500 tokens, 8 key
-                        # heads: 66 us a layer for the shared pass alone, 38 for a per-sequence pass that reads everything)
+                        # heads: 66 us a layer for the shared pass alone, 38 for a per-sequence pass that reads everything).
+                        # The two passes round their probabilities against different maxima; a router turns such last bits
+                        # into other experts, so models with experts keep the shared pass
                         n_full, priv_pages = 0, n_full + priv_pages
                     shared = self.pages.alloc(n_full)
                     gid = next_group

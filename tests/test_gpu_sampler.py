@@ -282,3 +282,49 @@ def test_single_samples_with_and_without_a_shared_header():
         assert same > 0
         # bf16 logits of the two orders of summation: the bound of the scoring test above
         assert np.abs(np.array(a["logprobs"][:same]) - np.array(b["logprobs"][:same])).max() < 0.08
+
+
+@pytest.mark.parametrize("Hq,Hkv,splits", [(32, 8, 1), (32, 4, 2), (16, 8, 4)])
+def test_cluster_join_has_the_bits_of_the_merge(Hq, Hkv, splits):
+    """What one launch joins is what partials and their merge give, to the bit: a router behind it turns last bits into experts."""
+    import ctypes
+    import math
+    from arctic_platform_b200.engine.sampler import _fn
+    from arctic_platform_b200.ops import _lib
+    dev, D, PAGE = "cuda", 128, 16
+    g = torch.Generator(device=dev).manual_seed(Hq + splits)
+    lens = [1, 15, 17, 64, 65, 1023, 300, 500, 777]
+    G, max_pages = len(lens), 64
+    kc, vc = (torch.randn(G * max_pages, Hkv, PAGE, D, device=dev, generator=g).bfloat16() for _ in range(2))
+    pages = torch.randperm(G * max_pages, device=dev, generator=g).to(torch.int32).view(G, max_pages)
+    q = torch.randn(G, Hq, D, device=dev, generator=g).bfloat16()
+    i32 = dict(device=dev, dtype=torch.int32)
+    start, count, kv_len = torch.arange(G, **i32), torch.ones(G, **i32), torch.tensor(lens, **i32)
+    one, two = (torch.empty(G, Hq, D, device=dev, dtype=torch.bfloat16) for _ in range(2))
+    po, pml = torch.zeros(G, Hq, splits, D, device=dev), torch.zeros(G, Hq, splits, 2, device=dev)
+    head = [_lib.ptr(t) for t in (q, start, count, pages)] + [max_pages] + [_lib.ptr(t) for t in (kv_len, kc, vc)]
+    tail = [G, Hq, Hkv, D, splits, 1 / math.sqrt(D), _lib.stream_ptr()]
+    _lib.check(_fn("dec_out")(*head, _lib.ptr(one), *tail), "paged_decode")
+    _lib.check(_fn("dec")(*head, _lib.ptr(po), _lib.ptr(pml), *tail), "paged_decode_partial")
+    _lib.check(_fn("merge")((ctypes.c_void_p * 4)(po.data_ptr(), 0, 0, 0), (ctypes.c_void_p * 4)(pml.data_ptr(), 0, 0, 0),
+                            (ctypes.c_int * 4)(splits, 0, 0, 0), 1, None, _lib.ptr(two), None, G, Hq, D, _lib.stream_ptr()), "merge")
+    _lib.check_status("paged_decode")
+    assert torch.equal(one, two)
+
+
+def test_expert_models_round_alike_for_one_and_for_two_samples():
+    """Prompts with one sample of a model with experts are decoded as those with several: another rounding of their probabilities
+    would choose other experts now and then.  Greedy samples of a prompt are equal, so are their log-probs, to the bit."""
+    from arctic_platform_b200.engine.sampler import SamplerEngine
+    from arctic_platform_b200.models.config import PRESETS
+    from arctic_platform_b200.models.decoder import DecoderLM
+    cfg = PRESETS["qwen3-moe-tiny"]
+    model = DecoderLM(cfg, "cuda", torch.bfloat16).init_weights(seed=5, std=0.05)
+    rng = np.random.default_rng(4)
+    prompts = [rng.integers(1, cfg.vocab_size, size=n).tolist() for n in (300, 37, 5, 160)]
+    outs = []
+    for n in (1, 2):
+        eng = SamplerEngine(cfg, "cuda", model=model, kv_cache_tokens=1 << 13, max_batch=8, max_seq_len=512)
+        outs.append(eng.generate(prompts, {"n": n, "temperature": 0.0, "max_tokens": 24})[::n])
+    for a, b in zip(*outs):
+        assert a["token_ids"] == b["token_ids"] and a["logprobs"] == b["logprobs"]
