@@ -328,9 +328,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
         tmem_st_32x32(t_s, pk);
         tmem_st_wait();
       }
+      // dO (and -delta, which comes with it) is seen before P^T is published: dV(i), which needs P^T alone of this group, gives dO's
+      // buffer back, and its barrier may then pass tile i + 1's phase before a warp that was held up here has looked at tile i's.
+      ok = wait(do_full, par, kTimeoutFull);
+      if (!ok) break;
       tc_fence_before();
       mbar_arrive(p_full);
-      ok = wait(do_full, par, kTimeoutFull) && wait(dp_full, par, kTimeoutTmemFull);
+      ok = wait(dp_full, par, kTimeoutTmemFull);
       if (!ok) break;
       const ulonglong2* ndelta = reinterpret_cast<const ulonglong2*>(smem_delta + s * 128 + grp * 64);
 #pragma unroll
