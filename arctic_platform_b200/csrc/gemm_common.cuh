@@ -26,6 +26,12 @@ __host__ __device__ inline bool is_glu_epilogue(int epi) {
   return epi == kEpiSwiGLU || epi == kEpiGeGLU || epi == kEpiClampGLU;
 }
 
+enum StagedOut : int {
+  kNotStaged = 0,
+  kStagedClipped = 1,  // the tensor map of C ends with row M
+  kStagedSlabs = 2,    // C is stacked (tile_ext): the map does not end with a slab
+};
+
 struct PeerTensorMaps {
   CUtensorMap m[8];
 };
@@ -70,7 +76,7 @@ struct GemmParams {
   int heads, a_step, c_step;
   const __nv_bfloat16* gate;   // kEpiSigmoidGate
   long long ldg;
-  int staged;              // one-CTA kernel: fp32 results leave by TMA (set by the launcher)
+  int staged;              // one-CTA kernel: fp32 results leave by TMA (StagedOut, set by the launcher)
   int chained;             // 1: launched in chained mode -- B (weights nobody in the chain writes) is prefetched
                            // before the wait for the previous kernel, everything else after it
 };

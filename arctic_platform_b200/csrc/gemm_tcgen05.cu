@@ -370,9 +370,10 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tma_a, const CUtens
           tmem_ld_32x32(taddr + c * 32, r);
           tmem_ld_wait();
         }
-        if (MASK == kF32Epi && Cfg::kStaged && p.staged) {
-          // a box of 32 x 32 per warp; what it holds beyond the tile's rows or columns is added as zeros
-          const int row0 = m0 + quarter * 32;
+        // a box of 32 x 32 per warp; columns that it holds beyond the tile's are added as zeros.  Rows: it belongs to the tile as a
+        // whole, or the map ends with the tile's rows; a box that would reach into another group's rows goes the other way.
+        const int row0 = m0 + quarter * 32;
+        if (MASK == kF32Epi && Cfg::kStaged && p.staged && (row0 + 32 <= m_end || (p.staged == kStagedClipped && m_end == p.M))) {
           if (row0 >= m_end) continue;
           const StagedBox out{smem_out + quarter * kStagedBoxBytes, lane};
           out.begin();
@@ -380,7 +381,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tma_a, const CUtens
           for (int u = 0; u < 8; ++u) {
             float4 f = make_float4(__uint_as_float(r[u * 4]) * p.alpha, __uint_as_float(r[u * 4 + 1]) * p.alpha,
                                    __uint_as_float(r[u * 4 + 2]) * p.alpha, __uint_as_float(r[u * 4 + 3]) * p.alpha);
-            if (!row_ok || u * 4 >= ncols) f = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (u * 4 >= ncols) f = make_float4(0.f, 0.f, 0.f, 0.f);
             out.put(u, *reinterpret_cast<const uint4*>(&f));
           }
           out.send(tma_c, col0, row0 + c_off, p.epi != kEpiF32);
@@ -455,16 +456,15 @@ static int launch_gemm_as(const CUtensorMap& ta, const CUtensorMap& tb, GemmPara
   if (max_ctas > 0 && grid > max_ctas) grid = max_ctas;
   if (grid <= 0) return 0;
   // fp32 results go out by TMA (a weight gradient of few rows is bound by them: as rows per thread every 16 bytes were an L1
-  // wavefront of their own).  Boxes have 32 rows and columns: slabs of a stacked C start at multiples of that, and a store (which
-  // cannot pad with zeros) ends with the tile.
+  // wavefront of their own).  A store cannot pad a tile with zeros, so it needs tiles of whole boxes and no groups.  Slabs of a
+  // stacked C lie at row offsets that only the table knows: their map has all the rows that an index can name, and the kernel sends
+  // no box that is not its slab's as a whole.
   CUtensorMap tc = ta;
   const bool add = p.epi == kEpiF32Atomic || p.epi == kEpiF32Accum;
   if (MASK == kF32Epi && Cfg::kStaged && p.C && p.heads == 0 && (p.ldc % 4) == 0 &&
-      (reinterpret_cast<uintptr_t>(p.C) & 15) == 0 && (!p.tile_ext || p.M % 32 == 0) &&
-      (add || (BN % 32 == 0 && !p.tile_map))) {
-    // with slabs, no box reaches beyond the rows of its own one, and their number is the caller's
-    const uint64_t c_rows = p.tile_ext && !p.num_tiles_dev ? uint64_t{1} << 24 : static_cast<uint64_t>(p.M);
-    if (make_tmap_2d(&tc, p.C, 4, c_rows, p.N, p.ldc, 32, 32) == 0) p.staged = 1;
+      (reinterpret_cast<uintptr_t>(p.C) & 15) == 0 && (add || (BN % 32 == 0 && !p.tile_map))) {
+    const uint64_t c_rows = p.tile_ext ? uint64_t{1} << 31 : static_cast<uint64_t>(p.M);
+    if (make_tmap_2d(&tc, p.C, 4, c_rows, p.N, p.ldc, 32, 32) == 0) p.staged = p.tile_ext ? kStagedSlabs : kStagedClipped;
   }
   return static_cast<int>(launch_kernel(gemm_bf16_kernel<BN, AR, MASK>, dim3(grid), dim3(kGemmThreads), Cfg::kSmemBytes, stream,
                                         ta, tb, tc, p));

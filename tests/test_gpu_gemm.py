@@ -274,3 +274,43 @@ def test_sums_of_few_tiles_are_cut_along_k(M, N, K):
     mag = a.double().abs() @ b.double().abs().T + c0.double().abs()
     assert ((out.double() - c0.double() - a.double() @ b.double().T).abs() <= 2 ** -21 * mag).all()
     _lib.check_status("gemm")
+
+
+@pytest.mark.parametrize("device_count", [False, True])
+@pytest.mark.parametrize("M,m_end", [(96, 96), (160, 160), (72, 72), (160, 136)])
+@pytest.mark.parametrize("epi", ["EPI_F32_ACCUM", "EPI_F32"])
+def test_slabs_of_a_stacked_result(epi, M, m_end, device_count):
+    """Grouped weight gradients: every group's tiles write its own slab of C, rows that end inside a 32-row box, with the number of
+    tiles on the host or on the device.  fp32 sums of K products: 2^-21 of the sum of magnitudes.  What is no tile's keeps its bits."""
+    from arctic_platform_b200.models.moe import _plan_fns
+    from arctic_platform_b200.ops import _lib, gemm
+    N, rows = 136, (64, 0, 192, 128)
+    E, R = len(rows), sum(rows)
+    g = torch.Generator(device="cuda").manual_seed(M + m_end)
+    dy, x = (torch.randn(R, c, generator=g, device="cuda").bfloat16() for c in (M, N))
+    c0 = torch.randn(E * M, N, generator=g, device="cuda")
+    out, tiles, ext, first = c0.clone(), [], [], 0
+    for e, r in enumerate(rows):
+        for m0 in range(0, m_end, 128):
+            for t in range((N + 127) // 128):
+                tiles.append([m0, m_end, 0, t])
+                ext.append([e * M, first // 64, (first + r) // 64, 0])
+        first += r
+    i32 = dict(device="cuda", dtype=torch.int32)
+    tiles, ext = torch.tensor(tiles, **i32), torch.tensor(ext, **i32)
+    count = torch.tensor([len(tiles)], **i32) if device_count else None
+    _lib.check(_plan_fns()["gemm"](_lib.ptr(dy), _lib.ptr(x), _lib.ptr(out), M, N, R, M, N, N, 1, 1, getattr(gemm, epi), 1.0,
+                                   _lib.ptr(tiles), _lib.ptr(ext), len(tiles), _lib.ptr(count), 0, 0, _lib.stream_ptr()), "grouped")
+    _lib.check_status("gemm")
+    first = 0
+    for e, r in enumerate(rows):
+        a, b = dy[first:first + r, :m_end].double(), x[first:first + r].double()
+        got, was = out[e * M:(e + 1) * M], c0[e * M:(e + 1) * M]
+        first += r
+        assert torch.equal(got[m_end:], was[m_end:])
+        if not r:                                        # a group without rows is left alone
+            assert torch.equal(got, was)
+            continue
+        add = was[:m_end].double() if epi == "EPI_F32_ACCUM" else torch.zeros(m_end, N, device="cuda", dtype=torch.float64)
+        mag = a.abs().T @ b.abs() + add.abs()
+        assert ((got[:m_end].double() - add - a.T @ b).abs() <= 2 ** -21 * mag).all()
