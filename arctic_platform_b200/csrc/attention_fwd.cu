@@ -335,7 +335,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           if (c < 3) tmem_ld_32x32(t_s + (c + 1) * 32, buf[(c + 1) & 1]);
-          mask(c, buf[c & 1]);
           uint32_t pk[16];
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
@@ -343,6 +342,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
                 xtc_fma2(xtc_pair(__uint_as_float(buf[c & 1][2 * i]), __uint_as_float(buf[c & 1][2 * i + 1])), c2, nm2));
             f.x = xtc_ex2(f.x);
             f.y = xtc_ex2(f.y);
+            if (masked) {            // the weight itself: a masked score times a scale of zero is no number
+              if (c * 32 + 2 * i >= limit) f.x = 0.f;
+              if (c * 32 + 2 * i + 1 >= limit) f.y = 0.f;
+            }
             rowsum += f.x + f.y;
             pk[i] = pack_bf16x2(f.x, f.y);
           }

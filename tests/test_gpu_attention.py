@@ -126,3 +126,25 @@ def _attention64(q, k, v, layout):
         seen = torch.arange(pl + ol, device=q.device)[None] <= pl + ol - ql + torch.arange(ql, device=q.device)[:, None]
         out.append(torch.einsum("hqk,khd->qhd", torch.softmax(s.masked_fill(~seen, float("-inf")), -1), vv))
     return torch.cat(out)
+
+
+@pytest.mark.parametrize("scale", [0.0, -0.05])
+def test_scales_that_are_not_positive(scale):
+    """A scale of zero weighs all visible keys alike, a negative one turns the order of the scores: blocks with and without masks,
+    forward and backward.  Tolerances as above (bf16 operands o, P and dS)."""
+    from arctic_platform_b200.ops import _lib
+    from arctic_platform_b200.ops.attention import AttnLayout, attention_ref, segment_attention
+    segs = np.array([[0, 200, 0, 0, 0, 200], [200, 70, 0, 200, 200, 70], [270, 129, 0, 0, 270, 129]], dtype=np.int32)
+    layout = AttnLayout(segs, 399)
+    torch.manual_seed(8)
+    q, k, v = (_rand((399, h, 128)).requires_grad_() for h in (4, 2, 2))
+    d_o = _rand((399, 4, 128))
+    o = segment_attention(q, k, v, layout, scale)
+    o.backward(d_o)
+    _lib.check_status("attention")
+    qr, kr, vr = (x.detach().double().requires_grad_() for x in (q, k, v))
+    ref = attention_ref(qr, kr, vr, layout, scale)
+    ref.backward(d_o.double())
+    assert (o.double() - ref.double()).norm() <= 2 ** -7 * ref.double().norm()
+    for got, want in ((q.grad, qr.grad), (k.grad, kr.grad), (v.grad, vr.grad)):
+        assert (got.double() - want.double()).norm() <= 2 ** -6 * want.double().norm() + 1e-6
