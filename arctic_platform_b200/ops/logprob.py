@@ -20,6 +20,7 @@ from typing import Optional, Tuple
 import torch
 
 from . import _lib, gemm
+from ..utils import memory_budget
 
 
 def logprobs_entropy_ref(hidden, weight, labels, inv_temperature=1.0, with_entropy=True, chunk: int = 4096):
@@ -80,12 +81,19 @@ def _fwd_cuda(hidden, weight, labels, inv_temp_t, inv_temp_s):
     return lp, ent, lse
 
 
-def _bwd_rows(N: int, V: int, budget: int = 5 << 30) -> int:
-    """Rows of d(logits) that are formed at a time: as many as ``budget`` bytes of bf16 hold, in chunks of equal size.  Every
-    chunk reads and writes the fp32 weight gradient once, and the tiles of a chunk's ``[rows, H]`` gradient should fill the
-    GPU several times over: at V = 151936, H = 2560 chunks of 4096 rows make 160 tiles on 74 CTA pairs (2.2 waves), chunks of
-    16384 rows 640 (8.6 waves)."""
-    parts = -(-N * V * 2 // budget)
+_BWD_ROWS = 4096        # rows of d(logits) that are formed at a time wherever memory is short
+
+
+def _bwd_rows(N: int, V: int, spare: int, budget: int = 5 << 30) -> int:
+    """Rows of d(logits) that are formed at a time: ``_BWD_ROWS``, or a multiple of it that ``budget`` bytes of bf16 hold where
+    ``spare`` bytes are there for what it takes beyond.  Every chunk reads and writes the fp32 weight gradient once, and the tiles
+    of a chunk's ``[rows, H]`` gradient should fill the GPU several times over: at V = 151936, H = 2560 chunks of 4096 rows make 160
+    tiles on 74 CTA pairs (2.2 waves), chunks of 16384 rows 640 (8.6 waves).  Chunks are of equal size."""
+    if N <= _BWD_ROWS:
+        return N
+    unit = _BWD_ROWS * V * 2
+    most = max(1, min(budget // unit, 1 + max(0, spare) // unit)) * _BWD_ROWS
+    parts = -(-N // most)
     return min(N, (-(-N // parts) + 255) // 256 * 256)
 
 
@@ -113,8 +121,12 @@ class _LmHeadLogprobFn(torch.autograd.Function):
         d_hidden = torch.empty_like(hidden)
         acc = getattr(weight, "grad_f32", None)
         dw32 = acc if acc is not None else torch.zeros((V, H), device=hidden.device, dtype=torch.float32)
-        chunk = ctx.bwd_chunk or _bwd_rows(N, V)
-        buf = torch.empty((min(chunk, N), V), device=hidden.device, dtype=torch.bfloat16)
+        chunk = ctx.bwd_chunk
+        if chunk is None:
+            chunk = _bwd_rows(N, V, memory_budget.spare_bytes(hidden.device) if N > _BWD_ROWS else 0)
+        # whole units, so that batches of other lengths find the block again
+        buf_rows = min(chunk, N) if ctx.bwd_chunk or N <= _BWD_ROWS else -(-chunk // _BWD_ROWS) * _BWD_ROWS
+        buf = torch.empty((buf_rows, V), device=hidden.device, dtype=torch.bfloat16)
         for s in range(0, N, chunk):
             n = min(chunk, N - s)
             h = hidden[s:s + n]

@@ -17,6 +17,9 @@ The trainer reports its footprint after every optimizer step (``note_training_pe
 that moment -- the caching allocator does not return blocks, so this is the training high-water mark, symmetric
 buffers included -- minus the KV bytes that were resident meanwhile.  ``kv_may_stay`` answers for the sampler.
 ``APB_SLEEP_KEEP_KV=0`` / ``1`` forces the answer.
+
+``spare_bytes`` is the other direction: how much a workspace may take beyond what it has to, so that the answer above does not
+change and nothing that fitted stops to fit.
 """
 from __future__ import annotations
 
@@ -27,6 +30,7 @@ import torch
 
 _train_peak: Dict[int, int] = {}      # device index -> bytes in use by everything but the KV cache, after a step
 _kv_resident: Dict[int, int] = {}     # device index -> bytes of KV cache currently allocated by samplers
+_kv_awake: Dict[int, int] = {}        # device index -> the most that it has been
 
 _trainers: Dict[int, int] = {}        # device index -> training engines built in this process
 _samplers: Dict[int, int] = {}        # device index -> sampler engines built in this process
@@ -57,7 +61,9 @@ def _index(device) -> int:
 
 
 def set_kv_resident(device, nbytes: int) -> None:
-    _kv_resident[_index(device)] = int(nbytes)
+    i = _index(device)
+    _kv_resident[i] = int(nbytes)
+    _kv_awake[i] = max(_kv_awake.get(i, 0), int(nbytes))
 
 
 def note_training_peak(device) -> None:
@@ -66,6 +72,18 @@ def note_training_peak(device) -> None:
     i = _index(device)
     free, total = torch.cuda.mem_get_info(i)
     _train_peak[i] = max(_train_peak.get(i, 0), total - free - _kv_resident.get(i, 0))
+
+
+def spare_bytes(device) -> int:
+    """Device memory that a workspace may use if it helps: what the driver has free and the caching allocator has unused, less the
+    headroom and the place of a KV cache that is asleep.  0 while a graph is captured (nothing is asked of the driver there)."""
+    if torch.cuda.is_current_stream_capturing():
+        return 0
+    i = _index(device)
+    free, total = torch.cuda.mem_get_info(i)
+    unused = torch.cuda.memory_reserved(i) - torch.cuda.memory_allocated(i)
+    asleep = max(0, _kv_awake.get(i, 0) - _kv_resident.get(i, 0))
+    return max(0, free + unused - asleep - int(HEADROOM * total))
 
 
 def kv_may_stay(device, kv_bytes: int) -> bool:

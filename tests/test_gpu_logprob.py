@@ -54,3 +54,34 @@ def test_row_and_column_remainders_of_pair_tiles(N, H, V):
         assert (got - ref).abs().max() <= 1e-4 * max(1.0, ref.abs().max().item())
     for got, ref in ((hidden.grad, hr.grad), (weight.grad, wr.grad)):
         assert (got.double() - ref).norm() <= 2 ** -7 * ref.norm()
+
+
+def test_gradients_where_memory_is_short():
+    """Without memory to spare d(logits) takes 4096 rows at a time; the gradients are those of one chunk but for the order of the
+    sums.  The tensor cores cut each step of 16 rows to the 24 bits of the running fp32 sum: N / 16 steps of 2^-23 at most.  The
+    hidden gradient is rounded to bf16 once on each side, 2^-9."""
+    from arctic_platform_b200.ops.logprob import lm_head_logprobs
+    from arctic_platform_b200.utils import memory_budget
+    N, H, V = 9000, 128, 32000
+    g = torch.Generator(device="cuda").manual_seed(2)
+    hidden = torch.randn(N, H, device="cuda", generator=g).bfloat16()
+    weight = (torch.randn(V, H, device="cuda", generator=g) * H ** -0.5).bfloat16()
+    labels = torch.randint(0, V, (N,), device="cuda", generator=g)
+    spare, got = memory_budget.spare_bytes, []
+    try:
+        for free in (0, 1 << 40):
+            memory_budget.spare_bytes = lambda device: free
+            h, w = hidden.clone().requires_grad_(), weight.clone().requires_grad_()
+            w.grad_f32 = torch.zeros(V, H, device="cuda")
+            lp, _ = lm_head_logprobs(h, w, labels)
+            torch.cuda.synchronize()
+            before = torch.cuda.memory_allocated()
+            torch.cuda.reset_peak_memory_stats()
+            lp.sum().backward()
+            got.append((h.grad, w.grad_f32, torch.cuda.max_memory_allocated() - before))
+    finally:
+        memory_budget.spare_bytes = spare
+    short, long = got
+    assert short[2] <= 4096 * V * 2 + (32 << 20) < long[2]
+    assert (short[1] - long[1]).norm() <= N / 16 * 2 ** -23 * long[1].norm()
+    assert (short[0].double() - long[0].double()).norm() <= 2 ** -8 * long[0].double().norm()
