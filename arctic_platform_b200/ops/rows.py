@@ -20,13 +20,24 @@ def rows_add(src: torch.Tensor, index: torch.Tensor, dst: torch.Tensor) -> None:
         c = ctypes
         _ADD = _lib.declare("apb_rows_add", [c.c_void_p, c.c_longlong, c.c_void_p, c.c_void_p, c.c_longlong, c.c_longlong, c.c_int,
                                              c.c_int, c.c_int, c.c_void_p])
-    _lib.check(_ADD(_lib.ptr(src), src.stride(0), _lib.ptr(index), _lib.ptr(dst), dst.stride(0), dst.shape[0],
+    _lib.check(_ADD(_lib.ptr(src), _ld(src), _lib.ptr(index), _lib.ptr(dst), dst.stride(0), dst.shape[0],
                     int(dst.dtype == torch.float32), src.shape[0], src.shape[1], _lib.stream_ptr()), "apb_rows_add")
 
 
 def _fits(t: torch.Tensor) -> bool:
     """Rows that the kernel addresses: whole vectors of 8 columns at 16-byte boundaries."""
     return t.is_cuda and t.dim() == 2 and t.stride(1) == 1 and t.shape[1] % 8 == 0 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0
+
+
+def _whole(t: torch.Tensor) -> torch.Tensor:
+    """Rows one behind the other from a 16-byte boundary on; a copy where a view is laid out otherwise."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
+def _ld(t: torch.Tensor) -> int:
+    """Elements between rows; a lone row may come with any stride."""
+    return t.stride(0) if t.shape[0] > 1 else t.shape[1]
 
 
 class _EmbeddingFn(torch.autograd.Function):
@@ -39,7 +50,7 @@ class _EmbeddingFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         (ids,) = ctx.saved_tensors
-        rows_add(dy.contiguous(), ids, ctx.weight.grad_f32)
+        rows_add(_whole(dy), ids, ctx.weight.grad_f32)
         return None, None
 
 
@@ -65,7 +76,7 @@ class _GatherFn(torch.autograd.Function):
     def backward(ctx, dy):
         (index,) = ctx.saved_tensors
         dx = torch.zeros(ctx.shape, device=dy.device, dtype=dy.dtype)
-        rows_add(dy.contiguous(), index, dx)
+        rows_add(_whole(dy), index, dx)
         return dx, None
 
 
@@ -109,17 +120,17 @@ def moe_place(chosen: torch.Tensor, experts: int, pad: int = 1):
 
 
 def _spread(x, place, rows: int, pad_rows: bool):
-    x = x.contiguous()
+    x = _whole(x)
     out = (torch.zeros if pad_rows else torch.empty)((rows, x.shape[1]), device=x.device, dtype=x.dtype)
-    _lib.check(_moe("spread")(_lib.ptr(x), x.stride(0), _lib.ptr(place), place.shape[0], place.shape[1], x.shape[1], _lib.ptr(out),
+    _lib.check(_moe("spread")(_lib.ptr(x), _ld(x), _lib.ptr(place), place.shape[0], place.shape[1], x.shape[1], _lib.ptr(out),
                               out.stride(0), _lib.stream_ptr()), "apb_moe_spread")
     return out
 
 
 def _collect(y, place, weight):
-    y = y.contiguous()
+    y = _whole(y)
     out = torch.empty((place.shape[0], y.shape[1]), device=y.device, dtype=y.dtype)
-    _lib.check(_moe("collect")(_lib.ptr(y), y.stride(0), _lib.ptr(place), _lib.ptr(weight), place.shape[0], place.shape[1], y.shape[1],
+    _lib.check(_moe("collect")(_lib.ptr(y), _ld(y), _lib.ptr(place), _lib.ptr(weight), place.shape[0], place.shape[1], y.shape[1],
                                _lib.ptr(out), out.stride(0), _lib.stream_ptr()), "apb_moe_collect")
     return out
 
@@ -139,7 +150,7 @@ class _SpreadFn(torch.autograd.Function):
 class _CollectFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, y, place, weight, pad_rows):
-        y, weight = y.contiguous(), weight.contiguous()
+        y, weight = _whole(y), weight.contiguous()
         ctx.save_for_backward(y, place, weight)
         ctx.pad_rows = pad_rows
         return _collect(y, place, weight)
@@ -147,10 +158,10 @@ class _CollectFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, d):
         y, place, weight = ctx.saved_tensors
-        d = d.contiguous()
+        d = _whole(d)
         dy = (torch.zeros_like if ctx.pad_rows else torch.empty_like)(y)
         dw = torch.empty_like(weight)
-        _lib.check(_moe("collect_bwd")(_lib.ptr(d), d.stride(0), _lib.ptr(y), y.stride(0), _lib.ptr(place), _lib.ptr(weight),
+        _lib.check(_moe("collect_bwd")(_lib.ptr(d), _ld(d), _lib.ptr(y), _ld(y), _lib.ptr(place), _lib.ptr(weight),
                                        place.shape[0], place.shape[1], y.shape[1], _lib.ptr(dy), _lib.ptr(dw), _lib.stream_ptr()),
                    "apb_moe_collect_bwd")
         return dy, None, dw, None

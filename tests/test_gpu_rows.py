@@ -76,3 +76,32 @@ def test_rows_to_experts_and_back(tokens, k, experts, cols, pad):
     dw = d.double()[:, None] * zr[at]
     assert ((w.grad - dw.sum(-1)).abs() <= cols * 2 ** -23 * dw.abs().sum(-1)).all()
     assert near(x.grad, dy.double()[at].sum(1), dy.double()[at].abs().sum(1))
+
+
+def test_rows_that_begin_anywhere():
+    """Views that start off a 16-byte boundary, a lone row with an odd stride: the same sums as aligned copies of them."""
+    from arctic_platform_b200.ops import rows as ops
+    g = torch.Generator(device="cuda").manual_seed(6)
+    off = lambda r, c: torch.randn(r * c + 1, device="cuda", generator=g).bfloat16()[1:].view(r, c)
+    x, d, index = off(40, 64), off(25, 64), torch.randperm(40, device="cuda", generator=g)[:25]
+    base = torch.randn(40, 64, device="cuda", generator=g).bfloat16().requires_grad_()
+    ops.gather_rows(base, index).backward(d)
+    assert torch.equal(base.grad[index], d)
+    weight = torch.nn.Parameter(torch.randn(40, 64, device="cuda", generator=g).bfloat16())
+    weight.grad_f32 = torch.zeros(40, 64, device="cuda")
+    ops.embedding(index, weight).backward(d)
+    assert torch.equal(weight.grad_f32[index], d.float())
+    chosen = torch.randint(0, 5, (40, 1), device="cuda", generator=g)
+    lone = torch.randn(1, 67, device="cuda", generator=g).bfloat16()[:, :64]
+    for src, c in ((x, chosen), (lone, chosen[:1])):
+        _, place = ops.moe_place(c, 5)
+        y = ops.moe_spread(src, place, len(c))
+        assert torch.equal(y[place[:, 0].long()], src)
+        w = torch.ones(len(c), 1, device="cuda")
+        z = off(len(c), 64)
+        z.copy_(y)
+        z.requires_grad_()
+        out = ops.moe_collect(z, place, w)
+        assert torch.equal(out, src)
+        out.backward(x[:len(c)])
+        assert torch.equal(z.grad[place[:, 0].long()], x[:len(c)])
