@@ -265,23 +265,32 @@ def test_sampling_when_several_ctas_take_a_row(B, V, pad):
 
 
 def test_single_samples_with_and_without_a_shared_header():
-    """One sample a prompt keeps its pages to itself: the same greedy tokens' log-probs with the shared pass on and off."""
+    """One sample a prompt keeps its pages to itself: with the shared pass on and off, every reported log-prob of all tokens equals
+    the model's own when the sequence is scored in one packed pass (bounds of the scoring test above)."""
+    from arctic_platform_b200.models.decoder import token_logprobs
     from arctic_platform_b200.ops import _lib
+    from arctic_platform_b200.rl.zorro_train.layout import build_packed_batch
     rng = np.random.default_rng(3)
     header = rng.integers(1, 200, size=48).tolist()
     prompts = [header + rng.integers(1, 200, size=k).tolist() for k in (5, 16, 33)]
     prompts += [rng.integers(1, 200, size=k).tolist() for k in (3, 16, 32, 75)]
-    outs = []
+    P, R = max(map(len, prompts)), 20
     for cascade in (True, False):
-        _, _, eng = _engine(cascade, True)
-        outs.append(eng.generate(prompts, {"n": 1, "temperature": 0.0, "max_tokens": 20}))
+        _, model, eng = _engine(cascade, True)
+        outs = eng.generate(prompts, {"n": 1, "temperature": 0.0, "max_tokens": R})
         _lib.check_status("generate")
         assert eng.pages.free_count() == eng.num_pages
-    for a, b in zip(*outs):
-        same = next((i for i, (x, y) in enumerate(zip(a["token_ids"], b["token_ids"])) if x != y), 20)
-        assert same > 0
-        # bf16 logits of the two orders of summation: the bound of the scoring test above
-        assert np.abs(np.array(a["logprobs"][:same]) - np.array(b["logprobs"][:same])).max() < 0.08
+        ids = torch.zeros((len(outs), P + R), dtype=torch.int64)
+        mask = torch.zeros_like(ids)
+        for i, (p, o) in enumerate(zip(prompts, outs)):
+            assert len(o["token_ids"]) == R
+            ids[i, P - len(p):] = torch.tensor(p + o["token_ids"])
+            mask[i, P - len(p):] = 1
+        pb = build_packed_batch(ids, mask, R, dedup=True).to("cuda")
+        with torch.no_grad():
+            lp, _ = token_logprobs(model, pb, 1.0)
+        diff = (torch.tensor([o["logprobs"] for o in outs]) - pb.scatter_to_grid(lp).cpu()).abs()
+        assert diff.max() < 0.08 and diff.mean() < 0.01
 
 
 @pytest.mark.parametrize("Hq,Hkv,splits", [(32, 8, 1), (32, 4, 2), (16, 8, 4)])
