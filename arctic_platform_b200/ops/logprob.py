@@ -82,9 +82,10 @@ def _fwd_cuda(hidden, weight, labels, inv_temp_t, inv_temp_s):
 
 
 _BWD_ROWS = 4096        # rows of d(logits) that are formed at a time wherever memory is short
+_BWD_BUDGET = 5 << 30   # bytes of d(logits) at most where it is not
 
 
-def _bwd_rows(N: int, V: int, spare: int, budget: int = 5 << 30) -> int:
+def _bwd_rows(N: int, V: int, spare: int, budget: int = _BWD_BUDGET) -> int:
     """Rows of d(logits) that are formed at a time: ``_BWD_ROWS``, or a multiple of it that ``budget`` bytes of bf16 hold where
     ``spare`` bytes are there for what it takes beyond.  Every chunk reads and writes the fp32 weight gradient once, and the tiles
     of a chunk's ``[rows, H]`` gradient should fill the GPU several times over: at V = 151936, H = 2560 chunks of 4096 rows make 160
@@ -123,7 +124,7 @@ class _LmHeadLogprobFn(torch.autograd.Function):
         dw32 = acc if acc is not None else torch.zeros((V, H), device=hidden.device, dtype=torch.float32)
         chunk = ctx.bwd_chunk
         if chunk is None:
-            chunk = _bwd_rows(N, V, memory_budget.spare_bytes(hidden.device) if N > _BWD_ROWS else 0)
+            chunk = _bwd_rows(N, V, memory_budget.spare_bytes(hidden.device, _BWD_BUDGET) if N > _BWD_ROWS else 0)
         # whole units, so that batches of other lengths find the block again
         buf_rows = min(chunk, N) if ctx.bwd_chunk or N <= _BWD_ROWS else -(-chunk // _BWD_ROWS) * _BWD_ROWS
         buf = torch.empty((buf_rows, V), device=hidden.device, dtype=torch.bfloat16)

@@ -70,7 +70,7 @@ def test_gradients_where_memory_is_short():
     spare, got = memory_budget.spare_bytes, []
     try:
         for free in (0, 1 << 40):
-            memory_budget.spare_bytes = lambda device: free
+            memory_budget.spare_bytes = lambda device, wanted: free
             h, w = hidden.clone().requires_grad_(), weight.clone().requires_grad_()
             w.grad_f32 = torch.zeros(V, H, device="cuda")
             lp, _ = lm_head_logprobs(h, w, labels)

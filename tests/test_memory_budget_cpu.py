@@ -23,22 +23,33 @@ def test_rows_of_dlogits(N, V, spare):
 
 def test_spare_memory(monkeypatch):
     gb = 1 << 30
-    state = {"free": 60 * gb, "capturing": False}
+    state = {"free": 60 * gb, "unused": 5 * gb, "capturing": False, "asked": 0}
+
+    def ask(i):
+        state["asked"] += 1
+        return state["free"], 100 * gb
+
+    current = lambda n: {"all": {"current": n}}
     monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: state["capturing"])
-    monkeypatch.setattr(torch.cuda, "mem_get_info", lambda i: (state["free"], 100 * gb))
-    monkeypatch.setattr(torch.cuda, "memory_reserved", lambda i: 30 * gb)
-    monkeypatch.setattr(torch.cuda, "memory_allocated", lambda i: 25 * gb)
+    monkeypatch.setattr(torch.cuda, "mem_get_info", ask)
+    monkeypatch.setattr(torch.cuda, "memory_stats_as_nested_dict",
+                        lambda i: {"reserved_bytes": current(25 * gb + state["unused"]), "allocated_bytes": current(25 * gb)})
     monkeypatch.setattr(memory_budget, "_kv_resident", {})
     monkeypatch.setattr(memory_budget, "_kv_awake", {})
-    dev = torch.device("cuda", 0)
-    assert memory_budget.spare_bytes(dev) == 65 * gb - 12 * gb
+    dev, most = torch.device("cuda", 0), 1000 * gb
+    assert memory_budget.spare_bytes(dev, most) == 65 * gb - 12 * gb
+    assert memory_budget.spare_bytes(dev, 3 * gb) == 3 * gb
     memory_budget.set_kv_resident(dev, 40 * gb)               # counted by the driver while it is there ...
     state["free"] = 20 * gb
-    assert memory_budget.spare_bytes(dev) == 25 * gb - 12 * gb
-    memory_budget.set_kv_resident(dev, 0)                     # ... and asleep its place stays its own
+    assert memory_budget.spare_bytes(dev, most) == 25 * gb - 12 * gb
+    memory_budget.set_kv_resident(dev, 0)                     # ... and asleep its place stays its own, given back to the driver
     state["free"] = 60 * gb
-    assert memory_budget.spare_bytes(dev) == 25 * gb - 12 * gb
-    state["free"] = 1 * gb
-    assert memory_budget.spare_bytes(dev) == 0
+    assert memory_budget.spare_bytes(dev, most) == 25 * gb - 12 * gb
+    state.update(free=20 * gb, unused=45 * gb)                # or kept by the caching allocator
+    assert memory_budget.spare_bytes(dev, most) == 25 * gb - 12 * gb
+    state["asked"] = 0
+    assert memory_budget.spare_bytes(dev, 5 * gb) == 5 * gb and state["asked"] == 0
+    state.update(free=1 * gb, unused=5 * gb)
+    assert memory_budget.spare_bytes(dev, most) == 0
     state.update(free=60 * gb, capturing=True)
-    assert memory_budget.spare_bytes(dev) == 0
+    assert memory_budget.spare_bytes(dev, most) == 0
