@@ -25,7 +25,7 @@
 // while one is worked on, because 128 registers hold O.  P*V of block j - 1 is read when S_j is there (it was issued
 // before S_j), so nobody waits for it.  Masks are applied only where a block has any.  Reading O behind every block,
 // masks everywhere, unpacked arithmetic and one CTA per tile took 7200 cycles per pair of blocks (8 x 4096 tokens,
-// 32 / 8 heads: 1.74 ms, 630 TFLOP/s), this 5500 (1.34 ms, 820; 32768 tokens 850 TFLOP/s).  Adding the previous P*V
+// 32 / 8 heads: 1.74 ms, 630 TFLOP/s), this 5500 (1.34 ms, 820; 32768 tokens 860 TFLOP/s).  Adding the previous P*V
 // between the exponentials instead, 16 columns at a time, spilled and took 1.46 ms.  Keeping O in tensor memory
 // behind a reference that lags the maximum took 4300 cycles, but rounds P and O differently from block to block;
 // routers downstream turn such last bits into other experts, so results stay those of the exact running maximum.

@@ -2,8 +2,9 @@
 // tensor memory), operands staged by TMA into a 128-byte-swizzled shared
 // memory ring.  One persistent CTA per SM, three warp roles:
 //   warp 0      TMA producer (one lane)
-//   warp 1      MMA issuer (one lane), owns the TMEM allocation
-//   warps 2..5  epilogue: TMEM -> registers -> global, one accumulator row per thread
+//   warp 1      MMA issuer (the whole warp walks the loop, one elected lane issues), owns the TMEM allocation
+//   warps 2..5  epilogue: TMEM -> registers, one accumulator row per thread; from there to global memory, or in fp32 through
+//               shared memory and TMA (stores, or additions for "+=")
 // Two accumulator buffers in TMEM let the epilogue of tile i overlap the main
 // loop of tile i+1.  Every wait is bounded (see common.cuh).
 //
@@ -471,7 +472,7 @@ static int launch_gemm_as(const CUtensorMap& ta, const CUtensorMap& tb, GemmPara
 }
 
 // The variant that holds the epilogue's code and little else (gate/up of 128 rows, 19456 x 2560: 38 us with the code of all kinds,
-// 32 with its own; 8 rows 40 and 27).  `few`: see GemmCfg; only for those kinds.
+// 32 with its own; 8 rows 40 and 27).  Only these kinds also have the variants of few rows (see GemmCfg).
 static bool own_variant(const GemmParams& p) {
   return ((kF32Epi >> p.epi) & 1u) || ((p.epi == kEpiSwiGLU || p.epi == kEpiBf16) && !p.bias);
 }

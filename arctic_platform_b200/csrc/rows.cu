@@ -2,8 +2,8 @@
 //
 // Bound by memory: the source is read once (16 bytes per thread) and leaves as vector reductions that the L2 carries out, so
 // nothing is sorted, no dense gradient of the table is formed, and rows that nobody names are not touched.  18432 rows of 2560
-// into a 151936-row fp32 embedding gradient: 0.06 ms against 3.6 ms of the sort, the dense bf16 gradient, its fp32 copy
-// and the sum with the accumulated gradient.
+// into a 151936-row fp32 embedding gradient: 0.10 ms (94 MB read, 189 MB added) against 3.6 ms of the sort, the dense bf16 gradient, its
+// fp32 copy and the sum with the accumulated gradient.  Rows that repeat are added in any order: their last bits vary from run to run.
 #include "common.cuh"
 #include "host_utils.cuh"
 

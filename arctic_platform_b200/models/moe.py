@@ -262,7 +262,8 @@ class _GroupedFFNPaddedFn(torch.autograd.Function):
 
 
 def padded_plan_supported(x: torch.Tensor, wgu: torch.Tensor) -> bool:
-    """The padded device-planned path needs the GPU, bf16 and at most 512 experts (one block builds the plan)."""
+    """The padded device-planned path needs the GPU, bf16 and at most 512 experts (the tables are built by a CTA per
+    expert that looks at all counts)."""
     E, I2, H = wgu.shape
     return (x.is_cuda and x.dtype == torch.bfloat16 and E <= 512 and H % 8 == 0 and (I2 // 2) % 8 == 0
             and os.environ.get("APB_MOE_PADDED", "1") != "0")

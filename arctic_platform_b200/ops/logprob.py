@@ -4,7 +4,7 @@
 ``log softmax(hidden @ weight^T * inv_temperature)[label]`` and optionally the entropy
 of that distribution.  On CUDA the forward runs the vocabulary GEMM on tcgen05 with an
 epilogue that reduces every 128-column tile to (max, sum-exp, sum p*logit, label
-logit) partials (``lmhead_logprob.cu``) followed by a small combine kernel; the
+logit) partials (``gemm_common.cuh``) followed by a small combine kernel; the
 backward recomputes logits one row-chunk at a time, forms d(logits) in bf16 and feeds
 two GEMMs (dH and dW).  The reference has three variants of this: full logits then a
 Triton cross-entropy (arctic_platform/common/utils/tiled_logits.py:74-139), chunked
