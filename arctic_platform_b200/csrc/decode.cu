@@ -8,10 +8,9 @@
 // are one contiguous 4 KB tile (D = 128).
 #include "common.cuh"
 #include "host_utils.cuh"
+#include "paged_mma.cuh"
 
 namespace apb {
-
-constexpr int kPage = 16;
 
 // k, v: [T, Hkv, D] (row stride ld elements); slots[t] = page * 16 + offset, or < 0 to skip.
 __global__ void kv_cache_write_kernel(const __nv_bfloat16* __restrict__ k, long long ldk,
@@ -224,50 +223,9 @@ paged_decode_kernel(const __nv_bfloat16* __restrict__ q, const int* __restrict__
 // cluster that joins them through shared memory and writes the normalised result (no partials in memory, no merge launch).
 // ---------------------------------------------------------------------------
 constexpr int kMmaStages = 3;
-constexpr int kMmaPageBytes = kPage * 128 * 2;                    // one K or V page of one head
 constexpr int kMmaWarpBytes = kMmaStages * 2 * kMmaPageBytes;     // K+V ring of one warp
 constexpr int kMmaSmem = 4 * kMmaWarpBytes;                       // 96 KB
 constexpr int kMaxSeqSplits = 4;                                  // parts that one cluster joins
-
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-__device__ __forceinline__ void ldsm_x4(uint32_t addr, uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
-               : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
-               : "r"(addr));
-}
-__device__ __forceinline__ void ldsm_x4_t(uint32_t addr, uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
-               : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
-               : "r"(addr));
-}
-__device__ __forceinline__ void mma_16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
-      "{%0, %1, %2, %3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-
-// One page (K and V, 4 KB each, contiguous in the cache) -> one ring stage; chunk c of row t lands at
-// t * 256 + ((c ^ (t & 7)) * 16) so that the 8 rows of an ldmatrix tile hit 8 different bank groups.
-__device__ __forceinline__ void decode_issue_page(uint32_t stage_addr, const __nv_bfloat16* kpage,
-                                                  const __nv_bfloat16* vpage, int lane) {
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int c = i * 32 + lane;  // 16-byte chunk 0..255 of the page
-    const int t = c >> 4, col = c & 15;
-    const uint32_t off = static_cast<uint32_t>(t * 256 + ((col ^ (t & 7)) << 4));
-    cp_async16(stage_addr + off, reinterpret_cast<const uint8_t*>(kpage) + c * 16);
-    cp_async16(stage_addr + kMmaPageBytes + off, reinterpret_cast<const uint8_t*>(vpage) + c * 16);
-  }
-}
 
 __global__ void __launch_bounds__(kDecThreads)
 paged_decode_mma_kernel(const __nv_bfloat16* __restrict__ q, const int* __restrict__ q_start,

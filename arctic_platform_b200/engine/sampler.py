@@ -38,7 +38,7 @@ from ..ops import _lib, gemm, norm
 from ..ops.attention import AttnLayout, attention_fwd_cuda
 from ..utils.transfer_stats import to_device, to_host
 
-from ..ops.forest_attention import ForestNode, forest_decode_attention, plan_forest
+from ..ops.forest_attention import ForestNode, forest_decode_attention, forest_decode_attention_passes, plan_forest
 
 PAGE = 16
 MIN_HEADER_PAGES = 4      # a common prefix shorter than this many pages is not worth a node of its own
@@ -356,9 +356,12 @@ class SamplerEngine:
         B, dev, c = self.max_batch, self.device, self.cfg
         i32, f32 = dict(device=dev, dtype=torch.int32), dict(device=dev, dtype=torch.float32)
         Hq, D = c.num_heads, c.head_dim
-        # partial results per source: header level, prompt level, private pass
-        self.part_o = [torch.empty((B, Hq, self.splits, D), **f32) for _ in range(3)]
-        self.part_ml = [torch.empty((B, Hq, self.splits, 2), **f32) for _ in range(3)]
+        # partial results per source: header level, prompt level, private pass.  Rows x parts of any call: small batches are cut
+        # into more parts than large ones
+        self._part_rows = max(self.splits * B, 256)
+        self.part_o = [torch.empty((self._part_rows, Hq, D), **f32) for _ in range(3)]
+        self.part_ml = [torch.empty((self._part_rows, Hq, 2), **f32) for _ in range(3)]
+        self.d_arrived = torch.zeros(2 * B * c.num_kv_heads, **i32)      # arrival counters of decode attention
         # fp32 split-K accumulators of the two skinny projections (kept zero between uses by the norm kernel)
         self.acc_o = torch.zeros((B, c.hidden_size), **f32)
         self.acc_d = torch.zeros((B, c.hidden_size), **f32)
@@ -442,19 +445,22 @@ class SamplerEngine:
         c = self.cfg
         scale = 1.0 / math.sqrt(c.head_dim)
         kc, vc = self.kcache[li], self.vcache[li]
+        out = torch.empty((B, c.num_heads, c.head_dim), device=self.device, dtype=torch.bfloat16)
         # per-sequence pass: one CTA per (sequence, kv head) already fills the GPU at rollout batch sizes, so the
         # KV range is split only when there are fewer CTAs than two waves of SMs
         seq_splits = max(1, min(self.splits, 296 // max(1, B * c.num_kv_heads)))
         if os.environ.get("APB_DECODE_SEQ_SPLITS"):               # tuning knob for A/B timing
             seq_splits = max(1, min(self.splits, int(os.environ["APB_DECODE_SEQ_SPLITS"])))
-        out = torch.empty((B, c.num_heads, c.head_dim), device=self.device, dtype=torch.bfloat16)
         if self._cascade_on() and self.n_groups > 0:
             # shared pass: as many KV splits as keep all its CTAs (nodes x KV heads x splits) within one wave of SMs
             nodes = self._group_bucket()
-            node_splits = max(1, min(self.splits, self._sm_count // max(1, nodes * c.num_kv_heads)))
-            return forest_decode_attention(q, kc, vc, self._forest_view(B), self.d_q_start, self.d_active,
-                                           self.d_priv_table, self.d_priv_len, self.part_o, self.part_ml, node_splits,
-                                           seq_splits, scale, out=out, n_nodes=nodes)
+            room = self._sm_count // max(1, nodes * c.num_kv_heads)
+            args = (q, kc, vc, self._forest_view(B), self.d_q_start, self.d_active, self.d_priv_table, self.d_priv_len, self.part_o,
+                    self.part_ml)
+            if c.is_moe:
+                return forest_decode_attention_passes(*args, max(1, min(self.splits, room)), seq_splits, scale, out=out, n_nodes=nodes)
+            return forest_decode_attention(*args, max(1, min(8, self._part_rows // B, room)), max(1, min(64, self._part_rows // B)),
+                                           scale, out=out, n_nodes=nodes, arrived=self.d_arrived)
         s = _lib.stream_ptr()
         if (c.head_dim == 128 and 16 % (c.num_heads // c.num_kv_heads) == 0 and seq_splits != 3
                 and not _lib.cuda_lib().apb_decode_scalar()):
@@ -728,6 +734,8 @@ class SamplerEngine:
         self._filter_on = bool((sp.top_k is not None and sp.top_k > 0) or sp.top_p < 1.0)
         self.d_topk.fill_(int(sp.top_k) if sp.top_k and sp.top_k > 0 else 0)
         self.d_topp.fill_(float(sp.top_p))
+        if getattr(self, "d_arrived", None) is not None:
+            self.d_arrived.zero_()         # a call that an error ended may have left arrivals behind
         prompts_np = [np.asarray(p, dtype=np.int64) for p in prompts]
         for p in prompts_np:
             if len(p) == 0:

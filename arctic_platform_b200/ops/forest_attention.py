@@ -3,9 +3,9 @@
 Sequences that decode together often share long prefixes -- the rollouts of one prompt share the prompt, and prompts
 of one task share a system / few-shot header -- so their KV pages form a forest: header -> prompt -> rollout.  Reading
 every sequence's full context per step re-reads the shared pages once per sequence.  Here every NODE of the forest is
-attended once per step by all sequences below it (``decode_prefix.cu``: their query rows form one 128-row tensor-core
-tile, the node's pages are streamed once), every sequence attends to its private pages by itself
-(``paged_decode_mma_kernel``), and a log-sum-exp merge joins a sequence's levels.  KV traffic per step drops from
+attended once per step by all sequences below it (``decode_attention.cu``: their query rows form one 128-row tensor-core
+tile, the node's pages are streamed once), every sequence attends to its private pages by itself, and a log-sum-exp merge
+joins a sequence's levels -- one launch, in which the last part of a sequence to finish does the merge.  KV traffic per step drops from
 ``sum over sequences of context length`` to ``sum over nodes of node length + private tokens``.
 
 The reference switches the same idea on in its sampler with ``use_fca`` ("forest cascade attention",
@@ -28,6 +28,7 @@ from . import _lib
 
 PAGE = 16
 MAX_SHARED_LEVELS = 3
+OWN_CHUNK = 4              # pages that a warp reads of a sequence's own, at least
 
 _FN = {}
 
@@ -38,6 +39,8 @@ def _fn(name: str):
         vp, i, ll, f = c.c_void_p, c.c_int, c.c_longlong, c.c_float
         _FN["dec"] = _lib.declare("apb_paged_decode_partial", [vp, vp, vp, vp, i, vp, vp, vp, vp, vp, i, i, i, i, i, f, vp])
         _FN["merge"] = _lib.declare("apb_decode_merge", [vp, vp, vp, i, vp, vp, vp, i, i, i, vp])
+        _FN["attn"] = _lib.declare("apb_decode_attention",
+                                   [vp] * 5 + [ll, i, i, i, i, f, i, i, i, vp, vp, vp, i] + [vp] * 8 + [i, vp, i, i, vp, vp, vp])
         _FN["prefix_tc"] = _lib.declare("apb_decode_prefix_tc",
                                         [vp, i, vp, vp, vp, i, vp, vp, vp, vp, ll, vp, vp, i, i, i, i, i, i, f, vp])
     return _FN[name]
@@ -118,18 +121,32 @@ def build_forest_tables(nodes: Sequence[ForestNode], num_slots: int, max_pages: 
     return ForestTables(t(qs), t(qc), t(pg), t(ln), t(lv), t(mask), G, nl, shared, covered)
 
 
+def _check_tables(q, forest: ForestTables, G: int, priv_start, priv_active, priv_table, priv_len, num_pages: int) -> None:
+    from ..utils import checked
+    if checked.active_for(q):
+        B = q.shape[0]
+        if G > 0:
+            checked.check_forest(forest.q_start[:G], forest.q_count[:G], forest.pages[:G], forest.kv_len[:G],
+                                 forest.level[:G], B, num_pages, forest.n_levels, 128, PAGE)
+        checked.check_range("priv_start", priv_start, 0, max(1, B), priv_active)
+        checked.check_page_table("priv_table", priv_table, priv_len, num_pages, PAGE, priv_active)
+
+
 def forest_decode_attention(q: torch.Tensor, kcache: torch.Tensor, vcache: torch.Tensor, forest: ForestTables,
                             priv_start: torch.Tensor, priv_active: torch.Tensor, priv_table: torch.Tensor,
                             priv_len: torch.Tensor, part_o: Sequence[torch.Tensor], part_ml: Sequence[torch.Tensor],
                             splits: int, seq_splits: int, scale: Optional[float] = None,
-                            out: Optional[torch.Tensor] = None, n_nodes: Optional[int] = None) -> torch.Tensor:
+                            out: Optional[torch.Tensor] = None, n_nodes: Optional[int] = None,
+                            arrived: Optional[torch.Tensor] = None, own_chunk: int = OWN_CHUNK) -> torch.Tensor:
     """``q [B, Hq, D]`` bf16 (one token per slot) -> ``[B, Hq, D]`` bf16.
 
     ``kcache / vcache [num_pages, Hkv, 16, D]`` (one layer).  ``forest``: shared nodes.  ``priv_*``: the per-sequence
     pass (``priv_start [B]`` = slot ids, ``priv_active [B]`` = 1 for live slots, ``priv_table [B, max_pages]``,
-    ``priv_len [B]``).  ``part_o[i] [B, Hq, splits, D]`` / ``part_ml[i] [B, Hq, splits, 2]`` fp32 scratch for source
-    ``i`` (shared levels first, the private pass last).  ``n_nodes`` bounds the launch grid (rows of the node tables
-    beyond the live nodes have ``q_count == 0`` and cost an empty CTA)."""
+    ``priv_len [B]``).  ``part_o[i]`` / ``part_ml[i]`` fp32 scratch for source ``i`` (shared levels first, the private pass
+    last): room for ``[B, Hq, splits, D]`` / ``[B, Hq, splits, 2]``, ``seq_splits`` in place of ``splits`` for the private pass,
+    whose pages are read in parts of at least ``own_chunk`` and at most ``seq_splits`` parts.  ``n_nodes`` bounds the launch grid
+    (rows of the node tables beyond the live nodes have ``q_count == 0`` and cost an empty CTA).  ``arrived``: int32 zeros, at
+    least ``2 * B * Hkv`` of them, that a caller keeps for its calls in one stream (they are zeros again after each)."""
     B, Hq, D = q.shape
     Hkv = kcache.shape[1]
     num_pages = kcache.shape[0]
@@ -140,21 +157,42 @@ def forest_decode_attention(q: torch.Tensor, kcache: torch.Tensor, vcache: torch
     G = forest.n_nodes if n_nodes is None else int(n_nodes)
     if out is None:
         out = torch.empty((B, Hq, D), device=q.device, dtype=torch.bfloat16)
-    from ..utils import checked
-    if checked.active_for(q):
-        if G > 0:
-            checked.check_forest(forest.q_start[:G], forest.q_count[:G], forest.pages[:G], forest.kv_len[:G],
-                                 forest.level[:G], B, num_pages, nl, 128, PAGE)
-        checked.check_range("priv_start", priv_start, 0, max(1, B), priv_active)
-        checked.check_page_table("priv_table", priv_table, priv_len, num_pages, PAGE, priv_active)
+    _check_tables(q, forest, G, priv_start, priv_active, priv_table, priv_len, num_pages)
+    if arrived is None:
+        arrived = torch.zeros(2 * B * Hkv, device=q.device, dtype=torch.int32)
+    o_lv = (ctypes.c_void_p * 3)(*[part_o[min(i, nl - 1)].data_ptr() for i in range(3)])
+    ml_lv = (ctypes.c_void_p * 3)(*[part_ml[min(i, nl - 1)].data_ptr() for i in range(3)])
+    _lib.check(_fn("attn")(_lib.ptr(q), _lib.ptr(kcache), _lib.ptr(vcache), _lib.ptr(out), _lib.ptr(arrived), num_pages, B, Hq, Hkv, D,
+                           scale, G, splits, nl, _lib.ptr(forest.q_start), _lib.ptr(forest.q_count), _lib.ptr(forest.pages),
+                           forest.pages.shape[1], _lib.ptr(forest.kv_len), _lib.ptr(forest.level), _lib.ptr(forest.row_mask), o_lv,
+                           ml_lv, _lib.ptr(priv_start), _lib.ptr(priv_active), _lib.ptr(priv_table), max_pages, _lib.ptr(priv_len),
+                           own_chunk, seq_splits, _lib.ptr(part_o[nl]), _lib.ptr(part_ml[nl]), s), "decode_attention")
+    return out
+
+
+def forest_decode_attention_passes(q, kcache, vcache, forest: ForestTables, priv_start, priv_active, priv_table, priv_len, part_o,
+                                   part_ml, splits: int, seq_splits: int, scale: Optional[float] = None,
+                                   out: Optional[torch.Tensor] = None, n_nodes: Optional[int] = None) -> torch.Tensor:
+    """The same attention in three launches (shared nodes, own pages, merge), twice as long and with other last bits: models with
+    experts keep it.  A router turns last bits into other experts now and then, and a greedy rollout behind another expert moves
+    by a fifth."""
+    B, Hq, D = q.shape
+    Hkv = kcache.shape[1]
+    scale = scale if scale is not None else 1.0 / math.sqrt(D)
+    s = _lib.stream_ptr()
+    nl = forest.n_levels
+    G = forest.n_nodes if n_nodes is None else int(n_nodes)
+    if out is None:
+        out = torch.empty((B, Hq, D), device=q.device, dtype=torch.bfloat16)
+    _check_tables(q, forest, G, priv_start, priv_active, priv_table, priv_len, kcache.shape[0])
     if G > 0:
         o_lv = (ctypes.c_void_p * 3)(*[part_o[min(i, nl - 1)].data_ptr() for i in range(3)])
         ml_lv = (ctypes.c_void_p * 3)(*[part_ml[min(i, nl - 1)].data_ptr() for i in range(3)])
         _lib.check(_fn("prefix_tc")(_lib.ptr(q), B, _lib.ptr(forest.q_start), _lib.ptr(forest.q_count),
                                     _lib.ptr(forest.pages), forest.pages.shape[1], _lib.ptr(forest.kv_len),
-                                    _lib.ptr(forest.level), _lib.ptr(kcache), _lib.ptr(vcache), num_pages, o_lv, ml_lv,
+                                    _lib.ptr(forest.level), _lib.ptr(kcache), _lib.ptr(vcache), kcache.shape[0], o_lv, ml_lv,
                                     nl, G, Hq, Hkv, D, splits, scale, s), "decode_prefix_tc")
-    _lib.check(_fn("dec")(_lib.ptr(q), _lib.ptr(priv_start), _lib.ptr(priv_active), _lib.ptr(priv_table), max_pages,
+    _lib.check(_fn("dec")(_lib.ptr(q), _lib.ptr(priv_start), _lib.ptr(priv_active), _lib.ptr(priv_table), priv_table.shape[1],
                           _lib.ptr(priv_len), _lib.ptr(kcache), _lib.ptr(vcache), _lib.ptr(part_o[nl]),
                           _lib.ptr(part_ml[nl]), B, Hq, Hkv, D, seq_splits, scale, s), "paged_decode(private)")
     n_src = nl + 1

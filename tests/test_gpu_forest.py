@@ -110,6 +110,48 @@ def test_three_level_forest_matches_dense_attention(Hq, Hkv):
     assert (out.float() - ref).abs().max().item() < 2e-2
 
 
+@pytest.mark.parametrize("Hq,Hkv,chunk,parts", [(32, 8, 4, 64), (32, 4, 16, 8), (16, 1, 1, 3), (8, 8, 2, 1)])
+def test_own_pages_in_parts_with_and_without_shared_nodes(Hq, Hkv, chunk, parts):
+    """Lengths at the edges of pages and parts, from nothing to more parts than allowed, an inactive entry; the same sequences once by
+    themselves and once below a node that all but one share, whose parts outnumber its blocks.  bf16 probabilities and outputs (2^-9
+    of a value each) against fp32; rows with nothing to see are zeros."""
+    from arctic_platform_b200.ops import _lib
+    from arctic_platform_b200.ops import forest_attention as fa
+    D = 128
+    lens = [0, 1, 15, 16, 17, 16 * chunk, 16 * chunk + 1, 16 * chunk * 2 + 5, 777, 1040, 300, 33]
+    B, dead = len(lens), 9
+    rows = min(B - 1, 128 // (Hq // Hkv))
+    g = torch.Generator(device="cuda").manual_seed(Hq + chunk)
+    max_pages, node_pages = 66, 20
+    kc, vc = (torch.randn((B * max_pages + node_pages, Hkv, PAGE, D), generator=g, device="cuda").bfloat16() for _ in range(2))
+    q = torch.randn((B, Hq, D), generator=g, device="cuda").bfloat16()
+    perm = torch.randperm(B * max_pages, generator=g, device="cuda").to(torch.int32)
+    table = perm.view(B, max_pages).contiguous()
+    node = np.arange(B * max_pages, B * max_pages + node_pages, dtype=np.int32)
+    i32 = dict(device="cuda", dtype=torch.int32)
+    active = torch.ones(B, **i32)
+    active[dead] = 0
+    arrived = torch.zeros(2 * B * Hkv, **i32)
+    for nodes in ([], [fa.ForestNode(0, list(range(rows)), node, node_pages * PAGE - 3)]):
+        forest = fa.build_forest_tables(nodes, B, max_pages, 128 // (Hq // Hkv), "cuda")
+        splits = 9
+        part_o = [torch.full((B, Hq, n, D), float("nan"), device="cuda") for n in (splits, parts)]
+        part_ml = [torch.full((B, Hq, n, 2), float("nan"), device="cuda") for n in (splits, parts)]
+        own = torch.tensor(lens, **i32)
+        for _ in range(2):                 # the second time from the counters that the first has left
+            out = fa.forest_decode_attention(q, kc, vc, forest, torch.arange(B, **i32), active, table, own, part_o, part_ml, splits,
+                                             parts, arrived=arrived, own_chunk=chunk)
+        _lib.check_status("decode attention")
+        assert not arrived.any()
+        shared = [(node, node_pages * PAGE - 3)]
+        ctx = [(shared if nodes and b < rows else []) + ([(table[b].cpu().numpy()[:(n + 15) // 16], n)] if b != dead else [])
+               for b, n in enumerate(lens)]
+        ref = fa.forest_decode_reference(q, kc, vc, ctx)
+        assert torch.isfinite(out.float()).all()
+        err = (out.float() - ref).norm(dim=-1)
+        assert (err <= 2 ** -7 * ref.norm(dim=-1)).all()
+
+
 def test_engine_discovers_shared_headers_and_samples_the_same_distribution():
     """Prompts that start with the same tokens are stored and attended through one header node.  Greedy generation with
     the forest equals greedy generation with plain per-sequence decoding, and the reported log-probs match a
