@@ -82,6 +82,13 @@ class SamplingParams:
         return sp
 
 
+_I32P = ctypes.POINTER(ctypes.c_int32)
+
+
+def _i32_ptr(a: np.ndarray):
+    return ctypes.cast(a.__array_interface__["data"][0], _I32P)
+
+
 class PageAllocator:
     """Reference-counted KV pages (C++ runtime, ``runtime.cpp``)."""
 
@@ -97,19 +104,19 @@ class PageAllocator:
         out = np.empty(max(n, 1), dtype=np.int32)
         if n == 0:
             return out[:0]
-        rc = self.rt.apb_rt_pages_alloc(self.h, n, out.ctypes.data_as(ctypes.POINTER(ctypes.c_int32)))
+        rc = self.rt.apb_rt_pages_alloc(self.h, n, _i32_ptr(out))
         return out[:n] if rc == 0 else None
 
     def retain(self, pages: np.ndarray) -> None:
         if len(pages):
             p = np.ascontiguousarray(pages, dtype=np.int32)
-            if self.rt.apb_rt_pages_retain(self.h, len(p), p.ctypes.data_as(ctypes.POINTER(ctypes.c_int32))) != 0:
+            if self.rt.apb_rt_pages_retain(self.h, len(p), _i32_ptr(p)) != 0:
                 raise RuntimeError("retain of a page that is not allocated")
 
     def release(self, pages: np.ndarray) -> None:
         if len(pages):
             p = np.ascontiguousarray(pages, dtype=np.int32)
-            if self.rt.apb_rt_pages_release(self.h, len(p), p.ctypes.data_as(ctypes.POINTER(ctypes.c_int32))) < 0:
+            if self.rt.apb_rt_pages_release(self.h, len(p), _i32_ptr(p)) < 0:
                 raise RuntimeError("release of a page that is not allocated")
 
     def __del__(self):
@@ -326,12 +333,12 @@ class SamplerEngine:
         # prefix forest (cascade): one table row per run of consecutive slots under a shared node; a sequence sits
         # under at most two shared nodes (header, prompt), so 2 * B rows always suffice
         self.n_node_rows = 2 * B
-        self.d_g_start = torch.zeros(self.n_node_rows, **i32)
-        self.d_g_count = torch.zeros(self.n_node_rows, **i32)
-        self.d_g_pages = torch.zeros((self.n_node_rows, self.max_pages), **i32)
-        self.d_g_len = torch.zeros(self.n_node_rows, **i32)
-        self.d_g_level = torch.zeros(self.n_node_rows, **i32)
-        self.d_row_mask = torch.full((B,), 1, **i32)
+        # ... in one buffer, so that a change of the forest is one copy
+        N = self.n_node_rows
+        self.d_forest = torch.zeros(B + N * (4 + self.max_pages), **i32)
+        self.d_row_mask = self.d_forest[:B].fill_(1)
+        self.d_g_start, self.d_g_count, self.d_g_len, self.d_g_level = self.d_forest[B:B + 4 * N].view(4, N)
+        self.d_g_pages = self.d_forest[B + 4 * N:].view(N, self.max_pages)
         self.n_levels = 1            # shared levels in use: 1 = prompt nodes only, 2 = header + prompt nodes
         self.forest_stats = {"shared_tokens": 0, "covered_tokens": 0}
         self.out_cap = 0
@@ -375,11 +382,12 @@ class SamplerEngine:
 
     # ------------------------------------------------------------------ layers (no autograd)
     @torch.no_grad()
-    def _block(self, li: int, x, stream, positions, slots, attn_fn):
+    def _block(self, li: int, x, stream, positions, slots, attn_fn, rows=None):
+        """One layer; with ``rows`` only these rows go on behind its attention."""
         c = self.cfg
         blk = self.model.blocks[li]
         if self.fp8:
-            return self._block_fp8(li, x, stream, positions, slots, attn_fn)
+            return self._block_fp8(li, x, stream, positions, slots, attn_fn, rows)
         h, stream = norm.rmsnorm(x, blk.ln1, c.rms_norm_eps, stream)
         qkv = gemm.matmul_nt(h, blk.wqkv)
         q, k, v = norm.qknorm_rope(qkv, blk.q_norm, blk.k_norm, *self.model.rope(self.device), positions, c.num_heads,
@@ -388,6 +396,8 @@ class SamplerEngine:
                               _lib.ptr(self.kcache[li]), _lib.ptr(self.vcache[li]), k.shape[0], c.num_kv_heads,
                               c.head_dim, _lib.stream_ptr()), "kv_cache_write")
         a = attn_fn(li, q, k, v)
+        if rows is not None:
+            a, stream = a.index_select(0, rows), stream.index_select(0, rows)
         o = self._tp_sum(gemm.matmul_nt(a.reshape(a.shape[0], -1), blk.wo))
         h2, stream = norm.rmsnorm(o, blk.ln2, c.rms_norm_eps, stream)
         if blk.mlp is not None:
@@ -421,7 +431,7 @@ class SamplerEngine:
         self._fp8_stale = False
 
     @torch.no_grad()
-    def _block_fp8(self, li: int, x, stream, positions, slots, attn_fn):
+    def _block_fp8(self, li: int, x, stream, positions, slots, attn_fn, rows=None):
         from ..ops.fp8 import fp8_linear
         c = self.cfg
         blk = self.model.blocks[li]
@@ -434,6 +444,8 @@ class SamplerEngine:
                               _lib.ptr(self.kcache[li]), _lib.ptr(self.vcache[li]), k.shape[0], c.num_kv_heads,
                               c.head_dim, _lib.stream_ptr()), "kv_cache_write")
         a = attn_fn(li, q, k, v)
+        if rows is not None:
+            a, stream = a.index_select(0, rows), stream.index_select(0, rows)
         o = self._tp_sum(fp8_linear(a.reshape(a.shape[0], -1).contiguous(), *w["wo"]))
         h2, stream = norm.rmsnorm(o, blk.ln2, c.rms_norm_eps, stream)
         act = norm.swiglu(fp8_linear(h2, *w["wgu"]))
@@ -768,6 +780,7 @@ class SamplerEngine:
         group_members: Dict[int, List[int]] = {}
         root_members: Dict[int, List[int]] = {}
         next_group = next_root = 0
+        retired = False
         while queue or live:
             # ---- admission: as many whole runs as fit in slots and pages
             admitted: List[dict] = []
@@ -812,17 +825,17 @@ class SamplerEngine:
                         # into other experts, so models with experts keep the shared pass
                         n_full, priv_pages = 0, n_full + priv_pages
                     shared = self.pages.alloc(n_full)
+                    own = self.pages.alloc(sp.n * priv_pages)
+                    self.pages.retain(np.tile(shared, sp.n - 1))
+                    # every sequence below the header holds a reference
+                    self.pages.retain(np.tile(header, sp.n - int(first_of_run)))
+                    first_of_run = False
                     gid = next_group
                     next_group += 1
                     mem = []
                     for si in range(sp.n):
                         slot = slots_free.pop(0)
-                        priv = self.pages.alloc(priv_pages)
-                        if si > 0:
-                            self.pages.retain(shared)
-                        if not first_of_run:
-                            self.pages.retain(header)          # every sequence below the header holds a reference
-                        first_of_run = False
+                        priv = own[si * priv_pages:(si + 1) * priv_pages]
                         live[slot] = _Seq(req=r, sample=si, prompt_len=P, max_new=sp.max_tokens, shared_pages=shared,
                                           private_pages=priv, group=gid, header_pages=header, root=rid)
                         mem.append(slot)
@@ -840,12 +853,16 @@ class SamplerEngine:
             bucket = next((b for b in (8, 16, 32, 64, 128, 256, 512, 1024) if b >= B), self.max_batch)
             bucket = min(bucket, self.max_batch)
             if B > 0:
-                self._set_groups(group_members, root_members, live)
+                if admitted or retired:
+                    self._set_groups(group_members, root_members, live)
                 self._run_steps(bucket, self.sync_interval)
             # ---- harvest
             fin = to_host(self.d_finished[:max(B, 1)]).numpy() if B else np.zeros(0, dtype=np.int32)
             done_slots = [s for s in list(live) if fin[s]]
+            retired = bool(done_slots)
             if done_slots:
+                done_t = self._upload(np.asarray(done_slots, dtype=np.int64))
+                freed: List[np.ndarray] = []
                 nout = to_host(self.d_out_idx[:B, 0]).numpy()
                 toks = to_host(self.d_out_tokens[:B]).numpy()
                 lps = to_host(self.d_out_lps[:B]).numpy()
@@ -857,9 +874,7 @@ class SamplerEngine:
                     results[sq.req * sp.n + sq.sample] = {
                         "token_ids": out, "logprobs": lps[s, :k].tolist(), "finish_reason": reason,
                         "prompt_len": sq.prompt_len, "prompt_index": sq.req, "text": None}
-                    self.pages.release(sq.private_pages)
-                    self.pages.release(sq.shared_pages)
-                    self.pages.release(sq.header_pages)
+                    freed += (sq.private_pages, sq.shared_pages, sq.header_pages)
                     group_members[sq.group].remove(s)
                     if not group_members[sq.group]:
                         del group_members[sq.group]
@@ -868,9 +883,9 @@ class SamplerEngine:
                         if not root_members[sq.root]:
                             del root_members[sq.root]
                     slots_free.append(s)
-                    self.d_finished[s] = 0
-                    self.d_len[s] = 0
-                    self.d_priv_len[s] = 0
+                self.pages.release(np.concatenate(freed))
+                for state in (self.d_finished, self.d_len, self.d_priv_len):
+                    state.index_fill_(0, done_t, 0)
         return results  # type: ignore[return-value]
 
     # ------------------------------------------------------------------ admission
@@ -914,7 +929,7 @@ class SamplerEngine:
         """Packs the admitted runs -- every header once, then every prompt's remainder with the header as its fully
         visible prefix -- runs the model over them, fills the KV pages and returns the final-norm hidden state of
         every prompt's last token, in the order of ``runs[*]["prompts"]``."""
-        toks, pos, slots, segs, last = [], [], [], [], []
+        toks, pos, slots, segs, last, tails = [], [], [], [], [], []
         t = 0
 
         def put(tokens: np.ndarray, p0: int, pages: np.ndarray):
@@ -938,26 +953,36 @@ class SamplerEngine:
                 pages = np.concatenate([s0.shared_pages, s0.private_pages])
                 q0 = t
                 put(rem, hlen, pages.astype(np.int64))
+                tails.append(len(segs))
                 segs.append((q0, len(rem), hstart if hlen else 0, hlen, q0, len(rem)))
                 last.append(t - 1)
-        ids = to_device(torch.from_numpy(np.concatenate(toks).astype(np.int64)), self.device)
-        positions = to_device(torch.from_numpy(np.concatenate(pos)), self.device)
-        slot_t = to_device(torch.from_numpy(np.concatenate(slots)), self.device)
+        blob = self._upload(np.concatenate([np.concatenate(toks), np.asarray(last, dtype=np.int64)]))
+        ids, last_t = blob[:t], blob[t:]
+        positions, slot_t = self._upload(np.concatenate(pos + slots)).view(2, t)
         layout = AttnLayout(np.asarray(segs, dtype=np.int32), t)
+        # only the last token of a prompt leaves the last layer: of the others its keys and values are wanted.  (Products of few rows
+        # may end in other last bits; behind routers those of models with experts have to stay.)
+        short = not self.cfg.is_moe
+        ends = [(at, 1, ps, pl, q0, ql) for at, (q0, ql, ps, pl, _, _) in zip(last, [segs[i] for i in tails])]
+        end_layout = AttnLayout(np.asarray(ends, dtype=np.int32), t)
         scale = 1.0 / math.sqrt(self.cfg.head_dim)
+        n_layers = self.cfg.num_layers
+        if self.device.type == "cuda":
+            for lay in (layout, end_layout)[:1 + int(short)]:      # work tables: their copies wait for the stream, which is idle here
+                lay.fwd_work(self.cfg.num_heads, self.cfg.num_kv_heads, ids.device)
 
         def attn(li, q, k, v):
-            o, _ = attention_fwd_cuda(q, k, v.contiguous() if v.stride(1) != v.shape[2] else v, layout, scale,
-                                      need_lse=False)
+            o, _ = attention_fwd_cuda(q, k, v.contiguous() if v.stride(1) != v.shape[2] else v,
+                                      end_layout if short and li + 1 == n_layers else layout, scale, need_lse=False)
             return o
 
         x = torch.nn.functional.embedding(ids, self.model.embed)
         stream = None
-        for li in range(self.cfg.num_layers):
-            x, stream = self._block(li, x, stream, positions, slot_t, attn)
-        last_t = to_device(torch.from_numpy(np.asarray(last, dtype=np.int64)), self.device)
-        h, _ = norm.rmsnorm(x.index_select(0, last_t), self.model.final_norm, self.cfg.rms_norm_eps,
-                            stream.index_select(0, last_t))
+        for li in range(n_layers):
+            x, stream = self._block(li, x, stream, positions, slot_t, attn, last_t if short and li + 1 == n_layers else None)
+        if not short:
+            x, stream = x.index_select(0, last_t), stream.index_select(0, last_t)
+        h, _ = norm.rmsnorm(x, self.model.final_norm, self.cfg.rms_norm_eps, stream)
         return h
 
     @torch.no_grad()
@@ -978,7 +1003,10 @@ class SamplerEngine:
             tok += n_tok
         for runs in batches:
             batch = [pm for run in runs for pm in run["prompts"]]
-            h = self._prefill_runs(runs, prompts_np, live)
+            # all that the host knows goes up before the prompts run, and nothing behind them makes it wait
+            rows = [gi for gi, (_, mem) in enumerate(batch) for _ in mem]
+            slots = [slot for _, mem in batch for slot in mem]
+            n = len(slots)
             # tail page copies for rollouts 1..n-1
             src, dst = [], []
             for gid, mem in batch:
@@ -987,15 +1015,36 @@ class SamplerEngine:
                     for slot in mem[1:]:
                         src.append(int(s0.private_pages[0]))
                         dst.append(int(live[slot].private_pages[0]))
+            pt = np.zeros((n, self.max_pages), dtype=np.int32)
+            pv = np.zeros((n, self.max_pages), dtype=np.int32)
+            plen = np.zeros(n, dtype=np.int32)
+            sh = np.zeros(n, dtype=np.int32)
+            for i, s in enumerate(slots):
+                sq = live[s]
+                n_hdr, n_sh, n_priv = len(sq.header_pages), len(sq.shared_pages), len(sq.private_pages)
+                pt[i, :n_hdr] = sq.header_pages
+                pt[i, n_hdr:n_hdr + n_sh] = sq.shared_pages
+                pt[i, n_hdr + n_sh:n_hdr + n_sh + n_priv] = sq.private_pages
+                pv[i, :n_priv] = sq.private_pages
+                sh[i] = (n_hdr + n_sh) * PAGE
+                plen[i] = sq.prompt_len - sh[i] + 1
+            from ..utils import checked
+            if checked.enabled():                   # host arrays: no synchronisation involved
+                checked.check_page_table("page_table", pt, plen + sh - 1, self.num_pages, PAGE)
+                checked.check_page_table("priv_table", pv, plen - 1, self.num_pages, PAGE)
+            longs = self._upload(np.asarray(rows + slots + src + dst, dtype=np.int64))
+            rows_t, st, src_t, dst_t = longs.split([n, n, len(src), len(src)])
+            ints = self._upload(np.concatenate([pt.reshape(-1), pv.reshape(-1), plen, sh,
+                                                np.asarray([live[s].prompt_len for s in slots], dtype=np.int32)]))
+            wide = n * self.max_pages
+            pt_t, pv_t, plen_t, sh_t, P_t = ints.split([wide, wide, n, n, n])
+            h = self._prefill_runs(runs, prompts_np, live)
             if src:
-                self._copy_pages(torch.tensor(src, device=self.device), torch.tensor(dst, device=self.device))
+                self._copy_pages(src_t, dst_t)
             self._fork_slots([(mem[0], mem[1:]) for _, mem in batch if len(mem) > 1])
             # first token of every rollout
-            rows = [gi for gi, (_, mem) in enumerate(batch) for _ in mem]
-            slots = [slot for _, mem in batch for slot in mem]
-            hrep = h.index_select(0, torch.tensor(rows, device=self.device))
+            hrep = h.index_select(0, rows_t)
             logits = self._output_logits(hrep.contiguous())
-            n = len(slots)
             temp = torch.full((n,), float(sp.temperature), device=self.device, dtype=torch.float32)
             tok0 = torch.empty(n, device=self.device, dtype=torch.int32)
             lp0 = torch.empty(n, device=self.device, dtype=torch.float32)
@@ -1011,8 +1060,6 @@ class SamplerEngine:
                 _lib.check(_fn("sample")(_lib.ptr(logits), logits.stride(0), _lib.ptr(temp), n, c.vocab_size, seed0,
                                          _lib.ptr(self.d_step), _lib.ptr(tok0), _lib.ptr(lp0), _lib.stream_ptr()), "sample")
             self.d_step += 1
-            st = torch.tensor(slots, device=self.device, dtype=torch.long)
-            P_t = torch.tensor([live[s].prompt_len for s in slots], device=self.device, dtype=torch.int32)
             stop_hit = (tok0[:, None] == self.d_stop[None, :]).any(1)
             fin = stop_hit | (sp.max_tokens <= 1)
             self.d_tokens[st] = tok0
@@ -1025,25 +1072,10 @@ class SamplerEngine:
             self.d_out_tokens[st, 0] = tok0
             self.d_out_lps[st, 0] = lp0
             self.d_out_idx[st, 0] = 1
-            pt = np.zeros((n, self.max_pages), dtype=np.int32)
-            pv = np.zeros((n, self.max_pages), dtype=np.int32)
-            plen = np.zeros(n, dtype=np.int32)
-            sh = np.zeros(n, dtype=np.int32)
-            for i, s in enumerate(slots):
-                sq = live[s]
-                allp = np.concatenate([sq.header_pages, sq.shared_pages, sq.private_pages])
-                pt[i, :len(allp)] = allp
-                pv[i, :len(sq.private_pages)] = sq.private_pages
-                sh[i] = (len(sq.header_pages) + len(sq.shared_pages)) * PAGE
-                plen[i] = sq.prompt_len - sh[i] + 1
-            from ..utils import checked
-            if checked.enabled():                   # host arrays: no synchronisation involved
-                checked.check_page_table("page_table", pt, plen + sh - 1, self.num_pages, PAGE)
-                checked.check_page_table("priv_table", pv, plen - 1, self.num_pages, PAGE)
-            self.d_page_table[st] = to_device(torch.from_numpy(pt), self.device)
-            self.d_priv_table[st] = to_device(torch.from_numpy(pv), self.device)
-            self.d_priv_len[st] = to_device(torch.from_numpy(plen), self.device)
-            self.d_shared_tokens[st] = to_device(torch.from_numpy(sh), self.device)
+            self.d_page_table[st] = pt_t.view(n, -1)
+            self.d_priv_table[st] = pv_t.view(n, -1)
+            self.d_priv_len[st] = plen_t
+            self.d_shared_tokens[st] = sh_t
 
     def _copy_pages(self, src: torch.Tensor, dst: torch.Tensor) -> None:
         """Copies KV pages (a prompt's partial last page to every rollout) in all layers."""
@@ -1076,15 +1108,19 @@ class SamplerEngine:
         self.n_groups, self.n_levels = G, nl
         self.forest_stats = {"shared_tokens": shared, "covered_tokens": covered}
 
-        def fill(dst: torch.Tensor, arr: np.ndarray):
-            buf = np.zeros(tuple(dst.shape), dtype=arr.dtype)
-            buf[:len(arr)] = arr[:len(buf)]
-            dst.copy_(to_device(torch.from_numpy(buf), self.device))
+        B, N = self.max_batch, self.n_node_rows
+        head = B + 4 * N
+        blob = np.zeros(head + G * self.max_pages, dtype=np.int32)      # pages of the rows in use
+        blob[:B] = mask
+        for i, arr in enumerate((qs, qc, ln, lv)):
+            blob[B + i * N:B + i * N + G] = arr[:G]
+        blob[head:] = pg[:G].reshape(-1)
+        self.d_forest[:len(blob)].copy_(self._upload(blob))
 
-        for dst, arr in ((self.d_g_start, qs), (self.d_g_count, qc), (self.d_g_len, ln), (self.d_g_level, lv),
-                         (self.d_g_pages, pg)):
-            fill(dst, arr)
-        self.d_row_mask.copy_(to_device(torch.from_numpy(mask), self.device))
+    def _upload(self, a: np.ndarray) -> torch.Tensor:
+        """A host array on the device.  The copy is staged at once and the host does not wait for the work queued in front of it
+        (``torch.tensor(..., device=...)`` and stores of single elements do)."""
+        return to_device(torch.from_numpy(a), self.device)
 
     # ------------------------------------------------------------------ weights / sleep / wake
     @torch.no_grad()
