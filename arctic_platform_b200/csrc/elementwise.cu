@@ -27,6 +27,19 @@ __device__ __forceinline__ void store8(__nv_bfloat16* p, const float (&f)[8]) {
   *reinterpret_cast<Bf16x8*>(p) = r;
 }
 
+__device__ __forceinline__ void unpack8(const uint4& r, float (&f)[8]) {
+  const uint32_t w[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 t = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[i]));
+    f[2 * i] = t.x;
+    f[2 * i + 1] = t.y;
+  }
+}
+__device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
+  return make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
+}
+
 template <int THREADS>
 __device__ __forceinline__ float block_sum(float v, float* scratch) {
   v = warp_sum(v);
@@ -45,6 +58,9 @@ __device__ __forceinline__ float block_sum(float v, float* scratch) {
 constexpr int kNormThreads = 256;
 constexpr int kNormMaxVec = 4;  // H <= 256 * 8 * 4 = 8192
 
+// A block has a row at a time; the next one's loads are on their way while it is reduced (18432 rows of 2560 with a residual, 377 MB:
+// 95 us when each row's loads waited for the row before, 78 now).  NV: 16-byte vectors of a row per thread.
+template <int NV>
 __global__ void __launch_bounds__(kNormThreads)
 rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res,
                    const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
@@ -53,12 +69,25 @@ rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
   pdl_entry();
   __shared__ float scratch[32];
   const int nvec = H / 8;
+  uint4 nx[NV], nr[NV];
+  auto request = [&](int row) {
+    const size_t base = static_cast<size_t>(row) * H;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int v = threadIdx.x + i * kNormThreads;
+      if (row < T && v < nvec) {
+        if (!x_f32) nx[i] = *reinterpret_cast<const uint4*>(x + base + v * 8);
+        if (res) nr[i] = *reinterpret_cast<const uint4*>(res + base + v * 8);
+      }
+    }
+  };
+  request(blockIdx.x);
   for (int row = blockIdx.x; row < T; row += gridDim.x) {
     const size_t base = static_cast<size_t>(row) * H;
-    float vals[kNormMaxVec][8];
+    float vals[NV][8];
     float ss = 0.f;
 #pragma unroll
-    for (int i = 0; i < kNormMaxVec; ++i) {
+    for (int i = 0; i < NV; ++i) {
       const int v = threadIdx.x + i * kNormThreads;
       if (v < nvec) {
         if (x_f32) {
@@ -70,29 +99,31 @@ rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
           xp[0] = make_float4(0.f, 0.f, 0.f, 0.f);
           xp[1] = make_float4(0.f, 0.f, 0.f, 0.f);
         } else {
-          load8(x + base + v * 8, vals[i]);
+          unpack8(nx[i], vals[i]);
         }
         if (res) {
           float r[8];
-          load8(res + base + v * 8, r);
+          unpack8(nr[i], r);
 #pragma unroll
           for (int j = 0; j < 8; ++j) vals[i][j] += r[j];
         }
         if (res_out) {
-          store8(res_out + base + v * 8, vals[i]);
           // the normalised value is computed from the rounded residual so that
           // forward and backward see the same stream
-          load8(res_out + base + v * 8, vals[i]);
+          const uint4 rounded = pack8(vals[i]);
+          *reinterpret_cast<uint4*>(res_out + base + v * 8) = rounded;
+          unpack8(rounded, vals[i]);
         }
 #pragma unroll
         for (int j = 0; j < 8; ++j) ss += vals[i][j] * vals[i][j];
       }
     }
+    request(row + gridDim.x);
     ss = block_sum<kNormThreads>(ss, scratch);
     const float rstd = rsqrtf(ss / H + eps);
     if (threadIdx.x == 0 && rstd_out) rstd_out[row] = rstd;
 #pragma unroll
-    for (int i = 0; i < kNormMaxVec; ++i) {
+    for (int i = 0; i < NV; ++i) {
       const int v = threadIdx.x + i * kNormThreads;
       if (v < nvec) {
         float wv[8], o[8];
@@ -107,6 +138,7 @@ rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
 
 // dx = rstd * (g - xhat * mean(g * xhat)) [+ dres], g = dy * w ; dw += sum_t dy * xhat
 // NV = 8-element vectors per thread (registers scale with it, so narrow rows keep more CTAs per SM).
+// The next row's loads are on their way while a row is reduced (18432 rows of 2560, 377 MB: 137 us without, 84 with).
 template <int NV>
 __global__ void __launch_bounds__(kNormThreads, NV <= 1 ? 3 : (NV <= 2 ? 2 : 1))
 rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
@@ -131,21 +163,37 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
       for (int j = 0; j < 8; ++j) wv[i][j] += w_offset;
     }
   }
+  uint4 nd[NV], nx[NV], nr[NV];
+  float n_rstd = 0.f;
+  auto request = [&](int row) {
+    if (row >= T) return;
+    const size_t base = static_cast<size_t>(row) * H;
+    n_rstd = rstd_in[row];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int v = threadIdx.x + i * kNormThreads;
+      if (v < nvec) {
+        nd[i] = *reinterpret_cast<const uint4*>(dy + base + v * 8);
+        nx[i] = *reinterpret_cast<const uint4*>(x + base + v * 8);
+        if (dres) nr[i] = *reinterpret_cast<const uint4*>(dres + base + v * 8);
+      }
+    }
+  };
+  request(blockIdx.x);
   for (int row = blockIdx.x; row < T; row += gridDim.x) {
     const size_t base = static_cast<size_t>(row) * H;
-    const float rstd = rstd_in[row];
-    float g[kNormMaxVec][8], xh[kNormMaxVec][8], rr[kNormMaxVec][8];
+    const float rstd = n_rstd;
+    float g[kNormMaxVec][8], xh[kNormMaxVec][8];
+    uint4 rr[kNormMaxVec];
     float dot = 0.f;
-    // all three inputs of the row are requested before the block-wide reduction: the upstream residual gradient
-    // used to be loaded after it, a second full memory latency per row
 #pragma unroll
     for (int i = 0; i < kNormMaxVec; ++i) {
       const int v = threadIdx.x + i * kNormThreads;
       if (v < nvec) {
         float d[8];
-        load8(dy + base + v * 8, d);
-        load8(x + base + v * 8, xh[i]);
-        if (dres) load8(dres + base + v * 8, rr[i]);
+        unpack8(nd[i], d);
+        unpack8(nx[i], xh[i]);
+        rr[i] = nr[i];
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           xh[i][j] *= rstd;
@@ -155,14 +203,16 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
         }
       }
     }
+    request(row + gridDim.x);
     dot = block_sum<kNormThreads>(dot, scratch) / H;
 #pragma unroll
     for (int i = 0; i < kNormMaxVec; ++i) {
       const int v = threadIdx.x + i * kNormThreads;
       if (v < nvec) {
-        float o[8];
+        float o[8], r[8];
+        unpack8(rr[i], r);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] = rstd * (g[i][j] - xh[i][j] * dot) + (dres ? rr[i][j] : 0.f);
+        for (int j = 0; j < 8; ++j) o[j] = rstd * (g[i][j] - xh[i][j] * dot) + (dres ? r[j] : 0.f);
         store8(dx + base + v * 8, o);
       }
     }
@@ -225,60 +275,97 @@ __device__ __forceinline__ void store_vec(__nv_bfloat16* p, const float (&v)[N])
 // the first `rot` dims with cos/sin tables [max_pos, rot/2] fp32.
 // Input rows: qkv[t] = [q heads | k heads | v heads]; outputs q_out[T,Hq,D],
 // k_out[T,Hkv,D].  wq/wk may be null (no per-head norm, rstd := 1).
-template <int D>
+// D / 16 lanes share one (token, head) and have 8 elements of each half of it, 16 bytes a load, as in the backward below.  Squares are
+// summed in the order that a warp per head summed them (two elements of each half a lane, then lanes 16, 8, 4, 2 and 1 apart), and
+// what is fused into one rounding is written out, so results keep the bits that routers downstream decide by.  18432 tokens, 32 + 8 heads of 128, 377 MB: 163 us with a warp per head and its 4-byte loads, 98 now.
+// ALIGNED: rows, weights and tables begin on 16-byte boundaries; otherwise element by element.
+template <int D, bool ALIGNED>
 __global__ void __launch_bounds__(256)
 qknorm_rope_fwd_kernel(const __nv_bfloat16* __restrict__ qkv, long long ld_qkv,
                        const __nv_bfloat16* __restrict__ wq, const __nv_bfloat16* __restrict__ wk,
                        const float* __restrict__ cos_t, const float* __restrict__ sin_t,
                        const int* __restrict__ pos, __nv_bfloat16* __restrict__ q_out,
                        __nv_bfloat16* __restrict__ k_out, int T, int Hq, int Hkv, int rot, float eps) {
-  constexpr int E = D / 32;  // elements per lane
-  const int lane = threadIdx.x & 31;
-  const long long gw = (blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) >> 5;
+  constexpr int LPI = D / 16;          // lanes per item
+  constexpr int IPW = 32 / LPI;        // items per warp
+  constexpr int E2 = D / 64;           // elements of a half that a lane of a whole warp would have
+  constexpr int OLD = 8 / E2;          // such lanes that a lane stands for
+  const int lane = threadIdx.x & 31, sub = lane % LPI;
   const int heads = Hq + Hkv;
-  if (gw >= static_cast<long long>(T) * heads) return;
-  const int t = static_cast<int>(gw / heads);
-  const int h = static_cast<int>(gw % heads);
+  const long long items = static_cast<long long>(T) * heads;
+  const long long it = ((blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) >> 5) * IPW + lane / LPI;
+  const bool valid = it < items;                       // the shuffles below need every lane of the warp
+  const long long itc = valid ? it : items - 1;
+  const int t = static_cast<int>(itc / heads);
+  const int h = static_cast<int>(itc - static_cast<long long>(t) * heads);
   const bool is_q = h < Hq;
   const __nv_bfloat16* src = qkv + t * ld_qkv + static_cast<long long>(h) * D;
   const __nv_bfloat16* w = is_q ? wq : wk;
   __nv_bfloat16* dst = is_q ? q_out + (static_cast<long long>(t) * Hq + h) * D
                             : k_out + (static_cast<long long>(t) * Hkv + (h - Hq)) * D;
-  // lane owns elements [lane*E/2 .. ) of the first half and the matching ones of the second half,
-  // so a rotate-half pair (i, i + D/2) sits in one lane.
-  constexpr int E2 = E / 2;
-  float a[E2], b[E2];
+  auto load = [](const __nv_bfloat16* from, float (&to)[8]) {
+    if constexpr (ALIGNED) {
+      load8(from, to);
+    } else {
 #pragma unroll
-  for (int j = 0; j < E2; ++j) {
-    a[j] = __bfloat162float(src[lane * E2 + j]);
-    b[j] = __bfloat162float(src[D / 2 + lane * E2 + j]);
-  }
-  float rstd = 1.f;
-  if (w) {
+      for (int j = 0; j < 8; ++j) to[j] = __bfloat162float(from[j]);
+    }
+  };
+  auto loadf = [](const float* from, float (&to)[8]) {
+    if constexpr (ALIGNED) {
+      *reinterpret_cast<float4*>(to) = *reinterpret_cast<const float4*>(from);
+      *reinterpret_cast<float4*>(to + 4) = *reinterpret_cast<const float4*>(from + 4);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) to[j] = from[j];
+    }
+  };
+  float a[8], b[8];
+  load(src + sub * 8, a);
+  load(src + D / 2 + sub * 8, b);
+  const bool norm = w != nullptr;
+  float part[OLD];
+#pragma unroll
+  for (int r = 0; r < OLD; ++r) {
     float ss = 0.f;
 #pragma unroll
-    for (int j = 0; j < E2; ++j) ss += a[j] * a[j] + b[j] * b[j];
-    ss = warp_sum(ss);
-    rstd = rsqrtf(ss / D + eps);
+    for (int j = r * E2; j < (r + 1) * E2; ++j) ss = __fadd_rn(ss, __fmaf_rn(a[j], a[j], __fmul_rn(b[j], b[j])));
+    part[r] = ss;
+  }
 #pragma unroll
-    for (int j = 0; j < E2; ++j) {
-      a[j] *= rstd * __bfloat162float(w[lane * E2 + j]);
-      b[j] *= rstd * __bfloat162float(w[D / 2 + lane * E2 + j]);
+  for (int o = LPI / 2; o > 0; o >>= 1)
+#pragma unroll
+    for (int r = 0; r < OLD; ++r) part[r] += __shfl_xor_sync(0xffffffffu, part[r], o);
+#pragma unroll
+  for (int o = OLD / 2; o > 0; o >>= 1)
+#pragma unroll
+    for (int r = 0; r < o; ++r) part[r] += part[r + o];
+  if (norm) {
+    const float rstd = rsqrtf(part[0] / D + eps);
+    float wa[8], wb[8];
+    load(w + sub * 8, wa);
+    load(w + D / 2 + sub * 8, wb);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      a[j] = __fmul_rn(a[j], __fmul_rn(rstd, wa[j]));
+      b[j] = __fmul_rn(b[j], __fmul_rn(rstd, wb[j]));
     }
   }
-  const int p = pos[t];
-  const int half = rot / 2;
+  if (rot == D) {
+    const long long at = static_cast<long long>(pos[t]) * (D / 2) + sub * 8;
+    alignas(16) float cs[8], sn[8];
+    loadf(cos_t + at, cs);
+    loadf(sin_t + at, sn);
 #pragma unroll
-  for (int j = 0; j < E2; ++j) {
-    const int i = lane * E2 + j;  // index inside the first half of the head
-    float oa = a[j], ob = b[j];
-    if (rot == D) {
-      const float c = cos_t[static_cast<long long>(p) * half + i], s = sin_t[static_cast<long long>(p) * half + i];
-      oa = a[j] * c - b[j] * s;
-      ob = b[j] * c + a[j] * s;
+    for (int j = 0; j < 8; ++j) {
+      const float oa = __fmaf_rn(a[j], cs[j], -__fmul_rn(b[j], sn[j])), ob = __fmaf_rn(a[j], sn[j], __fmul_rn(b[j], cs[j]));
+      a[j] = oa;
+      b[j] = ob;
     }
-    dst[i] = __float2bfloat16(oa);
-    dst[D / 2 + i] = __float2bfloat16(ob);
+  }
+  if (valid) {
+    store8(dst + sub * 8, a);
+    store8(dst + D / 2 + sub * 8, b);
   }
 }
 
@@ -456,35 +543,45 @@ __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfl
     store8(act + i * 8, o);
   }
 }
-__global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __nv_bfloat16* __restrict__ dact,
-                                  __nv_bfloat16* __restrict__ dgu, long long n_pairs8) {
-  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n_pairs8;
-       i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    float a[8], b[8], d[8], oa[8], ob[8];
-    load8(gu + i * 16, a);
-    load8(gu + i * 16 + 8, b);
-    load8(dact + i * 8, d);
+// Four pairs a thread and set, two sets a step: a warp's load is 512 bytes in a row and few registers are held, so that many loads are
+// in flight.  (18432 x 9728, 1.8 GB: 422 us with eight pairs, whose two loads are 32 bytes apart from lane to lane; 290 now.)
+__device__ __forceinline__ uint4 swiglu_bwd4(const uint4& r, const uint2& rd) {
+  float a[8], o[8];
+  unpack8(r, a);
+  const float2 d0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&rd.x));
+  const float2 d1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&rd.y));
+  const float d[4] = {d0.x, d0.y, d1.x, d1.y};
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      {
-        const float g = a[2 * j], u = a[2 * j + 1], s = 1.f / (1.f + __expf(-g));
-        oa[2 * j] = d[j] * u * s * (1.f + g * (1.f - s));
-        oa[2 * j + 1] = d[j] * g * s;
-      }
-      {
-        const float g = b[2 * j], u = b[2 * j + 1], s = 1.f / (1.f + __expf(-g));
-        ob[2 * j] = d[4 + j] * u * s * (1.f + g * (1.f - s));
-        ob[2 * j + 1] = d[4 + j] * g * s;
-      }
-    }
-    store8(dgu + i * 16, oa);
-    store8(dgu + i * 16 + 8, ob);
+  for (int j = 0; j < 4; ++j) {
+    const float g = a[2 * j], u = a[2 * j + 1], s = 1.f / (1.f + __expf(-g));
+    o[2 * j] = d[j] * u * s * (1.f + g * (1.f - s));
+    o[2 * j + 1] = d[j] * g * s;
   }
+  return pack8(o);
+}
+__global__ void __launch_bounds__(256)
+swiglu_bwd_kernel(const uint4* __restrict__ gu, const uint2* __restrict__ dact, uint4* __restrict__ dgu, long long n) {
+  const long long step = static_cast<long long>(gridDim.x) * blockDim.x;
+  long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+  for (; i + step < n; i += 2 * step) {
+    const uint4 r0 = gu[i], r1 = gu[i + step];
+    const uint2 d0 = dact[i], d1 = dact[i + step];
+    dgu[i] = swiglu_bwd4(r0, d0);
+    dgu[i + step] = swiglu_bwd4(r1, d1);
+  }
+  if (i < n) dgu[i] = swiglu_bwd4(gu[i], dact[i]);
 }
 
 }  // namespace apb
 
 // ---------------------------------------------------------------------------
+namespace apb {
+static decltype(&rmsnorm_fwd_kernel<1>) rmsnorm_fwd_variant(int H) {
+  const int nv = (H / 8 + kNormThreads - 1) / kNormThreads;
+  return nv <= 1 ? rmsnorm_fwd_kernel<1> : nv <= 2 ? rmsnorm_fwd_kernel<2> : rmsnorm_fwd_kernel<4>;
+}
+}  // namespace apb
+
 extern "C" {
 using namespace apb;
 
@@ -493,7 +590,7 @@ int apb_rmsnorm_fwd(const void* x, const void* res, const void* w, void* y, void
   if (T <= 0) return 0;
   if (H % 8 || H > kNormThreads * 8 * kNormMaxVec) return kBadArgument;
   const int grid = T < apb::sm_count() * 8 ? T : apb::sm_count() * 8;
-  return static_cast<int>(launch_kernel(rmsnorm_fwd_kernel, dim3(grid), dim3(kNormThreads), 0, s,
+  return static_cast<int>(launch_kernel(rmsnorm_fwd_variant(H), dim3(grid), dim3(kNormThreads), 0, s,
                                         static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(res),
                                         static_cast<const __nv_bfloat16*>(w), static_cast<__nv_bfloat16*>(y),
                                         static_cast<__nv_bfloat16*>(res_out), rstd, T, H, eps, w_offset,
@@ -507,7 +604,7 @@ int apb_rmsnorm_fwd_f32in(float* x_f32, const void* res, const void* w, void* y,
   if (T <= 0) return 0;
   if (H % 8 || H > kNormThreads * 8 * kNormMaxVec || !res_out) return kBadArgument;
   const int grid = T < apb::sm_count() * 8 ? T : apb::sm_count() * 8;
-  return static_cast<int>(launch_kernel(rmsnorm_fwd_kernel, dim3(grid), dim3(kNormThreads), 0, s,
+  return static_cast<int>(launch_kernel(rmsnorm_fwd_variant(H), dim3(grid), dim3(kNormThreads), 0, s,
                                         static_cast<const __nv_bfloat16*>(nullptr),
                                         static_cast<const __nv_bfloat16*>(res), static_cast<const __nv_bfloat16*>(w),
                                         static_cast<__nv_bfloat16*>(y), static_cast<__nv_bfloat16*>(res_out),
@@ -542,10 +639,14 @@ int apb_qknorm_rope_fwd(const void* qkv, long long ld_qkv, const void* wq, const
                         int D, int rot, float eps, cudaStream_t s) {
   if (T <= 0) return 0;
   if (rot != 0 && rot != D) return kBadArgument;
-  const long long warps = static_cast<long long>(T) * (Hq + Hkv);
-  const int grid = static_cast<int>((warps * 32 + 255) / 256);
+  const long long lanes = static_cast<long long>(T) * (Hq + Hkv) * (D / 16);
+  const int grid = static_cast<int>((lanes + 255) / 256);
+  const uintptr_t bases = reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(wq) | reinterpret_cast<uintptr_t>(wk) |
+                          reinterpret_cast<uintptr_t>(cos_t) | reinterpret_cast<uintptr_t>(sin_t);
+  const bool aligned = (bases & 15) == 0 && ld_qkv % 8 == 0;
+  if ((reinterpret_cast<uintptr_t>(q_out) | reinterpret_cast<uintptr_t>(k_out)) & 15) return kBadArgument;
 #define APB_LAUNCH_QK(DD)                                                                                   \
-  qknorm_rope_fwd_kernel<DD><<<grid, 256, 0, s>>>(                                                          \
+  (aligned ? qknorm_rope_fwd_kernel<DD, true> : qknorm_rope_fwd_kernel<DD, false>)<<<grid, 256, 0, s>>>(                                                          \
       static_cast<const __nv_bfloat16*>(qkv), ld_qkv, static_cast<const __nv_bfloat16*>(wq),               \
       static_cast<const __nv_bfloat16*>(wk), cos_t, sin_t, pos, static_cast<__nv_bfloat16*>(q_out),        \
       static_cast<__nv_bfloat16*>(k_out), T, Hq, Hkv, rot, eps)
@@ -598,12 +699,10 @@ int apb_swiglu_fwd(const void* gu, void* act, long long T, long long I, cudaStre
 }
 int apb_swiglu_bwd(const void* gu, const void* dact, void* dgu, long long T, long long I, cudaStream_t s) {
   if (I % 8) return kBadArgument;
-  const long long n = T * I / 8;
+  const long long n = T * I / 4;
   if (n <= 0) return 0;
   const int grid = static_cast<int>(n / 256 + 1 < apb::sm_count() * 16 ? n / 256 + 1 : apb::sm_count() * 16);
-  swiglu_bwd_kernel<<<grid, 256, 0, s>>>(static_cast<const __nv_bfloat16*>(gu),
-                                         static_cast<const __nv_bfloat16*>(dact),
-                                         static_cast<__nv_bfloat16*>(dgu), n);
+  swiglu_bwd_kernel<<<grid, 256, 0, s>>>(static_cast<const uint4*>(gu), static_cast<const uint2*>(dact), static_cast<uint4*>(dgu), n);
   return static_cast<int>(cudaGetLastError());
 }
 }

@@ -102,3 +102,62 @@ def test_delta_rule_scan_kernel_matches_the_token_by_token_recurrence(T, H, Dk, 
             loop_o, loop_S = gated_delta_rule_chunked(q, k, v, gate, beta, state)          # PyTorch loop
         for a, b in ((got_o, want_o), (got_S, want_S), (got_o, loop_o), (got_S, loop_S)):
             assert (a - b).abs().max() < 2e-3 * b.abs().max() + 1e-4
+
+
+@pytest.mark.parametrize("D", [64, 128, 256])
+@pytest.mark.parametrize("T,Hq,Hkv", [(1, 4, 2), (37, 3, 1), (513, 8, 2)])
+def test_qknorm_rope_of_rows_off_a_16_byte_boundary(D, T, Hq, Hkv):
+    """Rows, weights and tables that begin anywhere have the results of aligned ones, to the bit, with and without weights; both agree
+    with fp32 (bf16 outputs: 2^-8 of a value and a little for the sums)."""
+    from arctic_platform_b200.ops import norm
+    torch.manual_seed(D + T)
+    width = (Hq + 2 * Hkv) * D
+    wide = torch.randn(T, width + 13, device="cuda").bfloat16()
+    off = wide[:, 3:3 + width]
+    w = [torch.randn(2 * D + 5, device="cuda").bfloat16()[i * D + 1:(i + 1) * D + 1] for i in (0, 1)]
+    cos_t, sin_t = norm.rope_tables(700, D, 1e4, "cuda")
+    shift = [torch.cat([t.new_zeros(1), t.reshape(-1)])[1:].view_as(t) for t in (cos_t, sin_t)]
+    pos = torch.randint(0, 700, (T,), device="cuda", dtype=torch.int32)
+    for wq, wk in (w, (None, None)):
+        q0, k0, _ = norm.qknorm_rope(off.contiguous(), *(None if x is None else x.clone() for x in (wq, wk)), cos_t, sin_t, pos, Hq, Hkv, D)
+        q1, k1, _ = norm.qknorm_rope(off, wq, wk, *shift, pos, Hq, Hkv, D)
+        assert torch.equal(q0, q1) and torch.equal(k0, k1)
+        ref = norm.qknorm_rope_ref(off[:, :Hq * D].reshape(T, Hq, D).float(), off[:, Hq * D:(Hq + Hkv) * D].reshape(T, Hkv, D).float(),
+                                   wq, wk, cos_t, sin_t, pos, 1e-6)
+        for got, want in zip((q0, k0), ref):
+            assert (got.float() - want).abs().max() <= 2 ** -8 * want.abs().max() + 1e-4
+
+
+@pytest.mark.parametrize("H", [8, 1024, 2048, 2056, 2560, 4104, 8192])
+@pytest.mark.parametrize("T", [1, 1185, 2400])
+def test_rows_after_rows_in_one_block(H, T):
+    """RMSNorm forward and backward where a block walks several rows (1184 blocks and fewer), at the widths where the vectors per thread
+    change: as single rows give it, to the bit."""
+    from arctic_platform_b200.ops import norm
+    torch.manual_seed(H)
+    x, res, dy, dst = (torch.randn(T, H, device="cuda").bfloat16() for _ in range(4))
+    w = torch.randn(H, device="cuda").bfloat16()
+
+    def run(rows):
+        a, b = x[rows].clone().requires_grad_(), res[rows].clone().requires_grad_()
+        y, stream = norm.rmsnorm(a, w, 1e-6, b)
+        torch.autograd.backward([y, stream], [dy[rows], dst[rows]])
+        return y.detach(), stream.detach(), a.grad
+
+    whole = run(slice(0, T))
+    for r in {0, T // 2, T - 1}:
+        for got, want in zip(run(slice(r, r + 1)), whole):
+            assert torch.equal(got[0], want[r])
+
+
+@pytest.mark.parametrize("T,I", [(1, 8), (3, 1000), (700, 4864), (2049, 2056)])
+def test_swiglu_backward_two_sets_a_thread(T, I):
+    """Odd numbers of sets, fewer than threads and more than two rounds; bf16 results against fp32."""
+    from arctic_platform_b200.ops import norm
+    torch.manual_seed(T)
+    gu = torch.randn(T, 2 * I, device="cuda").bfloat16().requires_grad_()
+    d = torch.randn(T, I, device="cuda").bfloat16()
+    norm.swiglu(gu).backward(d)
+    ref = gu.detach().float().requires_grad_()
+    (torch.nn.functional.silu(ref[:, 0::2]) * ref[:, 1::2]).backward(d.float())
+    assert (gu.grad.float() - ref.grad).abs().max() <= 2 ** -8 * ref.grad.abs().max()
