@@ -106,24 +106,39 @@ __global__ void __launch_bounds__(256) grpo_token_loss_kernel(const GrpoArgs a) 
 // One warp per token.  scores = softmax(logits) or sigmoid(logits); selection on scores + bias; k rounds of warp
 // arg-max (ties go to the lower expert index, like a stable descending sort).  E <= 32 * kRouteMaxPerLane.
 constexpr int kRouteMaxPerLane = 16;
+//
+// With `weight`, the scores of the chosen experts go out too, with `renorm` (k <= 8) divided by their sum, times `scale`: conversion,
+// softmax, this kernel, a gather, a sum and a division were seven launches of 22 us in a decode step's layer, this is one of 4.  The
+// decision keeps the approximate exponential that it always had; weights take the exact one and sums in the order of the operations
+// that they replace, whose bits they have: a warp per row for the softmax, partial sums of every fourth weight for the division.
+template <typename LOGIT>
 __global__ void __launch_bounds__(256)
-moe_route_kernel(const float* __restrict__ logits, long long ld, const float* __restrict__ bias, int T, int E, int k,
-                 int sigmoid, long long* __restrict__ idx_out, int* __restrict__ counts) {
+moe_route_kernel(const LOGIT* __restrict__ logits, long long ld, const float* __restrict__ bias, int T, int E, int k,
+                 int sigmoid, long long* __restrict__ idx_out, int* __restrict__ counts, float* __restrict__ weight, int renorm,
+                 float scale) {
+  pdl_entry();
   const long long tok = (blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (tok >= T) return;
-  const float* row = logits + tok * ld;
+  const LOGIT* row = logits + tok * ld;
   float sc[kRouteMaxPerLane];
   float mx = -INFINITY;
 #pragma unroll
   for (int j = 0; j < kRouteMaxPerLane; ++j) {
     const int e = lane + 32 * j;
-    sc[j] = e < E ? row[e] : -INFINITY;
+    sc[j] = e < E ? static_cast<float>(row[e]) : -INFINITY;
     mx = fmaxf(mx, sc[j]);
   }
+  float exact_sum = 0.f;
   if (!sigmoid) {
     mx = warp_max(mx);
     float s = 0.f;
+    if (weight) {
+#pragma unroll
+      for (int j = 0; j < kRouteMaxPerLane; ++j)
+        if (lane + 32 * j < E) exact_sum += expf(sc[j] - mx);
+      exact_sum = warp_sum(exact_sum);
+    }
 #pragma unroll
     for (int j = 0; j < kRouteMaxPerLane; ++j) {
       const int e = lane + 32 * j;
@@ -143,6 +158,7 @@ moe_route_kernel(const float* __restrict__ logits, long long ld, const float* __
     const int e = lane + 32 * j;
     sc[j] = e < E ? sc[j] + (bias ? bias[e] : 0.f) : -INFINITY;
   }
+  float mine = 0.f;               // lane r: score of the r-th choice, for sums
   for (int r = 0; r < k; ++r) {
     float best = -INFINITY;
     int be = 0x7fffffff;
@@ -167,7 +183,22 @@ moe_route_kernel(const float* __restrict__ logits, long long ld, const float* __
       idx_out[tok * k + r] = be;
       if (counts) atomicAdd(counts + be, 1);
     }
-    if ((be & 31) == lane) sc[be >> 5] = -INFINITY;   // taken
+#pragma unroll
+    for (int j = 0; j < kRouteMaxPerLane; ++j)
+      if (be == lane + 32 * j) sc[j] = -INFINITY;   // taken
+    if (weight) {
+      const float x = static_cast<float>(row[be < E ? be : 0]);
+      const float score = sigmoid ? 1.f / (1.f + expf(-x)) : expf(x - mx) / exact_sum;
+      if (lane == r) mine = score;
+      if (lane == 0 && !renorm) weight[tok * k + r] = score * scale;
+    }
+  }
+  if (weight && renorm) {
+    float sum = mine + __shfl_down_sync(0xffffffffu, mine, 4);
+    sum += __shfl_down_sync(0xffffffffu, sum, 2);
+    sum += __shfl_down_sync(0xffffffffu, sum, 1);
+    sum = __shfl_sync(0xffffffffu, sum, 0);
+    if (lane < k) weight[tok * k + lane] = mine / (sum + 1e-20f) * scale;
   }
 }
 
@@ -178,18 +209,38 @@ __global__ void __launch_bounds__(256)
 moe_group_tiles_kernel(const int* __restrict__ counts, int E, int n_out1, int n_out2, int4* __restrict__ tiles1,
                        int4* __restrict__ tiles2, int max_tiles1, int max_tiles2, int* __restrict__ n_tiles,
                        int* __restrict__ offsets) {
+  pdl_entry();
   __shared__ int row_off[513];
   __shared__ int blk_off[513];
-  if (threadIdx.x == 0) {
-    int r = 0, b = 0;
-    for (int e = 0; e < E; ++e) {
-      row_off[e] = r;
-      blk_off[e] = b;
-      r += counts[e];
-      b += (counts[e] + 127) / 128;
+  __shared__ int2 warps[8];
+  // exclusive sums of two experts a thread (one thread that added all of them took 4 us of a decode step's layer)
+  const int e0 = 2 * threadIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int c0 = e0 < E ? counts[e0] : 0, c1 = e0 + 1 < E ? counts[e0 + 1] : 0;
+  const int b0 = (c0 + 127) / 128, b1 = (c1 + 127) / 128;
+  int r = c0 + c1, b = b0 + b1;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int tr = __shfl_up_sync(0xffffffffu, r, o), tb = __shfl_up_sync(0xffffffffu, b, o);
+    if (lane >= o) {
+      r += tr;
+      b += tb;
     }
-    row_off[E] = r;
-    blk_off[E] = b;
+  }
+  if (lane == 31) warps[warp] = make_int2(r, b);
+  __syncthreads();
+  for (int w = 0; w < warp; ++w) {
+    r += warps[w].x;
+    b += warps[w].y;
+  }
+  if (e0 < E) {
+    row_off[e0] = r - c0 - c1;
+    blk_off[e0] = b - b0 - b1;
+    row_off[e0 + 1] = r - c1;         // with an odd number of experts the totals
+    blk_off[e0 + 1] = b - b1;
+    if (e0 + 2 >= E) {
+      row_off[E] = r;
+      blk_off[E] = b;
+    }
   }
   __syncthreads();
   const int nt1 = (n_out1 + 127) / 128, nt2 = (n_out2 + 127) / 128;
@@ -317,9 +368,9 @@ int apb_moe_group_tiles(const int* counts, int E, int n_out1, int n_out2, void* 
                         int max_tiles2, int* n_tiles, int* offsets, cudaStream_t s) {
   using namespace apb;
   if (!counts || !tiles1 || !tiles2 || !n_tiles || E < 1 || E > 512) return kBadArgument;
-  moe_group_tiles_kernel<<<1, 256, 0, s>>>(counts, E, n_out1, n_out2, static_cast<int4*>(tiles1),
-                                           static_cast<int4*>(tiles2), max_tiles1, max_tiles2, n_tiles, offsets);
-  return static_cast<int>(cudaGetLastError());
+  return static_cast<int>(launch_kernel(moe_group_tiles_kernel, dim3(1), dim3(256), 0, s, counts, E, n_out1, n_out2,
+                                        static_cast<int4*>(tiles1), static_cast<int4*>(tiles2), max_tiles1, max_tiles2, n_tiles,
+                                        offsets));
 }
 
 // Token-mean GRPO / dual-clip PPO loss terms with gradient.  All vectors fp32 [n] on the device except mask (bytes).
@@ -346,8 +397,24 @@ int apb_moe_route(const float* logits, long long ld, const float* bias, int T, i
   if (T <= 0) return 0;
   if (!logits || !idx_out || E < 1 || E > 32 * kRouteMaxPerLane || k < 1 || k > E) return kBadArgument;
   const long long threads = static_cast<long long>(T) * 32;
-  moe_route_kernel<<<static_cast<int>((threads + 255) / 256), 256, 0, s>>>(logits, ld, bias, T, E, k, sigmoid, idx_out,
-                                                                            counts);
-  return static_cast<int>(cudaGetLastError());
+  return static_cast<int>(launch_kernel(moe_route_kernel<float>, dim3(static_cast<int>((threads + 255) / 256)), dim3(256), 0, s, logits,
+                                        ld, bias, T, E, k, sigmoid, idx_out, counts, static_cast<float*>(nullptr), 0, 1.f));
+}
+
+// The same with the weights of the chosen experts, weight [T, k] fp32; logits bf16 (bf16 = 1) or fp32.  renorm: divided by their sum,
+// k <= 8; times `scale` either way.
+int apb_moe_route_weights(const void* logits, int bf16, long long ld, const float* bias, int T, int E, int k, int sigmoid, int renorm,
+                          float scale, long long* idx_out, float* weight, cudaStream_t s) {
+  using namespace apb;
+  if (T <= 0) return 0;
+  if (!logits || !idx_out || !weight || E < 1 || E > 32 * kRouteMaxPerLane || k < 1 || k > E || (renorm && k > 8))
+    return kBadArgument;
+  const dim3 grid(static_cast<unsigned>((static_cast<long long>(T) * 32 + 255) / 256));
+  if (bf16)
+    return static_cast<int>(launch_kernel(moe_route_kernel<__nv_bfloat16>, grid, dim3(256), 0, s,
+                                          static_cast<const __nv_bfloat16*>(logits), ld, bias, T, E, k, sigmoid, idx_out,
+                                          static_cast<int*>(nullptr), weight, renorm, scale));
+  return static_cast<int>(launch_kernel(moe_route_kernel<float>, grid, dim3(256), 0, s, static_cast<const float*>(logits), ld, bias, T, E,
+                                        k, sigmoid, idx_out, static_cast<int*>(nullptr), weight, renorm, scale));
 }
 }

@@ -36,6 +36,11 @@ def route_topk(logits: torch.Tensor, k: int, renorm: bool, score_func: str = "so
     * ``routed_experts [T, k]`` replays a decision taken elsewhere (an earlier pass over the same tokens, an
       inference engine): the weights are gathered from the current scores, nothing is re-selected.
     (arctic_platform/model/implementations/qwen35/models/layers/moe.py:196-269, NemotronHRouter in the same file)."""
+    if (routed_experts is None and logits.is_cuda and n_group <= 1 and logits.dim() == 2 and logits.shape[-1] <= 512
+            and score_func in ("softmax", "sigmoid") and not (torch.is_grad_enabled() and logits.requires_grad)):
+        # without gradients: decision and scores from one kernel, the same bits
+        from ..ops.rl_ops import moe_route_weights
+        return moe_route_weights(logits, k, score_func, expert_bias, renorm, route_scale)
     x = logits.float()
     if score_func == "softmax":
         scores = torch.softmax(x, dim=-1)

@@ -22,6 +22,7 @@ def _fn(name: str):
         vp, i, ll, f = c.c_void_p, c.c_int, c.c_longlong, c.c_float
         _FN["grpo"] = _lib.declare("apb_grpo_token_loss", [vp, vp, vp, vp, vp, vp, vp, vp, ll, f, f, f, i, f, f, vp])
         _FN["route"] = _lib.declare("apb_moe_route", [vp, ll, vp, i, i, i, i, vp, vp, vp])
+        _FN["route_w"] = _lib.declare("apb_moe_route_weights", [vp, i, ll, vp, i, i, i, i, i, f, vp, vp, vp])
     return _FN[name]
 
 
@@ -86,3 +87,31 @@ def moe_route(logits: torch.Tensor, k: int, score_func: str = "softmax", bias: O
     _lib.check(_fn("route")(_lib.ptr(x), x.stride(0), _lib.ptr(b), T, E, k, 1 if score_func == "sigmoid" else 0,
                             _lib.ptr(idx), _lib.ptr(counts), _lib.stream_ptr()), "apb_moe_route")
     return idx
+
+
+@torch.no_grad()
+def moe_route_weights(logits: torch.Tensor, k: int, score_func: str = "softmax",
+                      bias: Optional[torch.Tensor] = None, renorm: bool = False,
+                      scale: float = 1.0) -> Tuple[torch.Tensor, torch.Tensor]:
+    """:func:`moe_route` and the chosen experts' scores in one launch: ``(weights [T, k] fp32, experts [T, k] int64)``, the scores divided
+    by their sum with ``renorm`` and multiplied by ``scale``.  ``logits`` bf16 or fp32; weights have the bits of ``torch.softmax`` /
+    ``torch.sigmoid`` in fp32, a gather, ``sum``, division and product."""
+    T, E = logits.shape
+    x = logits.detach()
+    if x.dtype not in (torch.bfloat16, torch.float32):
+        x = x.float()
+    if x.stride(1) != 1:
+        x = x.contiguous()
+    idx = torch.empty((T, k), device=x.device, dtype=torch.int64)
+    w = torch.empty((T, k), device=x.device, dtype=torch.float32)
+    b = None if bias is None else bias.detach().to(torch.float32).contiguous()
+    inside = k <= 8                        # whose order of sums the kernel knows
+    _lib.check(_fn("route_w")(_lib.ptr(x), int(x.dtype == torch.bfloat16), x.stride(0), _lib.ptr(b), T, E, k,
+                              int(score_func == "sigmoid"), int(renorm and inside), float(scale) if inside else 1.0, _lib.ptr(idx),
+                              _lib.ptr(w), _lib.stream_ptr()), "apb_moe_route_weights")
+    if not inside:
+        if renorm:
+            w = w / (w.sum(-1, keepdim=True) + 1e-20)
+        if scale != 1.0:
+            w = w * scale
+    return w, idx

@@ -147,3 +147,31 @@ def test_moe_layer_padded_plan_backward_matches_per_expert_fp32(tokens, experts,
     starved = (torch.bincount(idx.reshape(-1), minlength=experts) == 0).nonzero().flatten().tolist()
     for e in starved:                                              # experts without tokens: exactly zero gradient
         assert float(g_gu[e].abs().max()) == 0.0 and float(g_dn[e].abs().max()) == 0.0
+
+
+@pytest.mark.parametrize("E,k", [(8, 2), (60, 4), (128, 8), (512, 10), (33, 33)])
+@pytest.mark.parametrize("score", ["softmax", "sigmoid"])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_route_without_gradients_has_the_bits_of_the_pass_with_them(E, k, score, dtype):
+    """Decision and weights from one kernel where no gradient is wanted: those of the softmax, gather and division behind a decision, to
+    the bit, with and without a bias, normalised and scaled; rows with a stride."""
+    from arctic_platform_b200.models.moe import route_topk
+    torch.manual_seed(E)
+    x = (torch.randn(1037, E + 3, device="cuda") * 3).to(dtype)[:, :E]
+    bias = torch.randn(E, device="cuda")
+    for b, renorm, scale in ((None, True, 1.0), (bias, False, 2.5), (bias, True, 0.5)):
+        w0, i0 = route_topk(x.clone().requires_grad_(), k, renorm, score, scale, b)
+        w1, i1 = route_topk(x, k, renorm, score, scale, b)
+        assert torch.equal(i0, i1) and torch.equal(w0.detach(), w1)
+
+
+@pytest.mark.parametrize("E", [1, 2, 7, 64, 129, 511, 512])
+def test_group_tiles_of_any_number_of_experts(E):
+    """Prefix sums of two experts a thread: odd and even numbers, experts without rows, more than a block of rows."""
+    from arctic_platform_b200.models.moe import build_group_tiles, device_group_tiles
+    g = torch.Generator().manual_seed(E)
+    counts = torch.randint(0, 300, (E,), generator=g)
+    counts[::3] = 0
+    t1, t2, n, _, _ = device_group_tiles(counts.to(torch.int32).cuda(), int(counts.sum()), 384, 200)
+    for got, live, width in ((t1, int(n[0]), 384), (t2, int(n[1]), 200)):
+        assert torch.equal(got[:live].cpu(), build_group_tiles(counts, width, "cpu"))
