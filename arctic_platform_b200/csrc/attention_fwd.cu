@@ -28,14 +28,14 @@
 // 32 / 8 heads: 1.74 ms, 630 TFLOP/s), this 5500 (1.34 ms, 820; 32768 tokens 860 TFLOP/s).  Adding the previous P*V
 // between the exponentials instead, 16 columns at a time, spilled and took 1.46 ms.
 //
-// With LAG, O stays in tensor memory and weights are taken relative to a reference that follows a row's maximum only when it, or that
-// of another row of its warp, has moved by more than 2^8; O is rescaled on those occasions and read once per tile.  The largest weight
-// is then not 1 but rounded like the others; O is divided by the sum of the rounded weights, which makes up for it where few keys
-// share the weight (the exact sum goes into the LSE).  8 x 4096 tokens 1.11 ms instead of 1.34, one sequence of 32768 7.6 instead of
-// 10.2 (1150 TFLOP/s).  Errors of O against 64 bits, scores of standard deviation 0.3, 1 and 3: 2.02e-3, 2.01e-3, 1.87e-3, with the exact
-// maximum 2.04e-3, 1.99e-3, 1.77e-3 (dividing by the exact sum: 2.05e-3 at 3, and 1.03 ms).  Last bits are others from block to block,
-// which routers downstream turn into other experts: models with experts keep the exact running maximum.  A polynomial on the FMA pipe
-// for 1/8 to 1/2 of the exponentials made it no faster (1.05 to 1.16 ms against 1.04): they are not what a block waits for.
+// With TMEM_O, O stays in tensor memory, where the products add themselves up: it is rescaled only when the running maximum of one of a
+// warp's 32 rows has moved (nearly always in the first 32 blocks, in a tenth of them behind 256) and read once per tile, scores are read
+// once.  8 x 4096 tokens 1.11 ms instead of 1.33, one sequence of 32768 8.3 instead of 9.9 (1060 TFLOP/s), 12 x 300 46 us instead of 56.
+// Weights, row sums and maxima are those of the other form, and so are errors against 64 bits to four digits (scores of standard
+// deviation 0.3 to 5); O is added up by the tensor core, whose roundings differ, which routers downstream turn into other experts now
+// and then: models with experts keep O in registers.  Moving the reference only when it lags by 2^8 takes 1.03 ms, but rounds the
+// largest weight, which is 1 otherwise (error 2.05e-3 instead of 1.77e-3 at a deviation of 3).  Two buffers of 32 columns for the
+// rescaling spilled (1.25 ms); a polynomial on the FMA pipe for 1/8 to 1/2 of the exponentials gained nothing.
 #include "attention_common.cuh"
 #include "host_utils.cuh"
 
@@ -58,7 +58,6 @@ struct AttnFwdParams {
 constexpr int kAttnThreads = 384;
 constexpr int kAttnRegsIssue = 56, kAttnRegsSoftmax = 224;
 constexpr int kKvBlock = 128;
-constexpr float kAttnSlack = 8.f;       // log2 units by which a row's maximum may exceed its reference
 
 template <int D>
 struct AttnCfg {
@@ -81,7 +80,7 @@ struct AttnItem {
   }
 };
 
-template <int D, bool LAG>
+template <int D, bool TMEM_O>
 __global__ void __launch_bounds__(kAttnThreads, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant__ CUtensorMap tma_k,
                 const __grid_constant__ CUtensorMap tma_v, const AttnFwdParams p) {
@@ -242,7 +241,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
             if (!ok) break;
             ++done[g];
             if (elect_one()) {
-              issue_o(g, sv, !LAG || j == 0);
+              issue_o(g, sv, !TMEM_O || j == 0);
               if (more)
                 issue_s(g, sk);      // over P, which the product above reads first: the tensor core keeps the order of issue
               else
@@ -270,17 +269,17 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
     const uint64_t c2 = xtc_pair(p.scale_log2, p.scale_log2);
     uint32_t blocks = 0, items = 0;       // of this group so far
     bool ok = true;
-    uint64_t o[LAG ? 1 : D / 2];          // pairs of columns
+    uint64_t o[TMEM_O ? 1 : D / 2];          // pairs of columns
     uint32_t buf[2][32];
     for (int round = 0; round < rounds && ok; ++round) {
       const int at = item_at(round);
       if (at < 0) continue;
       const AttnItem w(p.work + static_cast<long long>(at) * 8);
       if (w.n_blocks == 0 || g >= w.n_groups) continue;
-      float m_run = -INFINITY, l_run = 0.f, alpha = 0.f;       // LAG: m_run is the reference, l_run the sum when all is done
-      uint64_t l2 = 0, lr2 = 0;       // LAG: sums of the weights and of the rounded weights, in two halves
+      float m_run = -INFINITY, l_run = 0.f, alpha = 0.f;       // TMEM_O: l_run is the sum when all is done
+      uint64_t l2 = 0;                // its sum so far, in two halves
 #pragma unroll
-      for (int i = 0; i < D / 2 && !LAG; ++i) o[i] = 0;
+      for (int i = 0; i < D / 2 && !TMEM_O; ++i) o[i] = 0;
       // o = o * alpha + P*V, 32 columns that are in `v`
       auto add = [&](int c, const uint32_t (&v)[32]) {
         const uint64_t a2 = xtc_pair(alpha, alpha);
@@ -302,7 +301,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
           limit = min(w.own_len - b0, row + w.diag - b0 + 1);
         }
         const bool masked = least < kKvBlock;
-        if constexpr (LAG) {
+        if constexpr (TMEM_O) {
           uint32_t v[4][32];
 #pragma unroll
           for (int c = 0; c < 4; ++c) tmem_ld_32x32(t_s + c * 32, v[c]);
@@ -318,25 +317,32 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
           for (int c = 0; c < kKvBlock; c += 2)
             mx[(c >> 1) & 3] = fmaxf(fmaxf(mx[(c >> 1) & 3], __uint_as_float(v[c / 32][c % 32])), __uint_as_float(v[c / 32][c % 32 + 1]));
           const float m_new = fmaxf(m_run, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * p.scale_log2);
-          if (__any_sync(0xffffffffu, m_new > m_run + kAttnSlack || m_run == -INFINITY)) {
+          if (__any_sync(0xffffffffu, m_new > m_run)) {
             if (j > 0) {           // O holds the blocks before this one: their product was issued ahead of this S
               alpha = m_run == -INFINITY ? 0.f : xtc_ex2(m_run - m_new);
               l2 = xtc_mul2(l2, xtc_pair(alpha, alpha));
-              lr2 = xtc_mul2(lr2, xtc_pair(alpha, alpha));
-#pragma unroll 1
-              for (int c = 0; c < D / 32; ++c) {
-                tmem_ld_32x32(t_o + c * 32, buf[0]);
-                tmem_ld_wait(buf[0]);
+              const uint64_t a2 = xtc_pair(alpha, alpha);
+              uint32_t r[2][16];
+              tmem_ld_32x16(t_o, r[0]);
+              tmem_ld_wait(r[0]);
 #pragma unroll
-                for (int i = 0; i < 32; ++i) buf[0][i] = __float_as_uint(__uint_as_float(buf[0][i]) * alpha);
-                tmem_st_32x32(t_o + c * 32, buf[0]);
+              for (int c = 0; c < D / 16; ++c) {
+                if (c + 1 < D / 16) tmem_ld_32x16(t_o + (c + 1) * 16, r[(c + 1) & 1]);
+#pragma unroll
+                for (int i = 0; i < 16; i += 2) {
+                  const float2 f = xtc_unpair(xtc_mul2(xtc_pair(__uint_as_float(r[c & 1][i]), __uint_as_float(r[c & 1][i + 1])), a2));
+                  r[c & 1][i] = __float_as_uint(f.x);
+                  r[c & 1][i + 1] = __float_as_uint(f.y);
+                }
+                tmem_st_32x16(t_o + c * 16, r[c & 1]);
+                if (c + 1 < D / 16) tmem_ld_wait(r[(c + 1) & 1]);
               }
             }
             m_run = m_new;
           }
           const float m_use = m_run == -INFINITY ? 0.f : m_run;
           const uint64_t nm2 = xtc_pair(-m_use, -m_use);
-          uint64_t sum[2] = {0, 0}, rounded[2] = {0, 0};
+          uint64_t sum[2] = {0, 0};
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
             uint32_t pk[16];
@@ -346,9 +352,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
                   xtc_fma2(xtc_pair(__uint_as_float(v[c][2 * i]), __uint_as_float(v[c][2 * i + 1])), c2, nm2));
               f.x = xtc_ex2(f.x);
               f.y = xtc_ex2(f.y);
-              if (p.lse) sum[i & 1] = xtc_add2(sum[i & 1], xtc_pair(f.x, f.y));
+              sum[i & 1] = xtc_add2(sum[i & 1], xtc_pair(f.x, f.y));
               pk[i] = pack_bf16x2(f.x, f.y);
-              rounded[i & 1] = xtc_add2(rounded[i & 1], xtc_pair(__uint_as_float(pk[i] << 16), __uint_as_float(pk[i] & 0xffff0000u)));
             }
             tmem_st_32x16(t_s + c * 16, pk);
           }
@@ -356,7 +361,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
           tc_fence_before();
           mbar_arrive(&p_full[g]);
           l2 = xtc_add2(l2, xtc_add2(sum[0], sum[1]));
-          lr2 = xtc_add2(lr2, xtc_add2(rounded[0], rounded[1]));
           continue;
         }
         auto mask = [&](int c, uint32_t (&v)[32]) {
@@ -428,12 +432,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
       ok = wait(&o_full[g], items & 1, kTimeoutTmemFull);
       if (!ok) break;
       ++items;
-      float l_norm = l_run;
-      if constexpr (LAG) {
+      if constexpr (TMEM_O) {
         const float2 l = xtc_unpair(l2);
         l_run = l.x + l.y;
-        const float2 lr = xtc_unpair(lr2);
-        l_norm = lr.x + lr.y;
       } else {
 #pragma unroll
         for (int c = 0; c < D / 32; ++c) {
@@ -443,10 +444,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant
         }
         tc_fence_before();
       }
-      const float inv = l_norm > 0.f ? 1.f / l_norm : 0.f;
+      const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
       const long long t = static_cast<long long>(w.q_row0) + row;
       __nv_bfloat16* dst = p.O + t * p.ldo + static_cast<long long>(w.head0 + g) * D;
-      if constexpr (LAG) {
+      if constexpr (TMEM_O) {
 #pragma unroll 1
         for (int c = 0; c < D / 32; ++c) {
           uint32_t r[32];
@@ -499,11 +500,11 @@ extern "C" {
 
 // q [T, Hq*D] (row stride ldq), k/v [T, Hkv*D] (ldk/ldv), o [T, Hq*D] (ldo), lse [Hq, T] fp32 or null.
 // work: device int32 [num_work][8] (see AttnFwdParams).  scale is the softmax scale (1/sqrt(D)).
-// lag: weights may be taken against a reference that follows a row's maximum (see the header); scales that are not positive take the
-// exact maximum either way, whose place among the scaled scores they change.
-int apb_attn_fwd_ref(const void* q, const void* k, const void* v, void* o, float* lse, const int* work, int num_work,
+// tmem_o: O may be added up in tensor memory (see the header); scales that are not positive, which change the place of the maximum among
+// the scores, take the other form either way.
+int apb_attn_fwd_form(const void* q, const void* k, const void* v, void* o, float* lse, const int* work, int num_work,
                      int T, int Hq, int Hkv, int D, long long ldq, long long ldk, long long ldv, long long ldo,
-                     float scale, int lag, cudaStream_t stream) {
+                     float scale, int tmem_o, cudaStream_t stream) {
   using namespace apb;
   if (num_work <= 0) return 0;
   if ((D != 128 && D != 64) || (ldq % 8) || (ldk % 8) || (ldv % 8) || (ldo % 8) || Hq % Hkv) return kBadArgument;
@@ -526,12 +527,12 @@ int apb_attn_fwd_ref(const void* q, const void* k, const void* v, void* o, float
   p.T = T;
   p.status = status_device_ptr();
   const int grid = num_work < sm_count() ? num_work : sm_count();
-  const bool follow = lag && scale > 0.f;
-  auto* kernel = D == 128 ? (follow ? attn_fwd_kernel<128, true> : attn_fwd_kernel<128, false>)
-                          : (follow ? attn_fwd_kernel<64, true> : attn_fwd_kernel<64, false>);
+  const bool in_tmem = tmem_o && scale > 0.f;
+  auto* kernel = D == 128 ? (in_tmem ? attn_fwd_kernel<128, true> : attn_fwd_kernel<128, false>)
+                          : (in_tmem ? attn_fwd_kernel<64, true> : attn_fwd_kernel<64, false>);
   const int smem = D == 128 ? AttnCfg<128>::kSmemBytes : AttnCfg<64>::kSmemBytes;
   static bool configured[4][64] = {{false}};
-  const int variant = (D == 128 ? 0 : 2) + (follow ? 1 : 0);
+  const int variant = (D == 128 ? 0 : 2) + (in_tmem ? 1 : 0);
   int dev = 0;
   cudaGetDevice(&dev);
   if (!configured[variant][dev & 63]) {
@@ -546,6 +547,6 @@ int apb_attn_fwd_ref(const void* q, const void* k, const void* v, void* o, float
 int apb_attn_fwd(const void* q, const void* k, const void* v, void* o, float* lse, const int* work, int num_work,
                  int T, int Hq, int Hkv, int D, long long ldq, long long ldk, long long ldv, long long ldo,
                  float scale, cudaStream_t stream) {
-  return apb_attn_fwd_ref(q, k, v, o, lse, work, num_work, T, Hq, Hkv, D, ldq, ldk, ldv, ldo, scale, 0, stream);
+  return apb_attn_fwd_form(q, k, v, o, lse, work, num_work, T, Hq, Hkv, D, ldq, ldk, ldv, ldo, scale, 0, stream);
 }
 }

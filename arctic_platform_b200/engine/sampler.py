@@ -974,7 +974,7 @@ class SamplerEngine:
         def attn(li, q, k, v):
             o, _ = attention_fwd_cuda(q, k, v.contiguous() if v.stride(1) != v.shape[2] else v,
                                       end_layout if short and li + 1 == n_layers else layout, scale, need_lse=False,
-                                      lag=not self.cfg.is_moe)
+                                      tmem_o=not self.cfg.is_moe)
             return o
 
         x = torch.nn.functional.embedding(ids, self.model.embed)

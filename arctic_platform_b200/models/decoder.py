@@ -141,7 +141,7 @@ class DecoderBlock(nn.Module):
                 from ..parallel.ulysses import ulysses_attention
                 a = ulysses_attention(q, k, v, layout, self.sp_group)
             else:
-                a = segment_attention(q, k, v, layout, lag=not self.cfg.is_moe)
+                a = segment_attention(q, k, v, layout, tmem_o=not self.cfg.is_moe)
             o = self._part("attn_proj", self._attn_out, a.reshape(a.shape[0], -1), h)
         o = self.tp_reduce(o)
         h2, stream = self._part("norm", self._norm, o, stream, self.ln2)
