@@ -5,7 +5,8 @@ of one task share a system / few-shot header -- so their KV pages form a forest:
 every sequence's full context per step re-reads the shared pages once per sequence.  Here every NODE of the forest is
 attended once per step by all sequences below it (``decode_attention.cu``: their query rows form one 128-row tensor-core
 tile, the node's pages are streamed once), every sequence attends to its private pages by itself, and a log-sum-exp merge
-joins a sequence's levels -- one launch, in which the last part of a sequence to finish does the merge.  KV traffic per step drops from
+joins a sequence's levels -- in one launch, in which the last part of a sequence to finish does the merge, where the caller keeps
+arrival counters for it, else in three.  KV traffic per step drops from
 ``sum over sequences of context length`` to ``sum over nodes of node length + private tokens``.
 
 The reference switches the same idea on in its sampler with ``use_fca`` ("forest cascade attention",
@@ -29,6 +30,7 @@ from . import _lib
 PAGE = 16
 MAX_SHARED_LEVELS = 3
 OWN_CHUNK = 4              # pages that a warp reads of a sequence's own, at least
+MAX_PARTS = 255            # of a node or a sequence, in the arrival counters of the one-launch form
 
 _FN = {}
 
@@ -143,12 +145,19 @@ def forest_decode_attention(q: torch.Tensor, kcache: torch.Tensor, vcache: torch
     ``kcache / vcache [num_pages, Hkv, 16, D]`` (one layer).  ``forest``: shared nodes.  ``priv_*``: the per-sequence
     pass (``priv_start [B]`` = slot ids, ``priv_active [B]`` = 1 for live slots, ``priv_table [B, max_pages]``,
     ``priv_len [B]``).  ``part_o[i]`` / ``part_ml[i]`` fp32 scratch for source ``i`` (shared levels first, the private pass
-    last): room for ``[B, Hq, splits, D]`` / ``[B, Hq, splits, 2]``, ``seq_splits`` in place of ``splits`` for the private pass,
-    whose pages are read in parts of at least ``own_chunk`` and at most ``seq_splits`` parts.  ``n_nodes`` bounds the launch grid
-    (rows of the node tables beyond the live nodes have ``q_count == 0`` and cost an empty CTA).  ``arrived``: int32 zeros, at
-    least ``2 * B * Hkv`` of them, that a caller keeps for its calls in one stream (they are zeros again after each)."""
+    last): room for ``[B, Hq, splits, D]`` / ``[B, Hq, splits, 2]``, ``seq_splits`` in place of ``splits`` for the private pass.
+    ``n_nodes`` bounds the launch grid (rows of the node tables beyond the live nodes have ``q_count == 0`` and cost an empty CTA).
+
+    ``arrived``: int32 zeros, at least ``2 * B * Hkv`` of them, that a caller keeps for its calls in one stream.  With them the
+    whole is one launch (private pages in parts of at least ``own_chunk``, at most ``seq_splits`` parts) that leaves them as zeros;
+    it asks more of the tables: every slot is in ``priv_start`` once, also those that are not live, and below one node per level at most.
+    After an error the counters have to be cleared.  Without them, and where a row's parts are more than its counter holds or there is
+    no ``row_mask``, it is :func:`forest_decode_attention_passes`."""
     B, Hq, D = q.shape
     Hkv = kcache.shape[1]
+    if arrived is None or forest.row_mask is None or max(splits, seq_splits) > MAX_PARTS or q.data_ptr() % 16:
+        return forest_decode_attention_passes(q, kcache, vcache, forest, priv_start, priv_active, priv_table, priv_len, part_o, part_ml,
+                                              splits, seq_splits, scale, out, n_nodes)
     num_pages = kcache.shape[0]
     max_pages = priv_table.shape[1]
     scale = scale if scale is not None else 1.0 / math.sqrt(D)
@@ -158,8 +167,6 @@ def forest_decode_attention(q: torch.Tensor, kcache: torch.Tensor, vcache: torch
     if out is None:
         out = torch.empty((B, Hq, D), device=q.device, dtype=torch.bfloat16)
     _check_tables(q, forest, G, priv_start, priv_active, priv_table, priv_len, num_pages)
-    if arrived is None:
-        arrived = torch.zeros(2 * B * Hkv, device=q.device, dtype=torch.int32)
     o_lv = (ctypes.c_void_p * 3)(*[part_o[min(i, nl - 1)].data_ptr() for i in range(3)])
     ml_lv = (ctypes.c_void_p * 3)(*[part_ml[min(i, nl - 1)].data_ptr() for i in range(3)])
     _lib.check(_fn("attn")(_lib.ptr(q), _lib.ptr(kcache), _lib.ptr(vcache), _lib.ptr(out), _lib.ptr(arrived), num_pages, B, Hq, Hkv, D,

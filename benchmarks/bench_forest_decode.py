@@ -75,13 +75,14 @@ def build_tree(roots, root_len, branches, branch_len, leaves, leaf_len, Hq, Hkv,
         "priv_table": torch.from_numpy(priv).to(device), "priv_len": torch.full((B,), leaf_len, **i32),
         "full_table": torch.from_numpy(full).to(device),
         "full_len": torch.full((B,), root_len + branch_len + leaf_len, **i32),
+        "arrived": torch.zeros(2 * B * Hkv, **i32),
     }
     return tabs
 
 
 def run_cascade(t, splits, part_o, part_ml, out):
     return fa.forest_decode_attention(t["q"], t["kc"], t["vc"], t["forest"], t["slot_ids"], t["ones"], t["priv_table"],
-                                      t["priv_len"], part_o, part_ml, splits, 1, out=out)
+                                      t["priv_len"], part_o, part_ml, splits, 1, out=out, arrived=t["arrived"])
 
 
 def run_flat(t, splits, part_o, part_ml, out):

@@ -152,6 +152,46 @@ def test_own_pages_in_parts_with_and_without_shared_nodes(Hq, Hkv, chunk, parts)
         assert (err <= 2 ** -7 * ref.norm(dim=-1)).all()
 
 
+@pytest.mark.parametrize("what", ["no mask", "many parts", "many own parts", "idle entries"])
+def test_calls_that_the_one_launch_form_does_not_take(what):
+    """Without a mask every source counts, parts may be more than 255, and what ``priv_start`` says of entries that are not live does
+    not matter: such calls have the results of the three launches, with counters and without (entries that are not live: without).
+    bf16 probabilities and outputs (2^-9 of a value each) against fp32."""
+    from arctic_platform_b200.ops import _lib
+    from arctic_platform_b200.ops import forest_attention as fa
+    B, Hq, Hkv, D, pages = 6, 8, 2, 128, 5
+    g = torch.Generator(device="cuda").manual_seed(len(what))
+    kc, vc = (torch.randn((B * pages + 9, Hkv, PAGE, D), generator=g, device="cuda").bfloat16() for _ in range(2))
+    q = torch.randn((B, Hq, D), generator=g, device="cuda").bfloat16()
+    i32 = dict(device="cuda", dtype=torch.int32)
+    table = torch.arange(B * pages, **i32).view(B, pages)
+    node = np.arange(B * pages, B * pages + 9, dtype=np.int32)
+    own = torch.tensor([70, 1, 80, 33, 16, 5], **i32)
+    forest = fa.build_forest_tables([fa.ForestNode(0, list(range(B)), node, 140)], B, 9, 32, "cuda")
+    start, active = torch.arange(B, **i32), torch.ones(B, **i32)
+    splits = parts = 2
+    live = list(range(B))
+    if what == "no mask":
+        forest.row_mask = None
+    elif what == "many parts":
+        splits = 300
+    elif what == "many own parts":
+        parts = 256
+    else:
+        active[1::2] = 0
+        start[1], start[3], start[5] = 0, -1, 1 << 20
+        live = [0, 2, 4]
+    part_o = [torch.full((B, Hq, n, D), float("nan"), device="cuda") for n in (splits, parts)]
+    part_ml = [torch.full((B, Hq, n, 2), float("nan"), device="cuda") for n in (splits, parts)]
+    ref = fa.forest_decode_reference(q, kc, vc, [[(node, 140), (table[b].cpu().numpy()[:(n + 15) // 16], n)]
+                                                for b, n in enumerate(own.tolist())])
+    for arrived in [None] + ([] if what == "idle entries" else [torch.zeros(2 * B * Hkv, **i32)]):
+        out = fa.forest_decode_attention(q, kc, vc, forest, start, active, table, own, part_o, part_ml, splits, parts, arrived=arrived)
+        _lib.check_status("decode attention")
+        err = (out[live].float() - ref[live]).norm(dim=-1)
+        assert (err <= 2 ** -7 * ref[live].norm(dim=-1)).all()
+
+
 def test_engine_discovers_shared_headers_and_samples_the_same_distribution():
     """Prompts that start with the same tokens are stored and attended through one header node.  Greedy generation with
     the forest equals greedy generation with plain per-sequence decoding, and the reported log-probs match a
