@@ -24,6 +24,7 @@ enum StatusCode : int {
   kTimeoutFlag = 105,      // wait on a global-memory flag (peer or local)
   kBadArgument = 201,
   kBadRouting = 202,       // a (rank, row) routing entry outside the group: the store was skipped
+  kBadTable = 203,         // a table names more rows than a tile has, or rows that are not there: they were left out
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {

@@ -208,6 +208,10 @@ __device__ __forceinline__ void own_pass(const DecodeAttnParams& p, uint32_t rin
       const int pages = (len + kPage - 1) / kPage;
       const int per = (pages + parts - 1) / parts, p0 = part * per, n = min(pages, p0 + per) - p0;     // n <= 0: nothing
       const int row = p.own_row[e];
+      if (row < 0 || row >= p.B) {       // also of an entry that is not active: its row's arrivals are counted
+        if (lane == 0 && p.status) atomicCAS(p.status, 0, kBadTable);
+        continue;
+      }
       const int* table = p.own_pages + static_cast<long long>(e) * p.own_max_pages + p0;
       int ids = lane < n ? table[lane] : 0;            // of pages [j & ~31, + 32)
       PagedHeads<H> acc;
@@ -315,8 +319,11 @@ decode_cascade_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_co
   const int g = unit % node_heads / p.Hkv;
   const int kvh = unit % p.Hkv;
   const int R = p.Hq / p.Hkv;
-  const int nq = has_unit ? p.q_count[g] : 0;
+  // what a table asks for beyond the tile or the batch is left out and reported: the output rows are staged for 128 and no more
+  const int asked = has_unit ? p.q_count[g] : 0;
   const int qs = has_unit ? p.q_start[g] : 0;
+  const int nq = qs < 0 ? 0 : min(min(asked, 128 / R), p.B - qs);
+  if (asked > 0 && nq != asked && threadIdx.x == 0 && p.status) atomicCAS(p.status, 0, kBadTable);
   const int len = has_unit ? p.kv_len[g] : 0;
   const int n_blocks_all = (len + 127) / 128;
   const int per = (n_blocks_all + p.splits - 1) / p.splits;
@@ -588,9 +595,11 @@ extern "C" {
 //   nodes (G of them, 0: none; q_count 0: unused): q_start, q_count, pages [G, max_pages], kv_len, level (or null), row_mask [B];
 //   `splits` parts per node, partials per level sh_o[l] [B, Hq, splits, 128], sh_ml[l] [B, Hq, splits, 2]; R * max(q_count) <= 128,
 //   rows of the same level are below one node at most;
-//   own pages: entry e < B is row own_row[e] (each row once), read when own_active[e] > 0: own_pages [B, own_max_pages], own_len, in
+//   what a table asks for beyond that, or beyond the batch, is left out and recorded in the status word;
+//   own pages: entry e < B is row own_row[e] (each row once, active or not), read when own_active[e] > 0: own_pages [B, own_max_pages], own_len, in
 //   parts of at least own_chunk pages, at most own_parts of them; own_o [B, Hq, own_parts, 128], own_ml [B, Hq, own_parts, 2].
-// arrived: 2 * B * Hkv zeros, which are zeros again afterwards.  Rows without anything to attend to are zeros.
+// arrived: 2 * B * Hkv zeros, which are zeros again afterwards (unless the tables broke these rules: then the caller clears them).
+// Rows without anything to attend to are zeros.
 int apb_decode_attention(const void* q, const void* kcache, const void* vcache, void* out, int* arrived, long long num_pages, int B,
                          int Hq, int Hkv, int D, float scale, int G, int splits, int n_levels, const int* q_start, const int* q_count,
                          const int* pages, int max_pages, const int* kv_len, const int* level, const int* row_mask,

@@ -192,6 +192,45 @@ def test_calls_that_the_one_launch_form_does_not_take(what):
         assert (err <= 2 ** -7 * ref[live].norm(dim=-1)).all()
 
 
+@pytest.mark.parametrize("what", ["rows", "batch", "start", "own row", "idle row"])
+def test_tables_beyond_the_tile_or_the_batch_are_reported(what):
+    """One launch: more sequences than a tile has rows, sequences behind the batch, own rows outside of it.  What does not fit is
+    left out, the status word says so, and with tables that hold and cleared counters the next call is right."""
+    from arctic_platform_b200.ops import _lib
+    from arctic_platform_b200.ops import forest_attention as fa
+    B, Hq, Hkv, D, pages = 40, 16, 4, 128, 2
+    g = torch.Generator(device="cuda").manual_seed(9)
+    kc, vc = (torch.randn((B * pages + 9, Hkv, PAGE, D), generator=g, device="cuda").bfloat16() for _ in range(2))
+    q = torch.randn((B, Hq, D), generator=g, device="cuda").bfloat16()
+    i32 = dict(device="cuda", dtype=torch.int32)
+    table = torch.arange(B * pages, **i32).view(B, pages)
+    node = np.arange(B * pages, B * pages + 9, dtype=np.int32)
+    own = torch.arange(B, **i32) % 32 + 1
+    arrived = torch.zeros(2 * B * Hkv, **i32)
+    part_o, part_ml = _scratch(B, Hq, D, 2)
+    for wrong in (True, False):
+        forest = fa.build_forest_tables([fa.ForestNode(0, list(range(B)), node, 140)], B, 9, 64 if wrong and what == "rows" else 32, "cuda")
+        start, active = torch.arange(B, **i32), torch.ones(B, **i32)
+        if wrong and what == "batch":
+            forest.q_count[1] += 3
+        elif wrong and what == "start":
+            forest.q_start[1] = -8
+        elif wrong and what == "own row":
+            start[7] = B
+        elif wrong and what == "idle row":
+            start[7], active[7] = -1, 0
+        out = fa.forest_decode_attention(q, kc, vc, forest, start, active, table, own, part_o, part_ml, 2, 2, arrived=arrived)
+        if wrong:
+            with pytest.raises(_lib.KernelError, match="203"):
+                _lib.check_status("decode attention")
+            arrived.zero_()
+    _lib.check_status("decode attention")
+    ref = fa.forest_decode_reference(q, kc, vc, [[(node, 140), (table[b].cpu().numpy()[:(n + 15) // 16], n)]
+                                                for b, n in enumerate(own.tolist())])
+    err = (out.float() - ref).norm(dim=-1)
+    assert (err <= 2 ** -7 * ref.norm(dim=-1)).all()
+
+
 def test_engine_discovers_shared_headers_and_samples_the_same_distribution():
     """Prompts that start with the same tokens are stored and attended through one header node.  Greedy generation with
     the forest equals greedy generation with plain per-sequence decoding, and the reported log-probs match a
