@@ -123,14 +123,19 @@ def build_forest_tables(nodes: Sequence[ForestNode], num_slots: int, max_pages: 
     return ForestTables(t(qs), t(qc), t(pg), t(ln), t(lv), t(mask), G, nl, shared, covered)
 
 
-def _check_tables(q, forest: ForestTables, G: int, priv_start, priv_active, priv_table, priv_len, num_pages: int) -> None:
+def _check_tables(q, Hkv: int, forest: ForestTables, G: int, priv_start, priv_active, priv_table, priv_len, num_pages: int,
+                  each_once: bool = False) -> None:
+    """``each_once``: every slot has to be in ``priv_start`` once, live or not (its arrivals are counted)."""
     from ..utils import checked
     if checked.active_for(q):
         B = q.shape[0]
         if G > 0:
             checked.check_forest(forest.q_start[:G], forest.q_count[:G], forest.pages[:G], forest.kv_len[:G],
-                                 forest.level[:G], B, num_pages, forest.n_levels, 128, PAGE)
-        checked.check_range("priv_start", priv_start, 0, max(1, B), priv_active)
+                                 forest.level[:G], B, num_pages, forest.n_levels, max(1, 128 * Hkv // q.shape[1]), PAGE)
+        if each_once:
+            checked.check_permutation("priv_start", priv_start, B)
+        else:
+            checked.check_range("priv_start", priv_start, 0, max(1, B), priv_active)
         checked.check_page_table("priv_table", priv_table, priv_len, num_pages, PAGE, priv_active)
 
 
@@ -166,7 +171,7 @@ def forest_decode_attention(q: torch.Tensor, kcache: torch.Tensor, vcache: torch
     G = forest.n_nodes if n_nodes is None else int(n_nodes)
     if out is None:
         out = torch.empty((B, Hq, D), device=q.device, dtype=torch.bfloat16)
-    _check_tables(q, forest, G, priv_start, priv_active, priv_table, priv_len, num_pages)
+    _check_tables(q, Hkv, forest, G, priv_start, priv_active, priv_table, priv_len, num_pages, each_once=True)
     o_lv = (ctypes.c_void_p * 3)(*[part_o[min(i, nl - 1)].data_ptr() for i in range(3)])
     ml_lv = (ctypes.c_void_p * 3)(*[part_ml[min(i, nl - 1)].data_ptr() for i in range(3)])
     _lib.check(_fn("attn")(_lib.ptr(q), _lib.ptr(kcache), _lib.ptr(vcache), _lib.ptr(out), _lib.ptr(arrived), num_pages, B, Hq, Hkv, D,
@@ -191,7 +196,7 @@ def forest_decode_attention_passes(q, kcache, vcache, forest: ForestTables, priv
     G = forest.n_nodes if n_nodes is None else int(n_nodes)
     if out is None:
         out = torch.empty((B, Hq, D), device=q.device, dtype=torch.bfloat16)
-    _check_tables(q, forest, G, priv_start, priv_active, priv_table, priv_len, kcache.shape[0])
+    _check_tables(q, Hkv, forest, G, priv_start, priv_active, priv_table, priv_len, kcache.shape[0])
     if G > 0:
         o_lv = (ctypes.c_void_p * 3)(*[part_o[min(i, nl - 1)].data_ptr() for i in range(3)])
         ml_lv = (ctypes.c_void_p * 3)(*[part_ml[min(i, nl - 1)].data_ptr() for i in range(3)])

@@ -112,8 +112,8 @@ def check_page_table(name: str, table: Any, lengths: Any, num_pages: int, page: 
 
 def check_forest(q_start: Any, q_count: Any, pages: Any, kv_len: Any, level: Any, num_slots: int, num_pages: int,
                  n_levels: int, max_rows: int = 128, page: int = 16) -> None:
-    """Node tables of the forest pass: slot runs inside the batch and at most one tile high, levels in range, page
-    lists long enough for the node's tokens and made of valid pages."""
+    """Node tables of the forest pass: slot runs inside the batch and at most one tile high, levels in range, no slot below
+    two nodes of a level, page lists long enough for the node's tokens and made of valid pages."""
     qs, qc = _as_tensor(q_start).long(), _as_tensor(q_count).long()
     live = qc > 0
     check_range("forest.q_count", qc, 0, max_rows + 1)
@@ -123,7 +123,25 @@ def check_forest(q_start: Any, q_count: Any, pages: Any, kv_len: Any, level: Any
         i = _first_bad(over)
         raise TableError(f"forest node {i}: slots {int(qs[i])}..{int(qs[i] + qc[i]) - 1} exceed the batch of {num_slots}")
     check_range("forest.level", level, 0, max(1, n_levels), live)
+    lv = _as_tensor(level).long()
+    for one in range(max(1, n_levels)):
+        at = torch.nonzero(live & (lv == one)).reshape(-1)
+        at = at[torch.argsort(qs[at], stable=True)]
+        clash = (qs[at] + qc[at])[:-1] > qs[at][1:]
+        if bool(clash.any()):
+            i = _first_bad(clash)
+            raise TableError(f"forest nodes {int(at[i])} and {int(at[i + 1])} of level {one} share slot {int(qs[at[i + 1]])}")
     check_page_table("forest.pages", pages, kv_len, num_pages, page, live)
+
+
+def check_permutation(name: str, table: Any, n: int) -> None:
+    """Every one of ``0 .. n - 1`` once."""
+    t = _as_tensor(table).reshape(-1)[:n].long()
+    check_range(name, t, 0, max(1, n))
+    seen = torch.bincount(t, minlength=n)
+    if bool((seen != 1).any()):
+        i = _first_bad(seen != 1)
+        raise TableError(f"{name} names {i} {int(seen[i])} times")
 
 
 def check_routing(dst_rank: Any, dst_row: Any, world: int, rows_cap: int, name: str = "routing") -> None:

@@ -66,6 +66,40 @@ def test_forest_tables_from_the_planner_pass_and_corruptions_are_named():
         checked.check_forest(qs, qc, pg, long, lv, num_slots=8, num_pages=8, n_levels=nl)
 
 
+def test_slots_below_two_nodes_of_a_level_and_rows_beyond_a_tile_are_refused():
+    """Decode attention joins a row when as many parts have arrived as its levels have: a slot below two nodes of one level (of
+    which its row has one place) or missing from the private pass would be joined early, late or never."""
+    from arctic_platform_b200.ops.forest_attention import ForestNode, _check_tables, build_forest_tables, plan_forest
+    page = np.arange(1, dtype=np.int32)
+    nodes = [ForestNode(0, [4, 5, 6], page, 9), ForestNode(1, [0, 1, 2], page, 9), ForestNode(1, [5], page, 9)]
+    qs, qc, pg, ln, lv, _mask, _G, nl, _s, _c = plan_forest(nodes, 8, 2, 32)
+    checked.check_forest(qs, qc, pg, ln, lv, 8, 4, nl)
+    qs, qc, pg, ln, lv, _mask, _G, nl, _s, _c = plan_forest(nodes + [ForestNode(1, [1], page, 9)], 8, 2, 32)
+    with pytest.raises(TableError, match="nodes 1 and 3 of level 1 share slot 1"):
+        checked.check_forest(qs, qc, pg, ln, lv, 8, 4, nl)
+    checked.check_permutation("start", [2, 0, 1], 3)
+    for bad, said in (([0, 0, 1], "start names 0 2 times"), ([0, 1, 3], "start"), ([-1, 0, 1], "start")):
+        with pytest.raises(TableError, match=said):
+            checked.check_permutation("start", bad, 3)
+    # the tile's height follows from the query heads of a key head, whatever the tables were cut for
+    B, Hkv = 40, 2
+    q = torch.zeros(B, 8, 128)
+    forest = build_forest_tables([ForestNode(0, range(B), page, 9)], B, 2, 128, "cpu")
+    start, one, table = torch.arange(B), torch.ones(B, dtype=torch.int32), torch.zeros(B, 1, dtype=torch.int32)
+    checked.force(True)
+    try:
+        with pytest.raises(TableError, match="q_count"):
+            _check_tables(q, Hkv, forest, 1, start, one, table, one, 4)
+        _check_tables(q[:, :6], Hkv, forest, 1, start, one, table, one, 4)        # 3 heads: 42 sequences a tile
+        idle = one.clone()
+        start[3], idle[3] = 0, 0
+        _check_tables(q[:, :6], Hkv, forest, 1, start, idle, table, one, 4)
+        with pytest.raises(TableError, match="priv_start names 0 2 times"):
+            _check_tables(q[:, :6], Hkv, forest, 1, start, idle, table, one, 4, each_once=True)
+    finally:
+        checked.force(None)
+
+
 def test_routing_tile_maps_and_copy_tables():
     checked.check_routing(torch.tensor([0, -1, 3]), torch.tensor([5, 10**6, 0]), world=4, rows_cap=8)
     with pytest.raises(TableError, match="dst_rank"):
