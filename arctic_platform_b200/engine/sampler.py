@@ -469,7 +469,7 @@ class SamplerEngine:
             room = self._sm_count // max(1, nodes * c.num_kv_heads)
             args = (q, kc, vc, self._forest_view(B), self.d_q_start, self.d_active, self.d_priv_table, self.d_priv_len, self.part_o,
                     self.part_ml)
-            if c.is_moe:
+            if c.is_moe or self._passes_asked_for():
                 return forest_decode_attention_passes(*args, max(1, min(self.splits, room)), seq_splits, scale, out=out, n_nodes=nodes)
             return forest_decode_attention(*args, max(1, min(8, self._part_rows // B, room)), max(1, min(64, self._part_rows // B)),
                                            scale, out=out, n_nodes=nodes, arrived=self.d_arrived)
@@ -492,6 +492,11 @@ class SamplerEngine:
         _lib.check(_fn("merge")(o_ptrs, ml_ptrs, sp, 1, None, _lib.ptr(out), None, B, c.num_heads, c.head_dim, s),
                    "decode_merge")
         return out
+
+    @staticmethod
+    def _passes_asked_for() -> bool:
+        """The two switches of the per-sequence pass (its splits, its scalar kernel) are switches of the three launches."""
+        return bool(os.environ.get("APB_DECODE_SEQ_SPLITS") or _lib.cuda_lib().apb_decode_scalar())
 
     def _cascade_on(self) -> bool:
         """The shared-node pass runs on 128-row tensor-core tiles: head_dim 128 and a query-head group that divides

@@ -261,3 +261,35 @@ def test_engine_discovers_shared_headers_and_samples_the_same_distribution():
     for a, b in zip(outs[True], outs[False]):
         assert a["prompt_index"] == b["prompt_index"] and a["token_ids"] == b["token_ids"]
         assert a["logprobs"] == pytest.approx(b["logprobs"], abs=5e-2)
+
+
+@pytest.mark.parametrize("switch", ["none", "splits", "scalar"])
+def test_switches_of_the_per_sequence_pass_reach_models_that_share_a_prompt(switch, monkeypatch):
+    """``APB_DECODE_SEQ_SPLITS`` and the scalar kernel belong to the three launches, so with either of them a rollout makes these; the
+    tokens are those of the one launch, log-probabilities agree to the roundings of bf16 probabilities."""
+    from arctic_platform_b200.engine import sampler
+    from arctic_platform_b200.models.config import PRESETS
+    from arctic_platform_b200.models.decoder import DecoderLM
+    from arctic_platform_b200.ops import _lib
+    cfg = PRESETS["qwen3-tiny-d128"]
+    model = DecoderLM(cfg, "cuda", torch.bfloat16).init_weights(seed=5)
+    prompt = torch.randint(1, cfg.vocab_size, (70,), generator=torch.Generator().manual_seed(2)).tolist()
+    eng = sampler.SamplerEngine(cfg, "cuda", model=model, kv_cache_tokens=1 << 12, max_batch=8, max_seq_len=128, use_cuda_graph=False)
+    sp = {"n": 4, "temperature": 0.0, "max_tokens": 6, "ignore_eos": True}
+    plain = eng.generate([prompt], sp)
+    seen = []
+    for name in ("forest_decode_attention", "forest_decode_attention_passes"):
+        monkeypatch.setattr(sampler, name, lambda *a, _f=getattr(sampler, name), _n=name, **k: seen.append((_n, a[11])) or _f(*a, **k))
+    if switch == "splits":
+        monkeypatch.setenv("APB_DECODE_SEQ_SPLITS", "3")
+    _lib.cuda_lib().apb_decode_use_scalar(int(switch == "scalar"))
+    try:
+        out = eng.generate([prompt], sp)
+    finally:
+        _lib.cuda_lib().apb_decode_use_scalar(0)
+    _lib.check_status("switches")
+    assert {n for n, _ in seen} == {"forest_decode_attention" if switch == "none" else "forest_decode_attention_passes"}
+    if switch == "splits":
+        assert {s for _, s in seen} == {3}
+    for a, b in zip(out, plain):
+        assert a["token_ids"] == b["token_ids"] and a["logprobs"] == pytest.approx(b["logprobs"], abs=5e-2)
