@@ -38,7 +38,8 @@ from ..ops import _lib, gemm, norm
 from ..ops.attention import AttnLayout, attention_fwd_cuda
 from ..utils.transfer_stats import to_device, to_host
 
-from ..ops.forest_attention import ForestNode, forest_decode_attention, forest_decode_attention_passes, plan_forest
+from ..ops.forest_attention import (ForestNode, forest_decode_attention, forest_decode_attention_passes, one_launch_pays,
+                                    plan_forest)
 
 PAGE = 16
 MIN_HEADER_PAGES = 4      # a common prefix shorter than this many pages is not worth a node of its own
@@ -137,6 +138,7 @@ class _Seq:
     group: int
     header_pages: np.ndarray = field(default_factory=lambda: np.zeros(0, dtype=np.int32))   # shared with other prompts
     root: int = -1               # id of the header node, -1 = none
+    own: int = 0                 # tokens on its own pages, the one being fed included
     out: List[int] = field(default_factory=list)
     lps: List[float] = field(default_factory=list)
     finish: Optional[str] = None
@@ -341,6 +343,7 @@ class SamplerEngine:
         self.d_g_pages = self.d_forest[B + 4 * N:].view(N, self.max_pages)
         self.n_levels = 1            # shared levels in use: 1 = prompt nodes only, 2 = header + prompt nodes
         self.forest_stats = {"shared_tokens": 0, "covered_tokens": 0}
+        self._one_launch = True      # decode attention of dense models over shared prompts: one launch or three
         self.out_cap = 0
         self.d_out_tokens = None
         self.d_out_lps = None
@@ -458,21 +461,17 @@ class SamplerEngine:
         scale = 1.0 / math.sqrt(c.head_dim)
         kc, vc = self.kcache[li], self.vcache[li]
         out = torch.empty((B, c.num_heads, c.head_dim), device=self.device, dtype=torch.bfloat16)
-        # per-sequence pass: one CTA per (sequence, kv head) already fills the GPU at rollout batch sizes, so the
-        # KV range is split only when there are fewer CTAs than two waves of SMs
-        seq_splits = max(1, min(self.splits, 296 // max(1, B * c.num_kv_heads)))
+        seq_splits = self._seq_splits(B)
         if os.environ.get("APB_DECODE_SEQ_SPLITS"):               # tuning knob for A/B timing
             seq_splits = max(1, min(self.splits, int(os.environ["APB_DECODE_SEQ_SPLITS"])))
         if self._cascade_on() and self.n_groups > 0:
-            # shared pass: as many KV splits as keep all its CTAs (nodes x KV heads x splits) within one wave of SMs
             nodes = self._group_bucket()
-            room = self._sm_count // max(1, nodes * c.num_kv_heads)
             args = (q, kc, vc, self._forest_view(B), self.d_q_start, self.d_active, self.d_priv_table, self.d_priv_len, self.part_o,
                     self.part_ml)
-            if c.is_moe or self._passes_asked_for():
-                return forest_decode_attention_passes(*args, max(1, min(self.splits, room)), seq_splits, scale, out=out, n_nodes=nodes)
-            return forest_decode_attention(*args, max(1, min(8, self._part_rows // B, room)), max(1, min(64, self._part_rows // B)),
-                                           scale, out=out, n_nodes=nodes, arrived=self.d_arrived)
+            one, three = self._forest_splits(B, nodes)
+            if c.is_moe or not self._one_launch or self._passes_asked_for():
+                return forest_decode_attention_passes(*args, three, seq_splits, scale, out=out, n_nodes=nodes)
+            return forest_decode_attention(*args, *one, scale, out=out, n_nodes=nodes, arrived=self.d_arrived)
         s = _lib.stream_ptr()
         if (c.head_dim == 128 and 16 % (c.num_heads // c.num_kv_heads) == 0 and seq_splits != 3
                 and not _lib.cuda_lib().apb_decode_scalar()):
@@ -492,6 +491,32 @@ class SamplerEngine:
         _lib.check(_fn("merge")(o_ptrs, ml_ptrs, sp, 1, None, _lib.ptr(out), None, B, c.num_heads, c.head_dim, s),
                    "decode_merge")
         return out
+
+    def _seq_splits(self, B: int) -> int:
+        """Parts of a sequence in the per-sequence pass: one CTA per (sequence, kv head) already fills the GPU at rollout batch sizes,
+        so the KV range is split only when there are fewer CTAs than two waves of SMs."""
+        return max(1, min(self.splits, 296 // max(1, B * self.cfg.num_kv_heads)))
+
+    def _forest_splits(self, B: int, nodes: int) -> Tuple[Tuple[int, int], int]:
+        """Parts of a node and of a sequence in the one-launch attention, parts of a node in the shared pass: as many as keep all
+        CTAs of the nodes (nodes x KV heads x parts) within one wave of SMs."""
+        room = self._sm_count // max(1, nodes * self.cfg.num_kv_heads)
+        fit = self._part_rows // B
+        return (max(1, min(8, fit, room)), max(1, min(64, fit))), max(1, min(self.splits, room))
+
+    def _choose_attention(self, B: int, live: Dict[int, _Seq]) -> None:
+        """One launch or three for the next steps, by the lengths that the host knows (a sequence that has ended since the last look
+        counts as if it went on)."""
+        self._one_launch = True
+        if self.cfg.is_moe or not self._cascade_on() or self.n_groups <= 0:
+            return
+        own = np.zeros(B, dtype=np.int64)
+        for slot, sq in live.items():
+            own[slot] = sq.own
+        nodes = self._group_bucket()
+        one, three = self._forest_splits(B, nodes)
+        self._one_launch = one_launch_pays(*self._node_runs, own, nodes, self.cfg.num_heads, self.cfg.num_kv_heads, *one, three,
+                                           self._seq_splits(B), self._sm_count)
 
     @staticmethod
     def _passes_asked_for() -> bool:
@@ -720,7 +745,8 @@ class SamplerEngine:
             for _ in range(n):
                 self._decode_step(B)
             return
-        key = (B, self._group_bucket() if self._cascade_on() else 0, self.n_levels, self._filter_on)
+        nodes = self._group_bucket() if self._cascade_on() else 0
+        key = (B, nodes, self.n_levels, self._filter_on, nodes == 0 or self._one_launch)
         g = self._graphs.get(key)
         if g is None:
             # the first steps run eagerly (kernel attribute set-up, device binding, allocator warm-up)
@@ -860,7 +886,12 @@ class SamplerEngine:
             if B > 0:
                 if admitted or retired:
                     self._set_groups(group_members, root_members, live)
+                if admitted:
+                    self._choose_attention(bucket, live)
                 self._run_steps(bucket, self.sync_interval)
+                for sq in live.values():
+                    sq.own += self.sync_interval
+                self._choose_attention(bucket, live)       # for the steps after these, while they run
             # ---- harvest
             fin = to_host(self.d_finished[:max(B, 1)]).numpy() if B else np.zeros(0, dtype=np.int32)
             done_slots = [s for s in list(live) if fin[s]]
@@ -1033,7 +1064,7 @@ class SamplerEngine:
                 pt[i, n_hdr + n_sh:n_hdr + n_sh + n_priv] = sq.private_pages
                 pv[i, :n_priv] = sq.private_pages
                 sh[i] = (n_hdr + n_sh) * PAGE
-                plen[i] = sq.prompt_len - sh[i] + 1
+                plen[i] = sq.own = sq.prompt_len - int(sh[i]) + 1
             from ..utils import checked
             if checked.enabled():                   # host arrays: no synchronisation involved
                 checked.check_page_table("page_table", pt, plen + sh - 1, self.num_pages, PAGE)
@@ -1112,6 +1143,7 @@ class SamplerEngine:
         if G > self.n_node_rows:
             raise RuntimeError(f"prefix forest needs {G} table rows, the engine holds {self.n_node_rows}")
         self.n_groups, self.n_levels = G, nl
+        self._node_runs = ln[:G], qc[:G]
         self.forest_stats = {"shared_tokens": shared, "covered_tokens": covered}
 
         B, N = self.max_batch, self.n_node_rows

@@ -293,3 +293,36 @@ def test_switches_of_the_per_sequence_pass_reach_models_that_share_a_prompt(swit
         assert {s for _, s in seen} == {3}
     for a, b in zip(out, plain):
         assert a["token_ids"] == b["token_ids"] and a["logprobs"] == pytest.approx(b["logprobs"], abs=5e-2)
+
+
+def test_rollout_moves_to_the_three_launches_where_they_are_faster(monkeypatch):
+    """A rollout in which the rule turns over between two looks at the finished flags (and back, for the next call) has the tokens of one
+    that keeps to either form, captured or not; the lengths that the rule is given are those on the device."""
+    from arctic_platform_b200.engine import sampler
+    from arctic_platform_b200.models.config import PRESETS
+    from arctic_platform_b200.models.decoder import DecoderLM
+    from arctic_platform_b200.ops import _lib
+    cfg = PRESETS["qwen3-tiny-d128"]
+    model = DecoderLM(cfg, "cuda", torch.bfloat16).init_weights(seed=5)
+    g = torch.Generator().manual_seed(3)
+    prompts = [torch.randint(1, cfg.vocab_size, (n,), generator=g).tolist() for n in (70, 33)]
+    sp = {"n": 3, "temperature": 0.0, "max_tokens": 40, "ignore_eos": True}
+    outs, told = {}, []
+    for name, rule in (("one", lambda own: True), ("three", lambda own: False), ("turns", lambda own: max(own) < 30)):
+        def pays(node_tokens, node_slots, own, *a, _r=rule):
+            assert len(node_tokens) == len(node_slots) == 2 and set(node_slots) == {3} and set(node_tokens) == {64, 32}
+            told.append(list(own))
+            return _r(own)
+        monkeypatch.setattr(sampler, "one_launch_pays", pays)
+        for graph in (False, True):
+            eng = sampler.SamplerEngine(cfg, "cuda", model=model, kv_cache_tokens=1 << 12, max_batch=8, max_seq_len=128, sync_interval=8,
+                                        use_cuda_graph=graph)
+            outs[name, graph] = [eng.generate(prompts, sp) for _ in range(2)]
+            assert len(eng._graphs) == (0 if not graph else 2 if name == "turns" else 1)
+        _lib.check_status("rollout")
+    want = outs["one", False][0]
+    for got in outs.values():
+        for call in got:
+            for a, b in zip(call, want):
+                assert a["token_ids"] == b["token_ids"] and a["logprobs"] == pytest.approx(b["logprobs"], abs=5e-2)
+    assert told[0][:6] == [70 % PAGE + 1] * 3 + [33 % PAGE + 1] * 3 and told[1][0] == told[0][0] + 8
