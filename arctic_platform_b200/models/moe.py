@@ -18,6 +18,7 @@ from typing import Optional, Tuple
 
 import torch
 from torch import nn
+from torch.autograd import forward_ad
 
 from ..ops import gemm, rows
 from .config import DecoderConfig
@@ -37,8 +38,9 @@ def route_topk(logits: torch.Tensor, k: int, renorm: bool, score_func: str = "so
       inference engine): the weights are gathered from the current scores, nothing is re-selected.
     (arctic_platform/model/implementations/qwen35/models/layers/moe.py:196-269, NemotronHRouter in the same file)."""
     if (routed_experts is None and logits.is_cuda and n_group <= 1 and logits.dim() == 2 and logits.shape[-1] <= 512
-            and score_func in ("softmax", "sigmoid") and not (torch.is_grad_enabled() and logits.requires_grad)):
-        # without gradients: decision and scores from one kernel, the same bits
+            and score_func in ("softmax", "sigmoid") and not (torch.is_grad_enabled() and logits.requires_grad)
+            and forward_ad.unpack_dual(logits).tangent is None):
+        # without gradients of either direction: decision and scores from one kernel, the same bits
         from ..ops.rl_ops import moe_route_weights
         return moe_route_weights(logits, k, score_func, expert_bias, renorm, route_scale)
     x = logits.float()

@@ -165,6 +165,31 @@ def test_route_without_gradients_has_the_bits_of_the_pass_with_them(E, k, score,
         assert torch.equal(i0, i1) and torch.equal(w0.detach(), w1)
 
 
+@pytest.mark.parametrize("score", ["softmax", "sigmoid"])
+@pytest.mark.parametrize("grad", [False, True])
+def test_route_keeps_a_forward_mode_tangent(score, grad):
+    """Weights of logits that carry a tangent carry one too, with and without gradients enabled: the derivative of scores, gather and
+    division in 64 bits (fp32 sums of up to 40 terms: 1e-5)."""
+    import torch.autograd.forward_ad as fw
+    from arctic_platform_b200.models.moe import route_topk
+    torch.manual_seed(4)
+    x, t = torch.randn(31, 40, device="cuda") * 2, torch.randn(31, 40, device="cuda")
+    with torch.set_grad_enabled(grad), fw.dual_level():
+        w, idx = route_topk(fw.make_dual(x, t), 5, True, score, 1.5)
+        got = fw.unpack_dual(w)
+        assert got.tangent is not None and got.tangent.dtype == torch.float32
+
+        def weights(y):
+            s = (torch.softmax(y, -1) if score == "softmax" else torch.sigmoid(y)).gather(-1, idx)
+            return s / s.sum(-1, keepdim=True) * 1.5
+
+    want, slope = torch.func.jvp(weights, (x.double(),), (t.double(),))
+    assert (got.primal - want).abs().max() <= 1e-5 and (got.tangent - slope).abs().max() <= 1e-5 * slope.abs().max()
+    with torch.set_grad_enabled(grad):
+        w0, idx0 = route_topk(x, 5, True, score, 1.5)
+    assert torch.equal(idx, idx0) and torch.equal(got.primal, w0)
+
+
 @pytest.mark.parametrize("E", [1, 2, 7, 64, 129, 511, 512])
 def test_group_tiles_of_any_number_of_experts(E):
     """Prefix sums of two experts a thread: odd and even numbers, experts without rows, more than a block of rows."""
