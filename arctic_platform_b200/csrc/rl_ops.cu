@@ -104,7 +104,8 @@ __global__ void __launch_bounds__(256) grpo_token_loss_kernel(const GrpoArgs a) 
 }
 
 // One warp per token.  scores = softmax(logits) or sigmoid(logits); selection on scores + bias; k rounds of warp
-// arg-max (ties go to the lower expert index, like a stable descending sort).  E <= 32 * kRouteMaxPerLane.
+// arg-max (ties go to the lower expert index, like a stable descending sort); where only NaN and -inf are left, the lowest expert that
+// is not taken, so that a choice always names an expert.  E <= 32 * kRouteMaxPerLane.
 constexpr int kRouteMaxPerLane = 16;
 //
 // With `weight`, the scores of the chosen experts go out too, with `renorm` (k <= 8) divided by their sum, times `scale`: conversion,
@@ -159,6 +160,7 @@ moe_route_kernel(const LOGIT* __restrict__ logits, long long ld, const float* __
     sc[j] = e < E ? sc[j] + (bias ? bias[e] : 0.f) : -INFINITY;
   }
   float mine = 0.f;               // lane r: score of the r-th choice, for sums
+  uint32_t taken = 0;             // bit j: expert lane + 32 j
   for (int r = 0; r < k; ++r) {
     float best = -INFINITY;
     int be = 0x7fffffff;
@@ -179,15 +181,22 @@ moe_route_kernel(const LOGIT* __restrict__ logits, long long ld, const float* __
         be = oe;
       }
     }
+    if (be >= E) {
+      const int j = __ffs(~taken) - 1;          // k <= E: some lane has one left
+      be = __reduce_min_sync(0xffffffffu, lane + 32 * j);
+    }
     if (lane == 0) {
       idx_out[tok * k + r] = be;
       if (counts) atomicAdd(counts + be, 1);
     }
 #pragma unroll
     for (int j = 0; j < kRouteMaxPerLane; ++j)
-      if (be == lane + 32 * j) sc[j] = -INFINITY;   // taken
+      if (be == lane + 32 * j) {
+        sc[j] = -INFINITY;
+        taken |= 1u << j;
+      }
     if (weight) {
-      const float x = static_cast<float>(row[be < E ? be : 0]);
+      const float x = static_cast<float>(row[be]);
       const float score = sigmoid ? 1.f / (1.f + expf(-x)) : expf(x - mx) / exact_sum;
       if (lane == r) mine = score;
       if (lane == 0 && !renorm) weight[tok * k + r] = score * scale;

@@ -165,6 +165,37 @@ def test_route_without_gradients_has_the_bits_of_the_pass_with_them(E, k, score,
         assert torch.equal(i0, i1) and torch.equal(w0.detach(), w1)
 
 
+@pytest.mark.parametrize("E,k", [(8, 3), (33, 33), (40, 6), (512, 10)])
+@pytest.mark.parametrize("grad", [False, True])
+def test_route_names_experts_whatever_the_logits_are(E, k, grad):
+    """NaN, infinities and a bias that leaves fewer experts than are chosen: every choice is one of the experts, none twice; scores that
+    are left are chosen in their order, ahead of the others; rows of plain numbers next to them choose as by themselves."""
+    from arctic_platform_b200.models.moe import route_topk
+    nan, inf = float("nan"), float("inf")
+    torch.manual_seed(E)
+    x = torch.randn(64, E, device="cuda")
+    plain = x.clone()
+    x[1::8] = nan
+    x[2::8, ::3] = nan
+    x[3::8] = -inf
+    x[4::8, 1] = inf
+    x[5::8, 2:] = -inf
+    shut = torch.full((E,), -inf, device="cuda")
+    shut[-2:] = 0
+    with torch.set_grad_enabled(grad):
+        for score in ("softmax", "sigmoid"):
+            for bias in (None, shut):
+                idx = route_topk(x.clone().requires_grad_(grad), k, True, score, 1.0, bias)[1]
+                assert ((idx >= 0) & (idx < E)).all() and (idx.sort(1).values.diff(dim=1) > 0).all()
+                alone = route_topk(plain[::8].clone().requires_grad_(grad), k, True, score, 1.0, bias)[1]
+                assert torch.equal(idx[::8], alone)
+                if bias is not None:
+                    assert torch.equal(alone[:, :2].sort(1).values, torch.tensor([[E - 2, E - 1]] * 8, device="cuda"))
+            if k <= E - (E + 2) // 3:
+                some = route_topk(x[2::8].clone().requires_grad_(grad), k, True, "sigmoid")[1]
+                assert torch.equal(some, x[2::8].nan_to_num(-1e9).topk(k, dim=1).indices)
+
+
 @pytest.mark.parametrize("score", ["softmax", "sigmoid"])
 @pytest.mark.parametrize("grad", [False, True])
 def test_route_keeps_a_forward_mode_tangent(score, grad):
