@@ -475,7 +475,7 @@ attn_delta_kernel(const __nv_bfloat16* __restrict__ o, long long ldo, const __nv
 
 extern "C" {
 
-// Backward of apb_attn_fwd for head_dim 128.
+// Backward of apb_attn_fwd_form for head_dim 128.
 //   q/o/d_o [T, Hq*D], k/v [T, Hkv*D] bf16 with row strides ld*; lse [Hq,T] from the forward.
 //   delta [Hq,T] fp32 scratch (written here); dq_acc [T, Hq*D] fp32 accumulator, zeroed by the caller;
 //   dk/dv [T, Hkv*D] bf16 outputs.  cta/list are the tables of apb_rt_attn_bwd_work.

@@ -543,10 +543,4 @@ int apb_attn_fwd_form(const void* q, const void* k, const void* v, void* o, floa
   kernel<<<grid, kAttnThreads, smem, stream>>>(tq, tk, tv, p);
   return static_cast<int>(cudaGetLastError());
 }
-
-int apb_attn_fwd(const void* q, const void* k, const void* v, void* o, float* lse, const int* work, int num_work,
-                 int T, int Hq, int Hkv, int D, long long ldq, long long ldk, long long ldv, long long ldo,
-                 float scale, cudaStream_t stream) {
-  return apb_attn_fwd_form(q, k, v, o, lse, work, num_work, T, Hq, Hkv, D, ldq, ldk, ldv, ldo, scale, 0, stream);
-}
 }

@@ -163,10 +163,12 @@ __device__ __forceinline__ int arrive_row(const DecodeAttnParams& p, int row, in
   return now >> 16;
 }
 
-// Own pages: warp `w` of `warps` takes every warps-th (sequence, part, key head).  A key head has 8 H query heads or less, STAGES
-// pages of the warp's ring.  Parts are as long as the work divided by the warps, a little longer until they are no more than the
-// warps: ragged lengths cost one round of nearly equal parts.
-template <int H, int STAGES, int KB>
+// Own pages: warp `w` of `warps` takes every warps-th (sequence, part, key head).  A key head has 8 H query heads or less.
+// Parts are as long as the work divided by the warps, a little longer until they are no more than the warps; where there are more
+// (sequence, key head) pairs than warps nothing is cut, and warps walk one or two whole sequences (16 % over an even split at 1024
+// pairs of equal length, more if lengths differ).  Which parts a row has thus depends on the lengths of all rows of the batch, and
+// with them its last bits.
+template <int H>
 __device__ __forceinline__ void own_pass(const DecodeAttnParams& p, uint32_t ring, int w, int warps, int lane) {
   const int R = p.Hq / p.Hkv, units = p.B * p.Hkv;
   auto tokens = [&](int e) { return e < p.B && p.own_active[e] > 0 ? max(0, p.own_len[e]) : 0; };
@@ -218,23 +220,23 @@ __device__ __forceinline__ void own_pass(const DecodeAttnParams& p, uint32_t rin
       acc.start(p.q + (static_cast<long long>(row) * p.Hq + kvh * R) * 128, n > 0 ? R : 0, lane);
       auto issue = [&](int j, int id) {
         const long long at = (static_cast<long long>(id) * p.Hkv + kvh) * (kPage * 128);
-        decode_issue_page(ring + (j % STAGES) * 2 * kMmaPageBytes, p.kcache + at, p.vcache + at, lane);
+        decode_issue_page(ring + (j % kDaOwnStages) * 2 * kMmaPageBytes, p.kcache + at, p.vcache + at, lane);
       };
-      for (int j = 0; j < STAGES - 1; ++j) {
+      for (int j = 0; j < kDaOwnStages - 1; ++j) {
         const int id = __shfl_sync(0xffffffffu, ids, j);
         if (j < n) issue(j, id);
         cp_async_commit();
       }
 #pragma unroll 1
       for (int j = 0; j < n; ++j) {
-        const int jn = j + STAGES - 1;
+        const int jn = j + kDaOwnStages - 1;
         if ((jn & 31) == 0) ids = jn + lane < n ? table[jn + lane] : 0;
         const int id = __shfl_sync(0xffffffffu, ids, jn & 31);
         if (jn < n) issue(jn, id);
         cp_async_commit();
-        cp_async_wait<STAGES - 1>();
+        cp_async_wait<kDaOwnStages - 1>();
         __syncwarp();
-        acc.page(ring + (j % STAGES) * 2 * kMmaPageBytes, len - (p0 + j) * kPage, p.scale_log2, lane);
+        acc.page(ring + (j % kDaOwnStages) * 2 * kMmaPageBytes, len - (p0 + j) * kPage, p.scale_log2, lane);
         __syncwarp();
       }
       cp_async_wait<0>();
@@ -283,7 +285,7 @@ __device__ __forceinline__ void own_pass(const DecodeAttnParams& p, uint32_t rin
         }
       }
       n_own = __shfl_sync(0xffffffffu, n_own, 0);
-      if (n_own > 0) join_heads<KB>(p, row, kvh, n_own, lane);
+      if (n_own > 0) join_heads<1>(p, row, kvh, n_own, lane);
     }
     before += here;
   }
@@ -576,7 +578,7 @@ decode_cascade_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_co
   } else {
     pdl_wait();
     const int w = warp - 2 - kDaSoftWarps;
-    own_pass<H, kDaOwnStages, 1>(p, smem_u32(smem_own) + w * kDaOwnRing, w * gridDim.x + blockIdx.x, gridDim.x * kDaOwnWarps, lane);
+    own_pass<H>(p, smem_u32(smem_own) + w * kDaOwnRing, w * gridDim.x + blockIdx.x, gridDim.x * kDaOwnWarps, lane);
   }
 
   tc_fence_before();

@@ -148,7 +148,7 @@ def attention_fwd_cuda(q, k, v, layout: AttnLayout, scale: float, need_lse: bool
     code = _fwd_fn()(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(o), _lib.ptr(lse), _lib.ptr(work),
                      work.shape[0], T, Hq, Hkv, D, q.stride(0), k.stride(0), v.stride(0), o.stride(0),
                      scale, int(tmem_o), _lib.stream_ptr())
-    _lib.check(code, "apb_attn_fwd")
+    _lib.check(code, "apb_attn_fwd_form")
     return o, lse
 
 
