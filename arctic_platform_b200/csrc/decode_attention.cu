@@ -15,9 +15,14 @@
 // A CTA of the shared form: warp 0 TMA producer, warp 1 MMA issuer, warps 2-9 softmax (a row belongs to two threads, each with 64 of a
 // block's 128 columns), warps 10-13 own pages.  As three launches -- shared pass with one thread per row, a pass of 96 KB CTAs over
 // the own pages that could not start beside it, a merge -- a layer of 8 prompts x 16 samples (2048 shared tokens, 17 own, 8 key heads)
-// took 24 + 19 + 6 us behind each other; the own pages are a few KB per warp and hide behind the shared ones here.
-// Together they take 26 us.  (Sequences that share nothing are left to paged_decode_mma_kernel, whose clusters join their parts
-// sooner than counters in memory do: 7 us against 10 for one sequence of 400 tokens, 33 against 36 for 41 of 500 to 1500.)
+// took 24 + 19 + 6 us behind each other; 17 own tokens are a few KB per warp and hide behind the shared ones here: 27 us together.
+// Long own contexts do not: four warps with one page ahead keep 32 KB under way per SM where paged_decode_mma_kernel has 128 KB, and at
+// 2048 own tokens the three launches take 194 us, this one 210 (lengths from 1 to 2048: 124 and 175).  The rollout engine takes the
+// one that is faster at the lengths at hand (one_launch_pays in ops/forest_attention.py).  (Sequences that share nothing are left to
+// paged_decode_mma_kernel, whose clusters join their parts sooner than counters in memory do: 7 us against 10 for one sequence of 400
+// tokens, 33 against 36 for 41 of 500 to 1500.)
+// Compiled for up to 8 query heads a key head it spills nothing, for 16 the walk over own pages spills 224 bytes (128 registers a
+// thread are all that 448 threads leave).
 //
 // The KV blocks of a node are software-pipelined: tensor memory holds TWO score buffers, the MMA warp issues Q K^T of block j+1 before
 // it waits for the probabilities of block j, and P V accumulates over all blocks in ONE output buffer in tensor memory that the

@@ -1004,7 +1004,8 @@ class SamplerEngine:
         scale = 1.0 / math.sqrt(self.cfg.head_dim)
         n_layers = self.cfg.num_layers
         if self.device.type == "cuda":
-            for lay in (layout, end_layout)[:1 + int(short)]:      # work tables: their copies wait for the stream, which is idle here
+            # work tables: their copies wait for the stream, so they go ahead of the prompts (of a second batch behind the first one's)
+            for lay in (layout, end_layout)[:1 + int(short)]:
                 lay.fwd_work(self.cfg.num_heads, self.cfg.num_kv_heads, ids.device)
 
         def attn(li, q, k, v):
@@ -1040,7 +1041,7 @@ class SamplerEngine:
             tok += n_tok
         for runs in batches:
             batch = [pm for run in runs for pm in run["prompts"]]
-            # all that the host knows goes up before the prompts run, and nothing behind them makes it wait
+            # all that the host knows goes up before the batch's prompts run, so that nothing has to wait behind them
             rows = [gi for gi, (_, mem) in enumerate(batch) for _ in mem]
             slots = [slot for _, mem in batch for slot in mem]
             n = len(slots)
@@ -1156,8 +1157,9 @@ class SamplerEngine:
         self.d_forest[:len(blob)].copy_(self._upload(blob))
 
     def _upload(self, a: np.ndarray) -> torch.Tensor:
-        """A host array on the device.  The copy is staged at once and the host does not wait for the work queued in front of it
-        (``torch.tensor(..., device=...)`` and stores of single elements do)."""
+        """A host array on the device, by a copy that does not ask for the work queued in front of it to end, as
+        ``torch.tensor(..., device=...)`` and stores of single elements do.  The source is pageable: the driver stages such copies
+        (8 x 16 samples: 5 ms of idle GPU a call instead of 11), but is free to wait."""
         return to_device(torch.from_numpy(a), self.device)
 
     # ------------------------------------------------------------------ weights / sleep / wake

@@ -185,9 +185,9 @@ def forest_decode_attention(q: torch.Tensor, kcache: torch.Tensor, vcache: torch
 def forest_decode_attention_passes(q, kcache, vcache, forest: ForestTables, priv_start, priv_active, priv_table, priv_len, part_o,
                                    part_ml, splits: int, seq_splits: int, scale: Optional[float] = None,
                                    out: Optional[torch.Tensor] = None, n_nodes: Optional[int] = None) -> torch.Tensor:
-    """The same attention in three launches (shared nodes, own pages, merge), twice as long and with other last bits: models with
-    experts keep it.  A router turns last bits into other experts now and then, and a greedy rollout behind another expert moves
-    by a fifth."""
+    """The same attention in three launches (shared nodes, own pages, merge), with other last bits.  Up to twice as long where own
+    pages are few, faster where they are many (:func:`one_launch_pays`).  Models with experts keep it: a router turns last bits into
+    other experts now and then, and a greedy rollout behind another expert moves by a fifth."""
     B, Hq, D = q.shape
     Hkv = kcache.shape[1]
     scale = scale if scale is not None else 1.0 / math.sqrt(D)
