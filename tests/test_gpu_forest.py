@@ -15,13 +15,23 @@ def _scratch(B, Hq, D, splits):
             [torch.empty((B, Hq, splits, 2), **f32) for _ in range(4)])
 
 
-def test_shared_pass_when_single_rows_meet_much_larger_scores_late():
+def _forms(B, Hkv):
+    """The op as three launches and as one, with the counters that the latter wants."""
+    from arctic_platform_b200.ops import forest_attention as fa
+    arrived = torch.zeros(2 * B * Hkv, device="cuda", dtype=torch.int32)
+    return {"three": fa.forest_decode_attention_passes,
+            "one": lambda *a, **k: fa.forest_decode_attention(*a, arrived=arrived, **k)}
+
+
+@pytest.mark.parametrize("form", ["three", "one"])
+@pytest.mark.parametrize("Hq,Hkv", [(32, 8), (32, 4), (16, 8)])
+def test_shared_pass_when_single_rows_meet_much_larger_scores_late(form, Hq, Hkv):
     """The running reference of a row moves when its scores outgrow it by 2^8; here some rows of a warp do, others never, in
     several blocks.  bf16 weights and outputs (2^-8 at most each, half of that in the
     mean) against fp32."""
     from arctic_platform_b200.ops import _lib
     from arctic_platform_b200.ops import forest_attention as fa
-    B, Hq, Hkv, D, tokens = 12, 32, 8, 128, 1216
+    B, D, tokens = 12, 128, 1216
     g = torch.Generator(device="cuda").manual_seed(5)
     n = tokens // PAGE
     kc, vc = (torch.randn((n + B, Hkv, PAGE, D), generator=g, device="cuda").to(torch.bfloat16) for _ in range(2))
@@ -32,20 +42,21 @@ def test_shared_pass_when_single_rows_meet_much_larger_scores_late():
     q = q.to(torch.bfloat16)
     pages = np.arange(n, dtype=np.int32)
     own = [np.array([n + b], dtype=np.int32) for b in range(B)]
-    forest = fa.build_forest_tables([fa.ForestNode(0, list(range(B)), pages, tokens)], B, n + 1, 32, "cuda")
+    forest = fa.build_forest_tables([fa.ForestNode(0, list(range(B)), pages, tokens)], B, n + 1, 128 * Hkv // Hq, "cuda")
     i32 = dict(device="cuda", dtype=torch.int32)
     table = torch.zeros((B, n + 1), **i32)
     table[:, 0] = torch.arange(n, n + B, **i32)
     part_o, part_ml = _scratch(B, Hq, D, 2)
-    out = fa.forest_decode_attention(q, kc, vc, forest, torch.arange(B, **i32), torch.ones(B, **i32), table,
-                                     torch.full((B,), 5, **i32), part_o, part_ml, 2, 2)
+    out = _forms(B, Hkv)[form](q, kc, vc, forest, torch.arange(B, **i32), torch.ones(B, **i32), table, torch.full((B,), 5, **i32), part_o,
+                               part_ml, 2, 2)
     _lib.check_status("forest")
     ref = fa.forest_decode_reference(q, kc, vc, [[(pages, tokens), (own[b], 5)] for b in range(B)])
     assert (out.float() - ref).norm() <= 2 ** -7 * ref.norm()
 
 
-@pytest.mark.parametrize("Hq,Hkv", [(32, 8), (16, 8), (8, 8)])
-def test_three_level_forest_matches_dense_attention(Hq, Hkv):
+@pytest.mark.parametrize("form", ["three", "one"])
+@pytest.mark.parametrize("Hq,Hkv", [(32, 8), (16, 8), (8, 8), (32, 4), (16, 1)])
+def test_three_level_forest_matches_dense_attention(Hq, Hkv, form):
     """Headers shared by several prompts, prompts shared by their rollouts, private tails; one sequence without a
     header, one prompt node whose slots are not consecutive, and a header with more sequences than one tile holds."""
     from arctic_platform_b200.ops import _lib
@@ -102,8 +113,8 @@ def test_three_level_forest_matches_dense_attention(Hq, Hkv):
     po, pml = _scratch(B, Hq, D, splits)
     for buf in po + pml:
         buf.fill_(float("nan"))                                            # stale partials must never be merged
-    out = fa.forest_decode_attention(q, kc, vc, forest, torch.arange(B, **i32), torch.ones(B, **i32),
-                                     torch.from_numpy(priv).cuda(), torch.from_numpy(plen).cuda(), po, pml, splits, 1)
+    out = _forms(B, Hkv)[form](q, kc, vc, forest, torch.arange(B, **i32), torch.ones(B, **i32), torch.from_numpy(priv).cuda(),
+                               torch.from_numpy(plen).cuda(), po, pml, splits, 1)
     _lib.check_status("forest")
     ref = fa.forest_decode_reference(q, kc, vc, ctx)
     assert torch.isfinite(out.float()).all()
@@ -326,3 +337,24 @@ def test_rollout_moves_to_the_three_launches_where_they_are_faster(monkeypatch):
             for a, b in zip(call, want):
                 assert a["token_ids"] == b["token_ids"] and a["logprobs"] == pytest.approx(b["logprobs"], abs=5e-2)
     assert told[0][:6] == [70 % PAGE + 1] * 3 + [33 % PAGE + 1] * 3 and told[1][0] == told[0][0] + 8
+
+
+def test_counters_that_a_failed_call_left_behind_do_not_reach_the_next_one():
+    """A call that an error ends between launches may leave arrivals: the next call begins with counters of zero."""
+    from arctic_platform_b200.engine import sampler
+    from arctic_platform_b200.models.config import PRESETS
+    from arctic_platform_b200.models.decoder import DecoderLM
+    from arctic_platform_b200.ops import _lib
+    cfg = PRESETS["qwen3-tiny-d128"]
+    model = DecoderLM(cfg, "cuda", torch.bfloat16).init_weights(seed=5)
+    prompt = torch.randint(1, cfg.vocab_size, (70,), generator=torch.Generator().manual_seed(2)).tolist()
+    eng = sampler.SamplerEngine(cfg, "cuda", model=model, kv_cache_tokens=1 << 12, max_batch=8, max_seq_len=128)
+    sp = {"n": 4, "temperature": 0.0, "max_tokens": 6, "ignore_eos": True}
+    want = eng.generate([prompt], sp)
+    assert eng._one_launch and not eng.d_arrived.any()
+    eng.d_arrived.copy_(torch.arange(eng.d_arrived.numel()) % 5)          # as from a kernel that gave up
+    got = eng.generate([prompt], sp)
+    _lib.check_status("after arrivals")
+    assert not eng.d_arrived.any()
+    for a, b in zip(got, want):
+        assert a["token_ids"] == b["token_ids"] and a["logprobs"] == pytest.approx(b["logprobs"], abs=5e-2)

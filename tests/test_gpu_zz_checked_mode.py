@@ -35,7 +35,8 @@ def test_sampler_with_forest_runs_clean_in_checked_mode(checked_on):
     assert [o["token_ids"] for o in outs[False]] == [o["token_ids"] for o in outs[True]]
 
 
-def test_forest_op_refuses_a_corrupted_table_before_launching(checked_on):
+@pytest.mark.parametrize("counters", [False, True])
+def test_forest_op_refuses_a_corrupted_table_before_launching(checked_on, counters):
     from arctic_platform_b200.ops.forest_attention import ForestNode, build_forest_tables, forest_decode_attention
     from arctic_platform_b200.ops import _lib
     B, Hq, Hkv, D, num_pages, max_pages = 8, 8, 2, 128, 32, 8
@@ -49,18 +50,19 @@ def test_forest_op_refuses_a_corrupted_table_before_launching(checked_on):
     start = torch.arange(B, device="cuda", dtype=torch.int32)
     active = torch.ones(B, device="cuda", dtype=torch.int32)
     splits = 2
+    kept = {"arrived": torch.zeros(2 * B * Hkv, device="cuda", dtype=torch.int32)} if counters else {}
     part_o = [torch.zeros(B, Hq, splits, D, device="cuda") for _ in range(2)]
     part_ml = [torch.zeros(B, Hq, splits, 2, device="cuda") for _ in range(2)]
-    out = forest_decode_attention(q, kc, vc, forest, start, active, priv_table, priv_len, part_o, part_ml, splits, splits)
+    out = forest_decode_attention(q, kc, vc, forest, start, active, priv_table, priv_len, part_o, part_ml, splits, splits, **kept)
     _lib.check_status("forest checked")
     assert torch.isfinite(out.float()).all()
     before = _lib.launch_count()
     priv_table[3, 0] = num_pages + 5                                   # a page id outside the cache
     with pytest.raises(checked_on.TableError, match=r"priv_table\[3, 0\]"):
-        forest_decode_attention(q, kc, vc, forest, start, active, priv_table, priv_len, part_o, part_ml, splits, splits)
+        forest_decode_attention(q, kc, vc, forest, start, active, priv_table, priv_len, part_o, part_ml, splits, splits, **kept)
     assert _lib.launch_count() == before                               # nothing ran with the bad table
     priv_table[3, 0] = 7
     forest.kv_len[0] = 16 * max_pages + 1                              # a node longer than its page list
     with pytest.raises(checked_on.TableError, match="pages"):
-        forest_decode_attention(q, kc, vc, forest, start, active, priv_table, priv_len, part_o, part_ml, splits, splits)
+        forest_decode_attention(q, kc, vc, forest, start, active, priv_table, priv_len, part_o, part_ml, splits, splits, **kept)
     assert _lib.launch_count() == before
