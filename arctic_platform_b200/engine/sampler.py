@@ -138,7 +138,6 @@ class _Seq:
     group: int
     header_pages: np.ndarray = field(default_factory=lambda: np.zeros(0, dtype=np.int32))   # shared with other prompts
     root: int = -1               # id of the header node, -1 = none
-    own: int = 0                 # tokens on its own pages, the one being fed included
     out: List[int] = field(default_factory=list)
     lps: List[float] = field(default_factory=list)
     finish: Optional[str] = None
@@ -344,6 +343,7 @@ class SamplerEngine:
         self.n_levels = 1            # shared levels in use: 1 = prompt nodes only, 2 = header + prompt nodes
         self.forest_stats = {"shared_tokens": 0, "covered_tokens": 0}
         self._one_launch = True      # decode attention of dense models over shared prompts: one launch or three
+        self._own = np.zeros(B, dtype=np.int32)      # tokens on a slot's own pages, the one being fed included (as d_priv_len)
         self.out_cap = 0
         self.d_out_tokens = None
         self.d_out_lps = None
@@ -504,18 +504,15 @@ class SamplerEngine:
         fit = self._part_rows // B
         return (max(1, min(8, fit, room)), max(1, min(64, fit))), max(1, min(self.splits, room))
 
-    def _choose_attention(self, B: int, live: Dict[int, _Seq]) -> None:
+    def _choose_attention(self, B: int) -> None:
         """One launch or three for the next steps, by the lengths that the host knows (a sequence that has ended since the last look
         counts as if it went on)."""
         self._one_launch = True
         if self.cfg.is_moe or not self._cascade_on() or self.n_groups <= 0:
             return
-        own = np.zeros(B, dtype=np.int64)
-        for slot, sq in live.items():
-            own[slot] = sq.own
         nodes = self._group_bucket()
         one, three = self._forest_splits(B, nodes)
-        self._one_launch = one_launch_pays(*self._node_runs, own, nodes, self.cfg.num_heads, self.cfg.num_kv_heads, *one, three,
+        self._one_launch = one_launch_pays(*self._node_runs, self._own[:B], nodes, self.cfg.num_heads, self.cfg.num_kv_heads, *one, three,
                                            self._seq_splits(B), self._sm_count)
 
     @staticmethod
@@ -779,6 +776,7 @@ class SamplerEngine:
         self.d_topp.fill_(float(sp.top_p))
         if getattr(self, "d_arrived", None) is not None:
             self.d_arrived.zero_()         # a call that an error ended may have left arrivals behind
+        self._own[:] = 0
         prompts_np = [np.asarray(p, dtype=np.int64) for p in prompts]
         for p in prompts_np:
             if len(p) == 0:
@@ -887,17 +885,17 @@ class SamplerEngine:
                 if admitted or retired:
                     self._set_groups(group_members, root_members, live)
                 if admitted:
-                    self._choose_attention(bucket, live)
+                    self._choose_attention(bucket)
                 self._run_steps(bucket, self.sync_interval)
-                for sq in live.values():
-                    sq.own += self.sync_interval
-                self._choose_attention(bucket, live)       # for the steps after these, while they run
+                self._own[self._own > 0] += self.sync_interval
+                self._choose_attention(bucket)             # for the steps after these, while they run
             # ---- harvest
             fin = to_host(self.d_finished[:max(B, 1)]).numpy() if B else np.zeros(0, dtype=np.int32)
             done_slots = [s for s in list(live) if fin[s]]
             retired = bool(done_slots)
             if done_slots:
                 done_t = self._upload(np.asarray(done_slots, dtype=np.int64))
+                self._own[done_slots] = 0
                 freed: List[np.ndarray] = []
                 nout = to_host(self.d_out_idx[:B, 0]).numpy()
                 toks = to_host(self.d_out_tokens[:B]).numpy()
@@ -1065,11 +1063,12 @@ class SamplerEngine:
                 pt[i, n_hdr + n_sh:n_hdr + n_sh + n_priv] = sq.private_pages
                 pv[i, :n_priv] = sq.private_pages
                 sh[i] = (n_hdr + n_sh) * PAGE
-                plen[i] = sq.own = sq.prompt_len - int(sh[i]) + 1
+                plen[i] = sq.prompt_len - sh[i] + 1
             from ..utils import checked
             if checked.enabled():                   # host arrays: no synchronisation involved
                 checked.check_page_table("page_table", pt, plen + sh - 1, self.num_pages, PAGE)
                 checked.check_page_table("priv_table", pv, plen - 1, self.num_pages, PAGE)
+            self._own[slots] = plen
             longs = self._upload(np.asarray(rows + slots + src + dst, dtype=np.int64))
             rows_t, st, src_t, dst_t = longs.split([n, n, len(src), len(src)])
             ints = self._upload(np.concatenate([pt.reshape(-1), pv.reshape(-1), plen, sh,

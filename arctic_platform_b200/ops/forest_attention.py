@@ -216,60 +216,20 @@ def forest_decode_attention_passes(q, kcache, vcache, forest: ForestTables, priv
     return out
 
 
-def _rounds(times: np.ndarray, sms: int) -> float:
-    """Blocks of the given times, in turn on ``sms`` places: the longest of each round."""
-    padded = np.zeros(-(-len(times) // sms) * sms)
-    padded[:len(times)] = times
-    return float(padded.reshape(-1, sms).max(1).sum())
-
-
 def one_launch_pays(node_tokens: np.ndarray, node_slots: np.ndarray, own_tokens: np.ndarray, node_rows: int, Hq: int, Hkv: int, splits: int,
                     own_parts: int, pass_splits: int, seq_splits: int, sms: int) -> bool:
     """Whether :func:`forest_decode_attention` with counters (``splits`` parts of a node, ``own_parts`` of a sequence at most) takes no
-    longer than the three launches (``pass_splits``, ``seq_splits``).
-
-    The one launch saves two ramps, has two threads per row of a node and hides short private pages behind the nodes.  But it reads
-    private pages with four warps an SM, each one page (8 KB) ahead, and leaves sequences whole where there are more of them than warps;
-    ``paged_decode_mma_kernel`` keeps four times as many bytes under way and runs at the copy rate.  And the last part of a node joins
-    all its rows in eight warps.  So it loses where a warp's chain of pages is long against the saving.  Where that is depends on everything else.
-    A layer in us, 32 / 8 heads, three launches against one: 8 prompts of 2048 x 16 samples with 17 own tokens 47 / 27, with 512
-    84 / 74, with 1024 121 / 120, with 2048 194 / 210, with 1 to 1024 83 / 101, with 1 to 2048 124 / 175; 40 prompts of 512 x 4
-    (512 tiles, 3.5 rounds of blocks) with 128 own 74 / 77, with 1024 156 / 234; one of 8192 x 2 with 2048 own 55 / 29; one of 416
-    x 32 with 8 own, 16 / 4 heads, 17 / 24.
-
-    Hence the sums below, in us, fitted to both times at 2600 sizes (2 to 256 sequences, 64 to 8192 shared and 8 to 2500 own tokens, equal
-    or not, all or a fifth of the slots live, 2 to 8 heads a key head): within 7 % in the mean.  At 1631 other sizes of these ranges what
-    they choose takes, in all, 0.7 % more than the better of the two, 14 % less than the three launches and 12 % less than the one.
+    longer than the three launches (``pass_splits``, ``seq_splits``): sums of what each form waits for, in the C++ runtime
+    (``runtime_decode.cpp``, where the measured times stand).
 
     ``node_tokens``, ``node_slots``: of each row of the node tables in use; ``own_tokens [B]``: private tokens of every slot, 0 for
     idle ones; ``node_rows``: table rows in the launch."""
-    B = len(own_tokens)
-    blocks, slots = -(-np.asarray(node_tokens) // 128), np.asarray(node_slots)
-    pages = -(-np.asarray(own_tokens) // PAGE)
-    each = int(pages.sum()) * Hkv / sms                                        # pages per SM
-    joined, rows = B * Hkv / 1024, -(-Hq // (4 * Hkv))                          # (slot, key head) pairs; rounds of four heads
-    three = (8.8 + _rounds(np.tile(np.repeat(3.15 + 2.25 * -(-blocks // pass_splits), Hkv), pass_splits), sms) + 0.158 * each
-             + 0.117 * int(pages.max(initial=0)) / seq_splits + 11.1 * joined)
-    # the chains of the one launch, as its kernel cuts them
-    units = node_rows * Hkv * splits
-    grid = max(units, min(-(-B * Hkv // 4), sms))
-    pages = np.maximum(pages, 1)
-    most, warps = int(pages.max(initial=1)), 4 * grid
-    chunk = max(OWN_CHUNK, -(-most // own_parts), -(-int(pages.sum()) * Hkv // warps))
-    for _ in range(12 if B <= 256 else 0):
-        if chunk >= most or int((-(-pages // chunk)).sum()) * Hkv <= warps:
-            break
-        chunk += max(1, chunk >> 4)
-    parts = -(-pages // chunk)
-    items = np.repeat(-(-pages // parts), parts * Hkv)
-    chains = np.zeros(-(-len(items) // warps) * warps, dtype=np.int64)
-    chains[:len(items)] = items
-    times = 5.7 + 0.59 * chains.reshape(-1, 4, grid).sum(0).max(0)
-    mine = np.zeros(node_rows)
-    mine[:len(blocks)] = 1.43 * -(-blocks // splits) + 0.6 * rows * -(-slots // 8) * (splits / 2 + 1)
-    times[:units] += np.tile(np.repeat(mine, Hkv), splits)
-    one = _rounds(times, sms) + 7.0 * joined + 0.54 * rows * int(parts.max(initial=1)) + 0.037 * each
-    return one <= three
+    tokens, slots, own = (np.ascontiguousarray(a, dtype=np.int32) for a in (node_tokens, node_slots, own_tokens))
+    rc = _lib.rt_lib().apb_rt_one_launch_pays(tokens.ctypes.data, slots.ctypes.data, len(tokens), own.ctypes.data, len(own), node_rows, Hq, Hkv,
+                                              splits, own_parts, OWN_CHUNK, pass_splits, seq_splits, sms)
+    if rc < 0:
+        raise ValueError("one_launch_pays: sizes out of range")
+    return bool(rc)
 
 
 def forest_decode_reference(q: torch.Tensor, kcache: torch.Tensor, vcache: torch.Tensor,

@@ -12,7 +12,8 @@ MEASURED = [
     (32, 8, 4, 8, 512, 512, 1.0, 28.6, 24.1), (32, 8, 40, 4, 512, 17, 1.0, 64.7, 56.7), (32, 8, 40, 4, 512, 256, 1.0, 84.3, 102.3),
     (32, 8, 64, 2, 1024, 1024, 1.0, 184.1, 165.7), (32, 8, 1, 8, 16384, 2048, 1.0, 98.0, 48.2), (16, 8, 1, 8, 512, 2048, 1.0, 25.3, 35.3),
     (32, 4, 4, 8, 512, 2048, 1.0, 42.5, 50.5), (32, 4, 8, 16, 2048, 128, 1.0, 38.5, 26.2),
-    (16, 4, 1, 32, 416, 8, 1.0, 17.1, 24.4), (32, 8, 1, 16, 2048, 17, 1.0, 21.2, 18.8), (64, 8, 4, 16, 3728, 15, 1.0, 42.1, 33.8),
+    (16, 4, 1, 32, 416, 8, 1.0, 17.1, 24.4), (16, 8, 64, 16, 256, 17, 1.0, 153.4, 250.8), (32, 8, 16, 32, 2048, 17, 1.0, 117.2, 80.4),
+    (32, 8, 1, 16, 2048, 17, 1.0, 21.2, 18.8), (64, 8, 4, 16, 3728, 15, 1.0, 42.1, 33.8),
 ]
 
 
@@ -39,3 +40,5 @@ def test_any_batch_has_an_answer(B, Hkv, nodes):
     for own in (np.zeros(B, dtype=np.int64), np.arange(B), np.full(B, 100000)):
         for splits in (1, 8):
             assert one_launch_pays(np.zeros(min(nodes, 3), dtype=np.int32), np.ones(min(nodes, 3), dtype=np.int32), own, nodes, 8 * Hkv, Hkv, splits, 4, 4, 1, 148) in (True, False)
+    with pytest.raises(ValueError, match="out of range"):
+        one_launch_pays(np.zeros(2), np.ones(2), np.ones(B), 1, 8 * Hkv, Hkv, 1, 4, 4, 1, 148)
