@@ -29,7 +29,7 @@ from arctic_platform_b200.ops import forest_attention as fa  # noqa: E402
 PAGE = fa.PAGE
 
 
-def build_tree(roots, root_len, branches, branch_len, leaves, leaf_len, Hq, Hkv, D, device, seed=0):
+def build_tree(roots, root_len, branches, branch_len, leaves, leaf_len, Hq, Hkv, D, device, seed=0, launches=3):
     """KV cache with random contents plus the tables of both kernels.  Slots are numbered depth first, so the
     sequences below every node are consecutive."""
     assert root_len % PAGE == 0 and branch_len % PAGE == 0, "shared nodes hold whole pages"
@@ -75,14 +75,14 @@ def build_tree(roots, root_len, branches, branch_len, leaves, leaf_len, Hq, Hkv,
         "priv_table": torch.from_numpy(priv).to(device), "priv_len": torch.full((B,), leaf_len, **i32),
         "full_table": torch.from_numpy(full).to(device),
         "full_len": torch.full((B,), root_len + branch_len + leaf_len, **i32),
-        "arrived": torch.zeros(2 * B * Hkv, **i32),
+        "arrived": torch.zeros(2 * B * Hkv, **i32), "launches": launches,
     }
     return tabs
 
 
 def run_cascade(t, splits, part_o, part_ml, out):
     return fa.forest_decode_attention(t["q"], t["kc"], t["vc"], t["forest"], t["slot_ids"], t["ones"], t["priv_table"],
-                                      t["priv_len"], part_o, part_ml, splits, 1, out=out, arrived=t["arrived"])
+                                      t["priv_len"], part_o, part_ml, splits, 1, out=out, arrived=t["arrived"] if t["launches"] == 1 else None)
 
 
 def run_flat(t, splits, part_o, part_ml, out):
@@ -135,6 +135,7 @@ def main():
     ap.add_argument("--splits", type=int, default=4)
     ap.add_argument("--iters", type=int, default=20)
     ap.add_argument("--hbm-gbs", type=float, default=6536.0)
+    ap.add_argument("--launches", type=int, default=3, choices=(1, 3), help="form of the cascade (shared pass, own pages, merge; or one)")
     ap.add_argument("--no-baseline", action="store_true")
     ap.add_argument("--check", action="store_true")
     args = ap.parse_args()
@@ -142,7 +143,7 @@ def main():
     Hq, Hkv, D = args.heads, args.kv_heads, 128
     res = {"bench": "forest_decode", "heads": [Hq, Hkv, D], "page": PAGE}
     if args.check:
-        t = build_tree(2, 256, 2, 64, 3, 40, Hq, Hkv, D, dev, seed=1)
+        t = build_tree(2, 256, 2, 64, 3, 40, Hq, Hkv, D, dev, seed=1, launches=args.launches)
         po, pml = scratch(t["B"], Hq, D, args.splits, dev)
         out = torch.empty_like(t["q"])
         ref = fa.forest_decode_reference(t["q"], t["kc"], t["vc"], t["contexts"])
@@ -151,7 +152,8 @@ def main():
         _lib.check_status("forest check")
         res["check_max_abs_err"] = {"cascade": e1, "flat": e2}
         assert e1 < 2e-2 and e2 < 2e-2, res
-    t = build_tree(args.roots, args.root_len, args.branches, args.branch_len, args.leaves, args.leaf_len, Hq, Hkv, D, dev)
+    t = build_tree(args.roots, args.root_len, args.branches, args.branch_len, args.leaves, args.leaf_len, Hq, Hkv, D, dev,
+                   launches=args.launches)
     B = t["B"]
     po, pml = scratch(B, Hq, D, args.splits, dev)
     out = torch.empty_like(t["q"])
