@@ -343,7 +343,8 @@ class SamplerEngine:
         self.n_levels = 1            # shared levels in use: 1 = prompt nodes only, 2 = header + prompt nodes
         self.forest_stats = {"shared_tokens": 0, "covered_tokens": 0}
         self._one_launch = True      # decode attention of dense models over shared prompts: one launch or three
-        self._own = np.zeros(B, dtype=np.int32)      # tokens on a slot's own pages, the one being fed included (as d_priv_len)
+        self._own = np.zeros(B, dtype=np.int32)      # tokens on a slot's own pages, the one being fed included (as d_priv_len),
+        self._left = np.zeros(B, dtype=np.int32)     # and steps that it has before it at most
         self.out_cap = 0
         self.d_out_tokens = None
         self.d_out_lps = None
@@ -505,14 +506,13 @@ class SamplerEngine:
         return (max(1, min(8, fit, room)), max(1, min(64, fit))), max(1, min(self.splits, room))
 
     def _choose_attention(self, B: int) -> None:
-        """One launch or three for the next steps, by the lengths that the host knows (a sequence that has ended since the last look
-        counts as if it went on)."""
+        """One launch or three until sequences join again, by the lengths that the host knows now and the steps that may follow."""
         self._one_launch = True
         if self.cfg.is_moe or not self._cascade_on() or self.n_groups <= 0:
             return
         nodes = self._group_bucket()
         one, three = self._forest_splits(B, nodes)
-        self._one_launch = one_launch_pays(*self._node_runs, self._own[:B], nodes, self.cfg.num_heads, self.cfg.num_kv_heads, *one, three,
+        self._one_launch = one_launch_pays(*self._node_runs, self._own[:B], self._left[:B], nodes, self.cfg.num_heads, self.cfg.num_kv_heads, *one, three,
                                            self._seq_splits(B), self._sm_count)
 
     @staticmethod
@@ -888,7 +888,7 @@ class SamplerEngine:
                     self._choose_attention(bucket)
                 self._run_steps(bucket, self.sync_interval)
                 self._own[self._own > 0] += self.sync_interval
-                self._choose_attention(bucket)             # for the steps after these, while they run
+                self._left -= self.sync_interval
             # ---- harvest
             fin = to_host(self.d_finished[:max(B, 1)]).numpy() if B else np.zeros(0, dtype=np.int32)
             done_slots = [s for s in list(live) if fin[s]]
@@ -1068,7 +1068,7 @@ class SamplerEngine:
             if checked.enabled():                   # host arrays: no synchronisation involved
                 checked.check_page_table("page_table", pt, plen + sh - 1, self.num_pages, PAGE)
                 checked.check_page_table("priv_table", pv, plen - 1, self.num_pages, PAGE)
-            self._own[slots] = plen
+            self._own[slots], self._left[slots] = plen, sp.max_tokens - 1
             longs = self._upload(np.asarray(rows + slots + src + dst, dtype=np.int64))
             rows_t, st, src_t, dst_t = longs.split([n, n, len(src), len(src)])
             ints = self._upload(np.concatenate([pt.reshape(-1), pv.reshape(-1), plen, sh,

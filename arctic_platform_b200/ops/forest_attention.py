@@ -216,17 +216,17 @@ def forest_decode_attention_passes(q, kcache, vcache, forest: ForestTables, priv
     return out
 
 
-def one_launch_pays(node_tokens: np.ndarray, node_slots: np.ndarray, own_tokens: np.ndarray, node_rows: int, Hq: int, Hkv: int, splits: int,
-                    own_parts: int, pass_splits: int, seq_splits: int, sms: int) -> bool:
+def one_launch_pays(node_tokens: np.ndarray, node_slots: np.ndarray, own_tokens: np.ndarray, left: np.ndarray, node_rows: int, Hq: int,
+                    Hkv: int, splits: int, own_parts: int, pass_splits: int, seq_splits: int, sms: int) -> bool:
     """Whether :func:`forest_decode_attention` with counters (``splits`` parts of a node, ``own_parts`` of a sequence at most) takes no
-    longer than the three launches (``pass_splits``, ``seq_splits``): sums of what each form waits for, in the C++ runtime
-    (``runtime_decode.cpp``, where the measured times stand).
+    longer than the three launches (``pass_splits``, ``seq_splits``) over the steps ahead: sums of what each form waits for, in the
+    C++ runtime (``runtime_decode.cpp``, where the measured times stand).
 
     ``node_tokens``, ``node_slots``: of each row of the node tables in use; ``own_tokens [B]``: private tokens of every slot, 0 for
-    idle ones; ``node_rows``: table rows in the launch."""
-    tokens, slots, own = (np.ascontiguousarray(a, dtype=np.int32) for a in (node_tokens, node_slots, own_tokens))
-    rc = _lib.rt_lib().apb_rt_one_launch_pays(tokens.ctypes.data, slots.ctypes.data, len(tokens), own.ctypes.data, len(own), node_rows, Hq, Hkv,
-                                              splits, own_parts, OWN_CHUNK, pass_splits, seq_splits, sms)
+    idle ones; ``left [B]``: steps that a slot still has before it (0: the lengths at hand); ``node_rows``: table rows in the launch."""
+    tokens, slots, own, steps = (np.ascontiguousarray(a, dtype=np.int32) for a in (node_tokens, node_slots, own_tokens, left))
+    rc = _lib.rt_lib().apb_rt_one_launch_pays(tokens.ctypes.data, slots.ctypes.data, len(tokens), own.ctypes.data, steps.ctypes.data, len(own),
+                                              node_rows, Hq, Hkv, splits, own_parts, OWN_CHUNK, pass_splits, seq_splits, sms)
     if rc < 0:
         raise ValueError("one_launch_pays: sizes out of range")
     return bool(rc)

@@ -29,7 +29,7 @@ def test_the_faster_form_is_chosen(case):
     runs = prompts * -(-samples // tile)
     node_rows = 1 << (runs - 1).bit_length()
     room, fit = sms // (node_rows * Hkv), max(4 * B, 256) // B
-    got = one_launch_pays(np.full(runs, shared), np.full(runs, min(samples, tile)), tokens, node_rows, Hq, Hkv, max(1, min(8, fit, room)),
+    got = one_launch_pays(np.full(runs, shared), np.full(runs, min(samples, tile)), tokens, np.zeros(B), node_rows, Hq, Hkv, max(1, min(8, fit, room)),
                           min(64, fit), max(1, min(4, room)), max(1, min(4, 296 // (B * Hkv))), sms)
     assert got == (one < three)
 
@@ -39,6 +39,24 @@ def test_any_batch_has_an_answer(B, Hkv, nodes):
     """No tokens, one slot, more slots than the kernel looks for better parts at, nodes of no tokens."""
     for own in (np.zeros(B, dtype=np.int64), np.arange(B), np.full(B, 100000)):
         for splits in (1, 8):
-            assert one_launch_pays(np.zeros(min(nodes, 3), dtype=np.int32), np.ones(min(nodes, 3), dtype=np.int32), own, nodes, 8 * Hkv, Hkv, splits, 4, 4, 1, 148) in (True, False)
+            assert one_launch_pays(np.zeros(min(nodes, 3), dtype=np.int32), np.ones(min(nodes, 3), dtype=np.int32), own, own[::-1], nodes, 8 * Hkv, Hkv,
+                                   splits, 4, 4, 1, 148) in (True, False)
     with pytest.raises(ValueError, match="out of range"):
-        one_launch_pays(np.zeros(2), np.ones(2), np.ones(B), 1, 8 * Hkv, Hkv, 1, 4, 4, 1, 148)
+        one_launch_pays(np.zeros(2), np.ones(2), np.ones(B), np.ones(B), 1, 8 * Hkv, Hkv, 1, 4, 4, 1, 148)
+
+
+@pytest.mark.parametrize("prompts,samples,shared,left,one", [(8, 16, 2048, 33, True), (8, 16, 2048, 2047, True), (40, 4, 512, 17, True),
+                                                            (40, 4, 512, 1024, False), (8, 16, 2048, 8000, False)])
+def test_the_choice_is_for_the_steps_ahead(prompts, samples, shared, left, one):
+    """From the first token on: what is saved while responses are short is set against what is lost when they are long.  A slot that has
+    no steps left counts as idle."""
+    B, sms = prompts * samples, 148
+    rows = 1 << (prompts - 1).bit_length()
+    room, fit = sms // (rows * 8), max(4 * B, 256) // B
+    sizes = (rows, 32, 8, max(1, min(8, fit, room)), min(64, fit), max(1, min(4, room)), max(1, min(4, 296 // (B * 8))), sms)
+    runs = np.full(prompts, shared), np.full(prompts, samples)
+    assert one_launch_pays(*runs, np.full(B, 1), np.full(B, left), *sizes) == one
+    long = np.full(B, 1)
+    long[::2] = 5000
+    ends = np.where(long > 1, -7, left)
+    assert one_launch_pays(*runs, long, ends, *sizes) == one_launch_pays(*runs, np.where(long > 1, 0, 1), np.full(B, left), *sizes)

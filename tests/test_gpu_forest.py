@@ -306,9 +306,9 @@ def test_switches_of_the_per_sequence_pass_reach_models_that_share_a_prompt(swit
         assert a["token_ids"] == b["token_ids"] and a["logprobs"] == pytest.approx(b["logprobs"], abs=5e-2)
 
 
-def test_rollout_moves_to_the_three_launches_where_they_are_faster(monkeypatch):
-    """A rollout in which the rule turns over between two looks at the finished flags (and back, for the next call) has the tokens of one
-    that keeps to either form, captured or not; the lengths that the rule is given are those on the device."""
+def test_rollout_chooses_a_form_when_sequences_join(monkeypatch):
+    """Rollouts that keep to either form, or take one and then the other as prompts join (4 slots, so the second prompt waits for the
+    first), have the same tokens, captured or not; the rule is asked when sequences have joined and told what is on the device."""
     from arctic_platform_b200.engine import sampler
     from arctic_platform_b200.models.config import PRESETS
     from arctic_platform_b200.models.decoder import DecoderLM
@@ -318,25 +318,28 @@ def test_rollout_moves_to_the_three_launches_where_they_are_faster(monkeypatch):
     g = torch.Generator().manual_seed(3)
     prompts = [torch.randint(1, cfg.vocab_size, (n,), generator=g).tolist() for n in (70, 33)]
     sp = {"n": 3, "temperature": 0.0, "max_tokens": 40, "ignore_eos": True}
-    outs, told = {}, []
-    for name, rule in (("one", lambda own: True), ("three", lambda own: False), ("turns", lambda own: max(own) < 30)):
-        def pays(node_tokens, node_slots, own, *a, _r=rule):
-            assert len(node_tokens) == len(node_slots) == 2 and set(node_slots) == {3} and set(node_tokens) == {64, 32}
-            told.append(list(own))
-            return _r(own)
-        monkeypatch.setattr(sampler, "one_launch_pays", pays)
+    outs = {}
+    for name, rule in (("one", lambda own: True), ("three", lambda own: False), ("turns", lambda own: own[0] == 70 % PAGE + 1)):
         for graph in (False, True):
-            eng = sampler.SamplerEngine(cfg, "cuda", model=model, kv_cache_tokens=1 << 12, max_batch=8, max_seq_len=128, sync_interval=8,
+            told = []
+            eng = sampler.SamplerEngine(cfg, "cuda", model=model, kv_cache_tokens=1 << 12, max_batch=4, max_seq_len=128, sync_interval=8,
                                         use_cuda_graph=graph)
+
+            def pays(node_tokens, node_slots, own, left, *sizes, _r=rule):
+                told.append((list(node_tokens), list(node_slots), list(own), list(left)))
+                assert eng.d_priv_len[:len(own)].tolist() == told[-1][2]
+                return _r(own)
+            monkeypatch.setattr(sampler, "one_launch_pays", pays)
             outs[name, graph] = [eng.generate(prompts, sp) for _ in range(2)]
             assert len(eng._graphs) == (0 if not graph else 2 if name == "turns" else 1)
+            want = [([64], [3], [70 % PAGE + 1] * 3 + [0], [39] * 3), ([32], [3], [33 % PAGE + 1] * 3 + [0], [39] * 3)]
+            assert [(a, b, c, d[:3]) for a, b, c, d in told] == want * 2
         _lib.check_status("rollout")
     want = outs["one", False][0]
     for got in outs.values():
         for call in got:
             for a, b in zip(call, want):
                 assert a["token_ids"] == b["token_ids"] and a["logprobs"] == pytest.approx(b["logprobs"], abs=5e-2)
-    assert told[0][:6] == [70 % PAGE + 1] * 3 + [33 % PAGE + 1] * 3 and told[1][0] == told[0][0] + 8
 
 
 def test_counters_that_a_failed_call_left_behind_do_not_reach_the_next_one():
