@@ -114,7 +114,9 @@ int32_t apb_rt_one_launch_pays(const int32_t* node_tokens, const int32_t* node_s
       seq_splits < 1 || sms < 1)
     return -1;
   const Launch p{node_tokens, node_slots, nodes, B, node_rows, Hq, Hkv, splits, own_parts, own_chunk, pass_splits, seq_splits, sms};
-  const int64_t longest = std::max(0, *std::max_element(left, left + B));
+  int64_t longest = 0;                    // of the slots in use: one whose sequence has ended early may have steps left
+  for (int e = 0; e < B; ++e)
+    if (own_tokens[e] > 0) longest = std::max<int64_t>(longest, left[e]);
   double three = 0, one = 0;
   std::vector<int64_t> pages(B);
   for (int k = 0; k < kStretches && (k == 0 || longest > 16); ++k) {

@@ -512,8 +512,8 @@ class SamplerEngine:
             return
         nodes = self._group_bucket()
         one, three = self._forest_splits(B, nodes)
-        self._one_launch = one_launch_pays(*self._node_runs, self._own[:B], self._left[:B], nodes, self.cfg.num_heads, self.cfg.num_kv_heads, *one, three,
-                                           self._seq_splits(B), self._sm_count)
+        self._one_launch = one_launch_pays(*self._node_runs, self._own[:B], self._left[:B], nodes, self.cfg.num_heads,
+                                           self.cfg.num_kv_heads, *one, three, self._seq_splits(B), self._sm_count)
 
     @staticmethod
     def _passes_asked_for() -> bool:
