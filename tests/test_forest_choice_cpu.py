@@ -62,4 +62,4 @@ def test_the_choice_is_for_the_steps_ahead(prompts, samples, shared, left, one):
     assert one_launch_pays(*runs, long, ends, *sizes) == one_launch_pays(*runs, np.where(long > 1, 0, 1), np.full(B, left), *sizes)
     some = np.full(B, 1)                 # a slot whose sequence has ended early may have steps left: they do not count
     some[-1] = 0
-    assert one_launch_pays(*runs, some, np.where(some > 0, left, 80000), *sizes) == one
+    assert one_launch_pays(*runs, some, np.where(some > 0, left, 80000), *sizes) == one_launch_pays(*runs, some, some * left, *sizes)
