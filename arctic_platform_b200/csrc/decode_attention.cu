@@ -312,9 +312,12 @@ decode_cascade_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_co
   uint64_t* q_full = bars + 2 * kDaSlots;
   uint64_t* s_full = q_full + 1;    // [2] MMA -> softmax: scores of block j are in S[j & 1]
   uint64_t* p_full = s_full + 2;    // [2] softmax -> MMA: probabilities of block j are in S[j & 1]
-  uint64_t* o_full = p_full + 2;    // [1] MMA -> softmax: P V of block j has been added to O (one phase per block)
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(o_full + 1);
-  static_assert((2 * kDaSlots + 6) * 8 + 4 <= kDaBarBytes, "barriers");
+  // [2] MMA -> softmax: P V of block j has been added to O.  A barrier for even blocks and one for odd ones: when the last block is
+  // waited for, no more is known than that the products up to the third last have landed (they are ahead of the last scores in
+  // the tensor core's order), and one barrier with a phase per block would take the third last's parity for the last one's.
+  uint64_t* o_full = p_full + 2;
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(o_full + 2);
+  static_assert((2 * kDaSlots + 7) * 8 + 4 <= kDaBarBytes, "barriers");
   float* halves = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bars) + kDaBarBytes);      // [2][2][128]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -348,8 +351,8 @@ decode_cascade_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_co
       for (int b = 0; b < 2; ++b) {
         mbar_init(&s_full[b], 1);
         mbar_init(&p_full[b], kDaSoftWarps * 32);
+        mbar_init(&o_full[b], 1);
       }
-      mbar_init(o_full, 1);
       mbar_fence_init();
     }
     if (warp == 1) {
@@ -446,7 +449,7 @@ decode_cascade_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_co
           for (int k = 0; k < 128 / 16; ++k)
             umma_bf16_ts(tmem_base + 256, tmem_base + b * 128 + k * 8, desc_v + slot * (kDaTile >> 4) + k * 128, idesc_o,
                          (j > 0 || k > 0) ? 1u : 0u);
-          tc_commit(o_full);
+          tc_commit(&o_full[b]);
           tc_commit(&kv_empty[slot]);
         }
         __syncwarp();
@@ -495,7 +498,7 @@ decode_cascade_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_co
             // row in tensor memory (once the previous block's P V has landed; block 0 has nothing to rescale)
             const float alpha = (m_ref == -INFINITY) ? 0.f : exp2f(m_ref - m_new);
             if (j > 0) {
-              ok = __all_sync(0xffffffffu, mbar_wait(o_full, (j - 1) & 1, p.status, kTimeoutTmemFull));
+              ok = __all_sync(0xffffffffu, mbar_wait(&o_full[b ^ 1], ((j - 1) >> 1) & 1, p.status, kTimeoutTmemFull));
               tc_fence_after();
               if (ok) {
 #pragma unroll 1
@@ -538,7 +541,8 @@ decode_cascade_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_co
       // bytes each
       float* stage = reinterpret_cast<float*>(smem_kv);
       if (n_blocks > 0) {
-        ok = ok && __all_sync(0xffffffffu, mbar_wait(o_full, (n_blocks - 1) & 1, p.status, kTimeoutTmemFull));
+        const int last = n_blocks - 1;
+        ok = ok && __all_sync(0xffffffffu, mbar_wait(&o_full[last & 1], (last >> 1) & 1, p.status, kTimeoutTmemFull));
         tc_fence_after();
         if (ok && live) {
 #pragma unroll

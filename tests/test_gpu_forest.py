@@ -361,3 +361,33 @@ def test_counters_that_a_failed_call_left_behind_do_not_reach_the_next_one():
     assert not eng.d_arrived.any()
     for a, b in zip(got, want):
         assert a["token_ids"] == b["token_ids"] and a["logprobs"] == pytest.approx(b["logprobs"], abs=5e-2)
+
+
+@pytest.mark.parametrize("form", ["three", "one"])
+@pytest.mark.parametrize("Hq,Hkv,samples,tokens", [(32, 8, 16, 2175), (32, 8, 8, 300), (32, 4, 16, 4000), (16, 2, 4, 1000)])
+def test_repeats_have_the_same_bits_whatever_arrives_first(form, Hq, Hkv, samples, tokens):
+    """Nodes whose pages come from memory late and in any order (caches of 180 MB in turn, more than the L2 holds): a product that is
+    read before it has landed changes the result.  Parts are joined in the order of their places, so repeats are equal to the bit; and
+    they are near fp32 (bf16 weights and outputs, 2^-9 of a value each)."""
+    from arctic_platform_b200.ops import _lib
+    from arctic_platform_b200.ops import forest_attention as fa
+    D, n = 128, (tokens + PAGE - 1) // PAGE
+    i32 = dict(device="cuda", dtype=torch.int32)
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    layers = -(-180_000_000 // (n * Hkv * PAGE * D * 4))
+    kc, vc = (torch.randn((layers, n + samples, Hkv, PAGE, D), generator=g, device="cuda").bfloat16() for _ in range(2))
+    q = torch.randn((samples, Hq, D), generator=g, device="cuda").bfloat16()
+    pages = np.arange(n, dtype=np.int32)
+    forest = fa.build_forest_tables([fa.ForestNode(0, list(range(samples)), pages, tokens)], samples, n, 128 * Hkv // Hq, "cuda")
+    table = torch.arange(n, n + samples, **i32).view(-1, 1)
+    splits = max(1, min(8, 148 // Hkv))
+    part_o, part_ml = _scratch(samples, Hq, D, splits)
+    run = _forms(samples, Hkv)[form]
+    args = (forest, torch.arange(samples, **i32), torch.ones(samples, **i32), table, torch.full((samples,), 9, **i32), part_o, part_ml, splits, 4)
+    first = [run(q, kc[i], vc[i], *args) for i in range(layers)]
+    for _ in range(max(3, 600 // layers)):
+        for i in range(layers):
+            assert torch.equal(run(q, kc[i], vc[i], *args), first[i])
+    _lib.check_status("forest")
+    ref = fa.forest_decode_reference(q, kc[0], vc[0], [[(pages, tokens), (np.array([n + b]), 9)] for b in range(samples)])
+    assert ((first[0].float() - ref).norm(dim=-1) <= 2 ** -7 * ref.norm(dim=-1)).all()
