@@ -61,7 +61,8 @@ decode_prefix_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
   uint64_t* q_full = bars + 2 * kDpSlots;
   uint64_t* s_full = q_full + 1;    // [2] MMA -> softmax: scores of block j are in S[j & 1]
   uint64_t* p_full = s_full + 2;    // [2] softmax -> MMA: probabilities of block j are in S[j & 1]
-  uint64_t* o_full = p_full + 2;    // [1] MMA -> softmax: P V of block j has been added to O (one phase per block)
+  // [2] MMA -> softmax: P V of block j has been added to O; one for even and one for odd blocks (see decode_attention.cu)
+  uint64_t* o_full = p_full + 2;
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(o_full + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -197,7 +198,7 @@ decode_prefix_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
           for (int k = 0; k < 128 / 16; ++k)
             umma_bf16_ts(tmem_base + 256, tmem_base + b * 128 + k * 8, desc_v + slot * (kDpTile >> 4) + k * 128, idesc_o,
                          (j > 0 || k > 0) ? 1u : 0u);
-          tc_commit(&o_full[0]);
+          tc_commit(&o_full[b]);
           tc_commit(&kv_empty[slot]);
         }
         __syncwarp();
@@ -238,7 +239,7 @@ decode_prefix_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
         // row in tensor memory (once the previous block's P V has landed; block 0 has nothing to rescale)
         const float alpha = (m_ref == -INFINITY) ? 0.f : exp2f(m_ref - m_new);
         if (j > 0) {
-          if (!mbar_wait(&o_full[0], (j - 1) & 1, p.status, kTimeoutTmemFull)) {
+          if (!mbar_wait(&o_full[b ^ 1], ((j - 1) >> 1) & 1, p.status, kTimeoutTmemFull)) {
             ok = false;
             break;
           }
@@ -280,7 +281,8 @@ decode_prefix_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
     // the output row: one read after the last P V
     float o_acc[D];
     if (ok && n_blocks > 0) {
-      ok = mbar_wait(&o_full[0], (n_blocks - 1) & 1, p.status, kTimeoutTmemFull);
+      const int last = n_blocks - 1;
+      ok = mbar_wait(&o_full[last & 1], (last >> 1) & 1, p.status, kTimeoutTmemFull);
       if (ok) {
         tc_fence_after();
 #pragma unroll
