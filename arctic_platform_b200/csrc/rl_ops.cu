@@ -191,10 +191,8 @@ moe_route_kernel(const LOGIT* __restrict__ logits, long long ld, const float* __
     }
 #pragma unroll
     for (int j = 0; j < kRouteMaxPerLane; ++j)
-      if (be == lane + 32 * j) {
-        sc[j] = -INFINITY;
-        taken |= 1u << j;
-      }
+      if (be == lane + 32 * j) sc[j] = -INFINITY;
+    if ((be & 31) == lane) taken |= 1u << (be >> 5);
     if (weight) {
       const float x = static_cast<float>(row[be]);
       const float score = sigmoid ? 1.f / (1.f + expf(-x)) : expf(x - mx) / exact_sum;
