@@ -18,7 +18,7 @@
 // took 24 + 19 + 6 us behind each other; 17 own tokens are a few KB per warp and hide behind the shared ones here: 27 us together.
 // Long own contexts do not: four warps with one page ahead keep 32 KB under way per SM where paged_decode_mma_kernel has 128 KB, and at
 // 2048 own tokens the three launches take 194 us, this one 210 (lengths from 1 to 2048: 124 and 175).  The rollout engine takes the
-// one that is faster at the lengths at hand (one_launch_pays in ops/forest_attention.py).  (Sequences that share nothing are left to
+// one that is faster for the responses ahead (runtime_decode.cpp).  (Sequences that share nothing are left to
 // paged_decode_mma_kernel, whose clusters join their parts sooner than counters in memory do: 7 us against 10 for one sequence of 400
 // tokens, 33 against 36 for 41 of 500 to 1500.)
 // Compiled for up to 8 query heads a key head it spills nothing, for 16 the walk over own pages spills 224 bytes (128 registers a

@@ -17,9 +17,10 @@
 // launches and 12 % less than one up to 256 slots, 8 % and 24 % less for more slots.  With a header above the prompts (959 sizes, none of
 // them fitted to): 0.9 % more than the better of the two, 17 % less than three launches and 4 % less than one.
 //
-// A rollout keeps to one form until sequences join it: the first steps of another form are captured in a graph of their own, which takes
+// A rollout keeps to one form until sequences join it: the first steps of another form are captured in a graph of their own, which took
 // 0.9 s in the middle of a rollout of the 4B model (128 sequences, 36 layers) -- more than the better form gives back behind the crossing
-// (2048 steps of 8 x 16 samples: 14.86 s with one launch, 15.29 with three, 14.99 with the better of the two at each step once both are captured).
+// (2048 steps of 8 x 16 samples: 14.86 s with one launch, 15.29 with three, 14.99 with the better of the two at each step once both are
+// captured).
 #include <algorithm>
 #include <cstdint>
 #include <vector>
